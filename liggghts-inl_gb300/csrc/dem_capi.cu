@@ -858,12 +858,8 @@ int dem_add_mesh(dem_handle *h, int ntri, const double *nodes, int wall_type, in
   CUDA_TRY(h, dalloc(L, &M.meta, mh.meta.size()));
   CUDA_TRY(h, cudaMemcpyAsync(M.meta, mh.meta.data(), mh.meta.size() * sizeof(int), cudaMemcpyHostToDevice, h->st));
   {
-    std::vector<float4> tf(2 * (size_t)ntri);
-    for (int t = 0; t < ntri; t++) {
-      const double *g = &mh.tri[(size_t)t * kTriStride];
-      tf[2 * (size_t)t] = make_float4((float)g[0], (float)g[1], (float)g[2], 0.f);
-      tf[2 * (size_t)t + 1] = make_float4((float)g[30], (float)g[31], (float)g[32], 0.f);
-    }
+    std::vector<float4> tf(kTrif * (size_t)ntri);
+    for (int t = 0; t < ntri; t++) tri_floats(&mh.tri[(size_t)t * kTriStride], &tf[kTrif * (size_t)t]);
     CUDA_TRY(h, dalloc(L, &M.trif, tf.size()));
     CUDA_TRY(h, cudaMemcpyAsync(M.trif, tf.data(), tf.size() * sizeof(float4), cudaMemcpyHostToDevice, h->st));
   }

@@ -160,6 +160,7 @@ constexpr int kMeshMaxCand = 24;
 constexpr int kMeshFastCand = 32;  // k_wall_force's tiled path (32-bit masks); more take the sequential path
 constexpr int kSlotKept = 1 << 30; // mesh_contacts: marks a slot touched in this evaluation
 constexpr int kTriStride = 40;     // doubles of geometry per triangle, see below
+constexpr int kTrif = 5;           // float4 of FP32 copies per triangle
 constexpr int kStatMeshSlots = 5;  // Ctrl::status: a mesh contact found no free slot (inconsistent slots)
 constexpr int kStatMeshReg = 6;    // Ctrl::status: triangle-cell registrations overflowed (halted, grown, resumed)
 constexpr int kStatMeshCand = 7;   // Ctrl::status: an atom has more candidate triangles than ccap (halted, grown,
@@ -172,7 +173,7 @@ struct MeshDev {
   int ntri, wall_type, rolling, moving;
   double distmax, tskin;  // FixNeighlistMesh: bounding-box growth and neighbuild threshold
   double *tri;        // [t*kTriStride]
-  float4 *trif;       // [2t]: node 0, [2t+1]: unit normal, FP32 copies (plane-distance prefilter)
+  float4 *trif;       // [kTrif*t + q]: FP32 copies for the candidate bounds, see tri_floats
   int *meta;          // [t]
   // fix move/mesh ... linear: every step nodes and centres move by dx =
   // dt*vel; node velocities are vel (0 during the setup force pass)

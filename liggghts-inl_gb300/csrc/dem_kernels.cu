@@ -801,11 +801,6 @@ __device__ __forceinline__ void mslot_swap(const MeshDev &M, size_t nmax, int i,
   }
 }
 
-// MeshMoverLinear::initial_integrate + MultiNodeMesh::move (nodes and
-// centres += dx, src/multi_node_mesh_I.h:502-520), then
-// MultiNodeMesh::decideRebuild (any node > skin/2 from its position at the
-// last build, src/multi_node_mesh_I.h:792-823); the decision is used by
-// k_decide only on steps that do not rebuild anyway (FixMesh::pre_force).
 // MathExtra::quatquat (src/math_extra.h:596-602) and
 // MathExtraLiggghts::vec_quat_rotate (src/math_extra_liggghts.h:455-471) in
 // the reference's operation order, exactly rounded: rotated nodes are
@@ -831,75 +826,102 @@ __device__ __forceinline__ void vec_quat_rotate_rn(double *v, const double *q) {
   v[2] = r[3];
 }
 
-// MeshMoverRotate::initial_integrate (src/mesh_mover_rotation.cpp:105-131):
-// nodes and centres (MultiNodeMesh::rotate(dQ, origin),
-// src/multi_node_mesh_I.h:643-668), the rotating element vectors edgeVec,
-// edgeNorm, surfaceNorm (CustomValueTracker::rotate), node velocities
-// 0 + w x (node - O); then the node-travel test of decideRebuild
-__global__ void k_mesh_rotate(Sys s, int k) {
-  Ctrl *c = s.ctrl;
-  if (c->halt) return;
-  const MeshDev &M = s.meshes[k];
+// One step of a moving mesh: 16 lanes per triangle, lane q taking one of its
+// vectors (nodes 0..2, edgeVec 3..5, edgeNorm 6..8, surfaceNorm 9), lane 10
+// the centre.  A quaternion rotation is a chain of some fifty FP64
+// instructions and most moving meshes have few triangles, so one thread per
+// triangle made ten such chains one after the other (a two-triangle paddle:
+// 23 us per step; one per lane: 6 us).  Returns whether a node moved more
+// than skin/2 since the last build.
+//   linear: MeshMoverLinear::initial_integrate + MultiNodeMesh::move (nodes and
+//     centres += dx, src/multi_node_mesh_I.h:502-520);
+//   rotating: MeshMoverRotate::initial_integrate
+//     (src/mesh_mover_rotation.cpp:105-131): nodes and centres
+//     (MultiNodeMesh::rotate(dQ, origin), src/multi_node_mesh_I.h:643-668), the
+//     rotating element vectors edgeVec, edgeNorm, surfaceNorm
+//     (CustomValueTracker::rotate), node velocities 0 + w x (node - O);
+// then the node-travel test of MultiNodeMesh::decideRebuild
+// (src/multi_node_mesh_I.h:792-823).
+__device__ __forceinline__ bool mesh_move_part(const Sys &s, const MeshDev &M, int t, int q) {
   const double trigger = __dmul_rn(__dmul_rn(0.25, s.skin), s.skin);
-  const double *o = M.rorig, *q = M.rq, *w = M.romega;
-  const bool trans = __dadd_rn(__dadd_rn(__dmul_rn(o[0], o[0]), __dmul_rn(o[1], o[1])), __dmul_rn(o[2], o[2])) > 0.;
-  const double third = 1. / 3.;
+  double *g = M.tri + (size_t)t * kTriStride;
+  const bool on = t < M.ntri && q < 11;
   bool moved = false;
-  GRID_STRIDE(t, M.ntri) {
-    double *g = M.tri + (size_t)t * kTriStride;
-    double cen[3] = {0., 0., 0.};
-    for (int j = 0; j < 3; j++) {
-      double nd[3] = {g[3 * j], g[3 * j + 1], g[3 * j + 2]};
-      if (trans)
-        for (int d = 0; d < 3; d++) nd[d] = __dsub_rn(nd[d], o[d]);
-      vec_quat_rotate_rn(nd, q);
-      if (trans)
-        for (int d = 0; d < 3; d++) nd[d] = __dadd_rn(nd[d], o[d]);
+  double out[3] = {0., 0., 0.};
+  int at = -1;  // where this lane's vector goes in the triangle's record
+  if (on && !M.rotating) {
+    if (q < 3 || q == 10) {
+      at = q < 3 ? 3 * q : 33;
+      for (int d = 0; d < 3; d++) out[d] = __dadd_rn(g[at + d], M.dx[d]);
+    }
+  } else if (on) {
+    const double *o = M.rorig, *rq = M.rq;
+    const bool trans =
+        __dadd_rn(__dadd_rn(__dmul_rn(o[0], o[0]), __dmul_rn(o[1], o[1])), __dmul_rn(o[2], o[2])) > 0.;
+    if (q < 10) {
+      at = 3 * q + (q == 9 ? 3 : 0);
+      for (int d = 0; d < 3; d++) out[d] = g[at + d];
+      if (q < 3 && trans)
+        for (int d = 0; d < 3; d++) out[d] = __dsub_rn(out[d], o[d]);
+      vec_quat_rotate_rn(out, rq);
+      if (q < 3 && trans)
+        for (int d = 0; d < 3; d++) out[d] = __dadd_rn(out[d], o[d]);
+    } else {
+      at = 33;
+      for (int j = 0; j < 3; j++) {
+        double nd[3] = {g[3 * j], g[3 * j + 1], g[3 * j + 2]};
+        if (trans)
+          for (int d = 0; d < 3; d++) nd[d] = __dsub_rn(nd[d], o[d]);
+        vec_quat_rotate_rn(nd, rq);
+        if (trans)
+          for (int d = 0; d < 3; d++) nd[d] = __dadd_rn(nd[d], o[d]);
+        for (int d = 0; d < 3; d++) out[d] = __dadd_rn(nd[d], out[d]);
+      }
+      const double third = 1. / 3.;
+      for (int d = 0; d < 3; d++) out[d] = __dmul_rn(third, out[d]);
+    }
+  }
+  __syncwarp();  // every lane has read the record before any writes it
+  if (at >= 0) {
+    for (int d = 0; d < 3; d++) g[at + d] = out[d];
+    if (q < 3) {
       double dsq = 0.0;
       for (int d = 0; d < 3; d++) {
-        g[3 * j + d] = nd[d];
-        cen[d] = __dadd_rn(nd[d], cen[d]);
-        const double e = __dadd_rn(nd[d], -M.node_last[(size_t)t * 9 + 3 * j + d]);
+        const double e = __dadd_rn(out[d], -M.node_last[(size_t)t * 9 + 3 * q + d]);
         dsq = d == 0 ? __dmul_rn(e, e) : __dadd_rn(dsq, __dmul_rn(e, e));
       }
-      moved |= dsq > trigger;
-      const double r[3] = {__dsub_rn(nd[0], o[0]), __dsub_rn(nd[1], o[1]), __dsub_rn(nd[2], o[2])};
-      double *v = M.nodev + (size_t)t * 9 + 3 * j;
-      v[0] = __dadd_rn(0.0, __dsub_rn(__dmul_rn(w[1], r[2]), __dmul_rn(w[2], r[1])));
-      v[1] = __dadd_rn(0.0, __dsub_rn(__dmul_rn(w[2], r[0]), __dmul_rn(w[0], r[2])));
-      v[2] = __dadd_rn(0.0, __dsub_rn(__dmul_rn(w[0], r[1]), __dmul_rn(w[1], r[0])));
+      moved = dsq > trigger;
+      if (M.rotating) {
+        const double *o = M.rorig, *w = M.romega;
+        const double r[3] = {__dsub_rn(out[0], o[0]), __dsub_rn(out[1], o[1]), __dsub_rn(out[2], o[2])};
+        double *v = M.nodev + (size_t)t * 9 + 3 * q;
+        v[0] = __dadd_rn(0.0, __dsub_rn(__dmul_rn(w[1], r[2]), __dmul_rn(w[2], r[1])));
+        v[1] = __dadd_rn(0.0, __dsub_rn(__dmul_rn(w[2], r[0]), __dmul_rn(w[0], r[2])));
+        v[2] = __dadd_rn(0.0, __dsub_rn(__dmul_rn(w[0], r[1]), __dmul_rn(w[1], r[0])));
+      }
     }
-    for (int d = 0; d < 3; d++) g[33 + d] = __dmul_rn(third, cen[d]);
-    for (int j = 0; j < 3; j++) vec_quat_rotate_rn(g + 9 + 3 * j, q);   // edgeVec
-    for (int j = 0; j < 3; j++) vec_quat_rotate_rn(g + 18 + 3 * j, q);  // edgeNorm
-    vec_quat_rotate_rn(g + 30, q);                                      // surfaceNorm
-    M.trif[2 * (size_t)t] = make_float4((float)g[0], (float)g[1], (float)g[2], 0.f);
-    M.trif[2 * (size_t)t + 1] = make_float4((float)g[30], (float)g[31], (float)g[32], 0.f);
+    // the FP32 copies: node 0, surface normal, edge normals (all zero where
+    // the triangle is too thin for the edge bounds, see tri_floats)
+    float4 *T = M.trif + kTrif * (size_t)t;
+    const int slot = q == 0 ? 0 : (q == 9 ? 1 : (q >= 6 && q < 9 ? q - 4 : -1));
+    if (slot >= 0) {
+      const float4 old = T[slot];
+      if (slot < 2 || old.x != 0.f || old.y != 0.f || old.z != 0.f)
+        T[slot] = make_float4((float)out[0], (float)out[1], (float)out[2], old.w);
+    }
   }
-  if (__any_sync(0xffffffffu, moved) && (threadIdx.x & 31) == 0) atomicOr(&c->mesh_moved, 1);
+  return moved;
 }
 
 __global__ void k_mesh_move(Sys s, int k) {
   Ctrl *c = s.ctrl;
   if (c->halt) return;
   const MeshDev &M = s.meshes[k];
-  const double trigger = __dmul_rn(__dmul_rn(0.25, s.skin), s.skin);
   bool moved = false;
-  GRID_STRIDE(t, M.ntri) {
-    double *g = M.tri + (size_t)t * kTriStride;
-    for (int q = 0; q < 3; q++) {
-      double dsq = 0.0;
-      for (int d = 0; d < 3; d++) {
-        const double x = __dadd_rn(g[3 * q + d], M.dx[d]);
-        g[3 * q + d] = x;
-        const double e = __dadd_rn(x, -M.node_last[(size_t)t * 9 + 3 * q + d]);
-        dsq = d == 0 ? __dmul_rn(e, e) : __dadd_rn(dsq, __dmul_rn(e, e));
-      }
-      moved |= dsq > trigger;
-    }
-    for (int d = 0; d < 3; d++) g[33 + d] = __dadd_rn(g[33 + d], M.dx[d]);
-    M.trif[2 * (size_t)t] = make_float4((float)g[0], (float)g[1], (float)g[2], 0.f);
-  }
+  const int per = (gridDim.x * blockDim.x) / 16;
+  // whole warps iterate together (mesh_move_part synchronises the warp)
+  for (int t0 = (blockIdx.x * blockDim.x + (threadIdx.x & ~31)) / 16; t0 < M.ntri; t0 += per)
+    moved |= mesh_move_part(s, M, t0 + ((threadIdx.x & 31) >> 4), threadIdx.x & 15);
   if (__any_sync(0xffffffffu, moved) && (threadIdx.x & 31) == 0) atomicOr(&c->mesh_moved, 1);
 }
 
@@ -1982,6 +2004,38 @@ __device__ __forceinline__ bool mesh_coplanar(const MeshDev &M, int a, int b) {
 // triangle id of a slot entry (-1: empty), without the kept mark
 __device__ __forceinline__ int slot_tri_of(int v) { return v < 0 ? -1 : (v & ~kSlotKept); }
 
+// FP32 test of candidate triangle t against an atom at xa within reach_f:
+// false only when the sphere is beyond the triangle.  Two bounds:
+//   plane  |sn.(x - n0)| > reach;
+//   edges  the triangle lies behind each of its edge planes (outward in-plane
+//          normal en_q), and a contact lies within sqrt(reach^2 - dn^2) of
+//          the centre's foot point, so en_q.(x - n_q) beyond that is none.
+// The margins cover the FP32 rounding of the copies and of this arithmetic (a
+// difference of coordinates is within 5*2^-24 of the sum of their magnitudes;
+// 2^-21 is four times that and more), and, for the edges, the 1e-8 by which
+// the reference widens its face region.  A rejected candidate would resolve
+// to deltan > 0, so leaving it out changes nothing.
+__device__ __forceinline__ bool tri_candidate_f(const MeshDev &M, int t, const float4 &xa, float reach_f) {
+  const float4 *T = M.trif + kTrif * (size_t)t;
+  const float4 n0 = T[0], sn = T[1];
+  const float wx = xa.x - n0.x, wy = xa.y - n0.y, wz = xa.z - n0.z;
+  const float dn = fabsf(sn.x * wx + sn.y * wy + sn.z * wz);
+  const float mag = fabsf(xa.x) + fabsf(xa.y) + fabsf(xa.z) + fabsf(n0.x) + fabsf(n0.y) + fabsf(n0.z);
+  const float hi = reach_f + mag * 0x1p-21f;
+  if (dn > hi) return false;
+  const float lo = fmaxf(0.0f, dn - mag * 0x1p-21f);
+  const float rho2 = (hi * hi - lo * lo) * (1.0f + 0x1p-20f) + hi * hi * 0x1p-20f;
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    const float4 e = T[2 + q];
+    const float d = e.x * wx + e.y * wy + e.z * wz - e.w;
+    const float m = (mag + fabsf(wx) + fabsf(wy) + fabsf(wz) + fabsf(e.w)) * 0x1p-21f + 4e-8f;
+    const float a = d - m;
+    if (a > 0.0f && a * a > rho2) return false;
+  }
+  return true;
+}
+
 // The closest-feature contacts of atom i with mesh k, one candidate at a
 // time in ascending triangle order (FixWallGran::post_force_mesh with
 // FixContactHistoryMesh::handleContact, coplanarContactAlready,
@@ -2006,20 +2060,12 @@ __device__ void mesh_contacts(const Sys &s, const AtomArrays &A, int i, int k, i
   // rounding of either side) skip the closest-feature resolution; the
   // resolution would return deltan > 0 and skip them as well
   const double reach = __dmul_rn(__dadd_rn(radi, fmax(0.0, __dmul_rn(cdm1, radi))), 1.0 + 1e-9);
-  // FP32 test first: the plane distance in FP32 is within 5*2^-24*S of the
-  // FP64 one (S: sum of the magnitudes of the atom's and node 0's
-  // coordinates), so a candidate farther than reach plus 2^-21*S is beyond
-  // reach in FP64 too; the rest take the FP64 path below
+  // FP32 bounds first (tri_candidate_f); the rest take the FP64 path below
   const float4 xa = s.xf[i];
   const float reach_f = (float)reach * (1.0f + 0x1p-20f);
   for (int q = 0; q < nc; q++) {
     const int t = M.cand[(size_t)q * nmax + i];
-    {
-      const float4 n0 = M.trif[2 * (size_t)t], sn = M.trif[2 * (size_t)t + 1];
-      const float dnf = sn.x * (xa.x - n0.x) + sn.y * (xa.y - n0.y) + sn.z * (xa.z - n0.z);
-      const float mag = fabsf(xa.x) + fabsf(xa.y) + fabsf(xa.z) + fabsf(n0.x) + fabsf(n0.y) + fabsf(n0.z);
-      if (fabsf(dnf) > reach_f + mag * 0x1p-21f) continue;
-    }
+    if (!tri_candidate_f(M, t, xa, reach_f)) continue;
     const double *g = M.tri + (size_t)t * kTriStride;
     {
       const double *sn = tri_sn(g), *n0 = tri_node(g, 0);
@@ -2089,12 +2135,12 @@ __device__ void mesh_contacts(const Sys &s, const AtomArrays &A, int i, int k, i
 // writes only the wall histories, mesh slots and fm/tm), so the two run side
 // by side; the per-atom kernel adds fm/tm.
 //
-// A block takes a tile of kWallTile listed atoms (one thread each) and, per
-// mesh, runs the FP64-heavy parts densely over the tile's work instead of
-// per atom (the FP64 pipe issues per warp instruction, and atoms differ in
-// their number of candidates and contacts):
-//   A  per atom, FP32: the candidates whose plane is within reach (see
-//      mesh_contacts), queued in ascending order;
+// A warp takes a tile of 32 listed atoms (one lane each) and, per mesh, runs
+// the FP64-heavy parts densely over the tile's work instead of per atom (the
+// FP64 pipe issues per warp instruction, and atoms differ in their number of
+// candidates and contacts):
+//   A  per atom, FP32: the candidates the triangle bounds cannot reject
+//      (tri_candidate_f), queued in ascending order;
 //   B  per queued candidate: exact plane test and closest feature
 //      (TriMesh::resolveTriSphereContactBary), kept when touching;
 //   C  per atom, integer work in candidate order: FixContactHistoryMesh's
@@ -2104,240 +2150,242 @@ __device__ void mesh_contacts(const Sys &s, const AtomArrays &A, int i, int k, i
 //      since that copy depends on the order of the contact updates;
 //   D  per contact: the contact law with the slot's history;
 //   E  per atom: contact forces summed in candidate order, slot clean-up.
-// A tile whose queue would exceed its capacity (cap entries, a launch
-// parameter) runs the sequential path for all its atoms.  Both paths give
-// the same result.  The queue lives in dynamic shared memory, kWallQ bytes
-// per entry: a smaller cap leaves room for more blocks beside the pair
-// kernel that runs concurrently.
-constexpr int kWallTile = 64;
-constexpr int kWallCapDefault = 6;  // queue entries per tile atom (LIGGGHTS_GB300_WALL_CAP)
+// Atoms without a touching candidate and without an occupied slot do nothing
+// after B (their slots are empty, with zero history).  A tile whose queue
+// would exceed its capacity (cap entries, a launch parameter) runs the
+// sequential path for all its atoms.  Both paths give the same result.
+//
+// The launch is bound by latency: the phases are one dependent chain, a few
+// warps per SM.  A warp per tile keeps the phases free of block barriers, and
+// the edge bounds leave B about one candidate per contact (with the plane
+// bound alone the conical mesh's tiles queued several per atom, three to five
+// FP64 passes of B).  Against 64-atom tiles with block barriers and the plane
+// bound: the 100,000-sphere hopper's step 84 -> 67 us, the 1M one's 0.318 ->
+// 0.309 ms (50 steps per call).
+constexpr int kWallTile = 32;
+constexpr int kWallWarps = 2;       // tiles (warps) per block
+constexpr int kWallCapDefault = 4;  // queue entries per tile atom (LIGGGHTS_GB300_WALL_CAP)
 constexpr int kWallRes = 7;  // doubles per queued candidate: deltan, delta[3], vwall[3]; then F[3], T[3]
 constexpr int kWallQ = kWallRes * 8 + 4 + 2;  // result doubles, state int, atom and candidate bytes
 
-__device__ __forceinline__ int wall_tile_scan(int v, int &total, int *wsum) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int inc = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int u = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += u;
+// one warp's queue of `cap` entries in shared memory
+struct WallQueue {
+  double *res;             // [cap * kWallRes]
+  int *st;                 // bit 0 touching, bit 1 face, bits 8+: contact slot + 1
+  unsigned char *qa, *qq;  // tile atom, candidate index
+};
+
+template <int NORMAL>
+__device__ __forceinline__ void wall_tile(const Sys &s, const AtomArrays &A, int base, int nl, int shearupdate,
+                                          int cap, const WallQueue &w, bool &meshbad) {
+  const size_t nmax = s.nmax;
+  const double cdm1 = s.cdf - 1.0;
+  const int a = threadIdx.x & 31;
+  const bool valid = base + a < nl;
+  const int i = valid ? s.mlist[base + a] : 0;
+  double v[3] = {0., 0., 0.}, om[3] = {0., 0., 0.}, xv[3] = {0., 0., 0.};
+  double fx = 0., fy = 0., fz = 0., tx = 0., ty = 0., tz = 0.;
+  if (valid) {
+    v[0] = A.vx[i]; v[1] = A.vy[i]; v[2] = A.vz[i];
+    om[0] = A.wx[i]; om[1] = A.wy[i]; om[2] = A.wz[i];
+    xv[0] = A.x[i]; xv[1] = A.y[i]; xv[2] = A.z[i];
+    const uint8_t bits = A.wbits[i];
+    for (int k = 0; k < s.nplanes; k++) {
+      double pfx = 0., pfy = 0., pfz = 0., ptx = 0., pty = 0., ptz = 0.;
+      if (bits & (1u << k)) plane_contact<NORMAL>(s, A, i, k, shearupdate, v, om, xv, pfx, pfy, pfz, ptx, pty, ptz);
+      fx += pfx; fy += pfy; fz += pfz;
+      tx += ptx; ty += pty; tz += ptz;
+      s.wforce[(size_t)(3 * k) * nmax + i] = pfx;
+      s.wforce[(size_t)(3 * k + 1) * nmax + i] = pfy;
+      s.wforce[(size_t)(3 * k + 2) * nmax + i] = pfz;
+    }
   }
-  if (lane == 31) wsum[warp] = inc;
-  __syncthreads();
-  int base = 0;
-  total = 0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
-    if (w < warp) base += wsum[w];
-    total += wsum[w];
+  for (int k = 0; k < s.nmeshes; k++) {
+    const MeshDev &M = s.meshes[k];
+    int *st = M.slot_tri[0];
+    double *sh = M.slot_hist[0];
+    // ---- A: FP32 candidate pass
+    const int nc = valid ? M.cand_n[i] : 0;
+    unsigned todo = 0u;
+    int np = 0;
+    const bool big = nc > kMeshFastCand;  // beyond the 32-bit masks: sequential path
+    if (nc > 0 && !big) {
+      np = M.npart[0][i];
+      const double radi = A.r[i];
+      const double reach = __dmul_rn(__dadd_rn(radi, fmax(0.0, __dmul_rn(cdm1, radi))), 1.0 + 1e-9);
+      const float4 xa = s.xf[i];
+      const float reach_f = (float)reach * (1.0f + 0x1p-20f);
+      int t = M.cand[i];
+      for (int q = 0; q < nc; q++) {
+        const int tn = q + 1 < nc ? M.cand[(size_t)(q + 1) * nmax + i] : 0;  // ahead of the triangle it names
+        if (tri_candidate_f(M, t, xa, reach_f)) todo |= 1u << q;
+        t = tn;
+      }
+    }
+    const int cnt = __popc(todo);
+    const int inc = warp_incl_scan(cnt);
+    const int total = __shfl_sync(0xffffffffu, inc, 31);
+    const int off = inc - cnt;
+    double msum[3] = {0., 0., 0.};
+    double *const wf = s.wforce + (size_t)(3 * (s.nplanes + k)) * nmax;
+    if (total > cap) {  // sequential path for this tile
+      if (nc > 0) mesh_contacts<NORMAL>(s, A, i, k, shearupdate, v, om, xv, fx, fy, fz, tx, ty, tz, meshbad, msum);
+      if (valid)
+        for (int d = 0; d < 3; d++) wf[(size_t)d * nmax + i] = msum[d];
+      __syncwarp();
+      continue;
+    }
+    {
+      unsigned m = todo;
+      for (int e = off; m; e++) {
+        w.qa[e] = (unsigned char)a;
+        w.qq[e] = (unsigned char)(__ffs(m) - 1);
+        m &= m - 1u;
+      }
+    }
+    __syncwarp();
+    // ---- B: exact plane test and closest feature per queued candidate
+    for (int e = a; e < total; e += kWallTile) {
+      const int ie = s.mlist[base + w.qa[e]];
+      const int t = M.cand[(size_t)w.qq[e] * nmax + ie];
+      const double *g = M.tri + (size_t)t * kTriStride;
+      const double xe[3] = {A.x[ie], A.y[ie], A.z[ie]};
+      const double re = A.r[ie];
+      const double reach_e = __dmul_rn(__dadd_rn(re, fmax(0.0, __dmul_rn(cdm1, re))), 1.0 + 1e-9);
+      int state = 0;
+      const double *snv = tri_sn(g), *n0 = tri_node(g, 0);
+      const double dn = snv[0] * (xe[0] - n0[0]) + snv[1] * (xe[1] - n0[1]) + snv[2] * (xe[2] - n0[2]);
+      if (!(fabs(dn) > reach_e)) {
+        double delta[3], bary[3];
+        int bs;
+        const double deltan = resolve_tri_sphere(g, M.meta[t], re, xe, delta, bary, bs);
+        if (!(deltan > s.cutneighmax) && (deltan <= 0 || deltan < cdm1 * re)) {
+          state = 1 | (bs == 7 ? 2 : 0);
+          double *r = w.res + (size_t)e * kWallRes;
+          r[0] = deltan;
+          r[1] = delta[0]; r[2] = delta[1]; r[3] = delta[2];
+          double vwall[3] = {0., 0., 0.};
+          if (M.moving && M.vel_on) mesh_vwall(M, t, bary, vwall);
+          r[4] = vwall[0]; r[5] = vwall[1]; r[6] = vwall[2];
+        }
+      }
+      w.st[e] = state;
+    }
+    __syncwarp();
+    // ---- C: slot semantics per atom, in candidate order
+    bool fallback = big;
+    unsigned keep = 0u;
+    int stl[kMeshFastCand];
+    bool work = np > 0 && !big;
+    for (int e = off; e < off + cnt; e++) work |= (w.st[e] & 1) != 0;
+    if (work) {
+      for (int u = 0; u < nc; u++) stl[u] = st[u * nmax + i];
+      unsigned fresh = 0u;
+      for (int e = off; e < off + cnt && !fallback; e++) {
+        if (!(w.st[e] & 1)) continue;
+        const int t = M.cand[(size_t)w.qq[e] * nmax + i];
+        int slot = -1;
+        for (int u = 0; u < nc; u++)
+          if (stl[u] == t) { slot = u; break; }
+        if (slot >= 0) {
+          keep |= 1u << slot;
+        } else {
+          const bool face = (w.st[e] & 2) != 0;
+          if (face) {  // coplanarContactAlready
+            bool already = false;
+            for (int u = 0; u < nc; u++)
+              if (stl[u] >= 0 && stl[u] != t && ((keep >> u) & 1u) && mesh_coplanar(M, stl[u], t)) already = true;
+            if (already) continue;
+          }
+          if (np >= nc) { meshbad = true; continue; }
+          for (int u = 0; u < nc; u++)
+            if (stl[u] == -1) { slot = u; break; }
+          if (face)  // checkCoplanarContactHistory would copy: order-dependent
+            for (int u = 0; u < nc; u++)
+              if (stl[u] >= 0 && stl[u] != t && mesh_coplanar(M, stl[u], t)) fallback = true;
+          if (fallback) break;
+          stl[slot] = t;
+          keep |= 1u << slot;
+          fresh |= 1u << slot;
+          np++;
+        }
+        w.st[e] |= (slot + 1) << 8;
+      }
+      if (fallback) {
+        for (int e = off; e < off + cnt; e++) w.st[e] &= 0xff;
+      } else {
+        for (int u = 0; u < nc; u++)
+          if ((fresh >> u) & 1u) {
+            st[u * nmax + i] = stl[u];
+            for (int d = 0; d < 3; d++) sh[(3 * u + d) * nmax + i] = 0.0;
+          }
+      }
+    }
+    __syncwarp();
+    // ---- D: contact law per contact
+    for (int e = a; e < total; e += kWallTile) {
+      const int slot = (w.st[e] >> 8) - 1;
+      if (slot < 0) continue;
+      const int ie = s.mlist[base + w.qa[e]];
+      double *r = w.res + (size_t)e * kWallRes;
+      const double delta[3] = {r[1], r[2], r[3]};
+      const double vwall[3] = {r[4], r[5], r[6]};
+      double ve[3] = {A.vx[ie], A.vy[ie], A.vz[ie]};
+      double oe[3] = {A.wx[ie], A.wy[ie], A.wz[ie]};
+      double cfx = 0., cfy = 0., cfz = 0., ctx = 0., cty = 0., ctz = 0.;
+      wall_force<NORMAL>(s, A, ie, r[0], delta, vwall, M.wall_type, M.rolling != 0,
+                         sh + (size_t)(3 * slot) * nmax + ie, nmax, shearupdate, ve, oe, cfx, cfy, cfz, ctx, cty,
+                         ctz);
+      r[0] = cfx; r[1] = cfy; r[2] = cfz;
+      r[3] = ctx; r[4] = cty; r[5] = ctz;
+    }
+    __syncwarp();
+    // ---- E: sums in candidate order, clean-up (or the sequential path)
+    if (fallback) {
+      mesh_contacts<NORMAL>(s, A, i, k, shearupdate, v, om, xv, fx, fy, fz, tx, ty, tz, meshbad, msum);
+    } else if (work) {
+      for (int e = off; e < off + cnt; e++) {
+        if ((w.st[e] >> 8) == 0) continue;
+        const double *r = w.res + (size_t)e * kWallRes;
+        fx += r[0]; fy += r[1]; fz += r[2];
+        tx += r[3]; ty += r[4]; tz += r[5];
+        msum[0] += r[0]; msum[1] += r[1]; msum[2] += r[2];
+      }
+      for (int u = 0; u < nc; u++)  // cleanUpContacts
+        if (!((keep >> u) & 1u) && stl[u] > -1) {
+          np--;
+          st[u * nmax + i] = -1;
+          for (int d = 0; d < 3; d++) sh[(3 * u + d) * nmax + i] = 0.0;
+        }
+      M.npart[0][i] = np;
+    }
+    if (valid)
+      for (int d = 0; d < 3; d++) wf[(size_t)d * nmax + i] = msum[d];
+    __syncwarp();
   }
-  __syncthreads();
-  return base + inc - v;
+  if (valid) {
+    A.fmx[i] = fx; A.fmy[i] = fy; A.fmz[i] = fz;
+    A.tmx[i] = tx; A.tmy[i] = ty; A.tmz[i] = tz;
+  }
 }
 
 template <int NORMAL>
-__global__ void __launch_bounds__(kWallTile) k_wall_force(Sys s, int shearupdate, int cap) {
-  extern __shared__ double wres[];             // [cap * kWallRes], then qst, qa, qq
-  int *qst = reinterpret_cast<int *>(wres + (size_t)cap * kWallRes);  // bit 0 touching, bit 1 face,
-                                                                       // bits 8+: contact slot + 1
-  unsigned char *qa = reinterpret_cast<unsigned char *>(qst + cap);
-  unsigned char *qq = qa + cap;
-  __shared__ int wsum[kWallTile / 32];
+__global__ void __launch_bounds__(kWallTile *kWallWarps) k_wall_force(Sys s, int shearupdate, int cap) {
+  extern __shared__ double wshared[];  // per warp: res [cap * kWallRes]; then st, qa, qq of every warp
   Ctrl *c = s.ctrl;
   if (c->halt) return;
-  const AtomArrays &A = s.atoms[0];
+  const int warp = threadIdx.x >> 5;
+  WallQueue w;
+  w.res = wshared + (size_t)warp * cap * kWallRes;
+  w.st = reinterpret_cast<int *>(wshared + (size_t)kWallWarps * cap * kWallRes) + warp * cap;
+  w.qa = reinterpret_cast<unsigned char *>(wshared + (size_t)kWallWarps * cap * kWallRes) +
+         (size_t)kWallWarps * cap * 4 + (size_t)warp * 2 * cap;
+  w.qq = w.qa + cap;
   const int nl = c->nmlist;
-  const size_t nmax = s.nmax;
-  const double cdm1 = s.cdf - 1.0;
   bool meshbad = false;
-  for (int base = blockIdx.x * kWallTile; base < nl; base += gridDim.x * kWallTile) {
-    const int a = threadIdx.x;
-    const bool valid = base + a < nl;
-    const int i = valid ? s.mlist[base + a] : 0;
-    double v[3] = {0., 0., 0.}, om[3] = {0., 0., 0.}, xv[3] = {0., 0., 0.};
-    double fx = 0., fy = 0., fz = 0., tx = 0., ty = 0., tz = 0.;
-    if (valid) {
-      v[0] = A.vx[i]; v[1] = A.vy[i]; v[2] = A.vz[i];
-      om[0] = A.wx[i]; om[1] = A.wy[i]; om[2] = A.wz[i];
-      xv[0] = A.x[i]; xv[1] = A.y[i]; xv[2] = A.z[i];
-      const uint8_t bits = A.wbits[i];
-      for (int w = 0; w < s.nplanes; w++) {
-        double pfx = 0., pfy = 0., pfz = 0., ptx = 0., pty = 0., ptz = 0.;
-        if (bits & (1u << w)) plane_contact<NORMAL>(s, A, i, w, shearupdate, v, om, xv, pfx, pfy, pfz, ptx, pty, ptz);
-        fx += pfx; fy += pfy; fz += pfz;
-        tx += ptx; ty += pty; tz += ptz;
-        s.wforce[(size_t)(3 * w) * nmax + i] = pfx;
-        s.wforce[(size_t)(3 * w + 1) * nmax + i] = pfy;
-        s.wforce[(size_t)(3 * w + 2) * nmax + i] = pfz;
-      }
-    }
-    for (int k = 0; k < s.nmeshes; k++) {
-      const MeshDev &M = s.meshes[k];
-      int *st = M.slot_tri[0];
-      double *sh = M.slot_hist[0];
-      // ---- A: FP32 candidate pass
-      const int nc = valid ? M.cand_n[i] : 0;
-      const double radi = valid ? A.r[i] : 0.0;
-      const double reach = __dmul_rn(__dadd_rn(radi, fmax(0.0, __dmul_rn(cdm1, radi))), 1.0 + 1e-9);
-      unsigned todo = 0u;
-      const bool big = nc > kMeshFastCand;  // beyond the 32-bit masks: sequential path
-      if (nc > 0 && !big) {
-        const float4 xa = s.xf[i];
-        const float reach_f = (float)reach * (1.0f + 0x1p-20f);
-        for (int q = 0; q < nc; q++) {
-          const int t = M.cand[(size_t)q * nmax + i];
-          const float4 n0 = M.trif[2 * (size_t)t], sn = M.trif[2 * (size_t)t + 1];
-          const float dn = sn.x * (xa.x - n0.x) + sn.y * (xa.y - n0.y) + sn.z * (xa.z - n0.z);
-          const float mag = fabsf(xa.x) + fabsf(xa.y) + fabsf(xa.z) + fabsf(n0.x) + fabsf(n0.y) + fabsf(n0.z);
-          if (!(fabsf(dn) > reach_f + mag * 0x1p-21f)) todo |= 1u << q;
-        }
-      }
-      const int cnt = __popc(todo);
-      int total;
-      const int off = wall_tile_scan(cnt, total, wsum);
-      double msum[3] = {0., 0., 0.};
-      double *const wf = s.wforce + (size_t)(3 * (s.nplanes + k)) * nmax;
-      if (total > cap) {  // sequential path for this tile
-        if (nc > 0) mesh_contacts<NORMAL>(s, A, i, k, shearupdate, v, om, xv, fx, fy, fz, tx, ty, tz, meshbad, msum);
-        if (valid)
-          for (int d = 0; d < 3; d++) wf[(size_t)d * nmax + i] = msum[d];
-        __syncthreads();
-        continue;
-      }
-      {
-        unsigned m = todo;
-        for (int e = off; m; e++) {
-          qa[e] = (unsigned char)a;
-          qq[e] = (unsigned char)(__ffs(m) - 1);
-          m &= m - 1u;
-        }
-      }
-      __syncthreads();
-      // ---- B: exact plane test and closest feature per queued candidate
-      for (int e = threadIdx.x; e < total; e += kWallTile) {
-        const int ie = s.mlist[base + qa[e]];
-        const int t = M.cand[(size_t)qq[e] * nmax + ie];
-        const double *g = M.tri + (size_t)t * kTriStride;
-        const double xe[3] = {A.x[ie], A.y[ie], A.z[ie]};
-        const double re = A.r[ie];
-        const double reach_e = __dmul_rn(__dadd_rn(re, fmax(0.0, __dmul_rn(cdm1, re))), 1.0 + 1e-9);
-        int state = 0;
-        const double *snv = tri_sn(g), *n0 = tri_node(g, 0);
-        const double dn = snv[0] * (xe[0] - n0[0]) + snv[1] * (xe[1] - n0[1]) + snv[2] * (xe[2] - n0[2]);
-        if (!(fabs(dn) > reach_e)) {
-          double delta[3], bary[3];
-          int bs;
-          const double deltan = resolve_tri_sphere(g, M.meta[t], re, xe, delta, bary, bs);
-          if (!(deltan > s.cutneighmax) && (deltan <= 0 || deltan < cdm1 * re)) {
-            state = 1 | (bs == 7 ? 2 : 0);
-            double *r = wres + (size_t)e * kWallRes;
-            r[0] = deltan;
-            r[1] = delta[0]; r[2] = delta[1]; r[3] = delta[2];
-            double vwall[3] = {0., 0., 0.};
-            if (M.moving && M.vel_on) mesh_vwall(M, t, bary, vwall);
-            r[4] = vwall[0]; r[5] = vwall[1]; r[6] = vwall[2];
-          }
-        }
-        qst[e] = state;
-      }
-      __syncthreads();
-      // ---- C: slot semantics per atom, in candidate order
-      bool fallback = big;
-      unsigned keep = 0u;
-      int np = 0;
-      if (nc > 0 && !big) {
-        np = M.npart[0][i];
-        int stl[kMeshFastCand];
-        for (int u = 0; u < nc; u++) stl[u] = st[u * nmax + i];
-        unsigned fresh = 0u;
-        for (int e = off; e < off + cnt && !fallback; e++) {
-          if (!(qst[e] & 1)) continue;
-          const int t = M.cand[(size_t)qq[e] * nmax + i];
-          int slot = -1;
-          for (int u = 0; u < nc; u++)
-            if (stl[u] == t) { slot = u; break; }
-          if (slot >= 0) {
-            keep |= 1u << slot;
-          } else {
-            const bool face = (qst[e] & 2) != 0;
-            if (face) {  // coplanarContactAlready
-              bool already = false;
-              for (int u = 0; u < nc; u++)
-                if (stl[u] >= 0 && stl[u] != t && ((keep >> u) & 1u) && mesh_coplanar(M, stl[u], t)) already = true;
-              if (already) continue;
-            }
-            if (np >= nc) { meshbad = true; continue; }
-            for (int u = 0; u < nc; u++)
-              if (stl[u] == -1) { slot = u; break; }
-            if (face)  // checkCoplanarContactHistory would copy: order-dependent
-              for (int u = 0; u < nc; u++)
-                if (stl[u] >= 0 && stl[u] != t && mesh_coplanar(M, stl[u], t)) fallback = true;
-            if (fallback) break;
-            stl[slot] = t;
-            keep |= 1u << slot;
-            fresh |= 1u << slot;
-            np++;
-          }
-          qst[e] |= (slot + 1) << 8;
-        }
-        if (fallback) {
-          for (int e = off; e < off + cnt; e++) qst[e] &= 0xff;
-        } else {
-          for (int u = 0; u < nc; u++)
-            if ((fresh >> u) & 1u) {
-              st[u * nmax + i] = stl[u];
-              for (int d = 0; d < 3; d++) sh[(3 * u + d) * nmax + i] = 0.0;
-            }
-        }
-      }
-      __syncthreads();
-      // ---- D: contact law per contact
-      for (int e = threadIdx.x; e < total; e += kWallTile) {
-        const int slot = (qst[e] >> 8) - 1;
-        if (slot < 0) continue;
-        const int ie = s.mlist[base + qa[e]];
-        double *r = wres + (size_t)e * kWallRes;
-        const double delta[3] = {r[1], r[2], r[3]};
-        const double vwall[3] = {r[4], r[5], r[6]};
-        double ve[3] = {A.vx[ie], A.vy[ie], A.vz[ie]};
-        double oe[3] = {A.wx[ie], A.wy[ie], A.wz[ie]};
-        double cfx = 0., cfy = 0., cfz = 0., ctx = 0., cty = 0., ctz = 0.;
-        wall_force<NORMAL>(s, A, ie, r[0], delta, vwall, M.wall_type, M.rolling != 0,
-                           sh + (size_t)(3 * slot) * nmax + ie, nmax, shearupdate, ve, oe, cfx, cfy, cfz, ctx,
-                           cty, ctz);
-        r[0] = cfx; r[1] = cfy; r[2] = cfz;
-        r[3] = ctx; r[4] = cty; r[5] = ctz;
-      }
-      __syncthreads();
-      // ---- E: sums in candidate order, clean-up (or the sequential path)
-      if (nc > 0) {
-        if (fallback) {
-          mesh_contacts<NORMAL>(s, A, i, k, shearupdate, v, om, xv, fx, fy, fz, tx, ty, tz, meshbad, msum);
-        } else {
-          for (int e = off; e < off + cnt; e++) {
-            if ((qst[e] >> 8) == 0) continue;
-            const double *r = wres + (size_t)e * kWallRes;
-            fx += r[0]; fy += r[1]; fz += r[2];
-            tx += r[3]; ty += r[4]; tz += r[5];
-            msum[0] += r[0]; msum[1] += r[1]; msum[2] += r[2];
-          }
-          for (int u = 0; u < nc; u++)  // cleanUpContacts
-            if (!((keep >> u) & 1u)) {
-              if (st[u * nmax + i] > -1) np--;
-              st[u * nmax + i] = -1;
-              for (int d = 0; d < 3; d++) sh[(3 * u + d) * nmax + i] = 0.0;
-            }
-          M.npart[0][i] = np;
-        }
-      }
-      if (valid)
-        for (int d = 0; d < 3; d++) wf[(size_t)d * nmax + i] = msum[d];
-      __syncthreads();
-    }
-    if (valid) {
-      A.fmx[i] = fx; A.fmy[i] = fy; A.fmz[i] = fz;
-      A.tmx[i] = tx; A.tmy[i] = ty; A.tmz[i] = tz;
-    }
-  }
+  for (int base = (blockIdx.x * kWallWarps + warp) * kWallTile; base < nl;
+       base += gridDim.x * kWallWarps * kWallTile)
+    wall_tile<NORMAL>(s, s.atoms[0], base, nl, shearupdate, cap, w, meshbad);
   if (__any_sync(0xffffffffu, meshbad) && (threadIdx.x & 31) == 0) atomicExch(&c->status, kStatMeshSlots);
 }
 
@@ -3144,15 +3192,15 @@ int launch_wall_force(const Sys &s, const LaunchCfg &lc, int shearupdate, cudaSt
   if (!cap_per_atom) {
     const char *e = getenv("LIGGGHTS_GB300_WALL_CAP");
     cap_per_atom = e ? std::max(1, std::min(16, atoi(e))) : kWallCapDefault;
-    const int bytes = cap_per_atom * kWallTile * kWallQ;
+    const int bytes = kWallWarps * cap_per_atom * kWallTile * kWallQ;
     cudaFuncSetAttribute(k_wall_force<kHertz>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     cudaFuncSetAttribute(k_wall_force<kHooke>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   }
   const int cap = cap_per_atom * kWallTile;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid_for(s.nmax, kWallTile, 2 * lc.max_grid));
-  cfg.blockDim = dim3(kWallTile);
-  cfg.dynamicSmemBytes = (size_t)cap * kWallQ;
+  cfg.gridDim = dim3(grid_for(s.nmax, kWallWarps * kWallTile, 2 * lc.max_grid));
+  cfg.blockDim = dim3(kWallWarps * kWallTile);
+  cfg.dynamicSmemBytes = (size_t)kWallWarps * cap * kWallQ;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributePriority;
@@ -3168,10 +3216,7 @@ int launch_mesh_move(const Sys &s, const LaunchCfg &lc, cudaStream_t st) {
   int nl = 0;
   for (int k = 0; k < s.nmeshes; k++) {
     if (!s.meshes[k].moving) continue;
-    if (s.meshes[k].rotating)
-      k_mesh_rotate<<<grid_for(s.meshes[k].ntri, 256, lc.max_grid), 256, 0, st>>>(s, k);
-    else
-      k_mesh_move<<<grid_for(s.meshes[k].ntri, 256, lc.max_grid), 256, 0, st>>>(s, k);
+    k_mesh_move<<<grid_for(16L * s.meshes[k].ntri, 256, lc.max_grid), 256, 0, st>>>(s, k);
     nl++;
   }
   return nl;

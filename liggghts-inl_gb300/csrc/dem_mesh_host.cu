@@ -267,6 +267,22 @@ Topo topology(const Geo &g, const std::vector<std::vector<int>> &near) {
 
 }  // namespace
 
+void tri_floats(const double *g, float4 *out) {
+  const double *n0 = g, *sn = g + 30;
+  out[0] = {(float)n0[0], (float)n0[1], (float)n0[2], 0.f};
+  out[1] = {(float)sn[0], (float)sn[1], (float)sn[2], 0.f};
+  double c[3];
+  cross(g + 9, g + 12, c);
+  const bool thin = !(mag(c) >= 1e-5);
+  for (int q = 0; q < 3; q++) {
+    const double *en = g + 18 + 3 * q, *nq = g + 3 * q;
+    double d[3];
+    sub(nq, n0, d);
+    if (thin) out[2 + q] = {0.f, 0.f, 0.f, 0.f};
+    else out[2 + q] = {(float)en[0], (float)en[1], (float)en[2], (float)dot(en, d)};
+  }
+}
+
 int mesh_prepare(int ntri, const double *nodes, const uint8_t *ea_in, const uint8_t *ca_in,
                  MeshHost &out) {
   if (ntri < 1 || !nodes) return DEM_ERR_BAD_ARG;
