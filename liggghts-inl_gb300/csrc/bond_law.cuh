@@ -71,7 +71,7 @@ __device__ __forceinline__ double bond_hyst(double th, double &hmax, double &hmi
 // h points at the pair's bond value 0 (device history d = 3); hs is the
 // stride between values.  Returns true when the pair is bonded and its
 // forces (o) replace the normal model's.
-__device__ bool bond_nonlinear(const Sys &s, const BondIn &b, double *h, size_t hs, int *flag,
+static __device__ bool bond_nonlinear(const Sys &s, const BondIn &b, double *h, size_t hs, int *flag,
                                bool update_history, long long ntimestep, ContactOut &o) {
   const int tp = b.tp;
   const double lambda = bond_tab(s, kBondLambda, tp);

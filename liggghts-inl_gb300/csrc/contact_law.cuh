@@ -101,6 +101,13 @@ struct ContactOut {
   double Tj[3];          // j_forces.delta_torque
 };
 
+// a > b for doubles that are not negative, on the integer pipe (their bit
+// patterns order the same way; a DSETP and the selects behind it hold the FP64
+// pipe for 108 cycles per warp)
+__device__ __forceinline__ bool gt_nonneg(double a, double b) {
+  return __double_as_longlong(a) > __double_as_longlong(b);
+}
+
 // shear[3] is the tangential history, updated in place when update_history.
 // base: forces and torques of a bonded pair (cohesion bond/nonlinear), which
 // replace the normal model's force before the tangential and rolling models
@@ -146,7 +153,7 @@ __device__ __forceinline__ void contact_law(const ContactIn &c, const TypePair &
     // the correctly rounded sqrt, with fewer FP64 instructions and no divide
     // (zero for a contact at zero overlap, as sqrt(0) gives)
     const double xr = c.reff * deltan;
-    const bool pos = xr > 0.0;
+    const bool pos = __double_as_longlong(xr) > 0;  // (on the integer pipe)
     const double rs = rsqrt(pos ? xr : 1.0);
     const double sqrtval = pos ? xr * rs : 0.0;
     const double q = pos ? rsqrt(rs) : 0.0;
@@ -178,7 +185,7 @@ __device__ __forceinline__ void contact_law(const ContactIn &c, const TypePair &
   const double ss = s0 * s0 + s1 * s1 + s2 * s2;
   const double Ft_friction = tp.mu * fabs(Fn);
   const double kt2ss = kt * kt * ss;
-  if (kt2ss > Ft_friction * Ft_friction) {
+  if (gt_nonneg(kt2ss, Ft_friction * Ft_friction)) {
     // sliding (ss > 0 here): cap the spring force at mu|Fn|;
     // mu|Fn| / (kt |shear|) with one reciprocal square root, no divide
     const double ratio = Ft_friction * rsqrt(kt2ss);
@@ -250,6 +257,151 @@ __device__ __forceinline__ void contact_law(const ContactIn &c, const TypePair &
     o.Tj[1] = -crj * tor2 + rt2;
     o.Tj[2] = -crj * tor3 + rt3;
   }
+}
+
+// contact_law for a pair of spheres without cohesion and rolling friction,
+// with the identities that save FP64 instructions (about 110 against 125 per
+// entry; each holds the pipe of its SM quarter for 64 cycles, whatever the
+// number of active lanes):
+//   * the surface velocity from en x (cri wi + crj wj): no 1/r on the radii,
+//     the vector sums as chains of fused multiply-adds;
+//   * one path for sticking and sliding: the spring of a sliding contact is
+//     cut to mu|Fn| (history and force alike), its damping drops out, so a
+//     warp with both kinds does not run two force evaluations;
+//   * kn*deltan formed once; comparisons of magnitudes on the integer pipe.
+// Each moves a result by rounding only.  With rolling friction the general
+// law stays (see plane_contact_fast on what CDT makes of a changed rounding).
+template <int NORMAL>
+__device__ __forceinline__ void pair_law(const ContactIn &c, const TypePair &tp, double dt, bool tdamp, bool limitf,
+                                         bool update_history, double shear[3], ContactOut &o) {
+  const double ex = c.en[0], ey = c.en[1], ez = c.en[2];
+  const double vn = c.vr[0] * ex + c.vr[1] * ey + c.vr[2] * ez;
+  const double deltan = __dadd_rn(c.radsum, -c.r);
+  const double cri = c.radi - 0.5 * deltan, crj = c.radj - 0.5 * deltan;
+  const double W0 = cri * c.wi[0] + crj * c.wj[0];
+  const double W1 = cri * c.wi[1] + crj * c.wj[1];
+  const double W2 = cri * c.wi[2] + crj * c.wj[2];
+  const double vt0 = fma(-ez, W1, fma(ey, W2, fma(-vn, ex, c.vr[0])));
+  const double vt1 = fma(-ex, W2, fma(ez, W0, fma(-vn, ey, c.vr[1])));
+  const double vt2 = fma(-ey, W0, fma(ex, W1, fma(-vn, ez, c.vr[2])));
+
+  // ---- normal model (see contact_law)
+  double kn, kt, gamman, gammat;
+  if (NORMAL == kHertz) {
+    const double xr = c.reff * deltan;
+    const bool pos = __double_as_longlong(xr) > 0;
+    const double rs = rsqrt(pos ? xr : 1.0);
+    const double sqrtval = pos ? xr * rs : 0.0;
+    const double q = pos ? rsqrt(rs) : 0.0;
+    kn = tp.Y43 * sqrtval;
+    kt = tp.G8 * sqrtval;
+    gamman = c.c0 * q;
+    gammat = c.c1 * q;
+  } else {
+    kn = c.c0;
+    kt = kn;
+    gamman = c.c1;
+    gammat = tdamp ? gamman : 0.0;
+  }
+  const double knd = kn * deltan;
+  double Fn = fma(-gamman, vn, knd);
+  if (limitf && Fn < 0.0) Fn = 0.0;
+
+  // ---- tangential history
+  double s0 = shear[0], s1 = shear[1], s2 = shear[2];
+  if (update_history) {
+    s0 = fma(vt0, dt, s0);
+    s1 = fma(vt1, dt, s1);
+    s2 = fma(vt2, dt, s2);
+    const double rsht = s0 * ex + s1 * ey + s2 * ez;
+    s0 = fma(-rsht, ex, s0);
+    s1 = fma(-rsht, ey, s1);
+    s2 = fma(-rsht, ez, s2);
+  }
+  const double kt2ss = kt * kt * (s0 * s0 + s1 * s1 + s2 * s2);
+  const double Ff = tp.mu * fabs(Fn);
+  if (gt_nonneg(kt2ss, Ff * Ff)) {  // sliding
+    const double ratio = Ff * rsqrt(kt2ss);
+    s0 *= ratio;
+    s1 *= ratio;
+    s2 *= ratio;
+    gammat = 0.0;
+  }
+  const double Ft0 = fma(-gammat, vt0, -(kt * s0));
+  const double Ft1 = fma(-gammat, vt1, -(kt * s1));
+  const double Ft2 = fma(-gammat, vt2, -(kt * s2));
+  if (update_history) {
+    shear[0] = s0;
+    shear[1] = s1;
+    shear[2] = s2;
+  }
+  const double tor0 = ey * Ft2 - ez * Ft1;
+  const double tor1 = ez * Ft0 - ex * Ft2;
+  const double tor2 = ex * Ft1 - ey * Ft0;
+  o.F[0] = fma(Fn, ex, Ft0);
+  o.F[1] = fma(Fn, ey, Ft1);
+  o.F[2] = fma(Fn, ez, Ft2);
+  o.Ti[0] = -cri * tor0;
+  o.Ti[1] = -cri * tor1;
+  o.Ti[2] = -cri * tor2;
+  o.Tj[0] = -crj * tor0;
+  o.Tj[1] = -crj * tor1;
+  o.Tj[2] = -crj * tor2;
+}
+
+// contact_law for a sphere on a plane normal to axis n (sign: the side it is
+// on), in the frame (n, t1, t2), cyclic axes: v and w are the velocity and
+// spin in that frame, sh the tangential history in t1 and t2 (its normal part
+// is zero after every update), F and T the results.  With en = +-e_n the
+// vector algebra falls away: about 50 FP64 instructions against 140 for the
+// general law.
+template <int NORMAL>
+__device__ __forceinline__ void plane_law(double sign, double radi, double deltan, const double v[3], const double w[3],
+                                          double c0, double c1, const TypePair &tp, double dt, bool tdamp,
+                                          bool limitf, bool update_history, double &s1, double &s2,
+                                          double F[3], double T[3]) {
+  const double vn = sign * v[0];
+  const double cri = radi - 0.5 * deltan, cs = sign * cri;
+  const double vt1 = fma(-cs, w[2], v[1]), vt2 = fma(cs, w[1], v[2]);
+  double kn, kt, gamman, gammat;
+  if (NORMAL == kHertz) {
+    const double xr = radi * deltan;
+    const bool pos = __double_as_longlong(xr) > 0;
+    const double rs = rsqrt(pos ? xr : 1.0);
+    const double sqrtval = pos ? xr * rs : 0.0;
+    const double q = pos ? rsqrt(rs) : 0.0;
+    kn = tp.Y43 * sqrtval;
+    kt = tp.G8 * sqrtval;
+    gamman = c0 * q;
+    gammat = c1 * q;
+  } else {
+    kn = c0;
+    kt = kn;
+    gamman = c1;
+    gammat = tdamp ? gamman : 0.0;
+  }
+  const double knd = kn * deltan;
+  double Fn = fma(-gamman, vn, knd);
+  if (limitf && Fn < 0.0) Fn = 0.0;
+  if (update_history) {
+    s1 = fma(vt1, dt, s1);
+    s2 = fma(vt2, dt, s2);
+  }
+  const double kt2ss = kt * kt * (s1 * s1 + s2 * s2);
+  const double Ff = tp.mu * fabs(Fn);
+  if (gt_nonneg(kt2ss, Ff * Ff)) {
+    const double ratio = Ff * rsqrt(kt2ss);
+    s1 *= ratio;
+    s2 *= ratio;
+    gammat = 0.0;
+  }
+  const double Ft1 = fma(-gammat, vt1, -(kt * s1)), Ft2 = fma(-gammat, vt2, -(kt * s2));
+  F[0] = sign * Fn;
+  F[1] = Ft1;
+  F[2] = Ft2;
+  T[0] = 0.0;
+  T[1] = cs * Ft2;
+  T[2] = -(cs * Ft1);
 }
 
 }  // namespace gb300

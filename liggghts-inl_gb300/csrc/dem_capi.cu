@@ -51,7 +51,10 @@ struct dem_handle {
   double *diag_buf = nullptr;  // dem_get_diagnostics partial sums
   LaunchCfg lc{152 * 8};
   float last_ms = 0.f;
+  // the control block as last read: every call that runs kernels ends by
+  // reading it, so between calls it equals the device's
   Ctrl host_ctrl{};
+  Ctrl *ctrl_pinned = nullptr;  // where the device's copy lands
   // per-kernel timing (dem_profile)
   bool profile = false;
   std::vector<cudaEvent_t> evpool;
@@ -63,7 +66,7 @@ struct dem_handle {
   cudaStream_t st2 = nullptr;
   cudaGraphExec_t gexec = nullptr;
   long long graph_gen = -1, sys_gen = 0;  // rebuilt when device pointers change
-  int graph_kps = 0, graph_kpr = 0;
+  StepCounts graph_counts;
   std::vector<MeshHost> mesh_host;
   std::vector<double> bond_tables;  // host copy for the cutoff derivation
   double cell_scale = 1.0;          // neighbour cell edge / cutneighmax (dem_set_tuning)
@@ -83,7 +86,8 @@ static int ensure_graph(dem_handle *h) {
     cudaGraphExecDestroy(h->gexec);
     h->gexec = nullptr;
   }
-  cudaError_t e = build_step_graph(h->s, h->lc, h->st, h->st2, &h->gexec, &h->graph_kps, &h->graph_kpr);
+  h->lc.np = h->host_ctrl.np;
+  cudaError_t e = build_step_graph(h->s, h->lc, h->st, h->st2, &h->gexec, &h->graph_counts);
   if (e != cudaSuccess) {
     h->err = std::string("build_step_graph: ") + cudaGetErrorString(e);
     return DEM_ERR_CUDA;
@@ -279,6 +283,7 @@ static int alloc_atoms(dem_handle *h, int nmax) {
     ar.take(&s.mlist, nmax);
     ar.take(&s.stash, (size_t)kStash * nmax);
     ar.take(&s.wforce, (size_t)3 * std::max(1, s.nplanes + s.nmeshes) * nmax);
+    ar.take(&s.wcon, (size_t)2 * std::max(1, s.nplanes + s.nmeshes) * nmax);
     ar.take(&s.order, nmax);
     ar.take(&s.pcount, nmax + 1);
     ar.take(&s.rev_count, nmax + 1);
@@ -404,8 +409,9 @@ static int alloc_pairs(dem_handle *h, int pcap, int keep_np) {
 }
 
 static int read_ctrl(dem_handle *h) {
-  CUDA_TRY(h, cudaMemcpyAsync(&h->host_ctrl, h->s.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, h->st));
+  CUDA_TRY(h, cudaMemcpyAsync(h->ctrl_pinned, h->s.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, h->st));
   CUDA_TRY(h, cudaStreamSynchronize(h->st));
+  h->host_ctrl = *h->ctrl_pinned;
   harvest(h);
   return DEM_OK;
 }
@@ -417,6 +423,7 @@ static int recover(dem_handle *h, bool *resumed) {
   int rc = read_ctrl(h);
   if (rc) return rc;
   Ctrl &c = h->host_ctrl;
+  if (c.status == kStatTimeout) return fail(h, DEM_ERR_TIMEOUT, "a wait of the fused step kernel gave up");
   if (c.status == kStatNan) return fail(h, DEM_ERR_NAN, "non-finite particle position");
   if (c.status == kStatMeshSlots)
     return fail(h, DEM_ERR_CAPACITY, "a mesh contact found no free history slot (inconsistent slots)");
@@ -507,7 +514,8 @@ int dem_create(const dem_config *cfg, dem_handle **out) {
   h->allocs_misc.push_back(s.ctrl);
   cudaMemset(s.ctrl, 0, sizeof(Ctrl));
   if (cudaMalloc(&h->chk, sizeof(UploadCheck)) != cudaSuccess ||
-      cudaMallocHost(&h->chk_host, sizeof(UploadCheck)) != cudaSuccess) {
+      cudaMallocHost(&h->chk_host, sizeof(UploadCheck)) != cudaSuccess ||
+      cudaMallocHost(&h->ctrl_pinned, sizeof(Ctrl)) != cudaSuccess) {
     delete h;
     return DEM_ERR_CUDA;
   }
@@ -566,6 +574,7 @@ int dem_destroy(dem_handle *h) {
   }
   if (h->stage) cudaFree(h->stage);
   if (h->chk_host) cudaFreeHost(h->chk_host);
+  if (h->ctrl_pinned) cudaFreeHost(h->ctrl_pinned);
   if (h->diag_buf) cudaFree(h->diag_buf);
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);
@@ -1345,7 +1354,7 @@ int dem_setup(dem_handle *h) {
   }
   h->kt.kernel_launches += launch_pair(h->s, h->lc, 0, h->st);
   h->kt.kernel_launches += launch_wall_force(h->s, h->lc, 0, h->st);
-  h->kt.kernel_launches += launch_particle(h->s, h->lc, kModeGather, 0, h->st);
+  h->kt.kernel_launches += launch_particle(h->s, h->lc, kModeGather, h->st);
   CUDA_TRY(h, cudaGetLastError());
   bool dummy;
   int rc = recover(h, &dummy);
@@ -1359,19 +1368,23 @@ int dem_step(dem_handle *h, int nsteps) {
   if (!h->setup_done) return fail(h, DEM_ERR_BAD_ARG, "dem_setup must precede dem_step");
   if (nsteps == 0) return DEM_OK;
   set_mesh_velocity_on(h, 1);
-  int rc = read_ctrl(h);
-  if (rc) return rc;
+  int rc = DEM_OK;
   const long long ts0 = h->host_ctrl.ntimestep;
+  const bool graph = h->use_graph && !h->profile;
+  if (graph && (rc = ensure_graph(h))) return rc;
   CUDA_TRY(h, cudaEventRecord(h->ev0, h->st));
   long long done = 0;  // steps whose rebuild+pair stage has been queued
   bool first = true;
-  const bool graph = h->use_graph && !h->profile;
+  bool closed = false;  // the last step's final_integrate has run
   while (done < nsteps) {
     const long long chunk = graph ? nsteps - done : std::min<long long>(kCheckEvery, nsteps - done);
     long long k0 = 0;
     mark_start(h);
-    if (first) {  // step 1 starts from stored forces: initial_integrate only
-      h->kt.kernel_launches += launch_particle(h->s, h->lc, kModeInitial, 1, h->st);
+    int phase = first ? kStepFirst : kStepGather;
+    // step 1 starts from stored forces: initial_integrate only.  The graph
+    // runs it too, unless staged atoms join between its drift and its decision
+    if (first && (!graph || h->pending_insert > 0)) {
+      h->kt.kernel_launches += launch_particle(h->s, h->lc, kModeInitial, h->st);
       h->kt.kernel_launches += launch_mesh_move(h->s, h->lc, h->st);
       if (h->pending_insert > 0) {  // staged atoms join now and force a rebuild
         h->kt.kernel_launches += launch_insert_commit(h->s, h->pending_insert, h->st);
@@ -1385,24 +1398,19 @@ int dem_step(dem_handle *h, int nsteps) {
       mark(h, 2);
       h->kt.kernel_launches += launch_wall_force(h->s, h->lc, 1, h->st);
       mark(h, 3);
-      first = false;
       k0 = 1;
+      phase = kStepGather;
     }
-    if (graph && chunk > k0) {
-      rc = ensure_graph(h);
-      if (rc) return rc;
-      rc = read_ctrl(h);
-      if (rc) return rc;
-      const long long rb0 = h->host_ctrl.nrebuilds;
-      h->kt.kernel_launches += launch_set_loop(h->s, (int)(chunk - k0), h->st);
+    first = false;
+    const long long rb0 = h->host_ctrl.nrebuilds;
+    const bool launched = graph && chunk > k0;
+    if (launched) {
+      h->kt.kernel_launches += launch_set_loop(h->s, (int)(chunk - k0), phase, h->st);
       CUDA_TRY(h, cudaGraphLaunch(h->gexec, h->st));
-      rc = read_ctrl(h);
-      if (rc) return rc;
-      const long long iters = std::min<long long>(chunk - k0, h->host_ctrl.ntimestep - (ts0 + done + k0));
-      h->kt.kernel_launches += iters * h->graph_kps + (h->host_ctrl.nrebuilds - rb0) * h->graph_kpr;
+      CUDA_TRY(h, cudaEventRecord(h->ev1, h->st));
     } else {
       for (long long k = k0; k < chunk; k++) {
-        h->kt.kernel_launches += launch_particle(h->s, h->lc, kModeGatherFinalInitial, 1, h->st);
+        h->kt.kernel_launches += launch_particle(h->s, h->lc, kModeGatherFinalInitial, h->st);
         h->kt.kernel_launches += launch_mesh_move(h->s, h->lc, h->st);
         mark(h, 0);
         h->kt.kernel_launches += launch_decide(h->s, h->st);
@@ -1418,6 +1426,12 @@ int dem_step(dem_handle *h, int nsteps) {
     bool resumed = false;
     rc = recover(h, &resumed);
     if (rc) return rc;
+    if (launched) {
+      const StepCounts &gc = h->graph_counts;
+      const long long iters = std::min<long long>(chunk - k0, h->host_ctrl.ntimestep - (ts0 + done + k0));
+      h->kt.kernel_launches += gc.call + std::max<long long>(0, iters - 1) * gc.step +
+                               (h->host_ctrl.nrebuilds - rb0) * gc.rebuild;
+    }
     if (resumed) {
       // the halted step's rebuild is now finished; compute its forces and
       // continue after it (later queued kernels were no-ops)
@@ -1432,21 +1446,23 @@ int dem_step(dem_handle *h, int nsteps) {
           h->kt.kernel_launches += launch_wall_force(h->s, h->lc, 1, h->st);
         }
       }
-      rc = read_ctrl(h);
-      if (rc) return rc;
+      if (graph && (rc = ensure_graph(h))) return rc;  // device pointers changed
       done = h->host_ctrl.ntimestep - ts0;
     } else {
       done += chunk;
+      closed = launched;
     }
   }
-  mark_start(h);
-  h->kt.kernel_launches += launch_particle(h->s, h->lc, kModeGatherFinal, 1, h->st);
-  mark(h, 0);
-  CUDA_TRY(h, cudaEventRecord(h->ev1, h->st));
-  CUDA_TRY(h, cudaGetLastError());
-  bool dummy;
-  rc = recover(h, &dummy);
-  if (rc) return rc;
+  if (!closed) {
+    mark_start(h);
+    h->kt.kernel_launches += launch_particle(h->s, h->lc, kModeGatherFinal, h->st);
+    mark(h, 0);
+    CUDA_TRY(h, cudaEventRecord(h->ev1, h->st));
+    CUDA_TRY(h, cudaGetLastError());
+    bool dummy;
+    rc = recover(h, &dummy);
+    if (rc) return rc;
+  }
   cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1);
   return DEM_OK;
 }
@@ -1501,8 +1517,6 @@ int dem_get_diagnostics(dem_handle *h, const double *region_lo, const double *re
 
 int dem_natoms(dem_handle *h, int *n) {
   if (!h || !n) return DEM_ERR_BAD_ARG;
-  int rc = read_ctrl(h);
-  if (rc) return rc;
   *n = h->host_ctrl.n;
   return DEM_OK;
 }
@@ -1510,8 +1524,7 @@ int dem_natoms(dem_handle *h, int *n) {
 int dem_download_atoms(dem_handle *h, int *tag, int *type, double *x, double *v, double *omega,
                        double *f, double *torque, double *radius, double *rmass) {
   if (!h || !h->have_atoms) return DEM_ERR_BAD_ARG;
-  int rc = read_ctrl(h);
-  if (rc) return rc;
+  int rc = DEM_OK;
   const int n = h->host_ctrl.n;
   if (n <= 0) return DEM_OK;
   AtomsOut out{tag, type, x, v, omega, f, torque, radius, rmass};

@@ -129,7 +129,16 @@ struct Ctrl {
   int ens_inplace;    // ensemble builds in place (atoms and list)
   int ens_relayout;   // ensemble builds in place for the atoms, list re-laid
   int pdone;          // blocks of k_particle done (the last one decides; graph steps)
+  // k_steps: what the launch starts with (kStep*), blocks that left, a wait
+  // gave up, the grid barrier's count (see grid_barrier)
+  int step_phase, bar_exit, bar_abort;
+  unsigned long long bar;
 };
+
+// Ctrl::step_phase: the first step of a call (no forces to gather), a step
+// that gathers the previous step's forces, resume with the forces after a
+// rebuild, all steps done
+enum { kStepFirst = 0, kStepGather = 1, kStepForces = 2, kStepDone = 3 };
 
 // Primitive wall of fix wall/gran (src/primitive_wall_definitions.h): a
 // plane normal to `axis` at pos, or a cylinder about `axis` of radius pos
@@ -160,6 +169,7 @@ constexpr int kMeshMaxCand = 24;
 constexpr int kMeshFastCand = 32;  // k_wall_force's tiled path (32-bit masks); more take the sequential path
 constexpr int kSlotKept = 1 << 30; // mesh_contacts: marks a slot touched in this evaluation
 constexpr int kTriStride = 40;     // doubles of geometry per triangle, see below
+constexpr int kStatTimeout = 8;    // Ctrl::status: a wait of k_steps gave up
 constexpr int kTrif = 5;           // float4 of FP32 copies per triangle
 constexpr int kStatMeshSlots = 5;  // Ctrl::status: a mesh contact found no free slot (inconsistent slots)
 constexpr int kStatMeshReg = 6;    // Ctrl::status: triangle-cell registrations overflowed (halted, grown, resumed)
@@ -220,6 +230,7 @@ struct Sys {
   float4 *xhf;      // FP32 copy of x at the last neighbour build (displacement prefilter)
   int *mlist;       // atoms with candidate mesh triangles [nmax]
   int *stash;       // [kStash*nmax]: entries found by the count pass, see kStash
+  double *wcon;     // [(2w+k)*nmax + i]: contact constants c0, c1 of listed atom i with wall w
   double *wforce;   // [(w*3+d)*nmax + i]: force of wall w (planes, then meshes) on listed
                     // atom i at the last force evaluation (diagnostics)
   // parameters

@@ -20,67 +20,9 @@
 #include "dem_device.cuh"
 #include "dem_kernels.h"
 #include "mesh_device.cuh"
+#include "step_device.cuh"
 
 namespace gb300 {
-
-#define GRID_STRIDE(i, n) for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
-
-__device__ __forceinline__ bool gated(const Ctrl *c) { return c->halt != 0 || c->rebuild == 0; }
-
-// Exact reference arithmetic (no contraction) for everything that decides
-// membership of the pair set.
-__device__ __forceinline__ double rsq_rn(double dx, double dy, double dz) {
-  return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-}
-
-__device__ __forceinline__ void shift_decode(int c, int &sx, int &sy, int &sz) {
-  sx = c % 3 - 1;
-  sy = (c / 3) % 3 - 1;
-  sz = c / 9 - 1;
-}
-
-// ghost image x_j + pbc*prd exactly as CommBrick::borders/forward_comm
-// (src/atom_vec_sphere.cpp:213-223): fl(x + (+-prd)) per shifted dimension.
-__device__ __forceinline__ void image(const Sys &s, int code, double &xj, double &yj, double &zj) {
-  if (code == kNoShift) return;
-  int sx, sy, sz;
-  shift_decode(code, sx, sy, sz);
-  // +-prd by selection: sx * prd would convert sx to FP64 and multiply on
-  // the FP64 pipe (and the compiler hoists that out of candidate loops)
-  if (sx) xj = __dadd_rn(xj, sx > 0 ? s.prd[0] : -s.prd[0]);
-  if (sy) yj = __dadd_rn(yj, sy > 0 ? s.prd[1] : -s.prd[1]);
-  if (sz) zj = __dadd_rn(zj, sz > 0 ? s.prd[2] : -s.prd[2]);
-}
-
-// Whether the periodic image of j (shift sv) exists as a ghost atom:
-// CommBrick::borders sends an atom across a periodic boundary only when it
-// lies within slab_offset + its radius of that boundary (the granular
-// criterion of CommBrick::decide, src/comm_brick.cpp:443,1613-1624).  With a
-// contact distance factor above 1 this band is narrower than the pair cutoff
-// and some periodic pairs near the cutoff do not exist in the reference.
-__device__ __forceinline__ bool ghost_exists(const Sys &s, const AtomArrays &A, int j, const int sv[3]) {
-  const double rad = A.r[j];
-  const double pos[3] = {A.x[j], A.y[j], A.z[j]};
-#pragma unroll
-  for (int d = 0; d < 3; d++) {
-    if (sv[d] > 0 && !(pos[d] <= __dadd_rn(__dadd_rn(s.boxlo[d], s.ghost_slab), rad))) return false;
-    if (sv[d] < 0 && !(pos[d] >= __dadd_rn(__dadd_rn(s.boxhi[d], -s.ghost_slab), -rad))) return false;
-  }
-  return true;
-}
-
-// The cells are wider than the neighbour cutoff by a relative 1e-9 at least,
-// far above the rounding of this product, so atoms within the cutoff are
-// never more than one cell apart; every kernel bins through this function.
-// FP32 image shift -1, 0 or +1 times the period, by selection (no conversion)
-__device__ __forceinline__ float fshift(int sv, float prd) { return sv == 0 ? 0.0f : (sv > 0 ? prd : -prd); }
-
-__device__ __forceinline__ int cell_coord(const Sys &s, double x, int d) {
-  int c = (int)((x - s.boxlo[d]) * s.icsz[d]);
-  c = c < 0 ? 0 : c;
-  c = c >= s.nc[d] ? s.nc[d] - 1 : c;
-  return c;
-}
 
 // ----------------------------------------------------------------------------
 // step control
@@ -156,7 +98,10 @@ __global__ void k_decide_loop(Sys s, cudaGraphConditionalHandle hreb, cudaGraphC
   }
 }
 
-__global__ void k_set_loop(Sys s, int n) { s.ctrl->loop_left = n; }
+__global__ void k_set_loop(Ctrl *c, int n, int phase) {
+  c->loop_left = n;
+  c->step_phase = phase;
+}
 
 __global__ void k_set_rebuild(Sys s, int v) {
   if (s.ctrl->halt) return;
@@ -178,16 +123,6 @@ __global__ void k_zero_gated(Sys s, int *a, int n) {
 // ----------------------------------------------------------------------------
 // exclusive scan (warp-shuffle prefix sums), 4096 items per block
 // ----------------------------------------------------------------------------
-
-__device__ __forceinline__ int warp_incl_scan(int x) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    int y = __shfl_up_sync(0xffffffffu, x, off);
-    if (lane >= off) x += y;
-  }
-  return x;
-}
 
 // out[k] = sum(in[0..k-1]) within the block's 4096 items; bsum[block] = total.
 // gate: 0 always runs; 1 only while the system rebuilds; 2 also not in an
@@ -801,118 +736,6 @@ __device__ __forceinline__ void mslot_swap(const MeshDev &M, size_t nmax, int i,
   }
 }
 
-// MathExtra::quatquat (src/math_extra.h:596-602) and
-// MathExtraLiggghts::vec_quat_rotate (src/math_extra_liggghts.h:455-471) in
-// the reference's operation order, exactly rounded: rotated nodes are
-// bit-identical to the reference's
-__device__ __forceinline__ void quatquat_rn(const double *a, const double *b, double *c) {
-  c[0] = __dsub_rn(__dsub_rn(__dsub_rn(__dmul_rn(a[0], b[0]), __dmul_rn(a[1], b[1])), __dmul_rn(a[2], b[2])),
-                   __dmul_rn(a[3], b[3]));
-  c[1] = __dsub_rn(__dadd_rn(__dadd_rn(__dmul_rn(a[0], b[1]), __dmul_rn(b[0], a[1])), __dmul_rn(a[2], b[3])),
-                   __dmul_rn(a[3], b[2]));
-  c[2] = __dsub_rn(__dadd_rn(__dadd_rn(__dmul_rn(a[0], b[2]), __dmul_rn(b[0], a[2])), __dmul_rn(a[3], b[1])),
-                   __dmul_rn(a[1], b[3]));
-  c[3] = __dsub_rn(__dadd_rn(__dadd_rn(__dmul_rn(a[0], b[3]), __dmul_rn(b[0], a[3])), __dmul_rn(a[1], b[2])),
-                   __dmul_rn(a[2], b[1]));
-}
-__device__ __forceinline__ void vec_quat_rotate_rn(double *v, const double *q) {
-  const double vq[4] = {0., v[0], v[1], v[2]};
-  const double qc[4] = {q[0], -q[1], -q[2], -q[3]};
-  double t[4], r[4];
-  quatquat_rn(q, vq, t);
-  quatquat_rn(t, qc, r);
-  v[0] = r[1];
-  v[1] = r[2];
-  v[2] = r[3];
-}
-
-// One step of a moving mesh: 16 lanes per triangle, lane q taking one of its
-// vectors (nodes 0..2, edgeVec 3..5, edgeNorm 6..8, surfaceNorm 9), lane 10
-// the centre.  A quaternion rotation is a chain of some fifty FP64
-// instructions and most moving meshes have few triangles, so one thread per
-// triangle made ten such chains one after the other (a two-triangle paddle:
-// 23 us per step; one per lane: 6 us).  Returns whether a node moved more
-// than skin/2 since the last build.
-//   linear: MeshMoverLinear::initial_integrate + MultiNodeMesh::move (nodes and
-//     centres += dx, src/multi_node_mesh_I.h:502-520);
-//   rotating: MeshMoverRotate::initial_integrate
-//     (src/mesh_mover_rotation.cpp:105-131): nodes and centres
-//     (MultiNodeMesh::rotate(dQ, origin), src/multi_node_mesh_I.h:643-668), the
-//     rotating element vectors edgeVec, edgeNorm, surfaceNorm
-//     (CustomValueTracker::rotate), node velocities 0 + w x (node - O);
-// then the node-travel test of MultiNodeMesh::decideRebuild
-// (src/multi_node_mesh_I.h:792-823).
-__device__ __forceinline__ bool mesh_move_part(const Sys &s, const MeshDev &M, int t, int q) {
-  const double trigger = __dmul_rn(__dmul_rn(0.25, s.skin), s.skin);
-  double *g = M.tri + (size_t)t * kTriStride;
-  const bool on = t < M.ntri && q < 11;
-  bool moved = false;
-  double out[3] = {0., 0., 0.};
-  int at = -1;  // where this lane's vector goes in the triangle's record
-  if (on && !M.rotating) {
-    if (q < 3 || q == 10) {
-      at = q < 3 ? 3 * q : 33;
-      for (int d = 0; d < 3; d++) out[d] = __dadd_rn(g[at + d], M.dx[d]);
-    }
-  } else if (on) {
-    const double *o = M.rorig, *rq = M.rq;
-    const bool trans =
-        __dadd_rn(__dadd_rn(__dmul_rn(o[0], o[0]), __dmul_rn(o[1], o[1])), __dmul_rn(o[2], o[2])) > 0.;
-    if (q < 10) {
-      at = 3 * q + (q == 9 ? 3 : 0);
-      for (int d = 0; d < 3; d++) out[d] = g[at + d];
-      if (q < 3 && trans)
-        for (int d = 0; d < 3; d++) out[d] = __dsub_rn(out[d], o[d]);
-      vec_quat_rotate_rn(out, rq);
-      if (q < 3 && trans)
-        for (int d = 0; d < 3; d++) out[d] = __dadd_rn(out[d], o[d]);
-    } else {
-      at = 33;
-      for (int j = 0; j < 3; j++) {
-        double nd[3] = {g[3 * j], g[3 * j + 1], g[3 * j + 2]};
-        if (trans)
-          for (int d = 0; d < 3; d++) nd[d] = __dsub_rn(nd[d], o[d]);
-        vec_quat_rotate_rn(nd, rq);
-        if (trans)
-          for (int d = 0; d < 3; d++) nd[d] = __dadd_rn(nd[d], o[d]);
-        for (int d = 0; d < 3; d++) out[d] = __dadd_rn(nd[d], out[d]);
-      }
-      const double third = 1. / 3.;
-      for (int d = 0; d < 3; d++) out[d] = __dmul_rn(third, out[d]);
-    }
-  }
-  __syncwarp();  // every lane has read the record before any writes it
-  if (at >= 0) {
-    for (int d = 0; d < 3; d++) g[at + d] = out[d];
-    if (q < 3) {
-      double dsq = 0.0;
-      for (int d = 0; d < 3; d++) {
-        const double e = __dadd_rn(out[d], -M.node_last[(size_t)t * 9 + 3 * q + d]);
-        dsq = d == 0 ? __dmul_rn(e, e) : __dadd_rn(dsq, __dmul_rn(e, e));
-      }
-      moved = dsq > trigger;
-      if (M.rotating) {
-        const double *o = M.rorig, *w = M.romega;
-        const double r[3] = {__dsub_rn(out[0], o[0]), __dsub_rn(out[1], o[1]), __dsub_rn(out[2], o[2])};
-        double *v = M.nodev + (size_t)t * 9 + 3 * q;
-        v[0] = __dadd_rn(0.0, __dsub_rn(__dmul_rn(w[1], r[2]), __dmul_rn(w[2], r[1])));
-        v[1] = __dadd_rn(0.0, __dsub_rn(__dmul_rn(w[2], r[0]), __dmul_rn(w[0], r[2])));
-        v[2] = __dadd_rn(0.0, __dsub_rn(__dmul_rn(w[0], r[1]), __dmul_rn(w[1], r[0])));
-      }
-    }
-    // the FP32 copies: node 0, surface normal, edge normals (all zero where
-    // the triangle is too thin for the edge bounds, see tri_floats)
-    float4 *T = M.trif + kTrif * (size_t)t;
-    const int slot = q == 0 ? 0 : (q == 9 ? 1 : (q >= 6 && q < 9 ? q - 4 : -1));
-    if (slot >= 0) {
-      const float4 old = T[slot];
-      if (slot < 2 || old.x != 0.f || old.y != 0.f || old.z != 0.f)
-        T[slot] = make_float4((float)out[0], (float)out[1], (float)out[2], old.w);
-    }
-  }
-  return moved;
-}
-
 __global__ void k_mesh_move(Sys s, int k) {
   Ctrl *c = s.ctrl;
   if (c->halt) return;
@@ -1061,14 +884,6 @@ __global__ void k_mesh_cand(Sys s, int k) {
   }
 }
 
-// end of atom i's owner row and of its partner list
-__device__ __forceinline__ int row_end(const Sys &s, const PairArrays &L, int i) {
-  return s.nsys ? L.rowe[i] : L.row[i + 1];
-}
-__device__ __forceinline__ int rev_end(const Sys &s, const PairArrays &L, int i) {
-  return s.nsys ? L.reve[i] : L.rev_start[i + 1];
-}
-
 // Entry of the old list for the atom pair (owner o, partner q) in old
 // indices: o's own row first, then the entries where o was the partner
 // (flip = true).  Only flagged entries carry history (pre_exchange keeps
@@ -1103,8 +918,23 @@ __global__ void __launch_bounds__(256) k_wall_list(Sys s) {
     const int i = base + threadIdx.x;
     bool has = false;
     if (i < n) {
-      has = (A.wbits[i] & 0x7fu) != 0;
-      for (int k = 0; k < s.nmeshes; k++) has |= s.meshes[k].cand_n[i] > 0;
+      const unsigned bits = A.wbits[i];
+      has = (bits & 0x7fu) != 0;
+      for (int w = 0; w < s.nplanes + s.nmeshes; w++) {
+        const bool mesh = w >= s.nplanes;
+        // (plane 7 shares its bit with the list mark, so that the wall tiles
+        // look at it for every listed atom)
+        const bool near = mesh ? s.meshes[w - s.nplanes].cand_n[i] > 0 : (w == 7 || ((bits >> w) & 1u));
+        has |= mesh && near;
+        if (!near) continue;
+        const int wt = mesh ? s.meshes[w - s.nplanes].wall_type : s.planes[w].wall_type;
+        const TypePair tp = load_typepair(s.params, s.ntypes, A.type[i], wt ? wt : A.type[i]);
+        double c0, c1;
+        if (s.normal == kHertz) contact_consts<kHertz>(tp, A.m[i], A.r[i], s.charVel, s.tdamp, c0, c1);
+        else contact_consts<kHooke>(tp, A.m[i], A.r[i], s.charVel, s.tdamp, c0, c1);
+        s.wcon[(size_t)(2 * w) * s.nmax + i] = c0;
+        s.wcon[(size_t)(2 * w + 1) * s.nmax + i] = c1;
+      }
       A.wbits[i] = has ? (uint8_t)(A.wbits[i] | 0x80u) : (uint8_t)(A.wbits[i] & 0x7fu);
     }
     const unsigned m = __ballot_sync(0xffffffffu, has);
@@ -1522,851 +1352,41 @@ __global__ void k_finish_rebuild(Sys s) {
   }
 }
 
-// ----------------------------------------------------------------------------
-// pair forces: one thread per half-list entry, results to the pair buffer
-// ----------------------------------------------------------------------------
-
-// The pair kernels test list entries per lane (phase 1) and queue the ones
-// that need the FP64 laws in a per-warp shared-memory queue (warp ballots),
-// so phase 2 runs on full warps: entries that need nothing cost no FP64
-// issue slots.  Results go to the entry's own slot, so the processing order
-// never changes a value.  kPairTile is k_pair_pf's block size.
-constexpr int kPairTile = 256;
-
-// The general kernel carries the bond law.  Blocks of 128 threads capped at
-// 128 registers (a few spilled) let four blocks share an SM (measured on the
-// 200k bonded fibre bed with one queue per tile: 0.55 ms with one 256-thread
-// block per SM, 0.41 ms with three 128-thread blocks, 0.35 ms with four;
-// 64-thread tiles 0.40 ms; with per-warp queues 0.27 ms).
-constexpr int kBandTile = 128;
-
-// the entry's result record: three whole 32-byte sectors in one go
-__device__ __forceinline__ void store_result(const Sys &s, int q, const ContactOut &o) {
-  double2 *r = reinterpret_cast<double2 *>(s.res + (size_t)kResStride * q);
-  r[0] = make_double2(o.F[0], o.F[1]);
-  r[1] = make_double2(o.F[2], o.Ti[0]);
-  r[2] = make_double2(o.Ti[1], o.Ti[2]);
-  r[3] = make_double2(o.Tj[0], o.Tj[1]);
-  r[4] = make_double2(o.Tj[2], 0.0);
-  r[5] = make_double2(0.0, 0.0);
-}
-
-// Phase 2 of k_pair for one queued entry q (delx, dely, delz, rsq_q from
-// its exact test): the bond law, the contact law, the result record
-template <int NORMAL, bool ROLL, bool BOND>
-__device__ __forceinline__ void band_entry(const Sys &s, int q, double delx, double dely, double delz,
-                                           double rsq_q, int shearupdate, long long ntimestep) {
-  const AtomArrays &A = s.atoms[0];
-  const PairArrays &L = s.pairs[0];
-  const size_t P = s.pcap;
-  const int i = L.i[q], j = L.j[q];
-  ContactIn ci;
-  ci.d[0] = delx;
-  ci.d[1] = dely;
-  ci.d[2] = delz;
-  ci.radi = A.r[i];
-  ci.radj = A.r[j];
-  ci.radsum = __dadd_rn(ci.radi, ci.radj);
-  ci.vr[0] = A.vx[i] - A.vx[j];
-  ci.vr[1] = A.vy[i] - A.vy[j];
-  ci.vr[2] = A.vz[i] - A.vz[j];
-  ci.wi[0] = A.wx[i]; ci.wi[1] = A.wy[i]; ci.wi[2] = A.wz[i];
-  ci.wj[0] = A.wx[j]; ci.wj[1] = A.wy[j]; ci.wj[2] = A.wz[j];
-  const bool touch = !BOND || rsq_q < __dmul_rn(ci.radsum, ci.radsum);
-  ContactOut bo;
-  bool bonded = false;
-  if (BOND) {
-    // evaluated in the reference's orientation: owner = lower lidx
-    // (periodic entries are directed and always owned by i)
-    const bool rev = L.sh[q] == kNoShift && A.lidx[i] > A.lidx[j];
-    const int a = rev ? j : i, b = rev ? i : j;
-    const double sg = rev ? -1.0 : 1.0;
-    BondIn bi;
-    bi.d[0] = sg * ci.d[0]; bi.d[1] = sg * ci.d[1]; bi.d[2] = sg * ci.d[2];
-    bi.rsq = rsq_q;
-    bi.radi = A.r[a];
-    bi.radj = A.r[b];
-    bi.vi[0] = A.vx[a]; bi.vi[1] = A.vy[a]; bi.vi[2] = A.vz[a];
-    bi.vj[0] = A.vx[b]; bi.vj[1] = A.vy[b]; bi.vj[2] = A.vz[b];
-    bi.wi[0] = A.wx[a]; bi.wi[1] = A.wy[a]; bi.wi[2] = A.wz[a];
-    bi.wj[0] = A.wx[b]; bi.wj[1] = A.wy[b]; bi.wj[2] = A.wz[b];
-    bi.xi[0] = A.x[a]; bi.xi[1] = A.y[a]; bi.xi[2] = A.z[a];
-    bi.tp = A.type[a] * (s.ntypes + 1) + A.type[b];
-    ContactOut bc;
-    bonded = bond_nonlinear(s, bi, L.hist + 3 * P + q, P, L.flag + q, shearupdate != 0, ntimestep, bc);
-    if (bonded) {  // back to the list's orientation (i owns the entry)
-      for (int k = 0; k < 3; k++) {
-        bo.F[k] = sg * bc.F[k];
-        bo.Ti[k] = rev ? bc.Tj[k] : bc.Ti[k];
-        bo.Tj[k] = rev ? bc.Ti[k] : bc.Tj[k];
-      }
-    }
+// entries of a grid-stride walk over the list, 32 per warp
+struct GridTiles {
+  long base, stride;
+  __device__ __forceinline__ GridTiles(int block) {
+    base = (long)blockIdx.x * block + (threadIdx.x & ~31);
+    stride = (long)gridDim.x * block;
+    base -= stride;
   }
-  ContactOut o;
-  if (touch) {
-    // r from 1/r: within an ulp of sqrt(rsq), which moves the overlap
-    // radsum - r by ~1e-13 of itself
-    ci.rinv = rsqrt(rsq_q);
-    ci.r = rsq_q * ci.rinv;
-    ci.reff = L.reff[q];
-    ci.c0 = L.c0[q];
-    ci.c1 = L.c1[q];
-    ci.en[0] = ci.d[0] * ci.rinv;
-    ci.en[1] = ci.d[1] * ci.rinv;
-    ci.en[2] = ci.d[2] * ci.rinv;
-    ci.deltan_wall = 0.0;
-    const TypePair tp = load_typepair(s.params, s.ntypes, A.type[i], A.type[j]);
-    double sh3[3] = {L.hist[q], L.hist[P + q], L.hist[2 * P + q]};
-    contact_law<NORMAL, false>(ci, tp, s.dt, s.tdamp, s.limitf, ROLL, shearupdate != 0, sh3, o,
-                               (BOND && bonded) ? &bo : nullptr);
-    if (shearupdate) {
-      L.hist[q] = sh3[0];
-      L.hist[P + q] = sh3[1];
-      L.hist[2 * P + q] = sh3[2];
-    }
-    L.flag[q] |= (kContactNormal | kContactTangential);
-  } else {
-    for (int k = 0; k < 3; k++) {
-      o.F[k] = bo.F[k];
-      o.Ti[k] = bo.Ti[k];
-      o.Tj[k] = bo.Tj[k];
-    }
+  __device__ __forceinline__ int operator()() {
+    base += stride;
+    return base < 0x7fffffffL ? (int)base : 0x7fffffff;
   }
-  if (touch || bonded) {
-    store_result(s, q, o);
-    s.active[q] = 1;
-  }
-}
+};
 
-// Phase 1 runs per lane on 32 consecutive entries of a warp at a time; the
-// entries that need phase 2 wait in the warp's shared-memory queue (with
-// their exact test's delta and rsq) until 32 have gathered, so the bond and
-// contact laws run on full warps.  The warps' remainders merge into one
-// block batch at the end.  Each entry's result goes to its own slot and
-// depends on no other entry, so the order changes no value.
 template <int NORMAL, bool ROLL, bool BOND>
 __global__ void __launch_bounds__(kBandTile, 4) k_pair(Sys s, int shearupdate) {
-  __shared__ int q_p[kBandTile / 32][64];
-  __shared__ double q_d[kBandTile / 32][4][64];
-  __shared__ int rest_p[kBandTile];
-  __shared__ double rest_d[4][kBandTile];
-  __shared__ int nrest;
+  __shared__ BandQueue q[kBandTile / 32];
+  __shared__ BandRest<kBandTile> rest;
   Ctrl *c = s.ctrl;
   if (c->halt) return;
-  const AtomArrays &A = s.atoms[0];
-  const PairArrays &L = s.pairs[0];
-  const int np = c->np;
-  const size_t P = s.pcap;
-  const double cdm = s.cdf * s.cdf;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned below = (1u << lane) - 1u;
-  int *qp = q_p[warp];
-  double(*qd)[64] = q_d[warp];
-  // cohesion bond/nonlinear: a bond can be created in this pass
   const long long ntimestep = BOND ? c->ntimestep : 0;
-  const bool may_create = BOND && shearupdate &&
-                          ((s.bond_flags & kBondCreateAlways) || ntimestep == s.bond_ts_create);
-  int qn = 0;  // the same in every lane
-  const long stride = (long)gridDim.x * kBandTile;
-  for (long base = (long)blockIdx.x * kBandTile + warp * 32; base < np; base += stride) {
-    const int p = (int)base + lane;
-    bool queue = false;
-    double delx = 0., dely = 0., delz = 0., rsq = 0.;
-    const int code = p < np ? L.sh[p] : kHole;
-    if (code == kHole && p < np) s.active[p] = 0;  // an unused entry of an ensemble segment
-    if (code != kHole) {
-      const int i = L.i[p], j = L.j[p];
-      double xj = A.x[j], yj = A.y[j], zj = A.z[j];
-      image(s, code, xj, yj, zj);
-      delx = __dadd_rn(A.x[i], -xj);
-      dely = __dadd_rn(A.y[i], -yj);
-      delz = __dadd_rn(A.z[i], -zj);
-      rsq = rsq_rn(delx, dely, delz);
-      const double radsum = __dadd_rn(A.r[i], A.r[j]);
-      queue = rsq < __dmul_rn(radsum, radsum);
-      if (!queue) {
-        s.active[p] = 0;
-        if (rsq < __dmul_rn(__dmul_rn(cdm, radsum), radsum)) {
-          // TangentialModel<TANGENTIAL_HISTORY>::surfacesClose
-          L.flag[p] &= ~kContactTangential;
-          L.hist[p] = 0.0;
-          L.hist[P + p] = 0.0;
-          L.hist[2 * P + p] = 0.0;
-          // CohesionModel::surfacesClose: bonded pairs (and pairs that may
-          // bond in this pass) are evaluated in phase 2
-          if (BOND && (may_create || L.hist[3 * P + p] >= 1.e-15)) {
-            const int tp = A.type[i] * (s.ntypes + 1) + A.type[j];
-            queue = __ldg(s.bondp + tp) >= 1.e-15;
-          }
-        }
-      }
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, queue);
-    if (queue) {
-      const int slot = qn + __popc(m & below);
-      qp[slot] = p;
-      qd[0][slot] = delx;
-      qd[1][slot] = dely;
-      qd[2][slot] = delz;
-      qd[3][slot] = rsq;
-    }
-    qn += __popc(m);
-    __syncwarp();
-    if (qn >= 32) {
-      band_entry<NORMAL, ROLL, BOND>(s, qp[lane], qd[0][lane], qd[1][lane], qd[2][lane], qd[3][lane], shearupdate,
-                                     ntimestep);
-      const int rem = qn - 32;
-      __syncwarp();
-      int vp = 0;
-      double v0 = 0., v1 = 0., v2 = 0., v3 = 0.;
-      if (lane < rem) {
-        vp = qp[32 + lane];
-        v0 = qd[0][32 + lane];
-        v1 = qd[1][32 + lane];
-        v2 = qd[2][32 + lane];
-        v3 = qd[3][32 + lane];
-      }
-      __syncwarp();
-      if (lane < rem) {
-        qp[lane] = vp;
-        qd[0][lane] = v0;
-        qd[1][lane] = v1;
-        qd[2][lane] = v2;
-        qd[3][lane] = v3;
-      }
-      qn = rem;
-      __syncwarp();
-    }
-  }
-  // the warps' remainders (at most 31 each) into one block batch
-  if (threadIdx.x == 0) nrest = 0;
-  __syncthreads();
-  int at = 0;
-  if (lane == 0 && qn) at = atomicAdd(&nrest, qn);
-  at = __shfl_sync(0xffffffffu, at, 0);
-  if (lane < qn) {
-    rest_p[at + lane] = qp[lane];
-    for (int k = 0; k < 4; k++) rest_d[k][at + lane] = qd[k][lane];
-  }
-  __syncthreads();
-  if (threadIdx.x < nrest)
-    band_entry<NORMAL, ROLL, BOND>(s, rest_p[threadIdx.x], rest_d[0][threadIdx.x], rest_d[1][threadIdx.x],
-                                   rest_d[2][threadIdx.x], rest_d[3][threadIdx.x], shearupdate, ntimestep);
-}
-
-// Pair forces without cohesion and with contact distance factor 1 (an entry
-// that is not touching needs no work).  A warp tests 32 consecutive entries
-// at a time in FP32 (x, y, z, r refreshed by every drift): entries apart by
-// more than the bound of the FP32 rounding (pf_margin_touch) only clear
-// their active flag.  The rest are queued in the warp's shared-memory queue;
-// whenever 32 have gathered, the warp runs the exact test and the FP64
-// contact law on all its lanes (the FP64 pipe issues per warp, so idle lanes
-// would waste it).  No block-wide barrier inside the loop: the warps of a
-// block reach their FP64 phases at different times (a block-wide queue
-// of 256 held all eight warps at three barriers per tile; the pair kernel
-// took 0.143 ms on the 1M-atom hopper that way, 0.136 ms this way).
-template <int NORMAL, bool ROLL>
-__device__ __forceinline__ void pair_entry(const Sys &s, int q, int shearupdate) {
-  const AtomArrays &A = s.atoms[0];
-  const PairArrays &L = s.pairs[0];
-  const size_t P = s.pcap;
-  const int i = L.i[q], j = L.j[q];
-  double xj = A.x[j], yj = A.y[j], zj = A.z[j];
-  image(s, L.sh[q], xj, yj, zj);
-  ContactIn ci;
-  ci.d[0] = __dadd_rn(A.x[i], -xj);
-  ci.d[1] = __dadd_rn(A.y[i], -yj);
-  ci.d[2] = __dadd_rn(A.z[i], -zj);
-  const double rsq = rsq_rn(ci.d[0], ci.d[1], ci.d[2]);
-  ci.radi = A.r[i];
-  ci.radj = A.r[j];
-  ci.radsum = __dadd_rn(ci.radi, ci.radj);
-  if (!(rsq < __dmul_rn(ci.radsum, ci.radsum))) {
-    s.active[q] = 0;
-    return;
-  }
-  ci.vr[0] = A.vx[i] - A.vx[j];
-  ci.vr[1] = A.vy[i] - A.vy[j];
-  ci.vr[2] = A.vz[i] - A.vz[j];
-  ci.wi[0] = A.wx[i]; ci.wi[1] = A.wy[i]; ci.wi[2] = A.wz[i];
-  ci.wj[0] = A.wx[j]; ci.wj[1] = A.wy[j]; ci.wj[2] = A.wz[j];
-  // r from 1/r: within an ulp of sqrt(rsq), which moves the overlap
-  // radsum - r by ~1e-13 of itself
-  ci.rinv = rsqrt(rsq);
-  ci.r = rsq * ci.rinv;
-  ci.reff = L.reff[q];
-  ci.c0 = L.c0[q];
-  ci.c1 = L.c1[q];
-  ci.en[0] = ci.d[0] * ci.rinv;
-  ci.en[1] = ci.d[1] * ci.rinv;
-  ci.en[2] = ci.d[2] * ci.rinv;
-  ci.deltan_wall = 0.0;
-  const TypePair tp = load_typepair(s.params, s.ntypes, A.type[i], A.type[j]);
-  double sh3[3] = {L.hist[q], L.hist[P + q], L.hist[2 * P + q]};
-  ContactOut o;
-  contact_law<NORMAL, false>(ci, tp, s.dt, s.tdamp, s.limitf, ROLL, shearupdate != 0, sh3, o);
-  if (shearupdate) {
-    L.hist[q] = sh3[0];
-    L.hist[P + q] = sh3[1];
-    L.hist[2 * P + q] = sh3[2];
-  }
-  L.flag[q] |= (kContactNormal | kContactTangential);
-  store_result(s, q, o);
-  s.active[q] = 1;
+  BandQueue &mine = q[threadIdx.x >> 5];
+  const int qn = band_tiles<NORMAL, ROLL, BOND>(s, c->np, shearupdate, ntimestep, mine, GridTiles(kBandTile));
+  band_rest<NORMAL, ROLL, BOND, kBandTile>(s, qn, shearupdate, ntimestep, mine, rest);
 }
 
 template <int NORMAL, bool ROLL, int MINB>
 __global__ void __launch_bounds__(kPairTile, MINB) k_pair_pf(Sys s, int shearupdate) {
   __shared__ int qbuf[kPairTile / 32][64];
+  __shared__ PfRest rest;
   Ctrl *c = s.ctrl;
   if (c->halt) return;
-  const PairArrays &L = s.pairs[0];
-  const int np = c->np;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned below = (1u << lane) - 1u;
-  int *q = qbuf[warp];
-  const float hi_f = 1.0f + s.pf_margin_touch;
-  const float px = s.prdf[0], py = s.prdf[1], pz = s.prdf[2];
-  int qn = 0;  // the same in every lane
-  const long stride = (long)gridDim.x * kPairTile;
-  for (long base = (long)blockIdx.x * kPairTile + warp * 32; base < np; base += stride) {
-    const int p = (int)base + lane;
-    bool maybe = false;
-    const int code = p < np ? L.sh[p] : kHole;
-    if (code != kHole) {
-      const float4 a = s.xf[L.i[p]], b = s.xf[L.j[p]];
-      float sx = 0.f, sy = 0.f, sz = 0.f;
-      if (code != kNoShift) {
-        sx = fshift(code % 3 - 1, px);
-        sy = fshift((code / 3) % 3 - 1, py);
-        sz = fshift(code / 9 - 1, pz);
-      }
-      const float fx = a.x - (b.x + sx), fy = a.y - (b.y + sy), fz = a.z - (b.z + sz);
-      const float rs = a.w + b.w;
-      maybe = !(fx * fx + fy * fy + fz * fz > rs * rs * hi_f);
-    }
-    if (!maybe && p < np) s.active[p] = 0;
-    const unsigned m = __ballot_sync(0xffffffffu, maybe);
-    if (maybe) q[qn + __popc(m & below)] = p;
-    qn += __popc(m);
-    __syncwarp();
-    if (qn >= 32) {
-      pair_entry<NORMAL, ROLL>(s, q[lane], shearupdate);
-      const int rem = qn - 32;
-      __syncwarp();
-      const int v = lane < rem ? q[32 + lane] : 0;
-      __syncwarp();
-      if (lane < rem) q[lane] = v;
-      qn = rem;
-      __syncwarp();
-    }
-  }
-  // the warps' remainders (at most 31 each) into one block queue, so that a
-  // block ends with one partial batch instead of one per warp
-  __shared__ int rest[kPairTile];
-  __shared__ int nrest;
-  if (threadIdx.x == 0) nrest = 0;
-  __syncthreads();
-  int at = 0;
-  if (lane == 0 && qn) at = atomicAdd(&nrest, qn);
-  at = __shfl_sync(0xffffffffu, at, 0);
-  if (lane < qn) rest[at + lane] = q[lane];
-  __syncthreads();
-  if (threadIdx.x < nrest) pair_entry<NORMAL, ROLL>(s, rest[threadIdx.x], shearupdate);
-}
-
-// ----------------------------------------------------------------------------
-// per-atom kernel: force gather + gravity + primitive walls + nve/sphere
-// ----------------------------------------------------------------------------
-
-// Walls::Granular::compute_force (src/fix_wall_gran_base.h:159-372) for one
-// wall contact: overlap -deltan, delta = closest wall point - centre, wall
-// velocity vwall; h points at the history (stride hs between components)
-template <int NORMAL>
-__device__ __forceinline__ void wall_force(const Sys &s, const AtomArrays &A, int i, double deltan,
-                                           const double delta[3], const double vwall[3],
-                                           int wall_type, bool rolling, double *h, size_t hs,
-                                           int shearupdate, const double v[3], const double om[3],
-                                           double &fx, double &fy, double &fz, double &tx,
-                                           double &ty, double &tz) {
-  const double radi = A.r[i];
-  if (deltan <= 0) {
-    ContactIn ci;
-    ci.radi = radi;
-    ci.radj = 0.0;
-    ci.deltan_wall = -deltan;
-    ci.d[0] = -delta[0];
-    ci.d[1] = -delta[1];
-    ci.d[2] = -delta[2];
-    ci.r = radi - ci.deltan_wall;
-    ci.rinv = 1.0 / ci.r;
-    ci.en[0] = ci.d[0] * ci.rinv;
-    ci.en[1] = ci.d[1] * ci.rinv;
-    ci.en[2] = ci.d[2] * ci.rinv;
-    ci.radsum = radi;
-    ci.reff = radi;
-    ci.vr[0] = v[0] - vwall[0];
-    ci.vr[1] = v[1] - vwall[1];
-    ci.vr[2] = v[2] - vwall[2];
-    ci.wi[0] = om[0]; ci.wi[1] = om[1]; ci.wi[2] = om[2];
-    ci.wj[0] = ci.wj[1] = ci.wj[2] = 0.0;
-    const TypePair tp = load_typepair(s.params, s.ntypes, A.type[i], wall_type);
-    contact_consts<NORMAL>(tp, A.m[i], radi, s.charVel, s.tdamp, ci.c0, ci.c1);
-    double sh3[3] = {h[0], h[hs], h[2 * hs]};
-    ContactOut o;
-    contact_law<NORMAL, true>(ci, tp, s.dt, s.tdamp, s.limitf, rolling, shearupdate != 0, sh3, o);
-    if (shearupdate) {
-      h[0] = sh3[0];
-      h[hs] = sh3[1];
-      h[2 * hs] = sh3[2];
-    }
-    fx += o.F[0]; fy += o.F[1]; fz += o.F[2];
-    tx += o.Ti[0]; ty += o.Ti[1]; tz += o.Ti[2];
-  } else {
-    h[0] = 0.0; h[hs] = 0.0; h[2 * hs] = 0.0;  // surfacesClose
-  }
-}
-
-template <int NORMAL>
-__device__ __forceinline__ void plane_contact(const Sys &s, const AtomArrays &A, int i, int w,
-                                              int shearupdate, double v[3], double om[3],
-                                              double xv[3], double &fx, double &fy, double &fz,
-                                              double &tx, double &ty, double &tz) {
-  const Plane &pl = s.planes[w];
-  const int ax = pl.axis, ay = (ax + 1) % 3, az = (ax + 2) % 3;
-  const double radi = A.r[i];
-  const double ppos = plane_pos(pl, A.type[i]);
-  double delta[3];
-  double deltan;
-  if (pl.kind == 1) {
-    // Cylinder<dim>::resolveContact, src/primitive_wall_definitions.h:170-190,
-    // in the reference's operations and order
-    const double dy = __dadd_rn(xv[ay], -pl.c1), dz = __dadd_rn(xv[az], -pl.c2);
-    const double dist = __dsqrt_rn(__dadd_rn(__dmul_rn(dy, dy), __dmul_rn(dz, dz)));
-    if (dist < 1e-13 && dist > -1e-13) {  // compDouble(dist, 0.0)
-      delta[0] = delta[1] = delta[2] = 0.;
-      deltan = 0.0;
-    } else if (dist > ppos) {
-      deltan = __dadd_rn(__dadd_rn(dist, -ppos), -radi);
-      const double fact = __ddiv_rn(__dadd_rn(dist, -ppos), dist);
-      delta[ax] = 0.;
-      delta[ay] = __dmul_rn(-dy, fact);
-      delta[az] = __dmul_rn(-dz, fact);
-    } else {
-      deltan = __dadd_rn(__dadd_rn(ppos, -dist), -radi);
-      const double fact = __ddiv_rn(__dadd_rn(ppos, -dist), dist);
-      delta[ax] = 0.;
-      delta[ay] = __dmul_rn(dy, fact);
-      delta[az] = __dmul_rn(dz, fact);
-    }
-  } else if (xv[ax] > ppos) {  // Plane<dim>::resolveContact, src/primitive_wall_definitions.h:123-140
-    delta[ax] = ppos - xv[ax];
-    deltan = xv[ax] - ppos - radi;
-  } else {
-    delta[ax] = ppos - xv[ax];
-    deltan = ppos - xv[ax] - radi;
-  }
-  if (pl.kind == 0) {
-    delta[ay] = 0.;
-    delta[az] = 0.;
-  }
-  if (deltan > s.cutneighmax) return;
-  double *h = A.whist + (size_t)(w * 3) * s.nmax + i;
-  const size_t hs = s.nmax;
-  const double cdm1 = s.cdf - 1.0;
-  if (deltan <= 0 || deltan < cdm1 * radi) {
-    const double vwall[3] = {0., 0., 0.};
-    wall_force<NORMAL>(s, A, i, deltan, delta, vwall, pl.wall_type ? pl.wall_type : A.type[i],
-                       pl.rolling != 0, h, hs, shearupdate, v, om, fx, fy, fz, tx, ty, tz);
-  } else {
-    h[0] = 0.0; h[hs] = 0.0; h[2 * hs] = 0.0;
-  }
-}
-
-// barycentric node velocity at the contact point (src/fix_wall_gran.cpp:929-934):
-// the linear mover's node velocities are all vel, the rotating mover's nodev
-__device__ __forceinline__ void mesh_vwall(const MeshDev &M, int t, const double bary[3], double vwall[3]) {
-  if (M.rotating) {
-    const double *vn = M.nodev + (size_t)t * 9;
-    for (int d = 0; d < 3; d++) vwall[d] = (bary[0] * vn[d] + bary[1] * vn[3 + d] + bary[2] * vn[6 + d]);
-  } else {
-    for (int d = 0; d < 3; d++) vwall[d] = (bary[0] * M.vel[d] + bary[1] * M.vel[d] + bary[2] * M.vel[d]);
-  }
-}
-
-// SurfaceMesh::areCoplanarNodeNeighs from the precomputed lists
-__device__ __forceinline__ bool mesh_coplanar(const MeshDev &M, int a, int b) {
-  for (int q = M.cn_start[a]; q < M.cn_start[a + 1]; q++)
-    if (M.cn_list[q] == b) return true;
-  return false;
-}
-
-// triangle id of a slot entry (-1: empty), without the kept mark
-__device__ __forceinline__ int slot_tri_of(int v) { return v < 0 ? -1 : (v & ~kSlotKept); }
-
-// FP32 test of candidate triangle t against an atom at xa within reach_f:
-// false only when the sphere is beyond the triangle.  Two bounds:
-//   plane  |sn.(x - n0)| > reach;
-//   edges  the triangle lies behind each of its edge planes (outward in-plane
-//          normal en_q), and a contact lies within sqrt(reach^2 - dn^2) of
-//          the centre's foot point, so en_q.(x - n_q) beyond that is none.
-// The margins cover the FP32 rounding of the copies and of this arithmetic (a
-// difference of coordinates is within 5*2^-24 of the sum of their magnitudes;
-// 2^-21 is four times that and more), and, for the edges, the 1e-8 by which
-// the reference widens its face region.  A rejected candidate would resolve
-// to deltan > 0, so leaving it out changes nothing.
-__device__ __forceinline__ bool tri_candidate_f(const MeshDev &M, int t, const float4 &xa, float reach_f) {
-  const float4 *T = M.trif + kTrif * (size_t)t;
-  const float4 n0 = T[0], sn = T[1];
-  const float wx = xa.x - n0.x, wy = xa.y - n0.y, wz = xa.z - n0.z;
-  const float dn = fabsf(sn.x * wx + sn.y * wy + sn.z * wz);
-  const float mag = fabsf(xa.x) + fabsf(xa.y) + fabsf(xa.z) + fabsf(n0.x) + fabsf(n0.y) + fabsf(n0.z);
-  const float hi = reach_f + mag * 0x1p-21f;
-  if (dn > hi) return false;
-  const float lo = fmaxf(0.0f, dn - mag * 0x1p-21f);
-  const float rho2 = (hi * hi - lo * lo) * (1.0f + 0x1p-20f) + hi * hi * 0x1p-20f;
-#pragma unroll
-  for (int q = 0; q < 3; q++) {
-    const float4 e = T[2 + q];
-    const float d = e.x * wx + e.y * wy + e.z * wz - e.w;
-    const float m = (mag + fabsf(wx) + fabsf(wy) + fabsf(wz) + fabsf(e.w)) * 0x1p-21f + 4e-8f;
-    const float a = d - m;
-    if (a > 0.0f && a * a > rho2) return false;
-  }
-  return true;
-}
-
-// The closest-feature contacts of atom i with mesh k, one candidate at a
-// time in ascending triangle order (FixWallGran::post_force_mesh with
-// FixContactHistoryMesh::handleContact, coplanarContactAlready,
-// checkCoplanarContactHistory and cleanUpContacts).  A slot touched in this
-// evaluation carries kSlotKept in slot_tri until the clean-up, so the number
-// of candidates has no fixed bound.
-template <int NORMAL>
-__device__ void mesh_contacts(const Sys &s, const AtomArrays &A, int i, int k, int shearupdate,
-                              double v[3], double om[3], double xv[3], double &fx, double &fy,
-                              double &fz, double &tx, double &ty, double &tz, bool &bad, double msum[3]) {
-  const MeshDev &M = s.meshes[k];
-  const int nc = M.cand_n[i];
-  if (nc == 0) return;
-  const size_t nmax = s.nmax;
-  int *st = M.slot_tri[0];
-  double *sh = M.slot_hist[0];
-  int np = M.npart[0][i];
-  const double radi = A.r[i];
-  const double cdm1 = s.cdf - 1.0;
-  // a triangle is at least as far as its plane: candidates whose plane is
-  // clearly beyond the contact range (relative margin 1e-9, far above the
-  // rounding of either side) skip the closest-feature resolution; the
-  // resolution would return deltan > 0 and skip them as well
-  const double reach = __dmul_rn(__dadd_rn(radi, fmax(0.0, __dmul_rn(cdm1, radi))), 1.0 + 1e-9);
-  // FP32 bounds first (tri_candidate_f); the rest take the FP64 path below
-  const float4 xa = s.xf[i];
-  const float reach_f = (float)reach * (1.0f + 0x1p-20f);
-  for (int q = 0; q < nc; q++) {
-    const int t = M.cand[(size_t)q * nmax + i];
-    if (!tri_candidate_f(M, t, xa, reach_f)) continue;
-    const double *g = M.tri + (size_t)t * kTriStride;
-    {
-      const double *sn = tri_sn(g), *n0 = tri_node(g, 0);
-      const double dn = sn[0] * (xv[0] - n0[0]) + sn[1] * (xv[1] - n0[1]) + sn[2] * (xv[2] - n0[2]);
-      if (fabs(dn) > reach) continue;
-    }
-    double delta[3], bary[3];
-    int bs;
-    const double deltan = resolve_tri_sphere(g, M.meta[t], radi, xv, delta, bary, bs);
-    if (deltan > s.cutneighmax) continue;
-    if (!(deltan <= 0 || deltan < cdm1 * radi)) continue;
-    int slot = -1;
-    for (int u = 0; u < nc; u++)
-      if (slot_tri_of(st[u * nmax + i]) == t) { slot = u; break; }
-    if (slot >= 0) {
-      st[slot * nmax + i] |= kSlotKept;
-    } else {
-      const bool face = bs == 7;
-      if (face) {  // coplanarContactAlready
-        bool already = false;
-        for (int u = 0; u < nc; u++) {
-          const int sv = st[u * nmax + i];
-          const int p = slot_tri_of(sv);
-          if (p >= 0 && p != t && (sv & kSlotKept) && mesh_coplanar(M, p, t)) already = true;
-        }
-        if (already) continue;
-      }
-      if (np >= nc) { bad = true; continue; }
-      for (int u = 0; u < nc; u++)
-        if (st[u * nmax + i] == -1) { slot = u; break; }
-      st[slot * nmax + i] = t | kSlotKept;
-      for (int d = 0; d < 3; d++) sh[(3 * slot + d) * nmax + i] = 0.0;
-      np++;
-      if (face)  // checkCoplanarContactHistory
-        for (int u = 0; u < nc; u++) {
-          const int p = slot_tri_of(st[u * nmax + i]);
-          if (p >= 0 && p != t && mesh_coplanar(M, p, t))
-            for (int d = 0; d < 3; d++) sh[(3 * slot + d) * nmax + i] = sh[(3 * u + d) * nmax + i];
-        }
-    }
-    double vwall[3] = {0., 0., 0.};
-    if (M.moving && M.vel_on) mesh_vwall(M, t, bary, vwall);
-    double cfx = 0., cfy = 0., cfz = 0., ctx = 0., cty = 0., ctz = 0.;
-    wall_force<NORMAL>(s, A, i, deltan, delta, vwall, M.wall_type, M.rolling != 0,
-                         sh + (size_t)(3 * slot) * nmax + i, nmax, shearupdate, v, om, cfx, cfy, cfz, ctx, cty, ctz);
-    fx += cfx; fy += cfy; fz += cfz;
-    tx += ctx; ty += cty; tz += ctz;
-    msum[0] += cfx; msum[1] += cfy; msum[2] += cfz;
-  }
-  for (int u = 0; u < nc; u++) {  // cleanUpContacts
-    const int sv = st[u * nmax + i];
-    if (sv >= 0 && (sv & kSlotKept)) {
-      st[u * nmax + i] = sv & ~kSlotKept;
-    } else {
-      if (sv > -1) np--;
-      st[u * nmax + i] = -1;
-      for (int d = 0; d < 3; d++) sh[(3 * u + d) * nmax + i] = 0.0;
-    }
-  }
-  M.npart[0][i] = np;
-}
-
-// FixWallGran::post_force_primitive / post_force_mesh for the atoms near a
-// wall (the compact list of k_wall_list): wall forces and torques of the
-// current state, planes then meshes in order, into fm/tm.  Independent of
-// the pair kernel of the same step (it reads positions and velocities and
-// writes only the wall histories, mesh slots and fm/tm), so the two run side
-// by side; the per-atom kernel adds fm/tm.
-//
-// A warp takes a tile of 32 listed atoms (one lane each) and, per mesh, runs
-// the FP64-heavy parts densely over the tile's work instead of per atom (the
-// FP64 pipe issues per warp instruction, and atoms differ in their number of
-// candidates and contacts):
-//   A  per atom, FP32: the candidates the triangle bounds cannot reject
-//      (tri_candidate_f), queued in ascending order;
-//   B  per queued candidate: exact plane test and closest feature
-//      (TriMesh::resolveTriSphereContactBary), kept when touching;
-//   C  per atom, integer work in candidate order: FixContactHistoryMesh's
-//      slot semantics (handleContact, coplanarContactAlready); an atom whose
-//      new face contact would copy a coplanar neighbour's history
-//      (checkCoplanarContactHistory) takes the sequential path instead,
-//      since that copy depends on the order of the contact updates;
-//   D  per contact: the contact law with the slot's history;
-//   E  per atom: contact forces summed in candidate order, slot clean-up.
-// Atoms without a touching candidate and without an occupied slot do nothing
-// after B (their slots are empty, with zero history).  A tile whose queue
-// would exceed its capacity (cap entries, a launch parameter) runs the
-// sequential path for all its atoms.  Both paths give the same result.
-//
-// The launch is bound by latency: the phases are one dependent chain, a few
-// warps per SM.  A warp per tile keeps the phases free of block barriers, and
-// the edge bounds leave B about one candidate per contact (with the plane
-// bound alone the conical mesh's tiles queued several per atom, three to five
-// FP64 passes of B).  Against 64-atom tiles with block barriers and the plane
-// bound: the 100,000-sphere hopper's step 84 -> 67 us, the 1M one's 0.318 ->
-// 0.309 ms (50 steps per call).
-constexpr int kWallTile = 32;
-constexpr int kWallWarps = 2;       // tiles (warps) per block
-constexpr int kWallCapDefault = 4;  // queue entries per tile atom (LIGGGHTS_GB300_WALL_CAP)
-constexpr int kWallRes = 7;  // doubles per queued candidate: deltan, delta[3], vwall[3]; then F[3], T[3]
-constexpr int kWallQ = kWallRes * 8 + 4 + 2;  // result doubles, state int, atom and candidate bytes
-
-// one warp's queue of `cap` entries in shared memory
-struct WallQueue {
-  double *res;             // [cap * kWallRes]
-  int *st;                 // bit 0 touching, bit 1 face, bits 8+: contact slot + 1
-  unsigned char *qa, *qq;  // tile atom, candidate index
-};
-
-template <int NORMAL>
-__device__ __forceinline__ void wall_tile(const Sys &s, const AtomArrays &A, int base, int nl, int shearupdate,
-                                          int cap, const WallQueue &w, bool &meshbad) {
-  const size_t nmax = s.nmax;
-  const double cdm1 = s.cdf - 1.0;
-  const int a = threadIdx.x & 31;
-  const bool valid = base + a < nl;
-  const int i = valid ? s.mlist[base + a] : 0;
-  double v[3] = {0., 0., 0.}, om[3] = {0., 0., 0.}, xv[3] = {0., 0., 0.};
-  double fx = 0., fy = 0., fz = 0., tx = 0., ty = 0., tz = 0.;
-  if (valid) {
-    v[0] = A.vx[i]; v[1] = A.vy[i]; v[2] = A.vz[i];
-    om[0] = A.wx[i]; om[1] = A.wy[i]; om[2] = A.wz[i];
-    xv[0] = A.x[i]; xv[1] = A.y[i]; xv[2] = A.z[i];
-    const uint8_t bits = A.wbits[i];
-    for (int k = 0; k < s.nplanes; k++) {
-      double pfx = 0., pfy = 0., pfz = 0., ptx = 0., pty = 0., ptz = 0.;
-      if (bits & (1u << k)) plane_contact<NORMAL>(s, A, i, k, shearupdate, v, om, xv, pfx, pfy, pfz, ptx, pty, ptz);
-      fx += pfx; fy += pfy; fz += pfz;
-      tx += ptx; ty += pty; tz += ptz;
-      s.wforce[(size_t)(3 * k) * nmax + i] = pfx;
-      s.wforce[(size_t)(3 * k + 1) * nmax + i] = pfy;
-      s.wforce[(size_t)(3 * k + 2) * nmax + i] = pfz;
-    }
-  }
-  for (int k = 0; k < s.nmeshes; k++) {
-    const MeshDev &M = s.meshes[k];
-    int *st = M.slot_tri[0];
-    double *sh = M.slot_hist[0];
-    // ---- A: FP32 candidate pass
-    const int nc = valid ? M.cand_n[i] : 0;
-    unsigned todo = 0u;
-    int np = 0;
-    const bool big = nc > kMeshFastCand;  // beyond the 32-bit masks: sequential path
-    if (nc > 0 && !big) {
-      np = M.npart[0][i];
-      const double radi = A.r[i];
-      const double reach = __dmul_rn(__dadd_rn(radi, fmax(0.0, __dmul_rn(cdm1, radi))), 1.0 + 1e-9);
-      const float4 xa = s.xf[i];
-      const float reach_f = (float)reach * (1.0f + 0x1p-20f);
-      int t = M.cand[i];
-      for (int q = 0; q < nc; q++) {
-        const int tn = q + 1 < nc ? M.cand[(size_t)(q + 1) * nmax + i] : 0;  // ahead of the triangle it names
-        if (tri_candidate_f(M, t, xa, reach_f)) todo |= 1u << q;
-        t = tn;
-      }
-    }
-    const int cnt = __popc(todo);
-    const int inc = warp_incl_scan(cnt);
-    const int total = __shfl_sync(0xffffffffu, inc, 31);
-    const int off = inc - cnt;
-    double msum[3] = {0., 0., 0.};
-    double *const wf = s.wforce + (size_t)(3 * (s.nplanes + k)) * nmax;
-    if (total > cap) {  // sequential path for this tile
-      if (nc > 0) mesh_contacts<NORMAL>(s, A, i, k, shearupdate, v, om, xv, fx, fy, fz, tx, ty, tz, meshbad, msum);
-      if (valid)
-        for (int d = 0; d < 3; d++) wf[(size_t)d * nmax + i] = msum[d];
-      __syncwarp();
-      continue;
-    }
-    {
-      unsigned m = todo;
-      for (int e = off; m; e++) {
-        w.qa[e] = (unsigned char)a;
-        w.qq[e] = (unsigned char)(__ffs(m) - 1);
-        m &= m - 1u;
-      }
-    }
-    __syncwarp();
-    // ---- B: exact plane test and closest feature per queued candidate
-    for (int e = a; e < total; e += kWallTile) {
-      const int ie = s.mlist[base + w.qa[e]];
-      const int t = M.cand[(size_t)w.qq[e] * nmax + ie];
-      const double *g = M.tri + (size_t)t * kTriStride;
-      const double xe[3] = {A.x[ie], A.y[ie], A.z[ie]};
-      const double re = A.r[ie];
-      const double reach_e = __dmul_rn(__dadd_rn(re, fmax(0.0, __dmul_rn(cdm1, re))), 1.0 + 1e-9);
-      int state = 0;
-      const double *snv = tri_sn(g), *n0 = tri_node(g, 0);
-      const double dn = snv[0] * (xe[0] - n0[0]) + snv[1] * (xe[1] - n0[1]) + snv[2] * (xe[2] - n0[2]);
-      if (!(fabs(dn) > reach_e)) {
-        double delta[3], bary[3];
-        int bs;
-        const double deltan = resolve_tri_sphere(g, M.meta[t], re, xe, delta, bary, bs);
-        if (!(deltan > s.cutneighmax) && (deltan <= 0 || deltan < cdm1 * re)) {
-          state = 1 | (bs == 7 ? 2 : 0);
-          double *r = w.res + (size_t)e * kWallRes;
-          r[0] = deltan;
-          r[1] = delta[0]; r[2] = delta[1]; r[3] = delta[2];
-          double vwall[3] = {0., 0., 0.};
-          if (M.moving && M.vel_on) mesh_vwall(M, t, bary, vwall);
-          r[4] = vwall[0]; r[5] = vwall[1]; r[6] = vwall[2];
-        }
-      }
-      w.st[e] = state;
-    }
-    __syncwarp();
-    // ---- C: slot semantics per atom, in candidate order
-    bool fallback = big;
-    unsigned keep = 0u;
-    int stl[kMeshFastCand];
-    bool work = np > 0 && !big;
-    for (int e = off; e < off + cnt; e++) work |= (w.st[e] & 1) != 0;
-    if (work) {
-      for (int u = 0; u < nc; u++) stl[u] = st[u * nmax + i];
-      unsigned fresh = 0u;
-      for (int e = off; e < off + cnt && !fallback; e++) {
-        if (!(w.st[e] & 1)) continue;
-        const int t = M.cand[(size_t)w.qq[e] * nmax + i];
-        int slot = -1;
-        for (int u = 0; u < nc; u++)
-          if (stl[u] == t) { slot = u; break; }
-        if (slot >= 0) {
-          keep |= 1u << slot;
-        } else {
-          const bool face = (w.st[e] & 2) != 0;
-          if (face) {  // coplanarContactAlready
-            bool already = false;
-            for (int u = 0; u < nc; u++)
-              if (stl[u] >= 0 && stl[u] != t && ((keep >> u) & 1u) && mesh_coplanar(M, stl[u], t)) already = true;
-            if (already) continue;
-          }
-          if (np >= nc) { meshbad = true; continue; }
-          for (int u = 0; u < nc; u++)
-            if (stl[u] == -1) { slot = u; break; }
-          if (face)  // checkCoplanarContactHistory would copy: order-dependent
-            for (int u = 0; u < nc; u++)
-              if (stl[u] >= 0 && stl[u] != t && mesh_coplanar(M, stl[u], t)) fallback = true;
-          if (fallback) break;
-          stl[slot] = t;
-          keep |= 1u << slot;
-          fresh |= 1u << slot;
-          np++;
-        }
-        w.st[e] |= (slot + 1) << 8;
-      }
-      if (fallback) {
-        for (int e = off; e < off + cnt; e++) w.st[e] &= 0xff;
-      } else {
-        for (int u = 0; u < nc; u++)
-          if ((fresh >> u) & 1u) {
-            st[u * nmax + i] = stl[u];
-            for (int d = 0; d < 3; d++) sh[(3 * u + d) * nmax + i] = 0.0;
-          }
-      }
-    }
-    __syncwarp();
-    // ---- D: contact law per contact
-    for (int e = a; e < total; e += kWallTile) {
-      const int slot = (w.st[e] >> 8) - 1;
-      if (slot < 0) continue;
-      const int ie = s.mlist[base + w.qa[e]];
-      double *r = w.res + (size_t)e * kWallRes;
-      const double delta[3] = {r[1], r[2], r[3]};
-      const double vwall[3] = {r[4], r[5], r[6]};
-      double ve[3] = {A.vx[ie], A.vy[ie], A.vz[ie]};
-      double oe[3] = {A.wx[ie], A.wy[ie], A.wz[ie]};
-      double cfx = 0., cfy = 0., cfz = 0., ctx = 0., cty = 0., ctz = 0.;
-      wall_force<NORMAL>(s, A, ie, r[0], delta, vwall, M.wall_type, M.rolling != 0,
-                         sh + (size_t)(3 * slot) * nmax + ie, nmax, shearupdate, ve, oe, cfx, cfy, cfz, ctx, cty,
-                         ctz);
-      r[0] = cfx; r[1] = cfy; r[2] = cfz;
-      r[3] = ctx; r[4] = cty; r[5] = ctz;
-    }
-    __syncwarp();
-    // ---- E: sums in candidate order, clean-up (or the sequential path)
-    if (fallback) {
-      mesh_contacts<NORMAL>(s, A, i, k, shearupdate, v, om, xv, fx, fy, fz, tx, ty, tz, meshbad, msum);
-    } else if (work) {
-      for (int e = off; e < off + cnt; e++) {
-        if ((w.st[e] >> 8) == 0) continue;
-        const double *r = w.res + (size_t)e * kWallRes;
-        fx += r[0]; fy += r[1]; fz += r[2];
-        tx += r[3]; ty += r[4]; tz += r[5];
-        msum[0] += r[0]; msum[1] += r[1]; msum[2] += r[2];
-      }
-      for (int u = 0; u < nc; u++)  // cleanUpContacts
-        if (!((keep >> u) & 1u) && stl[u] > -1) {
-          np--;
-          st[u * nmax + i] = -1;
-          for (int d = 0; d < 3; d++) sh[(3 * u + d) * nmax + i] = 0.0;
-        }
-      M.npart[0][i] = np;
-    }
-    if (valid)
-      for (int d = 0; d < 3; d++) wf[(size_t)d * nmax + i] = msum[d];
-    __syncwarp();
-  }
-  if (valid) {
-    A.fmx[i] = fx; A.fmy[i] = fy; A.fmz[i] = fz;
-    A.tmx[i] = tx; A.tmy[i] = ty; A.tmz[i] = tz;
-  }
+  int *q = qbuf[threadIdx.x >> 5];
+  const int qn = pf_tiles<NORMAL, ROLL>(s, c->np, shearupdate, q, GridTiles(kPairTile));
+  pf_rest<NORMAL, ROLL>(s, qn, shearupdate, q, rest);
 }
 
 template <int NORMAL>
@@ -2389,93 +1409,6 @@ __global__ void __launch_bounds__(kWallTile *kWallWarps) k_wall_force(Sys s, int
   if (__any_sync(0xffffffffu, meshbad) && (threadIdx.x & 31) == 0) atomicExch(&c->status, kStatMeshSlots);
 }
 
-// Force gather of one atom: its own row (ascending), then its reverse list
-// (ascending), the reference's per-atom order.  The FP64 pipe issues per warp
-// instruction, so additions inside a loop over all list entries cost one
-// issue per entry of the warp's longest row, active or not.  Here a first,
-// integer-only pass collects the active entries of up to 32 entries per list
-// as bit masks (gather_masks); one loop over the set bits then does the FP64
-// additions (gather_sum).  A reverse contribution adds the negated force
-// (sign bit flipped on the integer pipe: a + (-b) is exactly a - b) and Tj
-// instead of Ti.  k_particle hands the loops of a block's atoms to its
-// threads sorted by contact count, so that a warp's lanes run loops of equal
-// length (see there).
-__device__ __forceinline__ bool gather_masks(const Sys &s, const PairArrays &L, int i, int &pb, int &rb,
-                                             unsigned &om, unsigned &rm) {
-  pb = L.row[i];
-  rb = L.rev_start[i];
-  const int pe = row_end(s, L, i), re = rev_end(s, L, i);
-  if (pe - pb > 32 || re - rb > 32) return false;
-  om = 0u;
-  rm = 0u;
-  for (int k = 0; k < pe - pb; k++) om |= (s.active[pb + k] ? 1u : 0u) << k;
-  for (int k = 0; k < re - rb; k++) rm |= (s.active[L.rev[rb + k]] ? 1u : 0u) << k;
-  return true;
-}
-
-__device__ __forceinline__ void gather_sum(const Sys &s, const PairArrays &L, int pb, int rb, unsigned om,
-                                           unsigned rm, double &fx, double &fy, double &fz, double &tx, double &ty,
-                                           double &tz) {
-  const int cnt = __popc(om) + __popc(rm);
-  for (int t = 0; t < cnt; t++) {
-    int p;
-    unsigned long long sg;
-    int to;  // offset of the torque in the record: Ti (own row) or Tj (partner)
-    if (om) {
-      p = pb + __ffs(om) - 1;
-      om &= om - 1u;
-      sg = 0ull;
-      to = 3;
-    } else {
-      p = L.rev[rb + __ffs(rm) - 1];
-      rm &= rm - 1u;
-      sg = 0x8000000000000000ull;
-      to = 6;
-    }
-    const double *r = s.res + (size_t)kResStride * p;
-    fx += __longlong_as_double(__double_as_longlong(r[0]) ^ sg);
-    fy += __longlong_as_double(__double_as_longlong(r[1]) ^ sg);
-    fz += __longlong_as_double(__double_as_longlong(r[2]) ^ sg);
-    tx += r[to];
-    ty += r[to + 1];
-    tz += r[to + 2];
-  }
-}
-
-// lists longer than 32 entries: one pass over every entry
-__device__ __forceinline__ void gather_long(const Sys &s, const PairArrays &L, int i, double &fx, double &fy,
-                                            double &fz, double &tx, double &ty, double &tz) {
-  const int pb = L.row[i], pe = row_end(s, L, i);
-  const int rb = L.rev_start[i], re = rev_end(s, L, i);
-  for (int p = pb; p < pe; p++) {
-    if (!s.active[p]) continue;
-    const double *r = s.res + (size_t)kResStride * p;
-    fx += r[0]; fy += r[1]; fz += r[2];
-    tx += r[3]; ty += r[4]; tz += r[5];
-  }
-  for (int k = rb; k < re; k++) {
-    const int p = L.rev[k];
-    if (!s.active[p]) continue;
-    const double *r = s.res + (size_t)kResStride * p;
-    fx -= r[0]; fy -= r[1]; fz -= r[2];
-    tx += r[6]; ty += r[7]; tz += r[8];
-  }
-}
-
-// the block-level sort of k_particle's gather: loops of up to kGatherKeys-1
-// contacts by count, longer ones together in the last key
-constexpr int kGatherKeys = 32;
-constexpr int kParticleMaxThreads = 256;
-
-// Per atom: force gather, gravity, wall totals, nve/sphere, FP32 copy,
-// displacement check.  The gather runs in three block-wide phases, because a
-// warp's contact loops issue their FP64 additions once per contact of its
-// busiest atom: (1) every thread forms its atom's start sums (gravity) and
-// contact masks; (2) the atoms with contacts are sorted by their contact
-// count in shared memory; (3) thread t runs the loop of the t-th atom in that
-// order, so that a warp's lanes run loops of equal length, and the sums go
-// back to the owner.  Each atom's sum keeps its order and its one thread, so
-// the result does not depend on the sort or the launch shape.
 // Graph steps without moving meshes: the last block of k_particle to finish
 // takes the step's rebuild decision and sets the loop's conditionals, as
 // k_decide_loop does after it otherwise (one node and one dependency fewer
@@ -2485,181 +1418,9 @@ struct LoopCond {
   cudaGraphConditionalHandle hreb, hloop;
 };
 
-template <int NORMAL, bool GATHER, bool FINAL, bool INITIAL>
-__global__ void __launch_bounds__(kParticleMaxThreads, 4) k_particle(Sys s, int shearupdate, LoopCond lp) {
-  __shared__ double gsum[GATHER ? 6 : 1][GATHER ? kParticleMaxThreads : 1];
-  __shared__ int gpb[GATHER ? kParticleMaxThreads : 1], grb[GATHER ? kParticleMaxThreads : 1];
-  __shared__ unsigned gom[GATHER ? kParticleMaxThreads : 1], grm[GATHER ? kParticleMaxThreads : 1];
-  __shared__ short gsorted[GATHER ? kParticleMaxThreads : 1];
-  __shared__ int gcount[kGatherKeys], gfill[kGatherKeys], gstart[kGatherKeys], gnq;
+// the flags of a block's atoms, and (lp.on) the decision by the last block
+__device__ __forceinline__ void particle_end(const Sys &s, Ctrl *c, bool moved, bool bad, const LoopCond &lp) {
   __shared__ int last_block;
-  Ctrl *c = s.ctrl;
-  if (c->halt) {
-    if (lp.on && blockIdx.x == 0 && threadIdx.x == 0) {
-      cudaGraphSetConditional(lp.hreb, 0);
-      cudaGraphSetConditional(lp.hloop, 0);
-    }
-    return;
-  }
-  const AtomArrays &A = s.atoms[0];
-  const PairArrays &L = s.pairs[0];
-  const int n = c->n;
-  const double dtv = s.dt;
-  const double trigger = 0.25 * s.skin * s.skin;
-  const int tid = threadIdx.x;
-  bool moved = false, bad = false;
-  if (GATHER) {
-    if (tid < kGatherKeys) {
-      gcount[tid] = 0;
-      gfill[tid] = 0;
-    }
-    __syncthreads();
-  }
-  for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-    const int i = base + tid;
-    const bool valid = i < n;
-    double fx = 0.0, fy = 0.0, fz = 0.0, tx = 0.0, ty = 0.0, tz = 0.0;
-    double v[3] = {0.0, 0.0, 0.0}, om[3] = {0.0, 0.0, 0.0}, xv[3] = {0.0, 0.0, 0.0};
-    if (valid) {
-      v[0] = A.vx[i]; v[1] = A.vy[i]; v[2] = A.vz[i];
-      om[0] = A.wx[i]; om[1] = A.wy[i]; om[2] = A.wz[i];
-      xv[0] = A.x[i]; xv[1] = A.y[i]; xv[2] = A.z[i];
-    }
-    if (GATHER) {
-      // FixGravity::post_force (src/fix_gravity.cpp:329-337) adds m*g after
-      // the pair forces; starting the sum from it instead changes only the
-      // rounding order and saves three FP64 additions
-      if (valid && s.gravity_on) {
-        const double massone = A.m[i];
-        fx = __dmul_rn(massone, s.g[0]);
-        fy = __dmul_rn(massone, s.g[1]);
-        fz = __dmul_rn(massone, s.g[2]);
-      }
-      // (1) masks and counts; lists longer than 32 entries are summed here
-      // by the owner (gcount and gfill are zero: cleared after the last use)
-      int key = 0;
-      if (valid) {
-        int pb, rb;
-        unsigned mo, mr;
-        if (gather_masks(s, L, i, pb, rb, mo, mr)) {
-          const int cnt = __popc(mo) + __popc(mr);
-          if (cnt) {
-            key = cnt < kGatherKeys ? cnt : kGatherKeys - 1;
-            gpb[tid] = pb;
-            grb[tid] = rb;
-            gom[tid] = mo;
-            grm[tid] = mr;
-            gsum[0][tid] = fx; gsum[1][tid] = fy; gsum[2][tid] = fz;
-            gsum[3][tid] = tx; gsum[4][tid] = ty; gsum[5][tid] = tz;
-          }
-        } else {
-          gather_long(s, L, i, fx, fy, fz, tx, ty, tz);
-        }
-      }
-      // (2) counting sort of the block's atoms with contacts by their count
-      if (key) atomicAdd(&gcount[key], 1);
-      __syncthreads();
-      if (tid < 32) {
-        const int v0 = tid < kGatherKeys ? gcount[tid] : 0;
-        const int inc = warp_incl_scan(v0);
-        if (tid < kGatherKeys) gstart[tid] = inc - v0;
-        if (tid == 31) gnq = inc;
-      }
-      __syncthreads();
-      if (key) gsorted[gstart[key] + atomicAdd(&gfill[key], 1)] = (short)tid;
-      __syncthreads();
-      if (tid < kGatherKeys) {  // read by no one until the next block of atoms counts
-        gcount[tid] = 0;
-        gfill[tid] = 0;
-      }
-      // (3) the loops, one atom per thread in sorted order
-      if (tid < gnq) {
-        const int a = gsorted[tid];
-        double sx = gsum[0][a], sy = gsum[1][a], sz = gsum[2][a];
-        double qx = gsum[3][a], qy = gsum[4][a], qz = gsum[5][a];
-        gather_sum(s, L, gpb[a], grb[a], gom[a], grm[a], sx, sy, sz, qx, qy, qz);
-        gsum[0][a] = sx; gsum[1][a] = sy; gsum[2][a] = sz;
-        gsum[3][a] = qx; gsum[4][a] = qy; gsum[5][a] = qz;
-      }
-      __syncthreads();
-      if (key) {
-        fx = gsum[0][tid]; fy = gsum[1][tid]; fz = gsum[2][tid];
-        tx = gsum[3][tid]; ty = gsum[4][tid]; tz = gsum[5][tid];
-      }
-    }
-    if (!valid) continue;
-    if (GATHER) {
-      if (A.wbits[i] & 0x80u) {  // walls, computed by k_wall_force for this step
-        fx += A.fmx[i]; fy += A.fmy[i]; fz += A.fmz[i];
-        tx += A.tmx[i]; ty += A.tmy[i]; tz += A.tmz[i];
-      }
-      // the sums are kept for the download and the next call's first
-      // step; inside a run (FINAL && INITIAL) nothing reads them
-      if (!(FINAL && INITIAL)) {
-        A.fx[i] = fx; A.fy[i] = fy; A.fz[i] = fz;
-        A.tx[i] = tx; A.ty[i] = ty; A.tz[i] = tz;
-      }
-    } else {
-      fx = A.fx[i]; fy = A.fy[i]; fz = A.fz[i];
-      tx = A.tx[i]; ty = A.ty[i]; tz = A.tz[i];
-    }
-    if (FINAL || INITIAL) {
-      // FixNVESphere half-kicks and drift as fused multiply-adds: one FP64
-      // instruction each (the FP64 pipe bounds this kernel on GB300); the
-      // single rounding moves positions by at most an ulp from the reference.
-      // The final half-kick of step n and the initial one of step n+1 use
-      // the same force: fused into one FMA with 2*dtfm (2*dtir), exact
-      // scalings, one rounding instead of two.
-      const double dtfm = A.dtfm[i], dtir = A.dtir[i];
-      if (FINAL && INITIAL) {
-        v[0] = fma(2.0 * dtfm, fx, v[0]);
-        v[1] = fma(2.0 * dtfm, fy, v[1]);
-        v[2] = fma(2.0 * dtfm, fz, v[2]);
-        om[0] = fma(2.0 * dtir, tx, om[0]);
-        om[1] = fma(2.0 * dtir, ty, om[1]);
-        om[2] = fma(2.0 * dtir, tz, om[2]);
-      } else if (FINAL || INITIAL) {
-        v[0] = fma(dtfm, fx, v[0]);
-        v[1] = fma(dtfm, fy, v[1]);
-        v[2] = fma(dtfm, fz, v[2]);
-        om[0] = fma(dtir, tx, om[0]);
-        om[1] = fma(dtir, ty, om[1]);
-        om[2] = fma(dtir, tz, om[2]);
-      }
-      if (INITIAL) {
-        xv[0] = fma(dtv, v[0], xv[0]);
-        xv[1] = fma(dtv, v[1], xv[1]);
-        xv[2] = fma(dtv, v[2], xv[2]);
-        A.x[i] = xv[0]; A.y[i] = xv[1]; A.z[i] = xv[2];
-        // the FP32 radius of the copy does not change: no conversion
-        const float4 nf = make_float4((float)xv[0], (float)xv[1], (float)xv[2], s.xf[i].w);
-        s.xf[i] = nf;
-        // Neighbor::check_distance (src/neighbor.cpp:1426-1466) with an FP32
-        // prefilter: only displacements within the rounding band of skin/2
-        // take the exact FP64 test, so the decision is the reference's
-        const float4 hf = s.xhf[i];
-        const float ex = nf.x - hf.x, ey = nf.y - hf.y, ez = nf.z - hf.z;
-        const float rf2 = ex * ex + ey * ey + ez * ez;
-        bool mv = false;
-        if (rf2 > s.skin_hi2) {
-          mv = true;
-        } else if (rf2 > s.skin_lo2) {
-          const double dx = __dadd_rn(xv[0], -A.xh[i]);
-          const double dy = __dadd_rn(xv[1], -A.yh[i]);
-          const double dz = __dadd_rn(xv[2], -A.zh[i]);
-          if (rsq_rn(dx, dy, dz) > trigger) mv = true;
-        }
-        if (mv && s.nsys) s.sys_moved[A.type[i] - 1] = 1;  // this atom's system (ensembles)
-        moved |= mv;
-        // a non-finite coordinate converts to a non-finite float (so does one
-        // beyond the FP32 range, which no granular box reaches)
-        if (!(isfinite(nf.x) && isfinite(nf.y) && isfinite(nf.z))) bad = true;
-      }
-      A.vx[i] = v[0]; A.vy[i] = v[1]; A.vz[i] = v[2];
-      A.wx[i] = om[0]; A.wy[i] = om[1]; A.wz[i] = om[2];
-    }
-  }
-  (void)shearupdate;
   if (__any_sync(0xffffffffu, moved) && (threadIdx.x & 31) == 0) atomicOr(&c->moved, 1);
   if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) {
     atomicExch(&c->status, kStatNan);
@@ -2685,6 +1446,48 @@ __global__ void __launch_bounds__(kParticleMaxThreads, 4) k_particle(Sys s, int 
       }
     }
   }
+}
+
+__device__ __forceinline__ bool particle_halted(const Ctrl *c, const LoopCond &lp) {
+  if (!c->halt) return false;
+  if (lp.on && blockIdx.x == 0 && threadIdx.x == 0) {
+    cudaGraphSetConditional(lp.hreb, 0);
+    cudaGraphSetConditional(lp.hloop, 0);
+  }
+  return true;
+}
+
+template <bool GATHER, bool FINAL, bool INITIAL>
+__global__ void __launch_bounds__(kParticleMaxThreads, 4) k_particle(Sys s, LoopCond lp) {
+  __shared__ ParticleShared<kParticleMaxThreads> sm;
+  Ctrl *c = s.ctrl;
+  if (particle_halted(c, lp)) return;
+  const int n = c->n;
+  bool moved = false, bad = false;
+  if (GATHER) particle_clear(sm);
+  for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+    const int i = base + threadIdx.x;
+    particle_tile(s, sm, i, i < n, GATHER, FINAL, INITIAL, moved, bad);
+  }
+  particle_end(s, c, moved, bad, lp);
+}
+
+// The first step of a graph launch: from stored forces (a call's first step),
+// or gathering the previous step's (continuing a call after a capacity grew
+// or atoms were inserted), as Ctrl::step_phase says.
+__global__ void __launch_bounds__(kParticleMaxThreads, 4) k_particle_start(Sys s, LoopCond lp) {
+  __shared__ ParticleShared<kParticleMaxThreads> sm;
+  Ctrl *c = s.ctrl;
+  if (particle_halted(c, lp)) return;
+  const int n = c->n;
+  const bool gather = c->step_phase != kStepFirst;
+  bool moved = false, bad = false;
+  particle_clear(sm);
+  for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+    const int i = base + threadIdx.x;
+    particle_tile(s, sm, i, i < n, gather, gather, true, moved, bad);
+  }
+  particle_end(s, c, moved, bad, lp);
 }
 
 // ----------------------------------------------------------------------------
@@ -3081,22 +1884,33 @@ int launch_rebuild(const Sys &s, const LaunchCfg &lc, cudaStream_t st, int stage
   return nl + 4;
 }
 
-// Builds the executable graph of `steps 2..n` of dem_step:
-//   WHILE(loop) { k_particle(gather+final+initial) -> k_decide_loop ->
-//                 IF(rebuild) { rebuild kernels } -> k_pair }
-// (without moving meshes, the last block of k_particle decides instead of
-// k_decide_loop)
-// The host sets ctrl->loop_left with launch_set_loop() before each launch.
-static int launch_particle_lp(const Sys &s, const LaunchCfg &lc, int mode, int shearupdate, const LoopCond &lp,
-                              cudaStream_t st);
+// Builds the executable graph of one dem_step call; launch_set_loop sets the
+// number of steps and the phase it starts in before each launch.
+//
+// Fused (k_steps runs all steps up to the next rebuild):
+//   WHILE(loop) { k_steps -> IF(rebuild) { rebuild kernels } }
+// Separate kernels (ensembles, large systems):
+//   k_particle_start -> IF(rebuild) { rebuild kernels } -> pair || wall ->
+//   WHILE(loop) { k_particle(gather+final+initial) -> IF(rebuild) {...} -> pair || wall } ->
+//   k_particle(gather+final)
+// Without moving meshes the last block of the per-atom kernel takes the
+// decision, else k_decide_loop does after the mesh has moved.  The first
+// step's rebuild sits behind an IF node too: launched from the host its some
+// thirty kernels cost 67-150 us of each call while doing nothing.
+static int launch_particle_lp(const Sys &s, const LaunchCfg &lc, int mode, const LoopCond &lp, cudaStream_t st);
 
-cudaError_t build_step_graph(const Sys &s, const LaunchCfg &lc, cudaStream_t st, cudaStream_t st2,
-                             cudaGraphExec_t *exec, int *kernels_per_step, int *kernels_per_rebuild) {
+// Captures into one graph at a time on two streams and cleans up on failure.
+struct GraphBuilder {
+  const Sys &s;
+  const LaunchCfg &lc;
+  cudaStream_t st, st2;
   cudaGraph_t g = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
-  // every failure leaves through here: end a capture still open on either
-  // stream (its graph belongs to g), destroy the events and the graph
-  auto fail = [&](cudaError_t err) -> cudaError_t {
+  int kpr = 0;  // kernels of a rebuild
+
+  // ends a capture still open on either stream (its graph belongs to g),
+  // destroys the events and the graph
+  cudaError_t fail(cudaError_t err) {
     const cudaStream_t qs[2] = {st, st2};
     for (cudaStream_t q : qs) {
       cudaStreamCaptureStatus cs0 = cudaStreamCaptureStatusNone;
@@ -3105,79 +1919,132 @@ cudaError_t build_step_graph(const Sys &s, const LaunchCfg &lc, cudaStream_t st,
         cudaStreamEndCapture(q, &part);
       }
     }
+    done();
+    if (g) cudaGraphDestroy(g);
+    g = nullptr;
+    return err;
+  }
+  void done() {
     if (fork) cudaEventDestroy(fork);
     if (join) cudaEventDestroy(join);
-    if (g) cudaGraphDestroy(g);
-    return err;
-  };
-  cudaError_t e = cudaGraphCreate(&g, 0);
-  if (e != cudaSuccess) return fail(e);
-  cudaGraphConditionalHandle hloop, hreb;
-  if ((e = cudaGraphConditionalHandleCreate(&hloop, g, 1, cudaGraphCondAssignDefault)) != cudaSuccess) return fail(e);
-  if ((e = cudaGraphConditionalHandleCreate(&hreb, g, 0, cudaGraphCondAssignDefault)) != cudaSuccess) return fail(e);
-  cudaGraphNodeParams wp = {};
-  wp.type = cudaGraphNodeTypeConditional;
-  wp.conditional.handle = hloop;
-  wp.conditional.type = cudaGraphCondTypeWhile;
-  wp.conditional.size = 1;
-  cudaGraphNode_t wnode;
-  if ((e = cudaGraphAddNode(&wnode, g, nullptr, nullptr, 0, &wp)) != cudaSuccess) return fail(e);
-  cudaGraph_t body = wp.conditional.phGraph_out[0];
-  if ((e = cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
-    return fail(e);
-  bool moving = false;
-  for (int m = 0; m < s.nmeshes; m++) moving |= s.meshes[m].moving != 0;
-  int k = 0;
-  if (moving) {  // the mesh moves between the particle kernel and the decision
-    k += launch_particle(s, lc, kModeGatherFinalInitial, 1, st);
-    k += launch_mesh_move(s, lc, st);
-    k_decide_loop<<<1, sys_threads(s), 0, st>>>(s, hreb, hloop);
-    k++;
+    fork = join = nullptr;
+  }
+  cudaError_t begin(cudaGraph_t into) {
+    return cudaStreamBeginCaptureToGraph(st, into, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+  }
+  cudaError_t end() {
+    cudaGraph_t out = nullptr;
+    return cudaStreamEndCapture(st, &out);
+  }
+  // a conditional node behind what st has captured so far; its body in *body
+  cudaError_t conditional(cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type, cudaGraph_t *body) {
+    cudaStreamCaptureStatus cs;
+    const cudaGraphNode_t *deps = nullptr;
+    size_t nd = 0;
+    cudaGraph_t cg;
+    cudaError_t e = cudaStreamGetCaptureInfo(st, &cs, nullptr, &cg, &deps, nullptr, &nd);
+    if (e != cudaSuccess) return e;
+    cudaGraphNodeParams p = {};
+    p.type = cudaGraphNodeTypeConditional;
+    p.conditional.handle = h;
+    p.conditional.type = type;
+    p.conditional.size = 1;
+    cudaGraphNode_t node;
+    if ((e = cudaGraphAddNode(&node, cg, deps, nullptr, nd, &p)) != cudaSuccess) return e;
+    *body = p.conditional.phGraph_out[0];
+    return cudaStreamUpdateCaptureDependencies(st, &node, nullptr, 1, cudaStreamSetCaptureDependencies);
+  }
+  // IF(h) { rebuild kernels }
+  cudaError_t rebuild_if(cudaGraphConditionalHandle h) {
+    cudaGraph_t body, out = nullptr;
+    cudaError_t e = conditional(h, cudaGraphCondTypeIf, &body);
+    if (e != cudaSuccess) return e;
+    if ((e = cudaStreamBeginCaptureToGraph(st2, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
+        cudaSuccess)
+      return e;
+    kpr = launch_rebuild(s, lc, st2, 0);
+    return cudaStreamEndCapture(st2, &out);
+  }
+  // the pair kernel and the wall kernel of a step, side by side
+  cudaError_t forces(int *k) {
+    cudaError_t e;
+    const bool walls = s.nmeshes > 0 || s.nplanes > 0;
+    if (walls) {
+      if (!fork && (e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming)) != cudaSuccess) return e;
+      if (!join && (e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming)) != cudaSuccess) return e;
+      if ((e = cudaEventRecord(fork, st)) != cudaSuccess) return e;
+      if ((e = cudaStreamWaitEvent(st2, fork, 0)) != cudaSuccess) return e;
+      *k += launch_wall_force(s, lc, 1, st2);
+      if ((e = cudaEventRecord(join, st2)) != cudaSuccess) return e;
+    }
+    *k += launch_pair(s, lc, 1, st);
+    return walls ? cudaStreamWaitEvent(st, join, 0) : cudaSuccess;
+  }
+  // the per-atom kernel (start: the call's first step) with the decision
+  cudaError_t particle(bool start, cudaGraphConditionalHandle hreb, cudaGraphConditionalHandle hloop, int *k) {
+    bool moving = false;
+    for (int m = 0; m < s.nmeshes; m++) moving |= s.meshes[m].moving != 0;
+    const LoopCond lp{moving ? 0 : 1, hreb, hloop};
+    const int mode = start ? kModeStart : kModeGatherFinalInitial;
+    *k += launch_particle_lp(s, lc, mode, lp, st);
+    if (moving) {  // the mesh moves between the per-atom kernel and the decision
+      *k += launch_mesh_move(s, lc, st);
+      k_decide_loop<<<1, sys_threads(s), 0, st>>>(s, hreb, hloop);
+      (*k)++;
+    }
+    return cudaGetLastError();
+  }
+};
+
+cudaError_t build_step_graph(const Sys &s, const LaunchCfg &lc, cudaStream_t st, cudaStream_t st2,
+                             cudaGraphExec_t *exec, StepCounts *counts) {
+  GraphBuilder b{s, lc, st, st2};
+  cudaError_t e = cudaGraphCreate(&b.g, 0);
+  if (e != cudaSuccess) return b.fail(e);
+  cudaGraphConditionalHandle hloop, hreb, hreb0;
+  for (cudaGraphConditionalHandle *h : {&hloop, &hreb, &hreb0}) {
+    if (h == &hreb0 && fused_steps(s, lc)) continue;
+    if ((e = cudaGraphConditionalHandleCreate(h, b.g, h == &hloop ? 1 : 0, cudaGraphCondAssignDefault)) != cudaSuccess)
+      return b.fail(e);
+  }
+  *counts = StepCounts{};
+  cudaGraph_t body;
+  if ((e = b.begin(b.g)) != cudaSuccess) return b.fail(e);
+  if (fused_steps(s, lc)) {
+    if ((e = b.conditional(hloop, cudaGraphCondTypeWhile, &body)) != cudaSuccess) return b.fail(e);
+    if ((e = b.end()) != cudaSuccess) return b.fail(e);
+    if ((e = b.begin(body)) != cudaSuccess) return b.fail(e);
+    if ((e = launch_steps(s, lc, hreb, hloop, st)) != cudaSuccess) return b.fail(e);
+    if ((e = b.rebuild_if(hreb)) != cudaSuccess) return b.fail(e);
+    if ((e = b.end()) != cudaSuccess) return b.fail(e);
+    counts->call = 1;  // and one more launch per rebuild
+    counts->rebuild = b.kpr + 1;
   } else {
-    k += launch_particle_lp(s, lc, kModeGatherFinalInitial, 1, LoopCond{1, hreb, hloop}, st);
+    if ((e = b.particle(true, hreb0, hloop, &counts->call)) != cudaSuccess) return b.fail(e);
+    if ((e = b.rebuild_if(hreb0)) != cudaSuccess) return b.fail(e);
+    if ((e = b.forces(&counts->call)) != cudaSuccess) return b.fail(e);
+    if ((e = b.conditional(hloop, cudaGraphCondTypeWhile, &body)) != cudaSuccess) return b.fail(e);
+    counts->call += launch_particle(s, lc, kModeGatherFinal, st);
+    if ((e = b.end()) != cudaSuccess) return b.fail(e);
+    if ((e = b.begin(body)) != cudaSuccess) return b.fail(e);
+    if ((e = b.particle(false, hreb, hloop, &counts->step)) != cudaSuccess) return b.fail(e);
+    if ((e = b.rebuild_if(hreb)) != cudaSuccess) return b.fail(e);
+    if ((e = b.forces(&counts->step)) != cudaSuccess) return b.fail(e);
+    if ((e = b.end()) != cudaSuccess) return b.fail(e);
+    counts->rebuild = b.kpr;
   }
-  cudaStreamCaptureStatus cs;
-  const cudaGraphNode_t *deps = nullptr;
-  size_t nd = 0;
-  cudaGraph_t cg;
-  if ((e = cudaStreamGetCaptureInfo(st, &cs, nullptr, &cg, &deps, nullptr, &nd)) != cudaSuccess) return fail(e);
-  cudaGraphNodeParams ip = {};
-  ip.type = cudaGraphNodeTypeConditional;
-  ip.conditional.handle = hreb;
-  ip.conditional.type = cudaGraphCondTypeIf;
-  ip.conditional.size = 1;
-  cudaGraphNode_t inode;
-  if ((e = cudaGraphAddNode(&inode, cg, deps, nullptr, nd, &ip)) != cudaSuccess) return fail(e);
-  cudaGraph_t rbody = ip.conditional.phGraph_out[0];
-  if ((e = cudaStreamUpdateCaptureDependencies(st, &inode, nullptr, 1, cudaStreamSetCaptureDependencies)) != cudaSuccess)
-    return fail(e);
-  // the pair kernel and the wall kernel of the step run side by side
-  const bool walls = s.nmeshes > 0 || s.nplanes > 0;
-  if (walls) {
-    if ((e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming)) != cudaSuccess) return fail(e);
-    if ((e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming)) != cudaSuccess) return fail(e);
-    if ((e = cudaEventRecord(fork, st)) != cudaSuccess) return fail(e);
-    if ((e = cudaStreamWaitEvent(st2, fork, 0)) != cudaSuccess) return fail(e);
-    k += launch_wall_force(s, lc, 1, st2);
-    if ((e = cudaEventRecord(join, st2)) != cudaSuccess) return fail(e);
-  }
-  k += launch_pair(s, lc, 1, st);
-  if (walls && (e = cudaStreamWaitEvent(st, join, 0)) != cudaSuccess) return fail(e);
-  cudaGraph_t out = nullptr;
-  if ((e = cudaStreamEndCapture(st, &out)) != cudaSuccess) return fail(e);
-  if (fork) cudaEventDestroy(fork);
-  if (join) cudaEventDestroy(join);
-  fork = join = nullptr;
-  if ((e = cudaStreamBeginCaptureToGraph(st2, rbody, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
-    return fail(e);
-  const int kr = launch_rebuild(s, lc, st2, 0);
-  if ((e = cudaStreamEndCapture(st2, &out)) != cudaSuccess) return fail(e);
-  e = cudaGraphInstantiate(exec, g, 0);
-  cudaGraphDestroy(g);
-  g = nullptr;
-  *kernels_per_step = k;
-  *kernels_per_rebuild = kr;
+  e = cudaGraphInstantiate(exec, b.g, 0);
+  b.done();
+  cudaGraphDestroy(b.g);
   return e;
+}
+
+int wall_cap_per_atom() {
+  static const int cap = [] {
+    const char *e = getenv("LIGGGHTS_GB300_WALL_CAP");
+    return e ? std::max(1, std::min(16, atoi(e))) : kWallCapDefault;
+  }();
+  return cap;
 }
 
 // The wall kernel walks a short list (atoms near walls) with long per-atom
@@ -3187,20 +2054,15 @@ int launch_wall_force(const Sys &s, const LaunchCfg &lc, int shearupdate, cudaSt
   if (s.nmeshes == 0 && s.nplanes == 0) return 0;
   int lo = 0, hi = 0;
   cudaDeviceGetStreamPriorityRange(&lo, &hi);
-  // queue entries per tile: LIGGGHTS_GB300_WALL_CAP per atom (1..16)
-  static int cap_per_atom = 0;
-  if (!cap_per_atom) {
-    const char *e = getenv("LIGGGHTS_GB300_WALL_CAP");
-    cap_per_atom = e ? std::max(1, std::min(16, atoi(e))) : kWallCapDefault;
-    const int bytes = kWallWarps * cap_per_atom * kWallTile * kWallQ;
-    cudaFuncSetAttribute(k_wall_force<kHertz>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(k_wall_force<kHooke>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  }
+  const int cap_per_atom = wall_cap_per_atom();
+  const size_t bytes = (size_t)kWallWarps * cap_per_atom * kWallTile * kWallQ;
+  cudaFuncSetAttribute(k_wall_force<kHertz>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  cudaFuncSetAttribute(k_wall_force<kHooke>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   const int cap = cap_per_atom * kWallTile;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid_for(s.nmax, kWallWarps * kWallTile, 2 * lc.max_grid));
   cfg.blockDim = dim3(kWallWarps * kWallTile);
-  cfg.dynamicSmemBytes = (size_t)kWallWarps * cap * kWallQ;
+  cfg.dynamicSmemBytes = bytes;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributePriority;
@@ -3222,8 +2084,8 @@ int launch_mesh_move(const Sys &s, const LaunchCfg &lc, cudaStream_t st) {
   return nl;
 }
 
-int launch_set_loop(const Sys &s, int n, cudaStream_t st) {
-  k_set_loop<<<1, 1, 0, st>>>(s, n);
+int launch_set_loop(const Sys &s, int n, int phase, cudaStream_t st) {
+  k_set_loop<<<1, 1, 0, st>>>(s.ctrl, n, phase);
   return 1;
 }
 
@@ -3299,32 +2161,23 @@ int launch_pair(const Sys &s, const LaunchCfg &lc, int shearupdate, cudaStream_t
   return 1;
 }
 
-template <int NORMAL>
-static void launch_particle_n(const Sys &s, int g, int B, int mode, int shearupdate, const LoopCond &lp,
-                              cudaStream_t st) {
-  switch (mode) {
-    case kModeInitial: k_particle<NORMAL, false, false, true><<<g, B, 0, st>>>(s, shearupdate, lp); break;
-    case kModeGather: k_particle<NORMAL, true, false, false><<<g, B, 0, st>>>(s, shearupdate, lp); break;
-    case kModeGatherFinal: k_particle<NORMAL, true, true, false><<<g, B, 0, st>>>(s, shearupdate, lp); break;
-    case kModeGatherFinalInitial:
-      k_particle<NORMAL, true, true, true><<<g, B, 0, st>>>(s, shearupdate, lp);
-      break;
-  }
-}
-
-static int launch_particle_lp(const Sys &s, const LaunchCfg &lc, int mode, int shearupdate, const LoopCond &lp,
-                              cudaStream_t st) {
+static int launch_particle_lp(const Sys &s, const LaunchCfg &lc, int mode, const LoopCond &lp, cudaStream_t st) {
   // one particle per thread; smaller blocks give the same number of threads
   // in more, smaller blocks (each particle's sums do not depend on it)
   const int B = lc.particle_threads;
   const int g = grid_for(s.nmax, B, lc.max_grid * (256 / B));
-  if (s.normal == kHertz) launch_particle_n<kHertz>(s, g, B, mode, shearupdate, lp, st);
-  else launch_particle_n<kHooke>(s, g, B, mode, shearupdate, lp, st);
+  switch (mode) {
+    case kModeInitial: k_particle<false, false, true><<<g, B, 0, st>>>(s, lp); break;
+    case kModeGather: k_particle<true, false, false><<<g, B, 0, st>>>(s, lp); break;
+    case kModeGatherFinal: k_particle<true, true, false><<<g, B, 0, st>>>(s, lp); break;
+    case kModeGatherFinalInitial: k_particle<true, true, true><<<g, B, 0, st>>>(s, lp); break;
+    case kModeStart: k_particle_start<<<g, B, 0, st>>>(s, lp); break;
+  }
   return 1;
 }
 
-int launch_particle(const Sys &s, const LaunchCfg &lc, int mode, int shearupdate, cudaStream_t st) {
-  return launch_particle_lp(s, lc, mode, shearupdate, LoopCond{0, 0, 0}, st);
+int launch_particle(const Sys &s, const LaunchCfg &lc, int mode, cudaStream_t st) {
+  return launch_particle_lp(s, lc, mode, LoopCond{0, 0, 0}, st);
 }
 
 }  // namespace gb300

@@ -10,6 +10,7 @@ struct LaunchCfg {
   int max_grid;              // grid-stride kernels never launch more blocks of 256 than this
   int particle_threads = 256;  // threads per block of the per-particle kernel (64, 128, 256)
   int sms = 152;               // multiprocessors of the device
+  int np = 0;                  // list entries at the last build (what fused_steps goes by)
 };
 
 enum {
@@ -17,6 +18,8 @@ enum {
   kModeGather = 1,              // sum forces only (setup)
   kModeGatherFinal = 2,         // sum forces + final_integrate (last step of a call)
   kModeGatherFinalInitial = 3,  // sum forces + final(n) + initial(n+1) (steady state)
+  kModeStart = 4,               // first step of a graph launch: kModeInitial or kModeGatherFinalInitial, by
+                                // Ctrl::step_phase
 };
 
 struct InsertStage {  // new atoms, device arrays: x, v, w [3k], the rest [k]
@@ -66,16 +69,26 @@ int launch_set_rebuild(const Sys &s, int v, cudaStream_t st);
 // stage 2: resume after a mesh slot or registration overflow
 int launch_rebuild(const Sys &s, const LaunchCfg &lc, cudaStream_t st, int stage);
 int launch_pair(const Sys &s, const LaunchCfg &lc, int shearupdate, cudaStream_t st);
-int launch_particle(const Sys &s, const LaunchCfg &lc, int mode, int shearupdate, cudaStream_t st);
-int launch_set_loop(const Sys &s, int n, cudaStream_t st);
+int launch_particle(const Sys &s, const LaunchCfg &lc, int mode, cudaStream_t st);
+int launch_set_loop(const Sys &s, int n, int phase, cudaStream_t st);
 // wall (plane and mesh) forces of the current state, before the particle
 // kernel that gathers the step's forces; none without walls
 int launch_wall_force(const Sys &s, const LaunchCfg &lc, int shearupdate, cudaStream_t st);
 // fix move/mesh: moves the moving meshes by one step (after the drift)
 int launch_mesh_move(const Sys &s, const LaunchCfg &lc, cudaStream_t st);
-// Executable graph of the steady-state step loop (WHILE node over steps, IF
-// node around the rebuild); see dem_kernels.cu.
+// queue entries of the wall kernel per tile atom (LIGGGHTS_GB300_WALL_CAP)
+int wall_cap_per_atom();
+// Whether dem_step runs the steps in k_steps (dem_steps.cu) rather than as
+// separate kernels, and its launch inside the step graph.
+bool fused_steps(const Sys &s, const LaunchCfg &lc);
+cudaError_t launch_steps(const Sys &s, const LaunchCfg &lc, cudaGraphConditionalHandle hreb,
+                         cudaGraphConditionalHandle hloop, cudaStream_t st);
+// Executable graph of the step loop (WHILE node over steps, IF node around
+// the rebuild); see dem_kernels.cu.  launch_set_loop sets what it runs.
+struct StepCounts {  // kernels of a graph launch: per call, per further step, per rebuild
+  int call = 0, step = 0, rebuild = 0;
+};
 cudaError_t build_step_graph(const Sys &s, const LaunchCfg &lc, cudaStream_t st, cudaStream_t st2,
-                             cudaGraphExec_t *exec, int *kernels_per_step, int *kernels_per_rebuild);
+                             cudaGraphExec_t *exec, StepCounts *counts);
 
 }  // namespace gb300
