@@ -77,6 +77,7 @@ constexpr int kMaxGrid = 152 * 16;
 
 // parameter adjoints per entry / atom: Y, G, beta, mu, rolling coefficient
 constexpr int kTh = 5;
+constexpr int kARec = 16;  // doubles of ABar::rec per entry
 constexpr int kAMC = kMeshMaxCand;  // candidate triangles (= history slots) per atom and mesh
 constexpr int kAMeshes = 4;
 
@@ -98,6 +99,7 @@ struct AList {
   uint8_t *sh = nullptr;    // image code of the partner
   uint8_t *flag = nullptr;  // kContact* bits; nonzero: the entry's history is carried
   double *shear = nullptr;  // [3*p+k], evolving
+  double *pc = nullptr;     // [4*p]: reff, meff, sqrt(2 Y meff), sqrt(8 G meff) of the entry (LawPair)
   double *bond = nullptr;   // [kBondValues*p+k], evolving (bonds only)
   // mesh walls: candidates per (mesh, atom) at this build, ascending, and the
   // slot each slot came from at the build (-1: emptied)
@@ -131,16 +133,22 @@ struct ADev {
   // per-atom kick constants of the run: ka = dtf/m, kb = dtfrot/(r^2 m) and
   // the factors of their derivatives ka/m, kb/m, 2 kb/r
   double *ka, *kb, *kam, *kbm, *kbr;
+  // constants of the law (adjoint_law.cuh): of the material, and per atom
+  // 1/r, 1/m, sqrt(2 Y m), sqrt(8 G m) [4*i]
+  LawUniform lu;
+  double *ac;
   // list in use
   int np;
   const int *pi, *pj, *row, *rev_start, *rev;
   const uint8_t *sh;
   uint8_t *flag;
   double *shear;
+  const double *pc;
   double *bh;  // bond history of the list in use
   // pair outputs of the current force evaluation
   double *pF, *pTi, *pTj;
   uint8_t *active;  // touching or bonded: the entry's outputs count
+  double *wF, *wT;  // force and torque of the walls (planes, then meshes) [3*i+k]
   // cells
   int nc[3];
   double csz[3];
@@ -231,6 +239,10 @@ __global__ void ka_consts(ADev s) {
     s.kam[i] = a / m;
     s.kbm[i] = b / m;
     s.kbr[i] = 2.0 * b / r;
+    s.ac[4 * i] = 1.0 / r;
+    s.ac[4 * i + 1] = 1.0 / m;
+    s.ac[4 * i + 2] = sqrt(2.0 * s.Y * m);
+    s.ac[4 * i + 3] = sqrt(8.0 * s.G * m);
   }
 }
 
@@ -437,6 +449,12 @@ __global__ void ka_carry(ADev s, AList nw, AList old) {
           }
         }
     }
+    const double ri = s.r[i], rj = s.r[j], mi = s.m[i], mj = s.m[j];
+    const double meff = mi * mj / (mi + mj);
+    nw.pc[4 * (size_t)p] = ri * rj / (ri + rj);
+    nw.pc[4 * (size_t)p + 1] = meff;
+    nw.pc[4 * (size_t)p + 2] = sqrt(2.0 * s.Y * meff);
+    nw.pc[4 * (size_t)p + 3] = sqrt(8.0 * s.G * meff);
     nw.carry[p] = e < 0 ? -1 : (sgn > 0 ? e : -(e + 2));
     nw.flag[p] = e >= 0 ? 1 : 0;
     for (int k = 0; k < 3; k++) nw.shear[3 * p + k] = e >= 0 ? sgn * old.shear[3 * e + k] : 0.0;
@@ -475,7 +493,19 @@ __device__ __forceinline__ VjpIn pair_in(const ADev &s, const double *x, int p, 
   a.bonded = false;
   a.rolling = s.rolling != 0;
   a.mur = s.mur;
+  a.pre = true;
+  a.pu = s.lu;
+  const double *pc = s.pc + 4 * (size_t)p, *ci = s.ac + 4 * (size_t)i, *cj = s.ac + 4 * (size_t)j;
+  a.pp = LawPair{pc[0], pc[1], ci[0], cj[0], ci[1], cj[1], pc[2], pc[3]};
   return a;
+}
+
+// constants of atom i's contact with a wall
+__device__ __forceinline__ void wall_pre(const ADev &s, int i, VjpIn &a) {
+  a.pre = true;
+  a.pu = s.lu;
+  const double *c = s.ac + 4 * (size_t)i;
+  a.pp = LawPair{a.ri, a.mi, c[0], 0.0, c[1], 0.0, c[2], c[3]};
 }
 
 __device__ __forceinline__ bool pair_touch(const VjpIn &a) {
@@ -536,14 +566,18 @@ __device__ __forceinline__ bool wall_in(const ADev &s, const double *x, int w, i
   a.bonded = false;
   a.rolling = s.rolling != 0;
   a.mur = s.mur;
+  wall_pre(s, i, a);
   return true;
 }
 
 // adjoints of the run's state (the mesh reverse below and the reverse kernels)
 struct ABar {
   double *xb, *vb, *wb, *Fb, *Tb, *rb, *mb, *sb, *wsb;
-  // per-entry VJP outputs of the pair law
-  double *pd, *pv, *pwi, *pwj, *pri, *prj, *pmi, *pmj, *pth;  // pth [kTh*p]: Y, G, beta, mu, mur
+  // per-entry VJP outputs of the pair law, one 128-byte record each: adjoints
+  // of d[3], vr[3], wi[3], wj[3], ri, rj, mi, mj; pact: the entry has one
+  double *rec;
+  uint8_t *pact;
+  double *pth;  // [kTh*p]: Y, G, beta, mu, mur
   double *bb;   // [kBondValues*p] adjoint of the bond history (bonds only)
   double *wth;  // [kTh*i] wall parameter adjoints per atom
   double *th;   // [4] accumulated parameter adjoints
@@ -615,6 +649,7 @@ __device__ __forceinline__ void amesh_contact_in(const ADev &s, int i, const dou
   a.bonded = false;
   a.rolling = s.rolling != 0;
   a.mur = s.mur;
+  wall_pre(s, i, a);
 }
 
 // one evaluation of the slot logic and contact law for atom i and mesh m on
@@ -945,11 +980,10 @@ __global__ void kb_mesh_uncarry(int cnt, const int *map, const double *hb_new, d
 // BONDS: the system has cohesion bond/nonlinear (a separate instance keeps
 // the registers of the plain contact path low)
 template <bool BONDS, bool ROLL>
-__global__ void __launch_bounds__(kAB) ka_pair_force(ADev s, const double *vh, const double *wh, int upd,
-                                                     long long ntimestep, double *tape_sh, double *tape_bh) {
-  __shared__ int q[kAB];
-  __shared__ int wcnt[kAB / 32];
-  ABLOCKS(base, s.np) {
+__device__ __forceinline__ void pair_blocks(const ADev &s, int block, int blocks, int *q, int *wcnt, const double *vh,
+                                            const double *wh, int upd, long long ntimestep, double *tape_sh,
+                                            double *tape_bh) {
+  for (int base = block * kAB; base < s.np; base += blocks * kAB) {
     const int p0 = base + threadIdx.x;
     bool work = false;
     if (p0 < s.np) {  // tape and the FP32 candidate test; the rest runs queued
@@ -1010,81 +1044,18 @@ __global__ void __launch_bounds__(kAB) ka_pair_force(ADev s, const double *vh, c
   }
 }
 
-// total force/torque per atom: own row, reverse list (local entries), gravity,
-// planes; with final_kick the second half-kick v = vh + a F, w = wh + b T.
-// tape_ws receives the wall history before the update, wallF the wall forces,
-// tape_F/tape_T (if set) a copy of the forces and torques.
-// The next step's first half-kick and drift (ka_kick_drift without a wrap),
-// fused into the gather of a step when both lie in one segment: xref and the
-// t* records as there, nk = 1 to do it.
-struct NextKick {
-  const double *xref;
-  double *tx, *tv, *tw;
-  float4 *txf;
-  int on;
-};
-
+// walls of the current state, planes in order (the atoms touching plane w run
+// the law on dense warps), then meshes, summed into wF/wT.  tape_ws receives
+// the wall history before the update, wallF the wall forces.
 template <bool ROLL, bool MESH>
-__global__ void __launch_bounds__(kAB) ka_gather(ADev s, const double *vh, const double *wh, int upd,
-                                                 int final_kick, double *tape_ws, double *wallF, double *tape_F,
-                                                 double *tape_T, int *tape_mst, double *tape_msh, int *tape_mnp,
-                                                 long long ntimestep, NextKick nk) {
-  __shared__ int q[kAB];
-  __shared__ int wcnt[kAB / 32];
-  __shared__ double sF[3][kAB], sT[3][kAB];
-  ABLOCKS(base, s.n) {
+__device__ __forceinline__ void wall_blocks(const ADev &s, int block, int blocks, int *q, int *wcnt,
+                                            double (*sF)[kAB], double (*sT)[kAB], const double *vh, const double *wh,
+                                            int upd, double *tape_ws, double *wallF, int *tape_mst, double *tape_msh,
+                                            int *tape_mnp, long long ntimestep) {
+  for (int base = block * kAB; base < s.n; base += blocks * kAB) {
     const int i = base + threadIdx.x;
     const bool valid = i < s.n;
     double f[3] = {0., 0., 0.}, t[3] = {0., 0., 0.};
-    if (valid) {
-      // own row, then the local partner entries, each in ascending order; the
-      // active entries of lists of up to 32 are collected as bit masks first,
-      // so that the FP64 additions issue once per contact of the warp's
-      // busiest atom rather than once per entry of its longest list
-      const int pb = s.row[i], pe = s.row[i + 1], rb = s.rev_start[i], re = s.rev_start[i + 1];
-      if (pe - pb <= 32 && re - rb <= 32) {
-        unsigned mo = 0u, mr = 0u;
-        for (int k = 0; k < pe - pb; k++) mo |= (s.active[pb + k] ? 1u : 0u) << k;
-        for (int k = 0; k < re - rb; k++) {
-          const int p = s.rev[rb + k];
-          mr |= ((s.active[p] && s.sh[p] == kNoShift) ? 1u : 0u) << k;
-        }
-        while (mo) {
-          const int p = pb + __ffs(mo) - 1;
-          mo &= mo - 1u;
-          for (int k = 0; k < 3; k++) {
-            f[k] += s.pF[3 * p + k];
-            t[k] += s.pTi[3 * p + k];
-          }
-        }
-        while (mr) {
-          const int p = s.rev[rb + __ffs(mr) - 1];
-          mr &= mr - 1u;
-          for (int k = 0; k < 3; k++) {
-            f[k] -= s.pF[3 * p + k];
-            t[k] += s.pTj[3 * p + k];
-          }
-        }
-      } else {
-        for (int p = pb; p < pe; p++)
-          if (s.active[p])
-            for (int k = 0; k < 3; k++) {
-              f[k] += s.pF[3 * p + k];
-              t[k] += s.pTi[3 * p + k];
-            }
-        for (int qq = rb; qq < re; qq++) {
-          const int p = s.rev[qq];
-          if (!s.active[p] || s.sh[p] != kNoShift) continue;
-          for (int k = 0; k < 3; k++) {
-            f[k] -= s.pF[3 * p + k];
-            t[k] += s.pTj[3 * p + k];
-          }
-        }
-      }
-      if (s.gravity_on)
-        for (int k = 0; k < 3; k++) f[k] += s.m[i] * s.g[k];
-    }
-    // planes in order; the atoms touching plane w run the law on dense warps
     for (int w = 0; w < s.nplanes; w++) {
       bool touch = false;
       if (valid) {
@@ -1126,43 +1097,157 @@ __global__ void __launch_bounds__(kAB) ka_gather(ADev s, const double *vh, const
     }
     if (valid) {
       if (MESH) amesh_forward<ROLL>(s, i, s.x, vh, wh, upd, ntimestep, f, t, tape_mst, tape_msh, tape_mnp, wallF);
-      const double a = s.ka[i], b = s.kb[i];
       for (int k = 0; k < 3; k++) {
-        s.F[3 * i + k] = f[k];
-        s.T[3 * i + k] = t[k];
-        if (tape_F) {
-          tape_F[3 * i + k] = f[k];
-          tape_T[3 * i + k] = t[k];
-        }
-        if (final_kick) {
-          s.v[3 * i + k] = vh[3 * i + k] + a * f[k];
-          s.w[3 * i + k] = wh[3 * i + k] + b * t[k];
-        }
+        s.wF[3 * i + k] = f[k];
+        s.wT[3 * i + k] = t[k];
       }
-      if (nk.on) {  // the next step's first half-kick and drift, as ka_kick_drift
-        double dsq = 0.0;
+    }
+  }
+}
+
+// Pair and wall forces of one evaluation, side by side: the first gp blocks
+// take the list, the others (none without walls) the atoms' walls.  Both are
+// chains of FP64 instructions on few warps, so that side by side costs the
+// longer of the two (1,000 settling spheres: 8.4 us an evaluation, and 7.9 for
+// the gather; pairs alone and walls with the gather took 11.2 and 13.2).
+template <bool BONDS, bool ROLL, bool MESH>
+__global__ void __launch_bounds__(kAB) ka_forces(ADev s, int gp, const double *vh, const double *wh, int upd,
+                                                 long long ntimestep, double *tape_sh, double *tape_bh,
+                                                 double *tape_ws, double *wallF, int *tape_mst, double *tape_msh,
+                                                 int *tape_mnp) {
+  __shared__ int q[kAB];
+  __shared__ int wcnt[kAB / 32];
+  __shared__ double sF[3][kAB], sT[3][kAB];
+  if ((int)blockIdx.x < gp)
+    pair_blocks<BONDS, ROLL>(s, blockIdx.x, gp, q, wcnt, vh, wh, upd, ntimestep, tape_sh, tape_bh);
+  else
+    wall_blocks<ROLL, MESH>(s, blockIdx.x - gp, gridDim.x - gp, q, wcnt, sF, sT, vh, wh, upd, tape_ws, wallF, tape_mst,
+                            tape_msh, tape_mnp, ntimestep);
+}
+
+// The next step's first half-kick and drift (ka_kick_drift without a wrap),
+// fused into the gather of a step when both lie in one segment: xref and the
+// t* records as there, on = 1 to do it.
+struct NextKick {
+  const double *xref;
+  double *tx, *tv, *tw;
+  float4 *txf;
+  int on;
+};
+
+// Active entries of an atom's row and partner list (up to 32 each) as bit
+// masks, their flags loaded eight at a time without waiting for one another;
+// local: partner entries of images do not count.  false: longer lists.
+__device__ __forceinline__ bool entry_masks(const ADev &s, const uint8_t *active, bool local, int pb, int pe, int rb,
+                                            int re, unsigned &mo, unsigned &mr) {
+  if (pe - pb > 32 || re - rb > 32) return false;
+  mo = mr = 0u;
+  const int no = pe - pb, nr = re - rb;
+  for (int k0 = 0; k0 < max(no, nr); k0 += 8) {
+    int e[8];
+    bool ao[8], ar[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      e[k] = k0 + k < nr ? s.rev[rb + k0 + k] : -1;
+      ao[k] = k0 + k < no ? active[pb + k0 + k] != 0 : false;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) ar[k] = e[k] >= 0 ? active[e[k]] != 0 && (!local || s.sh[e[k]] == kNoShift) : false;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      mo |= (ao[k] ? 1u : 0u) << (k0 + k);
+      mr |= (ar[k] ? 1u : 0u) << (k0 + k);
+    }
+  }
+  return true;
+}
+
+// total force/torque per atom: own row, then the local partner entries, each
+// in ascending order, gravity, walls; with final_kick the second half-kick
+// v = vh + a F, w = wh + b T.  tape_F/tape_T (if set) receive a copy of the
+// forces and torques.
+__global__ void __launch_bounds__(kAB) ka_gather(ADev s, const double *vh, const double *wh, int final_kick,
+                                                 double *tape_F, double *tape_T, NextKick nk) {
+  AGRID(i, s.n) {
+    double f[3] = {0., 0., 0.}, t[3] = {0., 0., 0.};
+    const int pb = s.row[i], pe = s.row[i + 1], rb = s.rev_start[i], re = s.rev_start[i + 1];
+    unsigned mo, mr;
+    if (entry_masks(s, s.active, true, pb, pe, rb, re, mo, mr)) {
+      while (mo) {
+        const int p = pb + __ffs(mo) - 1;
+        mo &= mo - 1u;
         for (int k = 0; k < 3; k++) {
-          const double v = s.v[3 * i + k] + a * f[k];
-          const double w = s.w[3 * i + k] + b * t[k];
-          const double x = s.x[3 * i + k] + s.dt * v;
-          if (nk.xref) {
-            const double e = x - nk.xref[3 * i + k];
-            dsq += e * e;
-          }
-          s.v[3 * i + k] = v;
-          s.w[3 * i + k] = w;
-          s.x[3 * i + k] = x;
-          if (nk.tx) {
-            nk.tx[3 * i + k] = x;
-            nk.tv[3 * i + k] = v;
-            nk.tw[3 * i + k] = w;
-          }
+          f[k] += s.pF[3 * p + k];
+          t[k] += s.pTi[3 * p + k];
         }
-        const float4 f4 = make_float4((float)s.x[3 * i], (float)s.x[3 * i + 1], (float)s.x[3 * i + 2], (float)s.r[i]);
-        s.xf[i] = f4;
-        if (nk.txf) nk.txf[i] = f4;
-        if (dsq > 0.25 * s.skin * s.skin) s.err[0] = 1;
       }
+      while (mr) {
+        const int p = s.rev[rb + __ffs(mr) - 1];
+        mr &= mr - 1u;
+        for (int k = 0; k < 3; k++) {
+          f[k] -= s.pF[3 * p + k];
+          t[k] += s.pTj[3 * p + k];
+        }
+      }
+    } else {
+      for (int p = pb; p < pe; p++)
+        if (s.active[p])
+          for (int k = 0; k < 3; k++) {
+            f[k] += s.pF[3 * p + k];
+            t[k] += s.pTi[3 * p + k];
+          }
+      for (int qq = rb; qq < re; qq++) {
+        const int p = s.rev[qq];
+        if (!s.active[p] || s.sh[p] != kNoShift) continue;
+        for (int k = 0; k < 3; k++) {
+          f[k] -= s.pF[3 * p + k];
+          t[k] += s.pTj[3 * p + k];
+        }
+      }
+    }
+    if (s.gravity_on)
+      for (int k = 0; k < 3; k++) f[k] += s.m[i] * s.g[k];
+    if (s.nplanes > 0 || s.nmeshes > 0)
+      for (int k = 0; k < 3; k++) {
+        f[k] += s.wF[3 * i + k];
+        t[k] += s.wT[3 * i + k];
+      }
+    const double a = s.ka[i], b = s.kb[i];
+    for (int k = 0; k < 3; k++) {
+      s.F[3 * i + k] = f[k];
+      s.T[3 * i + k] = t[k];
+      if (tape_F) {
+        tape_F[3 * i + k] = f[k];
+        tape_T[3 * i + k] = t[k];
+      }
+      if (final_kick) {
+        s.v[3 * i + k] = vh[3 * i + k] + a * f[k];
+        s.w[3 * i + k] = wh[3 * i + k] + b * t[k];
+      }
+    }
+    if (nk.on) {  // the next step's first half-kick and drift, as ka_kick_drift
+      double dsq = 0.0;
+      for (int k = 0; k < 3; k++) {
+        const double v = s.v[3 * i + k] + a * f[k];
+        const double w = s.w[3 * i + k] + b * t[k];
+        const double x = s.x[3 * i + k] + s.dt * v;
+        if (nk.xref) {
+          const double e = x - nk.xref[3 * i + k];
+          dsq += e * e;
+        }
+        s.v[3 * i + k] = v;
+        s.w[3 * i + k] = w;
+        s.x[3 * i + k] = x;
+        if (nk.tx) {
+          nk.tx[3 * i + k] = x;
+          nk.tv[3 * i + k] = v;
+          nk.tw[3 * i + k] = w;
+        }
+      }
+      const float4 f4 = make_float4((float)s.x[3 * i], (float)s.x[3 * i + 1], (float)s.x[3 * i + 2], (float)s.r[i]);
+      s.xf[i] = f4;
+      if (nk.txf) nk.txf[i] = f4;
+      if (dsq > 0.25 * s.skin * s.skin) s.err[0] = 1;
     }
   }
 }
@@ -1209,39 +1294,53 @@ __global__ void ka_kick_drift(ADev s, const double *xref, int wrap, double *tx, 
 
 // ------------------------------------------------------------------ backward
 
-// gravity and walls of one force evaluation at positions x; vh/wh the
-// velocities the forces saw, ws_before the wall history before it; seed adds
-// d(loss)/d(normal wall force) on plane seed_w.  Fn1/Tn1 (if set): the
-// forces of this evaluation, whose second half-kick v' = vh + a F',
-// w' = wh + b T' is reversed first.  The wall parameter adjoints add to
-// B.wth.
+// The second half-kick v' = vh + a F', w' = wh + b T' of an evaluation, in
+// reverse: Fb += a vb, Tb += b wb and the radius and mass adjoints; then
+// gravity's mass adjoint.  fv = F'.vb, tw = T'.wb.  fresh: Fb, Tb start from
+// the next step's first half-kick (the same a vb, b wb), else from zero.
+__device__ __forceinline__ void kick_back(const ADev &s, const ABar &B, int i, const double vb[3], const double wb[3],
+                                          bool first, bool second, double fv, double tw, double rb, double mb) {
+  const double c = (first ? 1.0 : 0.0) + (second ? 1.0 : 0.0);
+  const double a = c * s.ka[i], b = c * s.kb[i];
+  double Fb[3];
+  for (int k = 0; k < 3; k++) {
+    Fb[k] = a * vb[k];
+    B.Fb[3 * i + k] = Fb[k];
+    B.Tb[3 * i + k] = b * wb[k];
+  }
+  mb += c * (-s.kam[i] * fv - s.kbm[i] * tw);
+  rb += c * (-s.kbr[i] * tw);
+  if (s.gravity_on) mb += s.g[0] * Fb[0] + s.g[1] * Fb[1] + s.g[2] * Fb[2];
+  B.rb[i] += rb;
+  B.mb[i] += mb;
+}
+
+// the last step's second half-kick, whose forces are Fn/Tn
+__global__ void kb_last_kick(ADev s, ABar B, const double *Fn, const double *Tn) {
+  AGRID(i, s.n) {
+    double vb[3], wb[3], fv = 0.0, tw = 0.0;
+    for (int k = 0; k < 3; k++) {
+      vb[k] = B.vb[3 * i + k];
+      wb[k] = B.wb[3 * i + k];
+      fv += Fn[3 * i + k] * vb[k];
+      tw += Tn[3 * i + k] * wb[k];
+    }
+    kick_back(s, B, i, vb, wb, false, true, fv, tw, 0.0, 0.0);
+  }
+}
+
+// walls of one force evaluation at positions x; vh/wh the velocities the
+// forces saw, ws_before the wall history before it; seed adds d(loss)/d(normal
+// wall force) on plane seed_w.  The wall parameter adjoints add to B.wth.
 template <bool ROLL, bool MESH>
-__global__ void __launch_bounds__(kAB) kb_walls(ADev s, ABar B, const double *x, const double *vh,
-                                                const double *wh, const double *ws_before, int upd, int seed_w,
-                                                double seed, const double *Fn1, const double *Tn1,
+__device__ __forceinline__ void wall_vjp_blocks(const ADev &s, const ABar &B, int block, int blocks, int *q, int *wcnt,
+                                                const double *x, const double *vh, const double *wh,
+                                                const double *ws_before, int upd, int seed_w, double seed,
                                                 const int *tmst, const double *tmsh, const int *tmnp,
                                                 long long ntimestep, int seed_axis) {
-  __shared__ int q[kAB];
-  __shared__ int wcnt[kAB / 32];
-  ABLOCKS(base, s.n) {
+  for (int base = block * kAB; base < s.n; base += blocks * kAB) {
     const int i = base + threadIdx.x;
     const bool valid = i < s.n;
-    if (valid) {
-      if (Fn1) {
-        const double a = s.ka[i], b = s.kb[i];
-        double fv = 0.0, tw = 0.0;
-        for (int k = 0; k < 3; k++) {
-          B.Fb[3 * i + k] += a * B.vb[3 * i + k];
-          B.Tb[3 * i + k] += b * B.wb[3 * i + k];
-          fv += Fn1[3 * i + k] * B.vb[3 * i + k];
-          tw += Tn1[3 * i + k] * B.wb[3 * i + k];
-        }
-        B.mb[i] += -s.kam[i] * fv - s.kbm[i] * tw;
-        B.rb[i] += -s.kbr[i] * tw;
-      }
-      if (s.gravity_on)
-        B.mb[i] += s.g[0] * B.Fb[3 * i] + s.g[1] * B.Fb[3 * i + 1] + s.g[2] * B.Fb[3 * i + 2];
-    }
     // planes in order; the atoms touching plane w run the VJP on dense warps
     for (int w = 0; w < s.nplanes; w++) {
       bool touch = false;
@@ -1303,17 +1402,16 @@ __global__ void __launch_bounds__(kAB) kb_walls(ADev s, ABar B, const double *x,
   }
 }
 
-// reverse of ka_pair_force for one evaluation at positions x (vh/wh the
+// reverse of pair_blocks for one evaluation at positions x (vh/wh the
 // velocities it saw, sh_before/bh_before the history before it); the input
-// adjoints of each entry go to the per-entry arrays, the history adjoints
-// B.sb/B.bb are replaced by those of the history before the evaluation
+// adjoints of each entry go to its record, the history adjoints B.sb/B.bb are
+// replaced by those of the history before the evaluation
 template <bool BONDS, bool ROLL>
-__global__ void __launch_bounds__(kAB) kb_pairs(ADev s, ABar B, const double *x, const float4 *xf,
-                                                const double *vh, const double *wh, const double *sh_before,
-                                                const double *bh_before, int upd, long long ntimestep) {
-  __shared__ int q[kAB];
-  __shared__ int wcnt[kAB / 32];
-  ABLOCKS(base, s.np) {
+__device__ __forceinline__ void pair_vjp_blocks(const ADev &s, const ABar &B, int block, int blocks, int *q, int *wcnt,
+                                                const double *x, const float4 *xf, const double *vh, const double *wh,
+                                                const double *sh_before, const double *bh_before, int upd,
+                                                long long ntimestep) {
+  for (int base = block * kAB; base < s.np; base += blocks * kAB) {
     const int p0 = base + threadIdx.x;
     bool work = false;
     if (p0 < s.np) {  // entries without a law evaluation: no input adjoints
@@ -1326,13 +1424,10 @@ __global__ void __launch_bounds__(kAB) kb_pairs(ADev s, ABar B, const double *x,
         band = pair_band(s, a);
         work = touch || (BONDS && band);
       }
-      if (!work) {
-        for (int k = 0; k < 3; k++) {
-          B.pd[3 * p0 + k] = B.pv[3 * p0 + k] = B.pwi[3 * p0 + k] = B.pwj[3 * p0 + k] = 0.0;
-          if (band) B.sb[3 * p0 + k] = 0.0;  // history cleared: no dependence
-        }  // else: history unchanged, its adjoint passes through
-        B.pri[p0] = B.prj[p0] = B.pmi[p0] = B.pmj[p0] = 0.0;
-      }
+      B.pact[p0] = work ? 1 : 0;
+      if (!work && band)
+        for (int k = 0; k < 3; k++) B.sb[3 * p0 + k] = 0.0;  // history cleared: no dependence
+      // (else: history unchanged, its adjoint passes through)
     }
     const int tot = block_queue(work, p0, q, wcnt);
     if (threadIdx.x < tot) {
@@ -1400,26 +1495,62 @@ __global__ void __launch_bounds__(kAB) kb_pairs(ADev s, ABar B, const double *x,
       } else if (band) {
         for (int k = 0; k < 3; k++) B.sb[3 * p + k] = 0.0;  // history cleared: no dependence
       }
+      double *r = B.rec + (size_t)kARec * p;
       for (int k = 0; k < 3; k++) {
-        B.pd[3 * p + k] = d[k];
-        B.pv[3 * p + k] = vr[k];
-        B.pwi[3 * p + k] = wi[k];
-        B.pwj[3 * p + k] = wj[k];
+        r[k] = d[k];
+        r[3 + k] = vr[k];
+        r[6 + k] = wi[k];
+        r[9 + k] = wj[k];
       }
-      B.pri[p] = ri;
-      B.prj[p] = rj;
-      B.pmi[p] = mi;
-      B.pmj[p] = mj;
+      r[12] = ri;
+      r[13] = rj;
+      r[14] = mi;
+      r[15] = mj;
       for (int k = 0; k < kTh; k++) B.pth[kTh * p + k] += th[k];  // summed over the segment's steps
     }
     __syncthreads();
   }
 }
 
-// per atom: pair adjoints in list order (own row, then reverse list), then
-// the drift x' = x + dt vh and the first half-kick vh = v + a F, wh = w + b T
-// with Fn/Tn the forces at the step's start; drift = 0 for the setup pass
-__global__ void kb_gather_kick(ADev s, ABar B, const double *Fn, const double *Tn, int drift) {
+// pairs and walls of one evaluation, side by side as in ka_forces: bound by the
+// length of the law's FP64 chain (64 cycles an instruction), so every division
+// and root that the law shares or inverts counts.  1,000 spheres: 12.9 us where
+// two launches took 20.2 and 6.7; 20,000: 25.5 us, of 26.2 and 7.1.
+template <bool BONDS, bool ROLL, bool MESH>
+__global__ void __launch_bounds__(kAB) kb_forces(ADev s, ABar B, int gp, const double *x, const float4 *xf,
+                                                 const double *vh, const double *wh, const double *sh_before,
+                                                 const double *bh_before, const double *ws_before, int upd, int seed_w,
+                                                 double seed, const int *tmst, const double *tmsh, const int *tmnp,
+                                                 long long ntimestep, int seed_axis) {
+  __shared__ int q[kAB];
+  __shared__ int wcnt[kAB / 32];
+  if ((int)blockIdx.x < gp)
+    pair_vjp_blocks<BONDS, ROLL>(s, B, blockIdx.x, gp, q, wcnt, x, xf, vh, wh, sh_before, bh_before, upd, ntimestep);
+  else
+    wall_vjp_blocks<ROLL, MESH>(s, B, blockIdx.x - gp, gridDim.x - gp, q, wcnt, x, vh, wh, ws_before, upd, seed_w, seed,
+                                tmst, tmsh, tmnp, ntimestep, seed_axis);
+}
+
+// adds the record of entry p (own: as owner, else as partner) to the sums
+__device__ __forceinline__ void add_record(const double *r, bool own, double xb[3], double vb[3], double wb[3],
+                                           double &rb, double &mb) {
+  const double sg = own ? 1.0 : -1.0;
+  for (int k = 0; k < 3; k++) {
+    xb[k] += sg * r[k];
+    vb[k] += sg * r[3 + k];
+    wb[k] += r[(own ? 6 : 9) + k];
+  }
+  rb += r[own ? 12 : 13];
+  mb += r[own ? 14 : 15];
+}
+
+// per atom: pair adjoints in list order (own row, then reverse list; entries
+// without a law evaluation have none), then the drift x' = x + dt vh and the
+// first half-kick vh = v + a F, wh = w + b T with Fn/Tn the forces at the
+// step's start, and (second) the second half-kick of the step before, which
+// has the same forces; drift = 0 for the setup pass
+__global__ void __launch_bounds__(kAB) kb_gather_kick(ADev s, ABar B, const double *Fn, const double *Tn, int drift,
+                                                      int second) {
   AGRID(i, s.n) {
     double xb[3], vb[3], wb[3], rb = 0.0, mb = 0.0;
     for (int k = 0; k < 3; k++) {
@@ -1427,49 +1558,35 @@ __global__ void kb_gather_kick(ADev s, ABar B, const double *Fn, const double *T
       vb[k] = B.vb[3 * i + k];
       wb[k] = B.wb[3 * i + k];
     }
-    for (int p = s.row[i]; p < s.row[i + 1]; p++) {
-      for (int k = 0; k < 3; k++) {
-        xb[k] += B.pd[3 * p + k];
-        vb[k] += B.pv[3 * p + k];
-        wb[k] += B.pwi[3 * p + k];
-      }
-      rb += B.pri[p];
-      mb += B.pmi[p];
+    const int pb = s.row[i], pe = s.row[i + 1], qb = s.rev_start[i], qe = s.rev_start[i + 1];
+    unsigned mo, mr;
+    if (entry_masks(s, B.pact, false, pb, pe, qb, qe, mo, mr)) {
+      for (; mo; mo &= mo - 1u) add_record(B.rec + (size_t)kARec * (pb + __ffs(mo) - 1), true, xb, vb, wb, rb, mb);
+      for (; mr; mr &= mr - 1u)
+        add_record(B.rec + (size_t)kARec * s.rev[qb + __ffs(mr) - 1], false, xb, vb, wb, rb, mb);
+    } else {
+      for (int p = pb; p < pe; p++)
+        if (B.pact[p]) add_record(B.rec + (size_t)kARec * p, true, xb, vb, wb, rb, mb);
+      for (int q = qb; q < qe; q++)
+        if (B.pact[s.rev[q]]) add_record(B.rec + (size_t)kARec * s.rev[q], false, xb, vb, wb, rb, mb);
     }
-    for (int q = s.rev_start[i]; q < s.rev_start[i + 1]; q++) {
-      const int p = s.rev[q];
-      for (int k = 0; k < 3; k++) {
-        xb[k] -= B.pd[3 * p + k];
-        vb[k] -= B.pv[3 * p + k];
-        wb[k] += B.pwj[3 * p + k];
-      }
-      rb += B.prj[p];
-      mb += B.pmj[p];
-    }
-    if (!drift) {  // setup force pass: adjoints of the initial state
-      for (int k = 0; k < 3; k++) {
-        B.xb[3 * i + k] = xb[k];
-        B.vb[3 * i + k] = vb[k];
-        B.wb[3 * i + k] = wb[k];
-      }
-      B.rb[i] += rb;
-      B.mb[i] += mb;
-      continue;
-    }
-    const double a = s.ka[i], b = s.kb[i];
     double fv = 0.0, tw = 0.0;
     for (int k = 0; k < 3; k++) {
-      vb[k] += s.dt * xb[k];
+      if (drift) vb[k] += s.dt * xb[k];
       B.xb[3 * i + k] = xb[k];
       B.vb[3 * i + k] = vb[k];
       B.wb[3 * i + k] = wb[k];
-      B.Fb[3 * i + k] = a * vb[k];
-      B.Tb[3 * i + k] = b * wb[k];
-      fv += Fn[3 * i + k] * vb[k];
-      tw += Tn[3 * i + k] * wb[k];
+      if (drift) {
+        fv += Fn[3 * i + k] * vb[k];
+        tw += Tn[3 * i + k] * wb[k];
+      }
     }
-    B.rb[i] += rb - s.kbr[i] * tw;
-    B.mb[i] += mb - s.kam[i] * fv - s.kbm[i] * tw;
+    if (drift) {
+      kick_back(s, B, i, vb, wb, true, second != 0, fv, tw, rb, mb);
+    } else {  // setup force pass: adjoints of the initial state
+      B.rb[i] += rb;
+      B.mb[i] += mb;
+    }
   }
 }
 
@@ -1683,6 +1800,7 @@ int build_list(dem_adjoint *h, AList &L, const AList &old, long long step) {
   AGET(h, L.rev, int, np);
   AGET(h, L.carry, int, np);
   AGET(h, L.shear, double, 3 * (size_t)np);
+  AGET(h, L.pc, double, 4 * (size_t)np);
   if (s.bonds) AGET(h, L.bond, double, (size_t)kBondValues * np);
   ka_pairs<true><<<grid_of(n), kAB, 0, st>>>(s, L.pi, L.pj, L.sh, L.row);
   ATRY(h, cudaMemsetAsync(h->rcnt, 0, (n + 1) * sizeof(int), st));
@@ -1716,6 +1834,7 @@ void use_list_on(ADev &s, const AList &L, double *shear, double *bond) {
   s.rev_start = L.rev_start;
   s.rev = L.rev;
   s.shear = shear;
+  s.pc = L.pc;
   s.mcn = L.mcn;
   s.mcand = L.mcand;
 }
@@ -1725,10 +1844,10 @@ void use_list(dem_adjoint *h, const AList &L, double *shear, double *bond) { use
 int ensure_pairs(dem_adjoint *h, int np) {
   if (np <= h->pcap) return DEM_OK;
   const int cap = std::max(np, 1024) + std::max(np, 1024) / 4;
-  double **d3[] = {&h->s.pF, &h->s.pTi, &h->s.pTj, &h->B.pd, &h->B.pv, &h->B.pwi, &h->B.pwj, &h->B.sb};
+  double **d3[] = {&h->s.pF, &h->s.pTi, &h->s.pTj, &h->B.sb};
   for (double **q : d3) ATRY(h, dmalloc(h->owned, q, 3 * (size_t)cap));
-  double **d1[] = {&h->B.pri, &h->B.prj, &h->B.pmi, &h->B.pmj};
-  for (double **q : d1) ATRY(h, dmalloc(h->owned, q, (size_t)cap));
+  ATRY(h, dmalloc(h->owned, &h->B.rec, (size_t)kARec * cap));
+  ATRY(h, dmalloc(h->owned, &h->B.pact, (size_t)cap));
   ATRY(h, dmalloc(h->owned, &h->B.pth, kTh * (size_t)cap));
   if (h->s.bonds) ATRY(h, dmalloc(h->owned, &h->B.bb, (size_t)kBondValues * cap));
   ATRY(h, dmalloc(h->owned, &h->s.active, (size_t)cap));
@@ -1749,26 +1868,32 @@ void derive(double E, double nu, double e, double &Y, double &G, double &beta, d
   dbde = (1.0 / e) * (M_PI * M_PI) / std::pow(lg * lg + M_PI * M_PI, 1.5);
 }
 
+// the instance for the run's bonds, rolling friction and meshes
+#define A_DISPATCH(K)                                                  \
+  do {                                                                 \
+    const int v_ = (s.bonds ? 4 : 0) | (s.rolling ? 2 : 0) | (s.nmeshes ? 1 : 0); \
+    if (v_ == 0) K(false, false, false);                               \
+    else if (v_ == 1) K(false, false, true);                           \
+    else if (v_ == 2) K(false, true, false);                           \
+    else if (v_ == 3) K(false, true, true);                            \
+    else if (v_ == 4) K(true, false, false);                           \
+    else if (v_ == 5) K(true, false, true);                            \
+    else if (v_ == 6) K(true, true, false);                            \
+    else K(true, true, true);                                          \
+  } while (0)
+
 // one force evaluation of state s on stream st
 void force_pass_on(const ADev &s, cudaStream_t st, const double *vh, const double *wh, int upd,
                    long long ntimestep, double *tape_sh, double *tape_bh, double *tape_ws, int final_kick,
                    double *wallF, double *tape_F = nullptr, double *tape_T = nullptr, int *tape_mst = nullptr,
                    double *tape_msh = nullptr, int *tape_mnp = nullptr, NextKick nk = NextKick{}) {
-  const int g = grid_of(s.np), ga = grid_of(s.n);
-  if (s.np > 0) {
-    if (s.bonds && s.rolling) ka_pair_force<true, true><<<g, kAB, 0, st>>>(s, vh, wh, upd, ntimestep, tape_sh, tape_bh);
-    else if (s.bonds) ka_pair_force<true, false><<<g, kAB, 0, st>>>(s, vh, wh, upd, ntimestep, tape_sh, tape_bh);
-    else if (s.rolling) ka_pair_force<false, true><<<g, kAB, 0, st>>>(s, vh, wh, upd, ntimestep, tape_sh, tape_bh);
-    else ka_pair_force<false, false><<<g, kAB, 0, st>>>(s, vh, wh, upd, ntimestep, tape_sh, tape_bh);
-  }
-#define A_GATHER(R, M)                                                                                        \
-  ka_gather<R, M><<<ga, kAB, 0, st>>>(s, vh, wh, upd, final_kick, tape_ws, wallF, tape_F, tape_T, tape_mst, tape_msh, \
-                                      tape_mnp, ntimestep, nk)
-  if (s.rolling && s.nmeshes) A_GATHER(true, true);
-  else if (s.rolling) A_GATHER(true, false);
-  else if (s.nmeshes) A_GATHER(false, true);
-  else A_GATHER(false, false);
-#undef A_GATHER
+  const int gp = s.np > 0 ? grid_of(s.np) : 0, gw = s.nplanes > 0 || s.nmeshes > 0 ? grid_of(s.n) : 0;
+#define A_FORCES(BD, R, M)                                                                                       \
+  ka_forces<BD, R, M><<<gp + gw, kAB, 0, st>>>(s, gp, vh, wh, upd, ntimestep, tape_sh, tape_bh, tape_ws, wallF, \
+                                               tape_mst, tape_msh, tape_mnp)
+  if (gp + gw > 0) A_DISPATCH(A_FORCES);
+#undef A_FORCES
+  ka_gather<<<grid_of(s.n), kAB, 0, st>>>(s, vh, wh, final_kick, tape_F, tape_T, nk);
 }
 
 void force_pass(dem_adjoint *h, const double *vh, const double *wh, int upd, long long ntimestep,
@@ -1779,33 +1904,18 @@ void force_pass(dem_adjoint *h, const double *vh, const double *wh, int upd, lon
                 tape_mst, tape_msh, tape_mnp, nk);
 }
 
-void pairs_vjp(dem_adjoint *h, const double *x, const float4 *xf, const double *vh, const double *wh,
-               const double *sh_before, const double *bh_before, int upd, long long ntimestep) {
+void forces_vjp(dem_adjoint *h, const double *x, const float4 *xf, const double *vh, const double *wh,
+                const double *sh_before, const double *bh_before, const double *ws_before, int upd, int seed_w,
+                double seed, const int *tmst, const double *tmsh, const int *tmnp, long long ntimestep,
+                int seed_axis = -1) {
   const ADev &s = h->s;
-  if (s.np <= 0) return;
-  const int g = grid_of(s.np);
-#define A_PAIRS(BD, R) \
-  kb_pairs<BD, R><<<g, kAB, 0, h->st>>>(s, h->B, x, xf, vh, wh, sh_before, bh_before, upd, ntimestep)
-  if (s.bonds && s.rolling) A_PAIRS(true, true);
-  else if (s.bonds) A_PAIRS(true, false);
-  else if (s.rolling) A_PAIRS(false, true);
-  else A_PAIRS(false, false);
-#undef A_PAIRS
-}
-
-void walls_vjp(dem_adjoint *h, const double *x, const double *vh, const double *wh, const double *ws_before, int upd,
-               int seed_w, double seed, const double *Fn1, const double *Tn1, const int *tmst, const double *tmsh,
-               const int *tmnp, long long ntimestep, int seed_axis = -1) {
-  const ADev &s = h->s;
-  const int g = grid_of(h->n);
-#define A_WALLS(R, M) \
-  kb_walls<R, M><<<g, kAB, 0, h->st>>>(s, h->B, x, vh, wh, ws_before, upd, seed_w, seed, Fn1, Tn1, tmst, tmsh, tmnp, \
-                                       ntimestep, seed_axis)
-  if (s.rolling && s.nmeshes) A_WALLS(true, true);
-  else if (s.rolling) A_WALLS(true, false);
-  else if (s.nmeshes) A_WALLS(false, true);
-  else A_WALLS(false, false);
-#undef A_WALLS
+  const int gp = s.np > 0 ? grid_of(s.np) : 0, gw = s.nplanes > 0 || s.nmeshes > 0 ? grid_of(h->n) : 0;
+  if (gp + gw == 0) return;
+#define A_VJP(BD, R, M)                                                                                             \
+  kb_forces<BD, R, M><<<gp + gw, kAB, 0, h->st>>>(s, h->B, gp, x, xf, vh, wh, sh_before, bh_before, ws_before, upd, \
+                                                  seed_w, seed, tmst, tmsh, tmnp, ntimestep, seed_axis)
+  A_DISPATCH(A_VJP);
+#undef A_VJP
 }
 
 void accumulate(dem_adjoint *h, const double *in, int cnt) {
@@ -2032,6 +2142,9 @@ int dem_adjoint_set_state(dem_adjoint *h, int n, const double *x, const double *
   const size_t W3 = 3 * (size_t)std::max(1, s.nplanes) * n;
   ATRY(h, dmalloc(h->owned, &s.ws, W3));
   ATRY(h, dmalloc(h->owned, &s.xf, (size_t)n));
+  ATRY(h, dmalloc(h->owned, &s.ac, 4 * (size_t)n));
+  ATRY(h, dmalloc(h->owned, &s.wF, 3 * (size_t)n));
+  ATRY(h, dmalloc(h->owned, &s.wT, 3 * (size_t)n));
   // mesh walls: the neighbour cutoff (Neighbor::cutneighmax, (maxrad_i +
   // maxrad_j) cdf + skin) bounds the contacts considered, and static meshes
   // take candidates within r cdf + skin/2 (FixNeighlistMesh::pre_force)
@@ -2106,6 +2219,7 @@ static int adj_run(dem_adjoint *h, double E, double e, double mu, const double *
   s.G = G;
   s.beta = beta;
   s.mu = mu;
+  s.lu = LawUniform{4.0 / 3.0 * Y, 8.0 * G, kLawK * beta, 1.0 / (8.0 * G), 0.5 / Y, 0.5 / G};
   const size_t S3 = 3 * (size_t)n, W3 = 3 * (size_t)std::max(1, s.nplanes) * n;
   ATRY(h, cudaMemcpyAsync(s.r, rr.data(), n * sizeof(double), cudaMemcpyHostToDevice, st));
   ATRY(h, cudaMemcpyAsync(s.m, mm.data(), n * sizeof(double), cudaMemcpyHostToDevice, st));
@@ -2378,6 +2492,8 @@ static int adj_run(dem_adjoint *h, double E, double e, double mu, const double *
     AGET(h, s2.pF, double, 3 * (size_t)maxnp);
     AGET(h, s2.pTi, double, 3 * (size_t)maxnp);
     AGET(h, s2.pTj, double, 3 * (size_t)maxnp);
+    AGET(h, s2.wF, double, S3);
+    AGET(h, s2.wT, double, S3);
     AGET(h, s2.active, uint8_t, (size_t)maxnp);
     if (s.nmeshes) {
       AGET(h, s2.mst, int, NBM * kAMC);
@@ -2477,16 +2593,16 @@ static int adj_run(dem_adjoint *h, double E, double e, double mu, const double *
     for (int t = last; t >= first; t--) {
       const int q = t - first;
       const double *xs = T.x + S3 * q, *vh = T.vh + S3 * q, *wh = T.wh + S3 * q;
-      walls_vjp(h, xs, vh, wh, T.ws + W3 * q, 1, t == nsteps ? lw : -1, t == nsteps ? fw_seed : 0.0, T.F + S3 * q,
-                T.T + S3 * q, s.nmeshes ? T.mst + NBM * kAMC * q : nullptr,
-                s.nmeshes ? T.msh + NBM * kAMC * 3 * q : nullptr, s.nmeshes ? T.mnp + NBM * q : nullptr, t,
-                loss->wall_axis);
-      if (s.np > 0)
-        pairs_vjp(h, xs, T.xf + (size_t)n * q, vh, wh, T.sh + 3 * PS * q,
-                  s.bonds ? T.bh + kBondValues * PS * q : nullptr, 1, t);
       const double *Fn = q > 0 ? T.F + S3 * (q - 1) : c.F;
       const double *Tn = q > 0 ? T.T + S3 * (q - 1) : c.T;
-      kb_gather_kick<<<grid_of(n), kAB, 0, st>>>(s, B, Fn, Tn, 1);
+      if (t == nsteps) kb_last_kick<<<grid_of(n), kAB, 0, st>>>(s, B, T.F + S3 * q, T.T + S3 * q);
+      forces_vjp(h, xs, T.xf + (size_t)n * q, vh, wh, T.sh + 3 * PS * q,
+                 s.bonds ? T.bh + kBondValues * PS * q : nullptr, T.ws + W3 * q, 1, t == nsteps ? lw : -1,
+                 t == nsteps ? fw_seed : 0.0, s.nmeshes ? T.mst + NBM * kAMC * q : nullptr,
+                 s.nmeshes ? T.msh + NBM * kAMC * 3 * q : nullptr, s.nmeshes ? T.mnp + NBM * q : nullptr, t,
+                 loss->wall_axis);
+      // (the step before step 1 is the setup pass, which has no half-kick)
+      kb_gather_kick<<<grid_of(n), kAB, 0, st>>>(s, B, Fn, Tn, 1, t > 1 ? 1 : 0);
     }
     if (k > 0) accumulate(h, B.pth, s.np);  // segment 0: after the setup pass below
     if (k > 0) {  // history adjoints back through the carry at this build
@@ -2515,9 +2631,8 @@ static int adj_run(dem_adjoint *h, double E, double e, double mu, const double *
     ATRY(h, cudaMemsetAsync(shr, 0, 3 * (size_t)maxnp * sizeof(double), st));
     if (s.bonds) ATRY(h, cudaMemsetAsync(bhr, 0, NB * sizeof(double), st));
     use_list(h, c.L, shr, bhr);
-    walls_vjp(h, c.x, c.v, c.w, tws0, 0, -1, 0.0, nullptr, nullptr, mst_e, msh_e, mnp_e, 0);
-    pairs_vjp(h, c.x, nullptr, c.v, c.w, shr, bhr, 0, 0);
-    kb_gather_kick<<<grid_of(n), kAB, 0, st>>>(s, B, nullptr, nullptr, 0);
+    forces_vjp(h, c.x, nullptr, c.v, c.w, shr, bhr, tws0, 0, -1, 0.0, mst_e, msh_e, mnp_e, 0);
+    kb_gather_kick<<<grid_of(n), kAB, 0, st>>>(s, B, nullptr, nullptr, 0, 0);
     accumulate(h, B.pth, s.np);  // segment 0's steps and the setup pass
     accumulate(h, B.wth, n);     // every step's wall contacts
   }
