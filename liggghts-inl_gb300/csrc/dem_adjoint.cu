@@ -154,6 +154,8 @@ struct ADev {
   double csz[3];
   int ncell;
   int *cell_of, *cell_count, *cell_start, *cell_fill, *order, *pcount;
+  int *rowcnt;      // [9*i + row]: entries of a stencil row
+  unsigned *stash;  // [(9*i + row)*kARow + k]: the first of them
   int *err;  // [0]: an atom moved more than skin/2 from its build position; [1]: mesh slots exceeded
   // mesh walls: meshes; FixNeighlistMesh's neighbour threshold (static: skin/2)
   int nmeshes;
@@ -227,6 +229,30 @@ __device__ __forceinline__ int block_queue(bool want, int item, int *q, int *wcn
   return tot;
 }
 
+// The list kernels queue from up to kAChunks runs of kAB entries before they run
+// the law: few entries of a list touch (5 % of the settling columns'), and a
+// block's law takes the same time for one of them as for a whole warp (an FP64
+// instruction holds its pipe for 64 cycles whatever the number of lanes).
+// Sized so that the grid is one wave of two blocks per SM (their registers):
+// 20,000 spheres took 25.5 us per reverse evaluation in two waves of blocks with
+// one run each, and take 17 with two runs a block.
+constexpr int kAChunks = 8;
+constexpr int kAWave = 280;  // list blocks; the rest of the wave is for the walls
+__host__ __device__ __forceinline__ int list_chunks(int np) {
+  const int c = ((np + kAB - 1) / kAB + kAWave - 1) / kAWave;
+  return c < 1 ? 1 : (c > kAChunks ? kAChunks : c);
+}
+
+// appends `item` of the lanes that want it to the block's queue of *cnt entries
+__device__ __forceinline__ void queue_append(bool want, int item, int *q, int *cnt) {
+  const int lane = threadIdx.x & 31;
+  const unsigned m = __ballot_sync(0xffffffffu, want);
+  int at = 0;
+  if (lane == 0 && m) at = atomicAdd(cnt, __popc(m));
+  at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+  if (want) q[at] = item;
+}
+
 // ---------------------------------------------------------------- list build
 // per-atom kick constants of FixNVESphere (src/fix_nve_sphere.cpp:134-244)
 // for the run's radii and masses
@@ -296,16 +322,30 @@ __global__ void ka_cellsort(ADev s) {
 
 // granular half list in input order: local pairs once (owner = lower index),
 // periodic images as directed entries of each owner; cutoff
-// (ri + rj) cdf + skin (src/neigh_gran.cpp:580-586)
-// candidates [qb, qe) of the cell-sorted order (s.order), all with image
-// code `code`
-// A candidate farther in FP32 (the mirror xf, refreshed by every drift and
-// wrap) than the cutoff plus fm, the bound of the mirror's rounding and of
-// this arithmetic, is beyond the exact cutoff too: it skips the FP64 test.
-template <bool FILL>
-__device__ __forceinline__ void ka_scan(const ADev &s, int i, const double xi[3], double ri, float4 fi,
-                                        float cdff, float skinm, int qb, int qe, int code, int &cnt, int &out,
-                                        int out_end, int *pi, int *pj, uint8_t *shc) {
+// (ri + rj) cdf + skin (src/neigh_gran.cpp:580-586).
+//
+// The 27 cells in the stencil's order (z, then y, then x offsets) form nine
+// rows; nine lanes take an atom's rows, three atoms per warp.  Along x the
+// unwrapped cells of a row are consecutive cells, whose atoms form one
+// contiguous run of the cell-sorted order (the same candidates in the same
+// order as cell by cell); a cell that wraps around a periodic x boundary is
+// scanned alone, with its image shift.  A lane loads four candidates at a time
+// (one after the other, and with one thread per atom, the search was a chain
+// of some sixty trips to L2: 38 us for 1,000 spheres and 46 for 20,000, twice per
+// build; now 7.5 and 13 once).  The count pass keeps each row's first kARow
+// entries (partner | image code << 27) for the fill (4 and 6 us).
+constexpr int kARow = 8;
+
+// candidates [qb, qe) of the cell-sorted order (s.order), all with image code
+// `code`; emit(j) for every entry, in order.  A candidate farther in FP32 (the
+// mirror xf, refreshed by every drift and wrap) than the cutoff plus fm, the
+// bound of the mirror's rounding and of this arithmetic, is beyond the exact
+// cutoff too, and one nearer than the cutoff minus fm within it: only the shell
+// between takes the FP64 test (some ten instructions of 64 cycles, for each
+// candidate of a warp on its own: 38 us of 20,000 spheres' search).
+template <class Emit>
+__device__ __forceinline__ void ka_scan(const ADev &s, int i, float4 fi, float cdff, float skinm, int qb, int qe,
+                                        int code, const Emit &emit) {
   float sxf = 0.f, syf = 0.f, szf = 0.f;
   if (code != kNoShift) {
     const int sx = code % 3 - 1, sy = (code / 3) % 3 - 1, sz = code / 9 - 1;
@@ -313,89 +353,113 @@ __device__ __forceinline__ void ka_scan(const ADev &s, int i, const double xi[3]
     syf = sy == 0 ? 0.f : (sy > 0 ? s.prdf[1] : -s.prdf[1]);
     szf = sz == 0 ? 0.f : (sz > 0 ? s.prdf[2] : -s.prdf[2]);
   }
-  for (int q = qb; q < qe; q++) {
-    const int j = s.order[q];
-    if (code == kNoShift && j <= i) continue;
-    const float4 b = s.xf[j];
-    const float fx = fi.x - (b.x + sxf), fy = fi.y - (b.y + syf), fz = fi.z - (b.z + szf);
-    const float rf = (fi.w + b.w) * cdff + skinm;
-    if (fx * fx + fy * fy + fz * fz > rf * rf) continue;
-    double xj[3] = {s.x[3 * j], s.x[3 * j + 1], s.x[3 * j + 2]};
-    a_image(s, code, xj);
-    const double dx = xi[0] - xj[0], dy = xi[1] - xj[1], dz = xi[2] - xj[2];
-    const double cs = (ri + s.r[j]) * s.cdf + s.skin;
-    if (dx * dx + dy * dy + dz * dz > cs * cs) continue;
-    if (!FILL) {
-      cnt++;
-      continue;
+  for (int q0 = qb; q0 < qe; q0 += 4) {
+    int jj[4];
+    float4 b[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) jj[k] = q0 + k < qe ? s.order[q0 + k] : -1;
+#pragma unroll
+    for (int k = 0; k < 4; k++) b[k] = jj[k] >= 0 ? s.xf[jj[k]] : fi;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int j = jj[k];
+      if (j < 0 || (code == kNoShift && j <= i)) continue;
+      const float fx = fi.x - (b[k].x + sxf), fy = fi.y - (b[k].y + syf), fz = fi.z - (b[k].z + szf);
+      const float rf = (fi.w + b[k].w) * cdff + skinm;
+      const float d2 = fx * fx + fy * fy + fz * fz, rl = rf - 2.f * s.fm;
+      if (d2 > rf * rf) continue;
+      if (rl > 0.f && d2 < rl * rl) {
+        emit(j, code);
+        continue;
+      }
+      double xj[3] = {s.x[3 * j], s.x[3 * j + 1], s.x[3 * j + 2]};
+      a_image(s, code, xj);
+      const double dx = s.x[3 * i] - xj[0], dy = s.x[3 * i + 1] - xj[1], dz = s.x[3 * i + 2] - xj[2];
+      const double cs = (s.r[i] + s.r[j]) * s.cdf + s.skin;
+      if (dx * dx + dy * dy + dz * dz > cs * cs) continue;
+      emit(j, code);
     }
-    if (out >= out_end) continue;
+  }
+}
+
+// row r (0..8) of atom i's stencil
+template <class Emit>
+__device__ __forceinline__ void ka_row(const ADev &s, int i, int r, const Emit &emit) {
+  const float cdff = (float)s.cdf, skinm = (float)s.skin + s.fm;
+  const float4 fi = s.xf[i];
+  const int cell = s.cell_of[i];
+  const int ci[3] = {cell % s.nc[0], cell / s.nc[0] % s.nc[1], cell / (s.nc[0] * s.nc[1])};
+  const int off[3] = {0, r % 3 - 1, r / 3 - 1};
+  int at[3] = {ci[0], 0, 0}, sv[3] = {0, 0, 0};
+  for (int d = 1; d < 3; d++) {
+    int c = ci[d] + off[d];
+    if (c < 0 || c >= s.nc[d]) {
+      if (!s.per[d]) return;
+      sv[d] = c < 0 ? -1 : 1;
+      c -= sv[d] * s.nc[d];
+    }
+    at[d] = c;
+  }
+  const int rowb = s.nc[0] * (at[1] + s.nc[1] * at[2]);
+  const int syz = 3 * (sv[1] + 1) + 9 * (sv[2] + 1);
+  const bool left = ci[0] > 0, right = ci[0] < s.nc[0] - 1;
+  if (!left && s.per[0])
+    ka_scan(s, i, fi, cdff, skinm, s.cell_start[rowb + s.nc[0] - 1], s.cell_start[rowb + s.nc[0]], syz, emit);
+  ka_scan(s, i, fi, cdff, skinm, s.cell_start[rowb + ci[0] - (left ? 1 : 0)],
+          s.cell_start[rowb + ci[0] + (right ? 2 : 1)], 1 + syz, emit);
+  if (!right && s.per[0]) ka_scan(s, i, fi, cdff, skinm, s.cell_start[rowb], s.cell_start[rowb + 1], 2 + syz, emit);
+}
+
+// atom and row of this lane; false: none (lanes 27..31, past the last atom)
+__device__ __forceinline__ bool ka_lane(int n, int &i, int &r) {
+  const int lane = threadIdx.x & 31;
+  i = (int)((blockIdx.x * blockDim.x + threadIdx.x) / 32) * 3 + lane / 9;
+  r = lane % 9;
+  return lane < 27 && i < n;
+}
+
+__global__ void ka_pairs_count(ADev s) {
+  int i, r, cnt = 0;
+  const bool on = ka_lane(s.n, i, r);
+  if (on) {
+    unsigned *st = s.stash + ((size_t)9 * i + r) * kARow;
+    ka_row(s, i, r, [&](int j, int code) {
+      if (cnt < kARow) st[cnt] = (unsigned)j | ((unsigned)code << 27);
+      cnt++;
+    });
+    s.rowcnt[(size_t)9 * i + r] = cnt;
+  }
+  const int lane = threadIdx.x & 31, base = lane / 9 * 9;
+  int tot = 0;
+  for (int k = 0; k < 9; k++) tot += __shfl_sync(0xffffffffu, cnt, (base + k) & 31);
+  if (on && r == 0) s.pcount[i] = tot;
+}
+
+__global__ void ka_pairs_fill(ADev s, int *pi, int *pj, uint8_t *shc, const int *row) {
+  int i, r;
+  const bool on = ka_lane(s.n, i, r);
+  const int cnt = on ? s.rowcnt[(size_t)9 * i + r] : 0;
+  const int lane = threadIdx.x & 31, base = lane / 9 * 9;
+  int out = 0;
+  for (int k = 0; k < 8; k++) {
+    const int c = __shfl_sync(0xffffffffu, cnt, (base + k) & 31);
+    if (k < r) out += c;
+  }
+  if (!on || cnt == 0) return;
+  out += row[i];
+  const int end = out + cnt;
+  auto put = [&](int j, int code) {
+    if (out >= end) return;  // (the passes agree)
     pi[out] = i;
     pj[out] = j;
     shc[out] = (uint8_t)code;
     out++;
-  }
-}
-
-// The 27 cells in the stencil's order (z, then y, then x offsets); along x
-// the unwrapped cells of a row are consecutive cells, whose atoms form one
-// contiguous run of the cell-sorted order, scanned in one loop (the same
-// candidates in the same order as cell by cell); a cell that wraps around a
-// periodic x boundary is scanned alone, with its image shift.
-template <bool FILL>
-__global__ void ka_pairs(ADev s, int *pi, int *pj, uint8_t *shc, const int *row) {
-  const float cdff = (float)s.cdf, skinm = (float)s.skin + s.fm;
-  AGRID(i, s.n) {
-    const double xi[3] = {s.x[3 * i], s.x[3 * i + 1], s.x[3 * i + 2]};
-    const double ri = s.r[i];
-    const float4 fi = s.xf[i];
-    int ci[3];
-    for (int d = 0; d < 3; d++) ci[d] = a_cell_coord(s, xi[d], d);
-    int cnt = 0, out = FILL ? row[i] : 0;
-    const int out_end = FILL ? row[i + 1] : 0;
-    int nb[3][3], sv3[3][3];
-    bool ok3[3][3];
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        int cc = ci[d] + k - 1, sv = 0;
-        bool ok = true;
-        if (cc < 0) {
-          ok = s.per[d] != 0;
-          cc += s.nc[d];
-          sv = -1;
-        } else if (cc >= s.nc[d]) {
-          ok = s.per[d] != 0;
-          cc -= s.nc[d];
-          sv = 1;
-        }
-        nb[d][k] = cc;
-        sv3[d][k] = sv;
-        ok3[d][k] = ok;
-      }
-    }
-    const bool lwrap = ok3[0][0] && sv3[0][0] != 0, rwrap = ok3[0][2] && sv3[0][2] != 0;
-    const int x0 = (ok3[0][0] && !lwrap) ? nb[0][0] : nb[0][1];
-    const int x1 = (ok3[0][2] && !rwrap) ? nb[0][2] : nb[0][1];
-#pragma unroll
-    for (int kz = 0; kz < 3; kz++) {
-#pragma unroll
-      for (int ky = 0; ky < 3; ky++) {
-        if (!ok3[2][kz] || !ok3[1][ky]) continue;
-        const int rowb = s.nc[0] * (nb[1][ky] + s.nc[1] * nb[2][kz]);
-        const int syz = 3 * (sv3[1][ky] + 1) + 9 * (sv3[2][kz] + 1);
-        if (lwrap)
-          ka_scan<FILL>(s, i, xi, ri, fi, cdff, skinm, s.cell_start[rowb + nb[0][0]],
-                        s.cell_start[rowb + nb[0][0] + 1], syz, cnt, out, out_end, pi, pj, shc);
-        ka_scan<FILL>(s, i, xi, ri, fi, cdff, skinm, s.cell_start[rowb + x0], s.cell_start[rowb + x1 + 1],
-                      1 + syz, cnt, out, out_end, pi, pj, shc);
-        if (rwrap)
-          ka_scan<FILL>(s, i, xi, ri, fi, cdff, skinm, s.cell_start[rowb + nb[0][2]],
-                        s.cell_start[rowb + nb[0][2] + 1], 2 + syz, cnt, out, out_end, pi, pj, shc);
-      }
-    }
-    if (!FILL) s.pcount[i] = cnt;
+  };
+  if (cnt <= kARow && s.n <= 1 << 27) {  // (an atom's index has 27 bits in a stashed entry)
+    const unsigned *st = s.stash + ((size_t)9 * i + r) * kARow;
+    for (int k = 0; k < cnt; k++) put(st[k] & 0x7ffffffu, st[k] >> 27);
+  } else {
+    ka_row(s, i, r, put);
   }
 }
 
@@ -983,21 +1047,28 @@ template <bool BONDS, bool ROLL>
 __device__ __forceinline__ void pair_blocks(const ADev &s, int block, int blocks, int *q, int *wcnt, const double *vh,
                                             const double *wh, int upd, long long ntimestep, double *tape_sh,
                                             double *tape_bh) {
-  for (int base = block * kAB; base < s.np; base += blocks * kAB) {
-    const int p0 = base + threadIdx.x;
-    bool work = false;
-    if (p0 < s.np) {  // tape and the FP32 candidate test; the rest runs queued
-      if (tape_sh)
-        for (int k = 0; k < 3; k++) tape_sh[3 * p0 + k] = s.shear[3 * p0 + k];
-      if (BONDS && tape_bh)
-        for (int k = 0; k < kBondValues; k++)
-          tape_bh[(size_t)kBondValues * p0 + k] = s.bh[(size_t)kBondValues * p0 + k];
-      work = pair_candidate(s, s.xf, p0);
-      if (!work) s.active[p0] = 0;  // beyond the contact distance: nothing changes
+  const int chunks = list_chunks(s.np);
+  for (long base = (long)block * chunks * kAB; base < s.np; base += (long)blocks * chunks * kAB) {
+    if (threadIdx.x == 0) wcnt[0] = 0;
+    __syncthreads();
+    for (int c = 0; c < chunks; c++) {
+      const int p0 = (int)min(base + c * kAB + threadIdx.x, (long)s.np);
+      bool work = false;
+      if (p0 < s.np) {  // tape and the FP32 candidate test; the rest runs queued
+        if (tape_sh)
+          for (int k = 0; k < 3; k++) tape_sh[3 * p0 + k] = s.shear[3 * p0 + k];
+        if (BONDS && tape_bh)
+          for (int k = 0; k < kBondValues; k++)
+            tape_bh[(size_t)kBondValues * p0 + k] = s.bh[(size_t)kBondValues * p0 + k];
+        work = pair_candidate(s, s.xf, p0);
+        if (!work) s.active[p0] = 0;  // beyond the contact distance: nothing changes
+      }
+      queue_append(work, p0, q, wcnt);
     }
-    const int tot = block_queue(work, p0, q, wcnt);
-    if (threadIdx.x < tot) {
-      const int p = q[threadIdx.x];
+    __syncthreads();
+    const int tot = wcnt[0];
+    for (int qi = threadIdx.x; qi < tot; qi += kAB) {
+      const int p = q[qi];
       VjpIn a = pair_in(s, s.x, p, vh, wh, s.shear);
       a.upd = upd != 0;
       const bool touch = pair_touch(a), band = pair_band(s, a);
@@ -1107,15 +1178,14 @@ __device__ __forceinline__ void wall_blocks(const ADev &s, int block, int blocks
 
 // Pair and wall forces of one evaluation, side by side: the first gp blocks
 // take the list, the others (none without walls) the atoms' walls.  Both are
-// chains of FP64 instructions on few warps, so that side by side costs the
-// longer of the two (1,000 settling spheres: 8.4 us an evaluation, and 7.9 for
-// the gather; pairs alone and walls with the gather took 11.2 and 13.2).
+// chains of FP64 instructions on few warps; one after the other, in two
+// launches, they took twice as long.
 template <bool BONDS, bool ROLL, bool MESH>
 __global__ void __launch_bounds__(kAB) ka_forces(ADev s, int gp, const double *vh, const double *wh, int upd,
                                                  long long ntimestep, double *tape_sh, double *tape_bh,
                                                  double *tape_ws, double *wallF, int *tape_mst, double *tape_msh,
                                                  int *tape_mnp) {
-  __shared__ int q[kAB];
+  __shared__ int q[kAB * kAChunks];
   __shared__ int wcnt[kAB / 32];
   __shared__ double sF[3][kAB], sT[3][kAB];
   if ((int)blockIdx.x < gp)
@@ -1250,6 +1320,20 @@ __global__ void __launch_bounds__(kAB) ka_gather(ADev s, const double *vh, const
       if (dsq > 0.25 * s.skin * s.skin) s.err[0] = 1;
     }
   }
+}
+
+// the state before a segment's first drift, into its checkpoint
+__global__ void ka_checkpoint(ADev s, size_t n3, size_t nw, double *x, double *v, double *w, double *F, double *T,
+                              double *ws) {
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n3; q += stride) {
+    x[q] = s.x[q];
+    v[q] = s.v[q];
+    w[q] = s.w[q];
+    F[q] = s.F[q];
+    T[q] = s.T[q];
+  }
+  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < nw; q += stride) ws[q] = s.ws[q];
 }
 
 // first half-kick and drift (v, w then hold vh, wh); xref: positions at the
@@ -1411,27 +1495,34 @@ __device__ __forceinline__ void pair_vjp_blocks(const ADev &s, const ABar &B, in
                                                 const double *x, const float4 *xf, const double *vh, const double *wh,
                                                 const double *sh_before, const double *bh_before, int upd,
                                                 long long ntimestep) {
-  for (int base = block * kAB; base < s.np; base += blocks * kAB) {
-    const int p0 = base + threadIdx.x;
-    bool work = false;
-    if (p0 < s.np) {  // entries without a law evaluation: no input adjoints
-      bool band = false;
-      if (xf) {  // FP32 candidate test (beyond it: not touching, not in the band)
-        work = pair_candidate(s, xf, p0);
-      } else {
-        const VjpIn a = pair_in(s, x, p0, vh, wh, sh_before);
-        const bool touch = pair_touch(a);
-        band = pair_band(s, a);
-        work = touch || (BONDS && band);
+  const int chunks = list_chunks(s.np);
+  for (long base = (long)block * chunks * kAB; base < s.np; base += (long)blocks * chunks * kAB) {
+    if (threadIdx.x == 0) wcnt[0] = 0;
+    __syncthreads();
+    for (int c = 0; c < chunks; c++) {
+      const int p0 = (int)min(base + c * kAB + threadIdx.x, (long)s.np);
+      bool work = false;
+      if (p0 < s.np) {  // entries without a law evaluation: no input adjoints
+        bool band = false;
+        if (xf) {  // FP32 candidate test (beyond it: not touching, not in the band)
+          work = pair_candidate(s, xf, p0);
+        } else {
+          const VjpIn a = pair_in(s, x, p0, vh, wh, sh_before);
+          const bool touch = pair_touch(a);
+          band = pair_band(s, a);
+          work = touch || (BONDS && band);
+        }
+        B.pact[p0] = work ? 1 : 0;
+        if (!work && band)
+          for (int k = 0; k < 3; k++) B.sb[3 * p0 + k] = 0.0;  // history cleared: no dependence
+        // (else: history unchanged, its adjoint passes through)
       }
-      B.pact[p0] = work ? 1 : 0;
-      if (!work && band)
-        for (int k = 0; k < 3; k++) B.sb[3 * p0 + k] = 0.0;  // history cleared: no dependence
-      // (else: history unchanged, its adjoint passes through)
+      queue_append(work, p0, q, wcnt);
     }
-    const int tot = block_queue(work, p0, q, wcnt);
-    if (threadIdx.x < tot) {
-      const int p = q[threadIdx.x];
+    __syncthreads();
+    const int tot = wcnt[0];
+    for (int qi = threadIdx.x; qi < tot; qi += kAB) {
+      const int p = q[qi];
       VjpIn a = pair_in(s, x, p, vh, wh, sh_before);
       a.upd = upd != 0;
       const int i = s.pi[p], j = s.pj[p];
@@ -1512,17 +1603,14 @@ __device__ __forceinline__ void pair_vjp_blocks(const ADev &s, const ABar &B, in
   }
 }
 
-// pairs and walls of one evaluation, side by side as in ka_forces: bound by the
-// length of the law's FP64 chain (64 cycles an instruction), so every division
-// and root that the law shares or inverts counts.  1,000 spheres: 12.9 us where
-// two launches took 20.2 and 6.7; 20,000: 25.5 us, of 26.2 and 7.1.
+// pairs and walls of one evaluation, side by side as in ka_forces
 template <bool BONDS, bool ROLL, bool MESH>
 __global__ void __launch_bounds__(kAB) kb_forces(ADev s, ABar B, int gp, const double *x, const float4 *xf,
                                                  const double *vh, const double *wh, const double *sh_before,
                                                  const double *bh_before, const double *ws_before, int upd, int seed_w,
                                                  double seed, const int *tmst, const double *tmsh, const int *tmnp,
                                                  long long ntimestep, int seed_axis) {
-  __shared__ int q[kAB];
+  __shared__ int q[kAB * kAChunks];
   __shared__ int wcnt[kAB / 32];
   if ((int)blockIdx.x < gp)
     pair_vjp_blocks<BONDS, ROLL>(s, B, blockIdx.x, gp, q, wcnt, x, xf, vh, wh, sh_before, bh_before, upd, ntimestep);
@@ -1610,7 +1698,15 @@ __global__ void kb_reduce_th(const double *in, int cnt, double *part) {
 __global__ void kb_accum_th(const double *part, int nb, double *acc) {
   if (threadIdx.x >= kTh) return;
   double v = acc[threadIdx.x];
-  for (int b = 0; b < nb; b++) v += part[kTh * b + threadIdx.x];
+  int b = 0;
+  for (; b + 16 <= nb; b += 16) {  // loads side by side, sums in order
+    double w[16];
+#pragma unroll
+    for (int k = 0; k < 16; k++) w[k] = part[kTh * (b + k) + threadIdx.x];
+#pragma unroll
+    for (int k = 0; k < 16; k++) v += w[k];
+  }
+  for (; b < nb; b++) v += part[kTh * b + threadIdx.x];
   acc[threadIdx.x] = v;
 }
 
@@ -1778,14 +1874,13 @@ int build_list(dem_adjoint *h, AList &L, const AList &old, long long step) {
   ADev &s = h->s;
   const int n = h->n;
   const cudaStream_t st = h->st;
-  ATRY(h, cudaMemsetAsync(s.cell_count, 0, (s.ncell + 2) * sizeof(int), st));
-  ATRY(h, cudaMemsetAsync(s.cell_fill, 0, (s.ncell + 2) * sizeof(int), st));
+  ATRY(h, cudaMemsetAsync(s.cell_count, 0, 2 * ((size_t)s.ncell + 2) * sizeof(int), st));  // and cell_fill
   ka_cell<<<grid_of(n), kAB, 0, st>>>(s);
   scan_exclusive(h->nosys, s.cell_count, s.cell_start, s.ncell + 1, h->scan_tmp, false, st);
   ka_scatter<<<grid_of(n), kAB, 0, st>>>(s);
   ka_cellsort<<<grid_of(s.ncell), kAB, 0, st>>>(s);
-  ka_pairs<false><<<grid_of(n), kAB, 0, st>>>(s, nullptr, nullptr, nullptr, nullptr);
-  ATRY(h, cudaMemsetAsync(s.pcount + n, 0, sizeof(int), st));
+  const int gr = (int)((((long)n + 2) / 3 * 32 + kAB - 1) / kAB);  // nine lanes per atom, three atoms per warp
+  ka_pairs_count<<<gr, kAB, 0, st>>>(s);
   AGET(h, L.row, int, n + 1);
   scan_exclusive(h->nosys, s.pcount, L.row, n + 1, h->scan_tmp, false, st);
   int np = 0;
@@ -1802,9 +1897,8 @@ int build_list(dem_adjoint *h, AList &L, const AList &old, long long step) {
   AGET(h, L.shear, double, 3 * (size_t)np);
   AGET(h, L.pc, double, 4 * (size_t)np);
   if (s.bonds) AGET(h, L.bond, double, (size_t)kBondValues * np);
-  ka_pairs<true><<<grid_of(n), kAB, 0, st>>>(s, L.pi, L.pj, L.sh, L.row);
-  ATRY(h, cudaMemsetAsync(h->rcnt, 0, (n + 1) * sizeof(int), st));
-  ATRY(h, cudaMemsetAsync(h->rfill, 0, (n + 1) * sizeof(int), st));
+  ka_pairs_fill<<<gr, kAB, 0, st>>>(s, L.pi, L.pj, L.sh, L.row);
+  ATRY(h, cudaMemsetAsync(h->rcnt, 0, 2 * ((size_t)n + 1) * sizeof(int), st));  // and rfill
   if (np > 0) ka_rev_count<<<grid_of(np), kAB, 0, st>>>(np, L.pj, h->rcnt);
   scan_exclusive(h->nosys, h->rcnt, L.rev_start, n + 1, h->scan_tmp, false, st);
   if (np > 0) {
@@ -1887,7 +1981,8 @@ void force_pass_on(const ADev &s, cudaStream_t st, const double *vh, const doubl
                    long long ntimestep, double *tape_sh, double *tape_bh, double *tape_ws, int final_kick,
                    double *wallF, double *tape_F = nullptr, double *tape_T = nullptr, int *tape_mst = nullptr,
                    double *tape_msh = nullptr, int *tape_mnp = nullptr, NextKick nk = NextKick{}) {
-  const int gp = s.np > 0 ? grid_of(s.np) : 0, gw = s.nplanes > 0 || s.nmeshes > 0 ? grid_of(s.n) : 0;
+  const int gp = s.np > 0 ? grid_of((s.np + list_chunks(s.np) - 1) / list_chunks(s.np)) : 0;
+  const int gw = s.nplanes > 0 || s.nmeshes > 0 ? grid_of(s.n) : 0;
 #define A_FORCES(BD, R, M)                                                                                       \
   ka_forces<BD, R, M><<<gp + gw, kAB, 0, st>>>(s, gp, vh, wh, upd, ntimestep, tape_sh, tape_bh, tape_ws, wallF, \
                                                tape_mst, tape_msh, tape_mnp)
@@ -1909,7 +2004,8 @@ void forces_vjp(dem_adjoint *h, const double *x, const float4 *xf, const double 
                 double seed, const int *tmst, const double *tmsh, const int *tmnp, long long ntimestep,
                 int seed_axis = -1) {
   const ADev &s = h->s;
-  const int gp = s.np > 0 ? grid_of(s.np) : 0, gw = s.nplanes > 0 || s.nmeshes > 0 ? grid_of(h->n) : 0;
+  const int gp = s.np > 0 ? grid_of((s.np + list_chunks(s.np) - 1) / list_chunks(s.np)) : 0;
+  const int gw = s.nplanes > 0 || s.nmeshes > 0 ? grid_of(h->n) : 0;
   if (gp + gw == 0) return;
 #define A_VJP(BD, R, M)                                                                                             \
   kb_forces<BD, R, M><<<gp + gw, kAB, 0, h->st>>>(s, h->B, gp, x, xf, vh, wh, sh_before, bh_before, ws_before, upd, \
@@ -2174,13 +2270,16 @@ int dem_adjoint_set_state(dem_adjoint *h, int n, const double *x, const double *
   ATRY(h, dmalloc(h->owned, &h->B.th, kTh));
   ATRY(h, dmalloc(h->owned, &h->part, kTh * (size_t)kMaxGrid));
   ATRY(h, dmalloc(h->owned, &s.cell_of, (size_t)n));
-  ATRY(h, dmalloc(h->owned, &s.cell_count, (size_t)ncell + 2));
+  ATRY(h, dmalloc(h->owned, &s.cell_count, 2 * ((size_t)ncell + 2)));
+  s.cell_fill = s.cell_count + ncell + 2;
   ATRY(h, dmalloc(h->owned, &s.cell_start, (size_t)ncell + 2));
-  ATRY(h, dmalloc(h->owned, &s.cell_fill, (size_t)ncell + 2));
   ATRY(h, dmalloc(h->owned, &s.order, (size_t)n));
   ATRY(h, dmalloc(h->owned, &s.pcount, (size_t)n + 1));
-  ATRY(h, dmalloc(h->owned, &h->rcnt, (size_t)n + 1));
-  ATRY(h, dmalloc(h->owned, &h->rfill, (size_t)n + 1));
+  ATRY(h, cudaMemset(s.pcount, 0, ((size_t)n + 1) * sizeof(int)));
+  ATRY(h, dmalloc(h->owned, &s.rowcnt, 9 * (size_t)n));
+  ATRY(h, dmalloc(h->owned, &s.stash, 9 * (size_t)kARow * n));
+  ATRY(h, dmalloc(h->owned, &h->rcnt, 2 * ((size_t)n + 1)));
+  h->rfill = h->rcnt + n + 1;
   ATRY(h, dmalloc(h->owned, &s.err, 4));
   const long maxlen = std::max<long>(n + 1, ncell + 2);
   ATRY(h, dmalloc(h->owned, &h->scan_tmp, (size_t)((maxlen + 4095) / 4096 + 2)));
@@ -2311,12 +2410,8 @@ static int adj_run(dem_adjoint *h, double E, double e, double mu, const double *
         AGET(h, T.mnp, int, NBM * nst);
       }
     }
-    copyd(h, c.x, s.x, S3);
-    copyd(h, c.v, s.v, S3);
-    copyd(h, c.w, s.w, S3);
-    copyd(h, c.F, s.F, S3);
-    copyd(h, c.T, s.T, S3);
-    copyd(h, c.ws, s.ws, W3);
+    ka_checkpoint<<<grid_of((long)std::max(S3, W3)), kAB, 0, st>>>(s, S3, s.nplanes ? W3 : 0, c.x, c.v, c.w, c.F, c.T,
+                                                                   c.ws);
     for (int t = first; t <= last; t++) {
       const bool build = (k > 0 && t == first);
       const int q = t - first;
