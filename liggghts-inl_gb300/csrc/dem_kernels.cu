@@ -1497,7 +1497,6 @@ __global__ void __launch_bounds__(kParticleMaxThreads, 4) k_particle(Sys s, Loop
   if (particle_halted(c, lp)) return;
   const int n = c->n;
   bool moved = false, bad = false;
-  if (GATHER) particle_clear(sm);
   for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     const int i = base + threadIdx.x;
     particle_tile(s, sm, i, i < n, GATHER, FINAL, INITIAL, moved, bad);
@@ -1515,7 +1514,6 @@ __global__ void __launch_bounds__(kParticleMaxThreads, 4) k_particle_start(Sys s
   const int n = c->n;
   const bool gather = c->step_phase != kStepFirst;
   bool moved = false, bad = false;
-  particle_clear(sm);
   for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     const int i = base + threadIdx.x;
     particle_tile(s, sm, i, i < n, gather, gather, true, moved, bad);

@@ -1160,9 +1160,7 @@ __device__ __forceinline__ void wall_tile(const Sys &s, const AtomArrays &A, int
 // as bit masks (gather_masks); one loop over the set bits then does the FP64
 // additions (gather_sum).  A reverse contribution adds the negated force
 // (sign bit flipped on the integer pipe: a + (-b) is exactly a - b) and Tj
-// instead of Ti.  k_particle hands the loops of a block's atoms to its
-// threads sorted by contact count, so that a warp's lanes run loops of equal
-// length (see there).
+// instead of Ti.  (particle_tile spreads the components over the lanes.)
 template <int GROUP>
 __device__ __forceinline__ bool gather_masks(const Sys &s, const PairArrays &L, int i, int &pb, int &rb,
                                              unsigned &om, unsigned &rm) {
@@ -1212,9 +1210,8 @@ __device__ __forceinline__ const double *gather_next(const Sys &s, const PairArr
   return s.res + (size_t)kResStride * p;
 }
 
-// AHEAD: the next record is loaded while this one is added (a record's loads
-// take twice as long as its six additions; six doubles more in registers)
-template <bool AHEAD>
+// the next record is loaded while this one is added (a record's loads take
+// twice as long as its six additions)
 __device__ __forceinline__ void gather_sum(const Sys &s, const PairArrays &L, int pb, int rb, unsigned om,
                                            unsigned rm, double &fx, double &fy, double &fz, double &tx, double &ty,
                                            double &tz) {
@@ -1222,7 +1219,7 @@ __device__ __forceinline__ void gather_sum(const Sys &s, const PairArrays &L, in
   unsigned long long sg = 0ull;
   int to = 3;
   double r[6];
-  if (AHEAD && cnt > 0) {
+  if (cnt > 0) {
     const double *q = gather_next(s, L, pb, rb, om, rm, sg, to);
     for (int k = 0; k < 3; k++) {
       r[k] = q[k];
@@ -1231,28 +1228,25 @@ __device__ __forceinline__ void gather_sum(const Sys &s, const PairArrays &L, in
   }
   for (int t = 0; t < cnt; t++) {
     double n[6];
-    const unsigned long long sc = sg;
-    if (AHEAD ? t + 1 < cnt : true) {
+    const unsigned long long su = sg;
+    if (t + 1 < cnt) {
       const double *q = gather_next(s, L, pb, rb, om, rm, sg, to);
       for (int k = 0; k < 3; k++) {
         n[k] = q[k];
         n[3 + k] = q[to + k];
       }
     }
-    const unsigned long long su = AHEAD ? sc : sg;
-    const double *u = AHEAD ? r : n;
-    fx += __longlong_as_double(__double_as_longlong(u[0]) ^ su);
-    fy += __longlong_as_double(__double_as_longlong(u[1]) ^ su);
-    fz += __longlong_as_double(__double_as_longlong(u[2]) ^ su);
-    tx += u[3];
-    ty += u[4];
-    tz += u[5];
-    if (AHEAD)
-      for (int k = 0; k < 6; k++) r[k] = n[k];
+    fx += __longlong_as_double(__double_as_longlong(r[0]) ^ su);
+    fy += __longlong_as_double(__double_as_longlong(r[1]) ^ su);
+    fz += __longlong_as_double(__double_as_longlong(r[2]) ^ su);
+    tx += r[3];
+    ty += r[4];
+    tz += r[5];
+    for (int k = 0; k < 6; k++) r[k] = n[k];
   }
 }
 
-// lists longer than 32 entries: one pass over every entry
+// lists that fit neither form: one pass over every entry
 __device__ __forceinline__ void gather_long(const Sys &s, const PairArrays &L, int i, double &fx, double &fy,
                                             double &fz, double &tx, double &ty, double &tz) {
   const int pb = L.row[i], pe = row_end(s, L, i);
@@ -1272,29 +1266,137 @@ __device__ __forceinline__ void gather_long(const Sys &s, const PairArrays &L, i
   }
 }
 
-// the block-level sort of k_particle's gather: loops of up to kGatherKeys-1
-// contacts by count, longer ones together in the last key
-constexpr int kGatherKeys = 32;
+// shared memory of particle_tile's gather, per warp: the atoms' contacts (own
+// entries from the front, the partner list's from the back), their sums, and
+// the atoms in the order of their contact counts
+constexpr int kGatherList = 16;
+constexpr int kGatherBatch = 4;  // records in flight per lane
+constexpr int kGatherSum = 7;  // doubles per atom: six and one that spreads the banks
 constexpr int kParticleMaxThreads = 256;
-
-// shared memory of particle_tile's sorted gather (counts and fills cleared
-// before a block's first tile, left cleared by every tile)
 template <int T>
 struct ParticleShared {
-  double gsum[6][T];
-  int gpb[T], grb[T];
-  unsigned gom[T], grm[T];
-  short gsorted[T];
-  int gcount[kGatherKeys], gfill[kGatherKeys], gstart[kGatherKeys], gnq;
+  int list[T / 32][kGatherList][32];
+  double sum[T / 32][32 * kGatherSum];
+  unsigned char order[T / 32][32];
 };
 
-template <int T>
-__device__ __forceinline__ void particle_clear(ParticleShared<T> &sm) {
-  if (threadIdx.x < kGatherKeys) {
-    sm.gcount[threadIdx.x] = 0;
-    sm.gfill[threadIdx.x] = 0;
+// the active entries of atom i into `list` (this lane's column, see above):
+// own count | total << 8, or -1 when they do not fit
+__device__ __forceinline__ int gather_list(const Sys &s, const PairArrays &L, int i, int (*list)[32], int lane) {
+  constexpr int kGroup = 4;
+  const int pb = L.row[i], rb = L.rev_start[i];
+  const int no = row_end(s, L, i) - pb, nr = rev_end(s, L, i) - rb;
+  int co = 0, cr = 0;
+  // the flags in groups of loads that do not wait for one another
+  for (int k0 = 0; k0 < max(no, nr); k0 += kGroup) {
+    int e[kGroup];
+    uint8_t ao[kGroup], ar[kGroup];
+#pragma unroll
+    for (int k = 0; k < kGroup; k++) {
+      e[k] = k0 + k < nr ? L.rev[rb + k0 + k] : -1;
+      ao[k] = k0 + k < no ? s.active[pb + k0 + k] : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < kGroup; k++) ar[k] = e[k] >= 0 ? s.active[e[k]] : 0;
+#pragma unroll
+    for (int k = 0; k < kGroup; k++) {
+      if (ao[k]) {
+        if (co + cr == kGatherList) return -1;
+        list[co++][lane] = pb + k0 + k;
+      }
+      if (ar[k]) {
+        if (co + cr == kGatherList) return -1;
+        list[kGatherList - 1 - cr++][lane] = e[k];
+      }
+    }
   }
-  __syncthreads();
+  return co | (co + cr) << 8;
+}
+
+// v += r where the program says so: left to itself the compiler adds first and
+// selects the result after, and an addition that is not needed holds the FP64
+// pipe as long as one that is
+__device__ __forceinline__ void add_now(double &v, double r) {
+  asm volatile("add.rn.f64 %0, %0, %1;" : "+d"(v) : "d"(r));
+}
+
+// the sums of a warp's atoms over their lists, started from and left in `sum`;
+// cnt: gather_list's result of this lane's atom
+__device__ __forceinline__ void gather_warp(const Sys &s, const int (*list)[32], double *sum, unsigned char *order,
+                                            int cnt, int lane) {
+  const int key = cnt < 0 ? 0 : cnt >> 8;
+  const int top = __reduce_max_sync(0xffffffffu, key);
+  if (top == 0) return;
+  unsigned more = 0u, same = 0u;  // lanes with a larger, with the same count
+  int nq = 0;
+  for (int k = 1; k <= top; k++) {
+    const unsigned b = __ballot_sync(0xffffffffu, key >= k);
+    if (k == 1) nq = __popc(b);
+    if (k == key) same = b;
+    if (k == key + 1) more = b;
+  }
+  if (key) order[__popc(more) + __popc(same & ~more & ((1u << lane) - 1u))] = (unsigned char)lane;
+  __syncwarp();
+  // one batch of records is loaded while the one before it is added
+  const int slot = lane / 6, comp = lane % 6;
+  // of a partner's entry the negated force, the other torque
+  const int torque = comp < 3 ? 0 : 3, flip = comp < 3 ? (int)0x80000000 : 0;
+  int a = 0, co = 0, n = 0, m = 0;  // the atom, its own count and total, the group's largest total
+  auto group = [&](int g) {
+    const bool on = lane < 30 && g + slot < nq;
+    a = on ? order[g + slot] : 0;
+    const int ca = __shfl_sync(0xffffffffu, cnt, a);
+    co = ca & 0xff;
+    n = on ? ca >> 8 : 0;
+    m = __shfl_sync(0xffffffffu, n, 0);
+  };
+  auto load = [&](double (&r)[kGatherBatch], int k0) {
+#pragma unroll
+    for (int k = 0; k < kGatherBatch; k++) {
+      const int t = k0 + k;
+      r[k] = -0.0;  // changes no sum
+      if (t < n) {
+        const bool own = t < co;
+        const int p = list[own ? t : kGatherList - 1 - (t - co)][a];
+        const double x = s.res[(size_t)kResStride * p + comp + (own ? 0 : torque)];
+        // (a constant sign bit would become a negation, which issues on the FP64 pipe)
+        r[k] = __hiloint2double(__double2hiint(x) ^ (own ? 0 : flip), __double2loint(x));
+      }
+    }
+  };
+  int g = 0, k0 = 0;
+  double r[kGatherBatch];
+  group(0);
+  load(r, 0);
+  double v = sum[a * kGatherSum + comp];
+  while (g < nq) {
+    const int left = m - k0, ga = a, gn = n;
+    const bool done = left <= kGatherBatch;
+    double q[kGatherBatch];
+    if (!done) {
+      k0 += kGatherBatch;
+      load(q, k0);
+    } else {
+      g += 5;
+      k0 = 0;
+      if (g < nq) {
+        group(g);
+        load(q, 0);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kGatherBatch; k++) {
+      if (k >= left) break;
+      add_now(v, r[k]);
+    }
+    if (done) {
+      if (gn) sum[ga * kGatherSum + comp] = v;
+      if (g < nq) v = sum[a * kGatherSum + comp];
+    }
+#pragma unroll
+    for (int k = 0; k < kGatherBatch; k++) r[k] = q[k];
+  }
+  __syncwarp();
 }
 
 // 2x of a normal double below the top of the range, by its exponent (exact;
@@ -1399,83 +1501,47 @@ __device__ __forceinline__ void particle_finish(const Sys &s, int i, bool gather
 }
 
 // Per atom: force gather, gravity, wall totals, nve/sphere, FP32 copy,
-// displacement check.  The gather runs in three block-wide phases, because a
-// warp's contact loops issue their FP64 additions once per contact of its
-// busiest atom: (1) every thread forms its atom's start sums (gravity) and
-// contact masks; (2) the atoms with contacts are sorted by their contact
-// count in shared memory; (3) thread t runs the loop of the t-th atom in that
-// order, so that a warp's lanes run loops of equal length, and the sums go
-// back to the owner.  Each atom's sum keeps its order and its one thread, so
-// the result does not depend on the sort or the launch shape.
-// Called by all threads of a block, thread tid with atom i (valid or none).
+// displacement check.  The FP64 pipe issues per warp instruction, so that a
+// gather with one lane per atom costs six additions per contact of the warp's
+// busiest atom.  Here a lane adds one of the six components of one atom: five
+// atoms at a time, taken in the order of their contact counts, so that the
+// lanes of a warp run loops of nearly equal length and a record is read by
+// neighbouring lanes.  Warps work on their own: they reach the FP64 pipe at
+// different times.  Each sum keeps its order, so the result does not depend on
+// any of this.  Bound by the FP64 pipe (55 % busy) and the latency of its four
+// dependent loads; measured against one lane per atom sorted over a block of
+// 256 (pipe 42-50 % busy, its warps all waiting for the same phase): 1,000,000
+// atoms in a hopper 101 -> 77 us, 400,000 packed 81 -> 71, 526,000 of an
+// ensemble 46 -> 39.  More blocks per SM (48 registers), larger batches and
+// prefetches of the atom's state were slower.
+// Called by all lanes of a warp, each with its atom i (valid or none).
 template <int T>
 __device__ __forceinline__ void particle_tile(const Sys &s, ParticleShared<T> &sm, int i, bool valid, bool gather,
                                               bool final, bool initial, bool &moved, bool &bad) {
   const AtomArrays &A = s.atoms[0];
   const PairArrays &L = s.pairs[0];
-  const int tid = threadIdx.x;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   double fx = 0.0, fy = 0.0, fz = 0.0, tx = 0.0, ty = 0.0, tz = 0.0;
-  double v[3] = {0.0, 0.0, 0.0}, om[3] = {0.0, 0.0, 0.0}, xv[3] = {0.0, 0.0, 0.0};
-  if (valid) {
-    v[0] = A.vx[i]; v[1] = A.vy[i]; v[2] = A.vz[i];
-    om[0] = A.wx[i]; om[1] = A.wy[i]; om[2] = A.wz[i];
-    xv[0] = A.x[i]; xv[1] = A.y[i]; xv[2] = A.z[i];
-  }
   if (gather) {
     if (valid && s.gravity_on) gravity_force(s, A.m[i], fx, fy, fz);
-    // (1) masks and counts; lists longer than 32 entries are summed here
-    // by the owner (sm.gcount and sm.gfill are zero: cleared after the last use)
-    int key = 0;
-    if (valid) {
-      int pb, rb;
-      unsigned mo, mr;
-      if (gather_masks<4>(s, L, i, pb, rb, mo, mr)) {
-        const int cnt = __popc(mo) + __popc(mr);
-        if (cnt) {
-          key = cnt < kGatherKeys ? cnt : kGatherKeys - 1;
-          sm.gpb[tid] = pb;
-          sm.grb[tid] = rb;
-          sm.gom[tid] = mo;
-          sm.grm[tid] = mr;
-          sm.gsum[0][tid] = fx; sm.gsum[1][tid] = fy; sm.gsum[2][tid] = fz;
-          sm.gsum[3][tid] = tx; sm.gsum[4][tid] = ty; sm.gsum[5][tid] = tz;
-        }
-      } else {
-        gather_long(s, L, i, fx, fy, fz, tx, ty, tz);
-      }
+    const int cnt = valid ? gather_list(s, L, i, sm.list[w], lane) : 0;
+    double *sum = &sm.sum[w][lane * kGatherSum];
+    if (cnt > 0) {
+      sum[0] = fx; sum[1] = fy; sum[2] = fz;
+      sum[3] = tx; sum[4] = ty; sum[5] = tz;
     }
-    // (2) counting sort of the block's atoms with contacts by their count
-    if (key) atomicAdd(&sm.gcount[key], 1);
-    __syncthreads();
-    if (tid < 32) {
-      const int v0 = tid < kGatherKeys ? sm.gcount[tid] : 0;
-      const int inc = warp_incl_scan(v0);
-      if (tid < kGatherKeys) sm.gstart[tid] = inc - v0;
-      if (tid == 31) sm.gnq = inc;
+    __syncwarp();
+    gather_warp(s, sm.list[w], sm.sum[w], sm.order[w], cnt, lane);
+    if (cnt > 0) {
+      fx = sum[0]; fy = sum[1]; fz = sum[2];
+      tx = sum[3]; ty = sum[4]; tz = sum[5];
     }
-    __syncthreads();
-    if (key) sm.gsorted[sm.gstart[key] + atomicAdd(&sm.gfill[key], 1)] = (short)tid;
-    __syncthreads();
-    if (tid < kGatherKeys) {  // read by no one until the next block of atoms counts
-      sm.gcount[tid] = 0;
-      sm.gfill[tid] = 0;
-    }
-    // (3) the loops, one atom per thread in sorted order
-    if (tid < sm.gnq) {
-      const int a = sm.gsorted[tid];
-      double sx = sm.gsum[0][a], sy = sm.gsum[1][a], sz = sm.gsum[2][a];
-      double qx = sm.gsum[3][a], qy = sm.gsum[4][a], qz = sm.gsum[5][a];
-      gather_sum<false>(s, L, sm.gpb[a], sm.grb[a], sm.gom[a], sm.grm[a], sx, sy, sz, qx, qy, qz);
-      sm.gsum[0][a] = sx; sm.gsum[1][a] = sy; sm.gsum[2][a] = sz;
-      sm.gsum[3][a] = qx; sm.gsum[4][a] = qy; sm.gsum[5][a] = qz;
-    }
-    __syncthreads();
-    if (key) {
-      fx = sm.gsum[0][tid]; fy = sm.gsum[1][tid]; fz = sm.gsum[2][tid];
-      tx = sm.gsum[3][tid]; ty = sm.gsum[4][tid]; tz = sm.gsum[5][tid];
-    }
+    if (cnt < 0) gather_long(s, L, i, fx, fy, fz, tx, ty, tz);
+    __syncwarp();
   }
   if (!valid) return;
+  double v[3] = {A.vx[i], A.vy[i], A.vz[i]}, om[3] = {A.wx[i], A.wy[i], A.wz[i]};
+  double xv[3] = {A.x[i], A.y[i], A.z[i]};
   if (gather) {
     if (A.wbits[i] & 0x80u) {  // walls, computed by the wall tiles for this step
       fx += A.fmx[i]; fy += A.fmy[i]; fz += A.fmz[i];
@@ -1523,10 +1589,8 @@ __device__ __forceinline__ void list_cache_load(const Sys &s, ListCache<T> &lc, 
   lc.cnt[tid] = cnt;
 }
 
-// particle_tile for k_steps: a warp handles its 32 atoms on its own.  With few
-// warps per SM the block-wide sort of particle_tile costs more (five barriers,
-// shared-memory round trips, all warps in the same phase) than the additions
-// that it saves, and each load that waits for another costs a trip to L2 (the
+// particle_tile for k_steps.  With few warps per SM the shared-memory round
+// trips of particle_tile cost more than the additions that they save, and each load that waits for another costs a trip to L2 (the
 // barriers leave nothing in L1): the list's indices come from the cache, what
 // does not depend on them is loaded together, and a contact's record is loaded
 // while the one before it is added.  Same sums in the same order.
@@ -1595,7 +1659,7 @@ __device__ __forceinline__ void particle_warp(const Sys &s, const ListCache<T> *
     } else {
       int pb, rb;
       unsigned mo, mr;
-      if (gather_masks<4>(s, L, i, pb, rb, mo, mr)) gather_sum<true>(s, L, pb, rb, mo, mr, f[0], f[1], f[2], f[3], f[4], f[5]);
+      if (gather_masks<4>(s, L, i, pb, rb, mo, mr)) gather_sum(s, L, pb, rb, mo, mr, f[0], f[1], f[2], f[3], f[4], f[5]);
       else gather_long(s, L, i, f[0], f[1], f[2], f[3], f[4], f[5]);
     }
     if (wall)
