@@ -108,6 +108,13 @@ __device__ __forceinline__ bool gt_nonneg(double a, double b) {
   return __double_as_longlong(a) > __double_as_longlong(b);
 }
 
+// A key that orders doubles as the comparison does, -0 and +0 alike (a NaN lies
+// beyond the infinities), for comparisons of any sign on the integer pipe.
+__device__ __forceinline__ long long order_key(double x) {
+  const long long b = __double_as_longlong(x);
+  return b < 0 ? (long long)(0x8000000000000000ull - (unsigned long long)b) : b;
+}
+
 // shear[3] is the tangential history, updated in place when update_history.
 // base: forces and torques of a bonded pair (cohesion bond/nonlinear), which
 // replace the normal model's force before the tangential and rolling models

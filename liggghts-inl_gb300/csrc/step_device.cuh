@@ -225,6 +225,12 @@ __device__ __forceinline__ void store_result(const Sys &s, int q, const ContactO
   r[5] = make_double2(0.0, 0.0);
 }
 
+// x with its sign bit flipped where `sign` has it (a variable: a constant one
+// would become a negation, which issues on the FP64 pipe, as a product does)
+__device__ __forceinline__ double with_sign(double x, int sign) {
+  return __hiloint2double(__double2hiint(x) ^ sign, __double2loint(x));
+}
+
 // Phase 2 of k_pair for one queued entry q (delx, dely, delz, rsq_q from
 // its exact test): the bond law, the contact law, the result record
 template <int NORMAL, bool ROLL, bool BOND>
@@ -246,7 +252,7 @@ __device__ __forceinline__ void band_entry(const Sys &s, int q, double delx, dou
   ci.vr[2] = A.vz[i] - A.vz[j];
   ci.wi[0] = A.wx[i]; ci.wi[1] = A.wy[i]; ci.wi[2] = A.wz[i];
   ci.wj[0] = A.wx[j]; ci.wj[1] = A.wy[j]; ci.wj[2] = A.wz[j];
-  const bool touch = !BOND || rsq_q < __dmul_rn(ci.radsum, ci.radsum);
+  const bool touch = !BOND || gt_nonneg(__dmul_rn(ci.radsum, ci.radsum), rsq_q);
   ContactOut bo;
   bool bonded = false;
   if (BOND) {
@@ -254,9 +260,9 @@ __device__ __forceinline__ void band_entry(const Sys &s, int q, double delx, dou
     // (periodic entries are directed and always owned by i)
     const bool rev = L.sh[q] == kNoShift && A.lidx[i] > A.lidx[j];
     const int a = rev ? j : i, b = rev ? i : j;
-    const double sg = rev ? -1.0 : 1.0;
+    const int sg = rev ? (int)0x80000000 : 0;  // turns a vector round
     BondIn bi;
-    bi.d[0] = sg * ci.d[0]; bi.d[1] = sg * ci.d[1]; bi.d[2] = sg * ci.d[2];
+    for (int k = 0; k < 3; k++) bi.d[k] = with_sign(ci.d[k], sg);
     bi.rsq = rsq_q;
     bi.radi = A.r[a];
     bi.radj = A.r[b];
@@ -270,7 +276,7 @@ __device__ __forceinline__ void band_entry(const Sys &s, int q, double delx, dou
     bonded = bond_nonlinear(s, bi, L.hist + 3 * P + q, P, L.flag + q, shearupdate != 0, ntimestep, bc);
     if (bonded) {  // back to the list's orientation (i owns the entry)
       for (int k = 0; k < 3; k++) {
-        bo.F[k] = sg * bc.F[k];
+        bo.F[k] = with_sign(bc.F[k], sg);
         bo.Ti[k] = rev ? bc.Tj[k] : bc.Ti[k];
         bo.Tj[k] = rev ? bc.Ti[k] : bc.Tj[k];
       }
@@ -350,10 +356,10 @@ __device__ __forceinline__ bool band_test(const Sys &s, int np, int p, double cd
     delz = __dadd_rn(A.z[i], -zj);
     rsq = rsq_rn(delx, dely, delz);
     const double radsum = __dadd_rn(A.r[i], A.r[j]);
-    queue = rsq < __dmul_rn(radsum, radsum);
+    queue = gt_nonneg(__dmul_rn(radsum, radsum), rsq);
     if (!queue) {
       s.active[p] = 0;
-      if (rsq < __dmul_rn(__dmul_rn(cdm, radsum), radsum)) {
+      if (gt_nonneg(__dmul_rn(__dmul_rn(cdm, radsum), radsum), rsq)) {
         // TangentialModel<TANGENTIAL_HISTORY>::surfacesClose
         L.flag[p] &= ~kContactTangential;
         L.hist[p] = 0.0;
@@ -361,9 +367,10 @@ __device__ __forceinline__ bool band_test(const Sys &s, int np, int p, double cd
         L.hist[2 * P + p] = 0.0;
         // CohesionModel::surfacesClose: bonded pairs (and pairs that may
         // bond in this pass) are evaluated in phase 2
-        if (BOND && (may_create || L.hist[3 * P + p] >= 1.e-15)) {
+        const long long tiny = order_key(1.e-15);
+        if (BOND && (may_create || order_key(L.hist[3 * P + p]) >= tiny)) {
           const int tp = A.type[i] * (s.ntypes + 1) + A.type[j];
-          queue = __ldg(s.bondp + tp) >= 1.e-15;
+          queue = order_key(__ldg(s.bondp + tp)) >= tiny;
         }
       }
     }

@@ -14,7 +14,8 @@ pytestmark = pytest.mark.gpu
 
 def _case(k, first):
     from gb300dem import workloads
-    c = workloads.lattice_case(4, 12, 12, 12, 2.05e-3, radius=(0.9e-3, 1.1e-3), dt=1e-6, skin=2e-4)
+    c = workloads.lattice_case(4, 12, 12, 12, 2.05e-3, radius=(0.9e-3, 1.1e-3), dt=1e-6, skin=2e-4,
+                               periodic=(0, 0, 0))
     R, r = 4e-3, 1e-3
     t = np.arange(k) + 0.5
     phi, z = np.pi * (1 + 5 ** 0.5) * t, 1 - 2 * t / k
