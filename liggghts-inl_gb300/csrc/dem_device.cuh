@@ -133,7 +133,11 @@ struct Ctrl {
   // gave up, the grid barrier's count (see grid_barrier)
   int step_phase, bar_exit, bar_abort;
   unsigned long long bar;
+  int hold;  // the unrolled step loop (see build_step_graph): kHold*
 };
+
+// Ctrl::hold: kernels of the step loop run; wait for the rebuild; all steps done
+enum { kHoldNone = 0, kHoldRebuild = 1, kHoldDone = 2 };
 
 // Ctrl::step_phase: the first step of a call (no forces to gather), a step
 // that gathers the previous step's forces, resume with the forces after a

@@ -78,24 +78,43 @@ __global__ void k_decide(Sys s) {
   decide_rebuild(s, c);
 }
 
-// k_decide for the graph-resident step loop: also drives the IF node around
-// the rebuild and the WHILE node around the whole step.
-__global__ void k_decide_loop(Sys s, cudaGraphConditionalHandle hreb, cudaGraphConditionalHandle hloop) {
-  Ctrl *c = s.ctrl;
-  if (c->halt) {
-    if (threadIdx.x == 0) {
-      cudaGraphSetConditional(hreb, 0);
-      cudaGraphSetConditional(hloop, 0);
-    }
-    return;
+// The conditionals of the graph-resident step loop.  on: the last block of
+// k_particle takes the decision (else k_decide_loop); gate: a step of the
+// unrolled loop, which may be held.
+struct LoopCond {
+  int on, gate;
+  cudaGraphConditionalHandle hreb, hloop;
+};
+
+// whether the loop's kernels are no-ops: halted, or held; ends the loop when
+// halted or out of steps (called by every thread, `lead` by one of them)
+__device__ __forceinline__ bool loop_held(const Ctrl *c, const LoopCond &lp, bool lead) {
+  const int hold = lp.gate ? c->hold : kHoldNone;
+  if (!c->halt && hold == kHoldNone) return false;
+  if (lead && (c->halt || hold == kHoldDone)) {
+    cudaGraphSetConditional(lp.hreb, 0);
+    cudaGraphSetConditional(lp.hloop, 0);
   }
+  return true;
+}
+
+// the decision of a loop step, by one thread behind decide_rebuild
+__device__ __forceinline__ void loop_decided(Ctrl *c, const LoopCond &lp, int reb) {
+  const int left = --c->loop_left;
+  c->hold = reb ? kHoldRebuild : (left > 0 ? kHoldNone : kHoldDone);
+  cudaGraphSetConditional(lp.hreb, reb ? 1u : 0u);
+  cudaGraphSetConditional(lp.hloop, reb || left > 0 ? 1u : 0u);
+}
+
+// k_decide for the step loop: also drives the IF node around the rebuild and
+// the WHILE node around the steps
+__global__ void k_decide_loop(Sys s, LoopCond lp) {
+  Ctrl *c = s.ctrl;
+  if (loop_held(c, lp, threadIdx.x == 0)) return;
+  __syncthreads();  // every thread has read the hold before it changes
   if (threadIdx.x == 0) c->ntimestep++;
   const int reb = decide_rebuild(s, c);
-  if (threadIdx.x == 0) {
-    c->loop_left--;
-    cudaGraphSetConditional(hreb, reb ? 1u : 0u);
-    cudaGraphSetConditional(hloop, c->loop_left > 0 ? 1u : 0u);
-  }
+  if (threadIdx.x == 0) loop_decided(c, lp, reb);
 }
 
 __global__ void k_set_loop(Ctrl *c, int n, int phase) {
@@ -769,9 +788,9 @@ __device__ __forceinline__ void mslot_swap(const MeshDev &M, size_t nmax, int i,
   }
 }
 
-__global__ void k_mesh_move(Sys s, int k) {
+__global__ void k_mesh_move(Sys s, int k, int gate) {
   Ctrl *c = s.ctrl;
-  if (c->halt) return;
+  if (c->halt || (gate && c->hold)) return;
   const MeshDev &M = s.meshes[k];
   bool moved = false;
   const int per = (gridDim.x * blockDim.x) / 16;
@@ -1382,6 +1401,7 @@ __global__ void k_finish_rebuild(Sys s) {
     if (!s.nsys) c->np_live = c->np_new;
     c->nrebuilds++;
     c->ago = 0;
+    c->hold = c->loop_left > 0 ? kHoldNone : kHoldDone;
   }
 }
 
@@ -1400,11 +1420,11 @@ struct GridTiles {
 };
 
 template <int NORMAL, bool ROLL, bool BOND>
-__global__ void __launch_bounds__(kBandTile, 4) k_pair(Sys s, int shearupdate) {
+__global__ void __launch_bounds__(kBandTile, 4) k_pair(Sys s, int shearupdate, int gate) {
   __shared__ BandQueue q[kBandTile / 32];
   __shared__ BandRest<kBandTile> rest;
   Ctrl *c = s.ctrl;
-  if (c->halt) return;
+  if (c->halt || (gate && c->hold)) return;
   const long long ntimestep = BOND ? c->ntimestep : 0;
   BandQueue &mine = q[threadIdx.x >> 5];
   const int qn = band_tiles<NORMAL, ROLL, BOND>(s, c->np, shearupdate, ntimestep, mine, GridTiles(kBandTile));
@@ -1412,21 +1432,21 @@ __global__ void __launch_bounds__(kBandTile, 4) k_pair(Sys s, int shearupdate) {
 }
 
 template <int NORMAL, bool ROLL, int MINB>
-__global__ void __launch_bounds__(kPairTile, MINB) k_pair_pf(Sys s, int shearupdate) {
+__global__ void __launch_bounds__(kPairTile, MINB) k_pair_pf(Sys s, int shearupdate, int gate) {
   __shared__ int qbuf[kPairTile / 32][64];
   __shared__ PfRest rest;
   Ctrl *c = s.ctrl;
-  if (c->halt) return;
+  if (c->halt || (gate && c->hold)) return;
   int *q = qbuf[threadIdx.x >> 5];
   const int qn = pf_tiles<NORMAL, ROLL>(s, c->np, shearupdate, q, GridTiles(kPairTile));
   pf_rest<NORMAL, ROLL>(s, qn, shearupdate, q, rest);
 }
 
 template <int NORMAL>
-__global__ void __launch_bounds__(kWallTile *kWallWarps) k_wall_force(Sys s, int shearupdate, int cap) {
+__global__ void __launch_bounds__(kWallTile *kWallWarps) k_wall_force(Sys s, int shearupdate, int cap, int gate) {
   extern __shared__ double wshared[];  // per warp: res [cap * kWallRes]; then st, qa, qq of every warp
   Ctrl *c = s.ctrl;
-  if (c->halt) return;
+  if (c->halt || (gate && c->hold)) return;
   const int warp = threadIdx.x >> 5;
   WallQueue w;
   w.res = wshared + (size_t)warp * cap * kWallRes;
@@ -1443,14 +1463,8 @@ __global__ void __launch_bounds__(kWallTile *kWallWarps) k_wall_force(Sys s, int
 }
 
 // Graph steps without moving meshes: the last block of k_particle to finish
-// takes the step's rebuild decision and sets the loop's conditionals, as
-// k_decide_loop does after it otherwise (one node and one dependency fewer
-// per step).
-struct LoopCond {
-  int on;
-  cudaGraphConditionalHandle hreb, hloop;
-};
-
+// takes the step's rebuild decision (LoopCond::on), as k_decide_loop does after
+// it otherwise (one node and one dependency fewer per step).
 // the flags of a block's atoms, and (lp.on) the decision by the last block
 __device__ __forceinline__ void particle_end(const Sys &s, Ctrl *c, bool moved, bool bad, const LoopCond &lp) {
   __shared__ int last_block;
@@ -1472,29 +1486,16 @@ __device__ __forceinline__ void particle_end(const Sys &s, Ctrl *c, bool moved, 
         c->ntimestep++;
       }
       const int reb = decide_rebuild(s, c);
-      if (threadIdx.x == 0) {
-        c->loop_left--;
-        cudaGraphSetConditional(lp.hreb, reb ? 1u : 0u);
-        cudaGraphSetConditional(lp.hloop, c->loop_left > 0 ? 1u : 0u);
-      }
+      if (threadIdx.x == 0) loop_decided(c, lp, reb);
     }
   }
-}
-
-__device__ __forceinline__ bool particle_halted(const Ctrl *c, const LoopCond &lp) {
-  if (!c->halt) return false;
-  if (lp.on && blockIdx.x == 0 && threadIdx.x == 0) {
-    cudaGraphSetConditional(lp.hreb, 0);
-    cudaGraphSetConditional(lp.hloop, 0);
-  }
-  return true;
 }
 
 template <bool GATHER, bool FINAL, bool INITIAL>
 __global__ void __launch_bounds__(kParticleMaxThreads, 4) k_particle(Sys s, LoopCond lp) {
   __shared__ ParticleShared<kParticleMaxThreads> sm;
   Ctrl *c = s.ctrl;
-  if (particle_halted(c, lp)) return;
+  if (loop_held(c, lp, (lp.on || lp.gate) && blockIdx.x == 0 && threadIdx.x == 0)) return;
   const int n = c->n;
   bool moved = false, bad = false;
   for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
@@ -1510,7 +1511,7 @@ __global__ void __launch_bounds__(kParticleMaxThreads, 4) k_particle(Sys s, Loop
 __global__ void __launch_bounds__(kParticleMaxThreads, 4) k_particle_start(Sys s, LoopCond lp) {
   __shared__ ParticleShared<kParticleMaxThreads> sm;
   Ctrl *c = s.ctrl;
-  if (particle_halted(c, lp)) return;
+  if (loop_held(c, lp, (lp.on || lp.gate) && blockIdx.x == 0 && threadIdx.x == 0)) return;
   const int n = c->n;
   const bool gather = c->step_phase != kStepFirst;
   bool moved = false, bad = false;
@@ -1928,14 +1929,25 @@ int launch_rebuild(const Sys &s, const LaunchCfg &lc, cudaStream_t st, int stage
 // Fused (k_steps runs all steps up to the next rebuild):
 //   WHILE(loop) { k_steps -> IF(rebuild) { rebuild kernels } }
 // Separate kernels (ensembles, large systems):
-//   k_particle_start -> IF(rebuild) { rebuild kernels } -> pair || wall ->
-//   WHILE(loop) { k_particle(gather+final+initial) -> IF(rebuild) {...} -> pair || wall } ->
-//   k_particle(gather+final)
+//   k_particle_start ->
+//   WHILE(loop) { IF(rebuild) { rebuild kernels } ->
+//                 kUnroll x (pair || wall -> k_particle(gather+final+initial)) } ->
+//   pair || wall -> k_particle(gather+final)
+// A step that decides to rebuild, and the last one, hold the rest of the loop's
+// kernels (Ctrl::hold): they are no-ops until the next iteration's rebuild, or
+// to the end.
 // Without moving meshes the last block of the per-atom kernel takes the
 // decision, else k_decide_loop does after the mesh has moved.  The first
 // step's rebuild sits behind an IF node too: launched from the host its some
 // thirty kernels cost 67-150 us of each call while doing nothing.
 static int launch_particle_lp(const Sys &s, const LaunchCfg &lc, int mode, const LoopCond &lp, cudaStream_t st);
+
+// steps per iteration: the WHILE and IF nodes cost some 10 us an iteration, a
+// held step's kernels 4 (they matter to ensembles, which rebuild every few
+// steps).  50 steps at 1, 4, 8: 1,000,000 in a hopper 13693, 13331, 13407 us;
+// 400,000 packed 24596, 24306, 24230; 100 steps of an ensemble of 48 14655,
+// 13872, 14076.
+constexpr int kUnroll = 4;
 
 // Captures into one graph at a time on two streams and cleans up on failure.
 struct GraphBuilder {
@@ -2004,7 +2016,7 @@ struct GraphBuilder {
     return cudaStreamEndCapture(st2, &out);
   }
   // the pair kernel and the wall kernel of a step, side by side
-  cudaError_t forces(int *k) {
+  cudaError_t forces(int gate, int *k) {
     cudaError_t e;
     const bool walls = s.nmeshes > 0 || s.nplanes > 0;
     if (walls) {
@@ -2012,22 +2024,22 @@ struct GraphBuilder {
       if (!join && (e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming)) != cudaSuccess) return e;
       if ((e = cudaEventRecord(fork, st)) != cudaSuccess) return e;
       if ((e = cudaStreamWaitEvent(st2, fork, 0)) != cudaSuccess) return e;
-      *k += launch_wall_force(s, lc, 1, st2);
+      *k += launch_wall_force(s, lc, 1, st2, gate);
       if ((e = cudaEventRecord(join, st2)) != cudaSuccess) return e;
     }
-    *k += launch_pair(s, lc, 1, st);
+    *k += launch_pair(s, lc, 1, st, gate);
     return walls ? cudaStreamWaitEvent(st, join, 0) : cudaSuccess;
   }
   // the per-atom kernel (start: the call's first step) with the decision
   cudaError_t particle(bool start, cudaGraphConditionalHandle hreb, cudaGraphConditionalHandle hloop, int *k) {
     bool moving = false;
     for (int m = 0; m < s.nmeshes; m++) moving |= s.meshes[m].moving != 0;
-    const LoopCond lp{moving ? 0 : 1, hreb, hloop};
+    const LoopCond lp{moving ? 0 : 1, start ? 0 : 1, hreb, hloop};
     const int mode = start ? kModeStart : kModeGatherFinalInitial;
     *k += launch_particle_lp(s, lc, mode, lp, st);
     if (moving) {  // the mesh moves between the per-atom kernel and the decision
-      *k += launch_mesh_move(s, lc, st);
-      k_decide_loop<<<1, sys_threads(s), 0, st>>>(s, hreb, hloop);
+      *k += launch_mesh_move(s, lc, st, lp.gate);
+      k_decide_loop<<<1, sys_threads(s), 0, st>>>(s, lp);
       (*k)++;
     }
     return cudaGetLastError();
@@ -2039,12 +2051,10 @@ cudaError_t build_step_graph(const Sys &s, const LaunchCfg &lc, cudaStream_t st,
   GraphBuilder b{s, lc, st, st2};
   cudaError_t e = cudaGraphCreate(&b.g, 0);
   if (e != cudaSuccess) return b.fail(e);
-  cudaGraphConditionalHandle hloop, hreb, hreb0;
-  for (cudaGraphConditionalHandle *h : {&hloop, &hreb, &hreb0}) {
-    if (h == &hreb0 && fused_steps(s, lc)) continue;
+  cudaGraphConditionalHandle hloop, hreb;
+  for (cudaGraphConditionalHandle *h : {&hloop, &hreb})
     if ((e = cudaGraphConditionalHandleCreate(h, b.g, h == &hloop ? 1 : 0, cudaGraphCondAssignDefault)) != cudaSuccess)
       return b.fail(e);
-  }
   *counts = StepCounts{};
   cudaGraph_t body;
   if ((e = b.begin(b.g)) != cudaSuccess) return b.fail(e);
@@ -2058,16 +2068,18 @@ cudaError_t build_step_graph(const Sys &s, const LaunchCfg &lc, cudaStream_t st,
     counts->call = 1;  // and one more launch per rebuild
     counts->rebuild = b.kpr + 1;
   } else {
-    if ((e = b.particle(true, hreb0, hloop, &counts->call)) != cudaSuccess) return b.fail(e);
-    if ((e = b.rebuild_if(hreb0)) != cudaSuccess) return b.fail(e);
-    if ((e = b.forces(&counts->call)) != cudaSuccess) return b.fail(e);
+    if ((e = b.particle(true, hreb, hloop, &counts->call)) != cudaSuccess) return b.fail(e);
     if ((e = b.conditional(hloop, cudaGraphCondTypeWhile, &body)) != cudaSuccess) return b.fail(e);
+    if ((e = b.forces(0, &counts->call)) != cudaSuccess) return b.fail(e);
     counts->call += launch_particle(s, lc, kModeGatherFinal, st);
     if ((e = b.end()) != cudaSuccess) return b.fail(e);
     if ((e = b.begin(body)) != cudaSuccess) return b.fail(e);
-    if ((e = b.particle(false, hreb, hloop, &counts->step)) != cudaSuccess) return b.fail(e);
     if ((e = b.rebuild_if(hreb)) != cudaSuccess) return b.fail(e);
-    if ((e = b.forces(&counts->step)) != cudaSuccess) return b.fail(e);
+    for (int u = 0; u < kUnroll; u++) {
+      counts->step = 0;
+      if ((e = b.forces(1, &counts->step)) != cudaSuccess) return b.fail(e);
+      if ((e = b.particle(false, hreb, hloop, &counts->step)) != cudaSuccess) return b.fail(e);
+    }
     if ((e = b.end()) != cudaSuccess) return b.fail(e);
     counts->rebuild = b.kpr;
   }
@@ -2088,7 +2100,7 @@ int wall_cap_per_atom() {
 // The wall kernel walks a short list (atoms near walls) with long per-atom
 // dependency chains; it is launched with the device's highest priority so
 // that its blocks start before those of the pair kernel beside it.
-int launch_wall_force(const Sys &s, const LaunchCfg &lc, int shearupdate, cudaStream_t st) {
+int launch_wall_force(const Sys &s, const LaunchCfg &lc, int shearupdate, cudaStream_t st, int gate) {
   if (s.nmeshes == 0 && s.nplanes == 0) return 0;
   int lo = 0, hi = 0;
   cudaDeviceGetStreamPriorityRange(&lo, &hi);
@@ -2107,16 +2119,16 @@ int launch_wall_force(const Sys &s, const LaunchCfg &lc, int shearupdate, cudaSt
   attr[0].val.priority = hi;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (s.normal == kHertz) cudaLaunchKernelEx(&cfg, k_wall_force<kHertz>, s, shearupdate, cap);
-  else cudaLaunchKernelEx(&cfg, k_wall_force<kHooke>, s, shearupdate, cap);
+  if (s.normal == kHertz) cudaLaunchKernelEx(&cfg, k_wall_force<kHertz>, s, shearupdate, cap, gate);
+  else cudaLaunchKernelEx(&cfg, k_wall_force<kHooke>, s, shearupdate, cap, gate);
   return 1;
 }
 
-int launch_mesh_move(const Sys &s, const LaunchCfg &lc, cudaStream_t st) {
+int launch_mesh_move(const Sys &s, const LaunchCfg &lc, cudaStream_t st, int gate) {
   int nl = 0;
   for (int k = 0; k < s.nmeshes; k++) {
     if (!s.meshes[k].moving) continue;
-    k_mesh_move<<<grid_for(16L * s.meshes[k].ntri, 256, lc.max_grid), 256, 0, st>>>(s, k);
+    k_mesh_move<<<grid_for(16L * s.meshes[k].ntri, 256, lc.max_grid), 256, 0, st>>>(s, k, gate);
     nl++;
   }
   return nl;
@@ -2136,18 +2148,18 @@ int launch_set_rebuild(const Sys &s, int v, cudaStream_t st) {
   return 1;
 }
 
-int launch_pair(const Sys &s, const LaunchCfg &lc, int shearupdate, cudaStream_t st) {
+int launch_pair(const Sys &s, const LaunchCfg &lc, int shearupdate, cudaStream_t st, int gate) {
   const int B = 256;
   const int g = grid_for(s.pcap, B, lc.max_grid);
   const int Bb = kBandTile;
   const int gb = grid_for(s.pcap, Bb, 2 * lc.max_grid);
   if (s.bond) {
     if (s.normal == kHertz) {
-      if (s.rolling) k_pair<kHertz, true, true><<<gb, Bb, 0, st>>>(s, shearupdate);
-      else k_pair<kHertz, false, true><<<gb, Bb, 0, st>>>(s, shearupdate);
+      if (s.rolling) k_pair<kHertz, true, true><<<gb, Bb, 0, st>>>(s, shearupdate, gate);
+      else k_pair<kHertz, false, true><<<gb, Bb, 0, st>>>(s, shearupdate, gate);
     } else {
-      if (s.rolling) k_pair<kHooke, true, true><<<gb, Bb, 0, st>>>(s, shearupdate);
-      else k_pair<kHooke, false, true><<<gb, Bb, 0, st>>>(s, shearupdate);
+      if (s.rolling) k_pair<kHooke, true, true><<<gb, Bb, 0, st>>>(s, shearupdate, gate);
+      else k_pair<kHooke, false, true><<<gb, Bb, 0, st>>>(s, shearupdate, gate);
     }
     return 1;
   }
@@ -2172,29 +2184,29 @@ int launch_pair(const Sys &s, const LaunchCfg &lc, int shearupdate, cudaStream_t
     const int gp = wave ? std::min(g, lc.sms * minb) : g;
     if (minb == 4) {
       if (s.normal == kHertz) {
-        if (s.rolling) k_pair_pf<kHertz, true, 4><<<gp, B, 0, st>>>(s, shearupdate);
-        else k_pair_pf<kHertz, false, 4><<<gp, B, 0, st>>>(s, shearupdate);
+        if (s.rolling) k_pair_pf<kHertz, true, 4><<<gp, B, 0, st>>>(s, shearupdate, gate);
+        else k_pair_pf<kHertz, false, 4><<<gp, B, 0, st>>>(s, shearupdate, gate);
       } else {
-        if (s.rolling) k_pair_pf<kHooke, true, 4><<<gp, B, 0, st>>>(s, shearupdate);
-        else k_pair_pf<kHooke, false, 4><<<gp, B, 0, st>>>(s, shearupdate);
+        if (s.rolling) k_pair_pf<kHooke, true, 4><<<gp, B, 0, st>>>(s, shearupdate, gate);
+        else k_pair_pf<kHooke, false, 4><<<gp, B, 0, st>>>(s, shearupdate, gate);
       }
     } else {
       if (s.normal == kHertz) {
-        if (s.rolling) k_pair_pf<kHertz, true, 3><<<gp, B, 0, st>>>(s, shearupdate);
-        else k_pair_pf<kHertz, false, 3><<<gp, B, 0, st>>>(s, shearupdate);
+        if (s.rolling) k_pair_pf<kHertz, true, 3><<<gp, B, 0, st>>>(s, shearupdate, gate);
+        else k_pair_pf<kHertz, false, 3><<<gp, B, 0, st>>>(s, shearupdate, gate);
       } else {
-        if (s.rolling) k_pair_pf<kHooke, true, 3><<<gp, B, 0, st>>>(s, shearupdate);
-        else k_pair_pf<kHooke, false, 3><<<gp, B, 0, st>>>(s, shearupdate);
+        if (s.rolling) k_pair_pf<kHooke, true, 3><<<gp, B, 0, st>>>(s, shearupdate, gate);
+        else k_pair_pf<kHooke, false, 3><<<gp, B, 0, st>>>(s, shearupdate, gate);
       }
     }
     return 1;
   }
   if (s.normal == kHertz) {
-    if (s.rolling) k_pair<kHertz, true, false><<<gb, Bb, 0, st>>>(s, shearupdate);
-    else k_pair<kHertz, false, false><<<gb, Bb, 0, st>>>(s, shearupdate);
+    if (s.rolling) k_pair<kHertz, true, false><<<gb, Bb, 0, st>>>(s, shearupdate, gate);
+    else k_pair<kHertz, false, false><<<gb, Bb, 0, st>>>(s, shearupdate, gate);
   } else {
-    if (s.rolling) k_pair<kHooke, true, false><<<gb, Bb, 0, st>>>(s, shearupdate);
-    else k_pair<kHooke, false, false><<<gb, Bb, 0, st>>>(s, shearupdate);
+    if (s.rolling) k_pair<kHooke, true, false><<<gb, Bb, 0, st>>>(s, shearupdate, gate);
+    else k_pair<kHooke, false, false><<<gb, Bb, 0, st>>>(s, shearupdate, gate);
   }
   return 1;
 }
@@ -2215,7 +2227,7 @@ static int launch_particle_lp(const Sys &s, const LaunchCfg &lc, int mode, const
 }
 
 int launch_particle(const Sys &s, const LaunchCfg &lc, int mode, cudaStream_t st) {
-  return launch_particle_lp(s, lc, mode, LoopCond{0, 0, 0}, st);
+  return launch_particle_lp(s, lc, mode, LoopCond{0, 0, 0, 0}, st);
 }
 
 }  // namespace gb300

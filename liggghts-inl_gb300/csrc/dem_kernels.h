@@ -68,14 +68,14 @@ int launch_set_rebuild(const Sys &s, int v, cudaStream_t st);
 // stage 0: full rebuild; stage 1: resume after a pair-capacity overflow;
 // stage 2: resume after a mesh slot or registration overflow
 int launch_rebuild(const Sys &s, const LaunchCfg &lc, cudaStream_t st, int stage);
-int launch_pair(const Sys &s, const LaunchCfg &lc, int shearupdate, cudaStream_t st);
+int launch_pair(const Sys &s, const LaunchCfg &lc, int shearupdate, cudaStream_t st, int gate = 0);
 int launch_particle(const Sys &s, const LaunchCfg &lc, int mode, cudaStream_t st);
 int launch_set_loop(const Sys &s, int n, int phase, cudaStream_t st);
 // wall (plane and mesh) forces of the current state, before the particle
 // kernel that gathers the step's forces; none without walls
-int launch_wall_force(const Sys &s, const LaunchCfg &lc, int shearupdate, cudaStream_t st);
+int launch_wall_force(const Sys &s, const LaunchCfg &lc, int shearupdate, cudaStream_t st, int gate = 0);
 // fix move/mesh: moves the moving meshes by one step (after the drift)
-int launch_mesh_move(const Sys &s, const LaunchCfg &lc, cudaStream_t st);
+int launch_mesh_move(const Sys &s, const LaunchCfg &lc, cudaStream_t st, int gate = 0);
 // queue entries of the wall kernel per tile atom (LIGGGHTS_GB300_WALL_CAP)
 int wall_cap_per_atom();
 // Whether dem_step runs the steps in k_steps (dem_steps.cu) rather than as
