@@ -266,6 +266,13 @@ __device__ __forceinline__ void contact_law(const ContactIn &c, const TypePair &
   }
 }
 
+// a b + c d with one product rounded; written out, so that every kernel that
+// inlines a law forms the same bits (which product the compiler rounds depends
+// on the code around it)
+__device__ __forceinline__ double two_products(double a, double b, double c, double d) {
+  return fma(c, d, __dmul_rn(a, b));
+}
+
 // contact_law for a pair of spheres without cohesion and rolling friction,
 // with the identities that save FP64 instructions (about 110 against 125 per
 // entry; each holds the pipe of its SM quarter for 64 cycles, whatever the
@@ -282,12 +289,12 @@ template <int NORMAL>
 __device__ __forceinline__ void pair_law(const ContactIn &c, const TypePair &tp, double dt, bool tdamp, bool limitf,
                                          bool update_history, double shear[3], ContactOut &o) {
   const double ex = c.en[0], ey = c.en[1], ez = c.en[2];
-  const double vn = c.vr[0] * ex + c.vr[1] * ey + c.vr[2] * ez;
+  const double vn = fma(c.vr[2], ez, two_products(c.vr[0], ex, c.vr[1], ey));
   const double deltan = __dadd_rn(c.radsum, -c.r);
   const double cri = c.radi - 0.5 * deltan, crj = c.radj - 0.5 * deltan;
-  const double W0 = cri * c.wi[0] + crj * c.wj[0];
-  const double W1 = cri * c.wi[1] + crj * c.wj[1];
-  const double W2 = cri * c.wi[2] + crj * c.wj[2];
+  const double W0 = two_products(cri, c.wi[0], crj, c.wj[0]);
+  const double W1 = two_products(cri, c.wi[1], crj, c.wj[1]);
+  const double W2 = two_products(cri, c.wi[2], crj, c.wj[2]);
   const double vt0 = fma(-ez, W1, fma(ey, W2, fma(-vn, ex, c.vr[0])));
   const double vt1 = fma(-ex, W2, fma(ez, W0, fma(-vn, ey, c.vr[1])));
   const double vt2 = fma(-ey, W0, fma(ex, W1, fma(-vn, ez, c.vr[2])));
@@ -320,12 +327,12 @@ __device__ __forceinline__ void pair_law(const ContactIn &c, const TypePair &tp,
     s0 = fma(vt0, dt, s0);
     s1 = fma(vt1, dt, s1);
     s2 = fma(vt2, dt, s2);
-    const double rsht = s0 * ex + s1 * ey + s2 * ez;
+    const double rsht = fma(s2, ez, two_products(s0, ex, s1, ey));
     s0 = fma(-rsht, ex, s0);
     s1 = fma(-rsht, ey, s1);
     s2 = fma(-rsht, ez, s2);
   }
-  const double kt2ss = kt * kt * (s0 * s0 + s1 * s1 + s2 * s2);
+  const double kt2ss = kt * kt * fma(s2, s2, two_products(s0, s0, s1, s1));
   const double Ff = tp.mu * fabs(Fn);
   if (gt_nonneg(kt2ss, Ff * Ff)) {  // sliding
     const double ratio = Ff * rsqrt(kt2ss);
@@ -342,9 +349,9 @@ __device__ __forceinline__ void pair_law(const ContactIn &c, const TypePair &tp,
     shear[1] = s1;
     shear[2] = s2;
   }
-  const double tor0 = ey * Ft2 - ez * Ft1;
-  const double tor1 = ez * Ft0 - ex * Ft2;
-  const double tor2 = ex * Ft1 - ey * Ft0;
+  const double tor0 = two_products(ey, Ft2, -ez, Ft1);
+  const double tor1 = two_products(ez, Ft0, -ex, Ft2);
+  const double tor2 = two_products(ex, Ft1, -ey, Ft0);
   o.F[0] = fma(Fn, ex, Ft0);
   o.F[1] = fma(Fn, ey, Ft1);
   o.F[2] = fma(Fn, ez, Ft2);
@@ -394,7 +401,7 @@ __device__ __forceinline__ void plane_law(double sign, double radi, double delta
     s1 = fma(vt1, dt, s1);
     s2 = fma(vt2, dt, s2);
   }
-  const double kt2ss = kt * kt * (s1 * s1 + s2 * s2);
+  const double kt2ss = kt * kt * two_products(s1, s1, s2, s2);
   const double Ff = tp.mu * fabs(Fn);
   if (gt_nonneg(kt2ss, Ff * Ff)) {
     const double ratio = Ff * rsqrt(kt2ss);

@@ -180,7 +180,7 @@ constexpr int kStatMeshReg = 6;    // Ctrl::status: triangle-cell registrations 
 constexpr int kStatMeshCand = 7;   // Ctrl::status: an atom has more candidate triangles than ccap (halted, grown,
                                    // resumed)
 // geometry layout per triangle: node[9] | edgeVec[9] | edgeNorm[9] |
-// edgeLen[3] | surfaceNorm[3] | center[3] | rBound | pad[3]
+// edgeLen[3] | surfaceNorm[3] | center[3] | rBound | barycentric limit -1e-8/(2 rBound) | pad[2]
 // meta per triangle: bits 0-1 obtuse node+1 (0 none), bits 2-4 edge active,
 // bits 5-7 corner active
 struct MeshDev {

@@ -802,9 +802,15 @@ __device__ __forceinline__ int slot_tri_of(int v) { return v < 0 ? -1 : (v & ~kS
 // 2^-21 is four times that and more), and, for the edges, the 1e-8 by which
 // the reference widens its face region.  A rejected candidate would resolve
 // to deltan > 0, so leaving it out changes nothing.
-__device__ __forceinline__ bool tri_candidate_f(const MeshDev &M, int t, const float4 &xa, float reach_f) {
-  const float4 *T = M.trif + kTrif * (size_t)t;
-  const float4 n0 = T[0], sn = T[1];
+struct TriF {
+  float4 v[kTrif];
+  __device__ __forceinline__ void load(const MeshDev &M, int t) {
+#pragma unroll
+    for (int k = 0; k < kTrif; k++) v[k] = M.trif[kTrif * (size_t)t + k];
+  }
+};
+__device__ __forceinline__ bool tri_candidate_f(const TriF &T, const float4 &xa, float reach_f) {
+  const float4 n0 = T.v[0], sn = T.v[1];
   const float wx = xa.x - n0.x, wy = xa.y - n0.y, wz = xa.z - n0.z;
   const float dn = fabsf(sn.x * wx + sn.y * wy + sn.z * wz);
   const float mag = fabsf(xa.x) + fabsf(xa.y) + fabsf(xa.z) + fabsf(n0.x) + fabsf(n0.y) + fabsf(n0.z);
@@ -814,7 +820,7 @@ __device__ __forceinline__ bool tri_candidate_f(const MeshDev &M, int t, const f
   const float rho2 = (hi * hi - lo * lo) * (1.0f + 0x1p-20f) + hi * hi * 0x1p-20f;
 #pragma unroll
   for (int q = 0; q < 3; q++) {
-    const float4 e = T[2 + q];
+    const float4 e = T.v[2 + q];
     const float d = e.x * wx + e.y * wy + e.z * wz - e.w;
     const float m = (mag + fabsf(wx) + fabsf(wy) + fabsf(wz) + fabsf(e.w)) * 0x1p-21f + 4e-8f;
     const float a = d - m;
@@ -829,13 +835,18 @@ __device__ __forceinline__ bool tri_candidate_f(const MeshDev &M, int t, const f
 // checkCoplanarContactHistory and cleanUpContacts).  A slot touched in this
 // evaluation carries kSlotKept in slot_tri until the clean-up, so the number
 // of candidates has no fixed bound.
+// acc: the atom's force and torque so far, added to, and the mesh's force.
+// Not inlined: a rare path (its code between the tiled path's would cost that
+// one instruction fetches, a quarter of its stalls).
 template <int NORMAL>
-__device__ void mesh_contacts(const Sys &s, const AtomArrays &A, int i, int k, int shearupdate,
-                              double v[3], double om[3], double xv[3], double &fx, double &fy,
-                              double &fz, double &tx, double &ty, double &tz, bool &bad, double msum[3]) {
+__device__ __noinline__ bool mesh_contacts(const Sys &s, int i, int k, int shearupdate, double acc[9]) {
   const MeshDev &M = s.meshes[k];
+  const AtomArrays &A = s.atoms[0];
   const int nc = M.cand_n[i];
-  if (nc == 0) return;
+  if (nc == 0) return false;
+  bool bad = false;
+  const double v[3] = {A.vx[i], A.vy[i], A.vz[i]}, om[3] = {A.wx[i], A.wy[i], A.wz[i]};
+  const double xv[3] = {A.x[i], A.y[i], A.z[i]};
   const size_t nmax = s.nmax;
   int *st = M.slot_tri[0];
   double *sh = M.slot_hist[0];
@@ -852,7 +863,9 @@ __device__ void mesh_contacts(const Sys &s, const AtomArrays &A, int i, int k, i
   const float reach_f = (float)reach * (1.0f + 0x1p-20f);
   for (int q = 0; q < nc; q++) {
     const int t = M.cand[(size_t)q * nmax + i];
-    if (!tri_candidate_f(M, t, xa, reach_f)) continue;
+    TriF T;
+    T.load(M, t);
+    if (!tri_candidate_f(T, xa, reach_f)) continue;
     const double *g = M.tri + (size_t)t * kTriStride;
     {
       const double *sn = tri_sn(g), *n0 = tri_node(g, 0);
@@ -900,9 +913,9 @@ __device__ void mesh_contacts(const Sys &s, const AtomArrays &A, int i, int k, i
     wall_consts(s, s.nplanes + k, i, c0, c1);
     wall_force<NORMAL>(s, A, i, deltan, delta, vwall, M.wall_type, M.rolling != 0, c0, c1,
                          sh + (size_t)(3 * slot) * nmax + i, nmax, shearupdate, v, om, cfx, cfy, cfz, ctx, cty, ctz);
-    fx += cfx; fy += cfy; fz += cfz;
-    tx += ctx; ty += cty; tz += ctz;
-    msum[0] += cfx; msum[1] += cfy; msum[2] += cfz;
+    acc[0] += cfx; acc[1] += cfy; acc[2] += cfz;
+    acc[3] += ctx; acc[4] += cty; acc[5] += ctz;
+    acc[6] += cfx; acc[7] += cfy; acc[8] += cfz;
   }
   for (int u = 0; u < nc; u++) {  // cleanUpContacts
     const int sv = st[u * nmax + i];
@@ -915,6 +928,7 @@ __device__ void mesh_contacts(const Sys &s, const AtomArrays &A, int i, int k, i
     }
   }
   M.npart[0][i] = np;
+  return bad;
 }
 
 // FixWallGran::post_force_primitive / post_force_mesh for the atoms near a
@@ -948,7 +962,12 @@ __device__ void mesh_contacts(const Sys &s, const AtomArrays &A, int i, int k, i
 // warps per SM.  A warp per tile keeps the phases free of block barriers, and
 // the edge bounds leave B about one candidate per contact (with the plane
 // bound alone the conical mesh's tiles queued several per atom, three to five
-// FP64 passes of B).  Against 64-atom tiles with block barriers and the plane
+// FP64 passes of B).  A runs over the tile's (atom, candidate) pairs, 32 at a
+// time, the next ones' triangles on their way, and sends for the records that B
+// will read; an atom at a time, it took 14 candidates' trips to L2 in a row.  C
+// and E walk the slots in use instead of all of them, and the sequential path is
+// a function of its own (instruction fetches were a quarter of the stalls):
+// 100,000 spheres' wall kernel 42 -> 35 us.  Against 64-atom tiles with block barriers and the plane
 // bound: the 100,000-sphere hopper's step 84 -> 67 us, the 1M one's 0.318 ->
 // 0.309 ms (50 steps per call).
 constexpr int kWallTile = 32;
@@ -992,23 +1011,54 @@ __device__ __forceinline__ void wall_tile(const Sys &s, const AtomArrays &A, int
     const MeshDev &M = s.meshes[k];
     int *st = M.slot_tri[0];
     double *sh = M.slot_hist[0];
+    const auto sequential = [&](double sum[3]) {
+      double acc[9] = {fx, fy, fz, tx, ty, tz, 0., 0., 0.};
+      meshbad |= mesh_contacts<NORMAL>(s, i, k, shearupdate, acc);
+      fx = acc[0]; fy = acc[1]; fz = acc[2];
+      tx = acc[3]; ty = acc[4]; tz = acc[5];
+      for (int d = 0; d < 3; d++) sum[d] = acc[6 + d];
+    };
     // ---- A: FP32 candidate pass
     const int nc = valid ? M.cand_n[i] : 0;
     unsigned todo = 0u;
     int np = 0;
     const bool big = nc > kMeshFastCand;  // beyond the 32-bit masks: sequential path
-    if (nc > 0 && !big) {
-      np = M.npart[0][i];
-      const double radi = A.r[i];
-      const double reach = __dmul_rn(__dadd_rn(radi, fmax(0.0, __dmul_rn(cdm1, radi))), 1.0 + 1e-9);
-      const float4 xa = s.xf[i];
-      const float reach_f = (float)reach * (1.0f + 0x1p-20f);
-      int t = M.cand[i];
-      for (int q = 0; q < nc; q++) {
-        const int tn = q + 1 < nc ? M.cand[(size_t)(q + 1) * nmax + i] : 0;  // ahead of the triangle it names
-        if (tri_candidate_f(M, t, xa, reach_f)) todo |= 1u << q;
-        t = tn;
+    const int na = big ? 0 : nc;
+    if (na > 0) np = M.npart[0][i];
+    {
+      const int last = warp_incl_scan(na), pairs = __shfl_sync(0xffffffffu, last, 31), beg = last - na;
+      const float4 xa = na > 0 ? s.xf[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float reach_f = xa.w * fmaxf(1.0f, s.cdff) * (1.0f + 0x1p-19f);
+      // a pair's atom (the first whose pairs end behind it), its candidate
+      const auto pair_of = [&](int f, int &o) {
+        o = 0;
+#pragma unroll
+        for (int h = 16; h > 0; h >>= 1)
+          if (__shfl_sync(0xffffffffu, last, o + h - 1) <= f) o += h;
+        const int io = __shfl_sync(0xffffffffu, i, o), q = f - __shfl_sync(0xffffffffu, beg, o);
+        return f < pairs ? M.cand[(size_t)q * nmax + io] : 0;
+      };
+      // lane a tests pair f0 + a; the next round's candidates are on their way
+      int on, tn = pair_of(a, on);
+      for (int f0 = 0; f0 < pairs; f0 += 32) {
+        const int o = on, t = tn;
+        TriF T;
+        T.load(M, t);
+        if (f0 + 32 < pairs) tn = pair_of(f0 + 32 + a, on);
+        const float4 xo = make_float4(__shfl_sync(0xffffffffu, xa.x, o), __shfl_sync(0xffffffffu, xa.y, o),
+                                      __shfl_sync(0xffffffffu, xa.z, o), 0.f);
+        const float ro = __shfl_sync(0xffffffffu, reach_f, o);
+        const bool pass = f0 + a < pairs && tri_candidate_f(T, xo, ro);
+        if (pass) {  // phase B reads its record
+          const char *g = reinterpret_cast<const char *>(M.tri + (size_t)t * kTriStride);
+          for (int k = 0; k < 3; k++) asm volatile("prefetch.global.L1 [%0];" ::"l"(g + 128 * k));
+          asm volatile("prefetch.global.L1 [%0];" ::"l"(M.meta + t));
+        }
+        const unsigned b = __ballot_sync(0xffffffffu, pass);
+        const int at = beg - f0;  // this lane's first pair in the ballot
+        if (at > -32 && at < 32) todo |= at >= 0 ? b >> at : b << -at;
       }
+      todo &= na >= 32 ? 0xffffffffu : (1u << na) - 1u;
     }
     const int cnt = __popc(todo);
     const int inc = warp_incl_scan(cnt);
@@ -1017,7 +1067,7 @@ __device__ __forceinline__ void wall_tile(const Sys &s, const AtomArrays &A, int
     double msum[3] = {0., 0., 0.};
     double *const wf = s.wforce + (size_t)(3 * (s.nplanes + k)) * nmax;
     if (total > cap) {  // sequential path for this tile
-      if (nc > 0) mesh_contacts<NORMAL>(s, A, i, k, shearupdate, v, om, xv, fx, fy, fz, tx, ty, tz, meshbad, msum);
+      if (nc > 0) sequential(msum);
       if (valid)
         for (int d = 0; d < 3; d++) wf[(size_t)d * nmax + i] = msum[d];
       __syncwarp();
@@ -1039,11 +1089,8 @@ __device__ __forceinline__ void wall_tile(const Sys &s, const AtomArrays &A, int
       const double *g = M.tri + (size_t)t * kTriStride;
       const double xe[3] = {A.x[ie], A.y[ie], A.z[ie]};
       const double re = A.r[ie];
-      const double reach_e = __dmul_rn(__dadd_rn(re, fmax(0.0, __dmul_rn(cdm1, re))), 1.0 + 1e-9);
       int state = 0;
-      const double *snv = tri_sn(g), *n0 = tri_node(g, 0);
-      const double dn = snv[0] * (xe[0] - n0[0]) + snv[1] * (xe[1] - n0[1]) + snv[2] * (xe[2] - n0[2]);
-      if (!(fabs(dn) > reach_e)) {
+      {
         double delta[3], bary[3];
         int bs;
         const double deltan = resolve_tri_sphere(g, M.meta[t], re, xe, delta, bary, bs);
@@ -1063,36 +1110,40 @@ __device__ __forceinline__ void wall_tile(const Sys &s, const AtomArrays &A, int
     // ---- C: slot semantics per atom, in candidate order
     bool fallback = big;
     unsigned keep = 0u;
+    unsigned occ = 0u;  // slots in use
     int stl[kMeshFastCand];
     bool work = np > 0 && !big;
     for (int e = off; e < off + cnt; e++) work |= (w.st[e] & 1) != 0;
     if (work) {
-      for (int u = 0; u < nc; u++) stl[u] = st[u * nmax + i];
       unsigned fresh = 0u;
+#pragma unroll 4
+      for (int u = 0; u < nc; u++) {
+        const int v = st[u * nmax + i];
+        stl[u] = v;
+        occ |= (v >= 0 ? 1u : 0u) << u;
+      }
       for (int e = off; e < off + cnt && !fallback; e++) {
         if (!(w.st[e] & 1)) continue;
         const int t = M.cand[(size_t)w.qq[e] * nmax + i];
         int slot = -1;
-        for (int u = 0; u < nc; u++)
-          if (stl[u] == t) { slot = u; break; }
+        for (unsigned m = occ; m; m &= m - 1u)
+          if (stl[__ffs(m) - 1] == t) { slot = __ffs(m) - 1; break; }
         if (slot >= 0) {
           keep |= 1u << slot;
         } else {
           const bool face = (w.st[e] & 2) != 0;
           if (face) {  // coplanarContactAlready
             bool already = false;
-            for (int u = 0; u < nc; u++)
-              if (stl[u] >= 0 && stl[u] != t && ((keep >> u) & 1u) && mesh_coplanar(M, stl[u], t)) already = true;
+            for (unsigned m = occ & keep; m; m &= m - 1u) already |= mesh_coplanar(M, stl[__ffs(m) - 1], t);
             if (already) continue;
           }
-          if (np >= nc) { meshbad = true; continue; }
-          for (int u = 0; u < nc; u++)
-            if (stl[u] == -1) { slot = u; break; }
+          slot = __ffs(~occ) - 1;
+          if (np >= nc || slot < 0 || slot >= nc) { meshbad = true; continue; }
           if (face)  // checkCoplanarContactHistory would copy: order-dependent
-            for (int u = 0; u < nc; u++)
-              if (stl[u] >= 0 && stl[u] != t && mesh_coplanar(M, stl[u], t)) fallback = true;
+            for (unsigned m = occ; m; m &= m - 1u) fallback |= mesh_coplanar(M, stl[__ffs(m) - 1], t);
           if (fallback) break;
           stl[slot] = t;
+          occ |= 1u << slot;
           keep |= 1u << slot;
           fresh |= 1u << slot;
           np++;
@@ -1102,11 +1153,11 @@ __device__ __forceinline__ void wall_tile(const Sys &s, const AtomArrays &A, int
       if (fallback) {
         for (int e = off; e < off + cnt; e++) w.st[e] &= 0xff;
       } else {
-        for (int u = 0; u < nc; u++)
-          if ((fresh >> u) & 1u) {
-            st[u * nmax + i] = stl[u];
-            for (int d = 0; d < 3; d++) sh[(3 * u + d) * nmax + i] = 0.0;
-          }
+        for (unsigned m = fresh; m; m &= m - 1u) {
+          const int u = __ffs(m) - 1;
+          st[u * nmax + i] = stl[u];
+          for (int d = 0; d < 3; d++) sh[(3 * u + d) * nmax + i] = 0.0;
+        }
       }
     }
     __syncwarp();
@@ -1132,7 +1183,7 @@ __device__ __forceinline__ void wall_tile(const Sys &s, const AtomArrays &A, int
     __syncwarp();
     // ---- E: sums in candidate order, clean-up (or the sequential path)
     if (fallback) {
-      mesh_contacts<NORMAL>(s, A, i, k, shearupdate, v, om, xv, fx, fy, fz, tx, ty, tz, meshbad, msum);
+      sequential(msum);
     } else if (work) {
       for (int e = off; e < off + cnt; e++) {
         if ((w.st[e] >> 8) == 0) continue;
@@ -1141,12 +1192,12 @@ __device__ __forceinline__ void wall_tile(const Sys &s, const AtomArrays &A, int
         tx += r[3]; ty += r[4]; tz += r[5];
         msum[0] += r[0]; msum[1] += r[1]; msum[2] += r[2];
       }
-      for (int u = 0; u < nc; u++)  // cleanUpContacts
-        if (!((keep >> u) & 1u) && stl[u] > -1) {
-          np--;
-          st[u * nmax + i] = -1;
-          for (int d = 0; d < 3; d++) sh[(3 * u + d) * nmax + i] = 0.0;
-        }
+      for (unsigned m = occ & ~keep; m; m &= m - 1u) {  // cleanUpContacts
+        const int u = __ffs(m) - 1;
+        np--;
+        st[u * nmax + i] = -1;
+        for (int d = 0; d < 3; d++) sh[(3 * u + d) * nmax + i] = 0.0;
+      }
       M.npart[0][i] = np;
     }
     if (valid)
