@@ -299,20 +299,25 @@ StepKernel step_kernel(const Sys &s, size_t *shared) {
 }  // namespace
 
 // Up to 330,000 list entries (about 115,000 spheres of a loose packing, 57,000
-// of a dense one).  Us per step, fused against separate kernels, on one GB300:
-//   loose column   20k spheres 18 / 30   100k 39 / 50   200k 68 / 77
-//   dense bed      20k 44 / 53           60k 86 / 87    150k 185 / 167
-//   hopper mesh    20k 41 / 51           50k 44 / 55    100k 59 / 57
-//   bonded fibres  10k 40 / 51           100k 179 / 199 200k 315 / 315
+// of a dense one), with mesh walls and no bonds up to 160,000.  Us per step,
+// fused against separate kernels, on one GB300:
+//   loose column   80k spheres 39 / 44   100k 45 / 48   120k 53 / 52   200k 74 / 73
+//   dense bed      15k 46 / 50           35k 66 / 65    50k 81 / 81    100k 150 / 127
+//   hooke          60k 24 / 32           99k 37 / 37    200k 65 / 58
+//   bonded fibres  30k 50 / 73           60k 93 / 113
+//   hopper mesh    20k 35 / 42           60k 42 / 42    80k 53 / 45    200k 105 / 80
+//   mixer mesh     40k 27 / 35           80k 38 / 39
 // Above it the separate kernels win: each is compiled for its own registers,
 // with twice the warps per SM to hide loads and fill the FP64 pipes, and the
-// nodes' latency is small beside them.  Ensembles decide per system
+// nodes' latency is small beside them; a mesh's wall kernel runs beside the pair
+// kernel, while here its tiles hold up the blocks that have them.  (With bonds
+// the pair law is the longer one.)  Ensembles decide per system
 // (decide_rebuild) and keep the separate kernels.
 // LIGGGHTS_GB300_FUSED_STEPS=0|1: never, always (tests).
 bool fused_steps(const Sys &s, const LaunchCfg &lc) {
   if (s.nsys) return false;
   if (const char *e = getenv("LIGGGHTS_GB300_FUSED_STEPS")) return atoi(e) != 0;
-  return lc.np <= 330000;
+  return lc.np <= (s.nmeshes > 0 && !s.bond ? 160000 : 330000);
 }
 
 cudaError_t launch_steps(const Sys &s, const LaunchCfg &lc, cudaGraphConditionalHandle hreb,
