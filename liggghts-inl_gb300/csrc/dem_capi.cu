@@ -29,6 +29,30 @@ static_assert(kMaxScan < (1L << 24), "the neighbour stash packs atom indices in 
 constexpr long kMaxCells = 16000000L;
 }  // namespace
 
+// One device allocation that its user sizes again and again: an upload of the
+// same number of atoms finds its arrays where they were (five allocations and
+// their releases took 0.3 ms of a 300,000-atom upload's 1.1, and the step graph,
+// which holds the pointers, was built anew).  Never kept at more than twice the
+// need plus 1 MB.
+struct Slab {
+  void *p = nullptr;
+  size_t cap = 0;
+  void release() {
+    if (p) cudaFree(p);
+    p = nullptr;
+    cap = 0;
+  }
+  bool fits(size_t need) const { return p && cap >= need && cap <= 2 * need + (1u << 20); }
+  cudaError_t fit(size_t need) {
+    if (fits(need)) return cudaSuccess;
+    release();
+    cudaError_t e = cudaMalloc(&p, need);
+    if (e != cudaSuccess) p = nullptr;
+    else cap = need;
+    return e;
+  }
+};
+
 struct dem_handle {
   dem_config cfg{};
   Sys s{};
@@ -37,8 +61,9 @@ struct dem_handle {
   int device = 0;
   std::string err;
   bool have_params = false, have_atoms = false, setup_done = false;
-  std::vector<void *> allocs_atoms, allocs_pairs, allocs_misc, allocs_cells;
-  std::vector<void *> allocs_mslots[kMaxMeshes], allocs_tclist[kMaxMeshes];  // grown on overflow
+  std::vector<void *> allocs_misc;
+  Slab atoms_slab, pairs_slab, cells_slab;
+  Slab mslots_slab[kMaxMeshes], tclist_slab[kMaxMeshes];  // grown on overflow
   // atom transfers: kernels read and write the caller's arrays directly
   // when the device reaches pageable host memory through the host's page
   // tables (cudaDevAttrPageableMemoryAccessUsesHostPageTables, Grace
@@ -65,7 +90,8 @@ struct dem_handle {
   bool use_graph = true;
   cudaStream_t st2 = nullptr;
   cudaGraphExec_t gexec = nullptr;
-  long long graph_gen = -1, sys_gen = 0;  // rebuilt when device pointers change
+  long long graph_gen = -1, sys_gen = 0;  // looked at again when something that it holds may have changed
+  std::vector<unsigned char> graph_holds;  // what it was built from (see ensure_graph)
   StepCounts graph_counts;
   std::vector<MeshHost> mesh_host;
   std::vector<double> bond_tables;  // host copy for the cutoff derivation
@@ -82,17 +108,28 @@ struct dem_handle {
 
 static int ensure_graph(dem_handle *h) {
   if (h->gexec && h->graph_gen == h->sys_gen) return DEM_OK;
+  h->lc.np = h->host_ctrl.np;
+  // the kernels' arguments and the launch settings: the same bytes give the
+  // same graph (0.25 ms to build), as after the next upload of as many atoms
+  const int cfg[4] = {h->lc.max_grid, h->lc.particle_threads, h->lc.sms, step_loop_key(h->s, h->lc)};
+  std::vector<unsigned char> holds(sizeof(Sys) + sizeof cfg);
+  std::memcpy(holds.data(), &h->s, sizeof(Sys));
+  std::memcpy(holds.data() + sizeof(Sys), cfg, sizeof cfg);
+  if (h->gexec && holds == h->graph_holds) {
+    h->graph_gen = h->sys_gen;
+    return DEM_OK;
+  }
   if (h->gexec) {
     cudaGraphExecDestroy(h->gexec);
     h->gexec = nullptr;
   }
-  h->lc.np = h->host_ctrl.np;
   cudaError_t e = build_step_graph(h->s, h->lc, h->st, h->st2, &h->gexec, &h->graph_counts);
   if (e != cudaSuccess) {
     h->err = std::string("build_step_graph: ") + cudaGetErrorString(e);
     return DEM_ERR_CUDA;
   }
   h->graph_gen = h->sys_gen;
+  h->graph_holds.swap(holds);
   return DEM_OK;
 }
 
@@ -159,13 +196,10 @@ struct Arena {
     if (base) *p = reinterpret_cast<T *>(base + off);
     off += std::max<size_t>(n, 1) * sizeof(T);
   }
-  cudaError_t commit(std::vector<void *> &list) {
-    void *q = nullptr;
-    cudaError_t e = cudaMalloc(&q, std::max<size_t>(off, 256));
-    if (e == cudaSuccess) {
-      list.push_back(q);
-      base = static_cast<char *>(q);
-    }
+  size_t need() const { return std::max<size_t>(off, 256); }
+  cudaError_t commit(Slab &slab) {
+    cudaError_t e = slab.fit(need());
+    if (e == cudaSuccess) base = static_cast<char *>(slab.p);
     off = 0;
     return e;
   }
@@ -185,7 +219,6 @@ static int alloc_mesh_slots(dem_handle *h, int k, int cap, bool keep) {
   MeshDev &M = s.meshes[k];
   const size_t nmax = s.nmax;
   MeshDev N = M;
-  std::vector<void *> nl;
   auto carve = [&](Arena &ar) {
     ar.take(&N.cand_n, nmax);
     ar.take(&N.cand, (size_t)cap * nmax);
@@ -198,7 +231,9 @@ static int alloc_mesh_slots(dem_handle *h, int k, int cap, bool keep) {
   };
   Arena ar;
   carve(ar);
-  CUDA_TRY(h, ar.commit(nl));
+  const bool reuse = !keep && h->mslots_slab[k].fits(ar.need());
+  Slab grown;  // beside the current arrays, which may be copied from
+  CUDA_TRY(h, ar.commit(reuse ? h->mslots_slab[k] : grown));
   carve(ar);
   const size_t old = keep ? (size_t)std::min(M.ccap, cap) : 0;
   if (keep) {
@@ -217,9 +252,11 @@ static int alloc_mesh_slots(dem_handle *h, int k, int cap, bool keep) {
   CUDA_TRY(h, cudaMemsetAsync(N.slot_tri[0] + old * nmax, 0xff, ((size_t)cap - old) * nmax * sizeof(int), h->st));
   CUDA_TRY(h, cudaMemsetAsync(N.slot_hist[0] + 3 * old * nmax, 0, 3 * ((size_t)cap - old) * nmax * sizeof(double),
                               h->st));
-  CUDA_TRY(h, cudaStreamSynchronize(h->st));  // the old arrays are read until here
-  free_list(h->allocs_mslots[k]);
-  h->allocs_mslots[k] = nl;
+  if (!reuse) {
+    CUDA_TRY(h, cudaStreamSynchronize(h->st));  // the old arrays are read until here
+    h->mslots_slab[k].release();
+    h->mslots_slab[k] = grown;
+  }
   M.cand_n = N.cand_n;
   M.cand = N.cand;
   for (int b = 0; b < 2; b++) {
@@ -237,20 +274,21 @@ static int alloc_mesh_slots(dem_handle *h, int k, int cap, bool keep) {
 // triangle lists) at M.tc_cap entries.
 static int alloc_tc_list(dem_handle *h, int k) {
   MeshDev &M = h->s.meshes[k];
-  std::vector<void *> nl;
-  int *p = nullptr;
-  CUDA_TRY(h, dalloc(nl, &p, (size_t)M.tc_cap));
-  CUDA_TRY(h, cudaStreamSynchronize(h->st));
-  free_list(h->allocs_tclist[k]);
-  h->allocs_tclist[k] = nl;
-  M.tc_list = p;
+  const size_t need = (size_t)M.tc_cap * sizeof(int);
+  if (!h->tclist_slab[k].fits(need)) {
+    Slab grown;
+    CUDA_TRY(h, grown.fit(need));
+    CUDA_TRY(h, cudaStreamSynchronize(h->st));
+    h->tclist_slab[k].release();
+    h->tclist_slab[k] = grown;
+  }
+  M.tc_list = static_cast<int *>(h->tclist_slab[k].p);
   h->sys_gen++;
   return DEM_OK;
 }
 
 static int alloc_atoms(dem_handle *h, int nmax) {
   Sys &s = h->s;
-  free_list(h->allocs_atoms);
   h->sys_gen++;
   s.nmax = nmax;
   auto carve = [&](Arena &ar) {
@@ -291,7 +329,7 @@ static int alloc_atoms(dem_handle *h, int nmax) {
   };
   Arena ar;
   carve(ar);
-  CUDA_TRY(h, ar.commit(h->allocs_atoms));
+  CUDA_TRY(h, ar.commit(h->atoms_slab));
   carve(ar);
   for (int b = 0; b < 2; b++) {
     PairArrays &P = s.pairs[b];
@@ -315,7 +353,6 @@ static int alloc_atoms(dem_handle *h, int nmax) {
 // block sums, the triangle-to-cell lists.
 static int alloc_cells(dem_handle *h) {
   Sys &s = h->s;
-  free_list(h->allocs_cells);
   auto carve = [&](Arena &ar) {
     ar.take(&s.cell_count, (size_t)s.ncell + 2);
     ar.take(&s.cell_start, (size_t)s.ncell + 2);
@@ -331,7 +368,7 @@ static int alloc_cells(dem_handle *h) {
   };
   Arena ar;
   carve(ar);
-  CUDA_TRY(h, ar.commit(h->allocs_cells));
+  CUDA_TRY(h, ar.commit(h->cells_slab));
   carve(ar);
   for (int k = 0; k < s.nmeshes; k++) {
     int rc = alloc_tc_list(h, k);
@@ -356,7 +393,6 @@ static int ensure_stage(dem_handle *h, size_t bytes) {
 // (Re)allocates every pcap-sized array; keeps the current list (pairs[0]).
 static int alloc_pairs(dem_handle *h, int pcap, int keep_np) {
   Sys &s = h->s;
-  std::vector<void *> nl;
   PairArrays np_[2];
   double *rres = nullptr;
   uint8_t *act = nullptr;
@@ -379,7 +415,9 @@ static int alloc_pairs(dem_handle *h, int pcap, int keep_np) {
   };
   Arena ar;
   carve(ar);
-  CUDA_TRY(h, ar.commit(nl));
+  const bool reuse = keep_np == 0 && h->pairs_slab.fits(ar.need());
+  Slab grown;  // beside the current list, which may be copied from
+  CUDA_TRY(h, ar.commit(reuse ? h->pairs_slab : grown));
   carve(ar);
   if (keep_np > 0 && s.pcap > 0) {
     const PairArrays &O = s.pairs[0];
@@ -397,8 +435,10 @@ static int alloc_pairs(dem_handle *h, int pcap, int keep_np) {
     CUDA_TRY(h, cudaMemcpyAsync(N.c1, O.c1, k * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
     CUDA_TRY(h, cudaMemcpyAsync(N.rev, O.rev, k * sizeof(int), cudaMemcpyDeviceToDevice, h->st));
   }
-  free_list(h->allocs_pairs);
-  h->allocs_pairs = nl;
+  if (!reuse) {
+    h->pairs_slab.release();
+    h->pairs_slab = grown;
+  }
   s.pairs[0] = np_[0];
   s.pairs[1] = np_[1];
   s.res = rres;
@@ -564,13 +604,11 @@ static inline int dev_hist_index(const Sys &s, int r) {
 int dem_destroy(dem_handle *h) {
   if (!h) return DEM_ERR_BAD_ARG;
   if (h->st) cudaStreamSynchronize(h->st);
-  free_list(h->allocs_pairs);
-  free_list(h->allocs_atoms);
   free_list(h->allocs_misc);
-  free_list(h->allocs_cells);
+  for (Slab *q : {&h->atoms_slab, &h->pairs_slab, &h->cells_slab}) q->release();
   for (int k = 0; k < kMaxMeshes; k++) {
-    free_list(h->allocs_mslots[k]);
-    free_list(h->allocs_tclist[k]);
+    h->mslots_slab[k].release();
+    h->tclist_slab[k].release();
   }
   if (h->stage) cudaFree(h->stage);
   if (h->chk_host) cudaFreeHost(h->chk_host);

@@ -81,6 +81,8 @@ int wall_cap_per_atom();
 // Whether dem_step runs the steps in k_steps (dem_steps.cu) rather than as
 // separate kernels, and its launch inside the step graph.
 bool fused_steps(const Sys &s, const LaunchCfg &lc);
+// what else the step graph depends on: 0 for the separate kernels, else k_steps' limit
+int step_loop_key(const Sys &s, const LaunchCfg &lc);
 cudaError_t launch_steps(const Sys &s, const LaunchCfg &lc, cudaGraphConditionalHandle hreb,
                          cudaGraphConditionalHandle hloop, cudaStream_t st);
 // Executable graph of the step loop (WHILE node over steps, IF node around

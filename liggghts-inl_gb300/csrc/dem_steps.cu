@@ -320,6 +320,13 @@ bool fused_steps(const Sys &s, const LaunchCfg &lc) {
   return lc.np <= (s.nmeshes > 0 && !s.bond ? 160000 : 330000);
 }
 
+static int barrier_polls() {
+  const char *polls = getenv("LIGGGHTS_GB300_BARRIER_POLLS");
+  return polls ? std::max(1, atoi(polls)) : kBarrierPolls;
+}
+
+int step_loop_key(const Sys &s, const LaunchCfg &lc) { return fused_steps(s, lc) ? barrier_polls() : 0; }
+
 cudaError_t launch_steps(const Sys &s, const LaunchCfg &lc, cudaGraphConditionalHandle hreb,
                          cudaGraphConditionalHandle hloop, cudaStream_t st) {
   size_t shared = 0;
@@ -343,8 +350,7 @@ cudaError_t launch_steps(const Sys &s, const LaunchCfg &lc, cudaGraphConditional
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const char *polls = getenv("LIGGGHTS_GB300_BARRIER_POLLS");
-  return cudaLaunchKernelEx(&cfg, k, s, wall_cap, polls ? std::max(1, atoi(polls)) : kBarrierPolls, hreb, hloop);
+  return cudaLaunchKernelEx(&cfg, k, s, wall_cap, barrier_polls(), hreb, hloop);
 }
 
 }  // namespace gb300
