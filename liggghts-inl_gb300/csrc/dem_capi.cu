@@ -588,6 +588,9 @@ int dem_create(const dem_config *cfg, dem_handle **out) {
   s.tdamp = cfg->tangential_damping;
   s.limitf = cfg->limit_force;
   s.gravity_on = cfg->gravity_on;
+  s.gcount = 0;
+  for (int d = 0; d < 3; d++)
+    if (s.g[d] != 0.0 || std::signbit(s.g[d])) s.gaxis[s.gcount++] = d;
   s.bond = cfg->cohesion_model == DEM_COHESION_BOND_NONLINEAR ? 1 : 0;
   s.dnum = s.bond ? kDnumBond : kDnumShear;
   *out = h;

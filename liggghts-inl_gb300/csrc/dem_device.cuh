@@ -283,6 +283,7 @@ struct Sys {
   int neigh_every, neigh_delay, neigh_check;
   int normal, rolling, tdamp, limitf;
   int gravity_on;
+  int gcount, gaxis[3];  // the components of g that are not +0
   double g[3];
   double charVel;
   int nplanes;

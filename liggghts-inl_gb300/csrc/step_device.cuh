@@ -520,16 +520,13 @@ __device__ __forceinline__ void pair_entry(const Sys &s, int q, int i, int j, in
   s.active[q] = 1;
 }
 
-// FP32 touching test of entry p (x, y, z, r refreshed by every drift): false
-// when the pair is apart by more than the bound of the FP32 rounding.
-__device__ __forceinline__ bool pf_test(const Sys &s, int np, int p, int &i, int &j, int &code) {
-  const PairArrays &L = s.pairs[0];
+// FP32 touching test of entry p between i and j (x, y, z, r refreshed by every
+// drift): false when the pair is apart by more than the bound of the FP32
+// rounding; code kHole: no entry.
+__device__ __forceinline__ bool pf_near(const Sys &s, int np, int p, int i, int j, int code) {
   const float hi_f = 1.0f + s.pf_margin_touch;
   bool maybe = false;
-  code = p < np ? L.sh[p] : kHole;
   if (code != kHole) {
-    i = L.i[p];
-    j = L.j[p];
     const float4 a = s.xf[i], b = s.xf[j];
     float sx = 0.f, sy = 0.f, sz = 0.f;
     if (code != kNoShift) {
@@ -543,6 +540,17 @@ __device__ __forceinline__ bool pf_test(const Sys &s, int np, int p, int &i, int
   }
   if (!maybe && p < np) s.active[p] = 0;
   return maybe;
+}
+__device__ __forceinline__ void pf_load(const Sys &s, int np, int p, int &i, int &j, int &code) {
+  const PairArrays &L = s.pairs[0];
+  const bool on = p < np;
+  code = on ? L.sh[p] : kHole;
+  i = on ? L.i[p] : 0;
+  j = on ? L.j[p] : 0;
+}
+__device__ __forceinline__ bool pf_test(const Sys &s, int np, int p, int &i, int &j, int &code) {
+  pf_load(s, np, p, i, j, code);
+  return pf_near(s, np, p, i, j, code);
 }
 
 template <int NORMAL, bool ROLL>
@@ -558,10 +566,13 @@ __device__ __forceinline__ int pf_tiles(const Sys &s, int np, int shearupdate, i
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
   int qn = 0;  // the same in every lane
-  for (int base = next(); base < np; base = next()) {
-    const int p = base + lane;
-    int i, j, code;
-    const bool maybe = pf_test(s, np, p, i, j, code);
+  int base = next(), i = 0, j = 0, code = kHole;
+  if (base < np) pf_load(s, np, base + lane, i, j, code);
+  while (base < np) {
+    const int p = base + lane, pi = i, pj = j, pc = code;
+    base = next();
+    if (base < np) pf_load(s, np, base + lane, i, j, code);  // on its way during this tile's test
+    const bool maybe = pf_near(s, np, p, pi, pj, pc);
     const unsigned m = __ballot_sync(0xffffffffu, maybe);
     if (maybe) q[qn + __popc(m & below)] = p;
     qn += __popc(m);
@@ -1457,37 +1468,55 @@ __device__ __forceinline__ void gather_warp(const Sys &s, const int (*list)[32],
   __syncwarp();
 }
 
-// 2x of a normal double below the top of the range, by its exponent (exact;
-// the multiplication would hold the FP64 pipe)
+// 2x by the bits (exact; a multiplication, even one that is predicated off,
+// holds the FP64 pipe): the exponent up by one, a denormal's mantissa (or zero)
+// to the left, infinity from the top binade on
 __device__ __forceinline__ double twice(double x) {
-  const int hi = __double2hiint(x);
-  const unsigned e = hi & 0x7ff00000u;
-  if (e - 0x00100000u >= 0x7fd00000u) return 2.0 * x;  // zero, denormal, or the result out of range
-  return __hiloint2double(hi + 0x00100000, __double2loint(x));
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), e = hi & 0x7ff00000u;
+  unsigned h = hi + 0x00100000u, l = lo;
+  if (e == 0u) {
+    h = (hi & 0x80000000u) | (__funnelshift_l(lo, hi, 1) & 0x7fffffffu);
+    l = lo << 1;
+  } else if (e == 0x7fe00000u) {
+    h = (hi & 0x80000000u) | 0x7ff00000u;
+    l = 0u;
+  } else if (e == 0x7ff00000u) {
+    h = hi;
+  }
+  return __hiloint2double((int)h, (int)l);
 }
 
-// (float)x, round to nearest even, on the integer pipe (the conversion
-// instruction issues on the FP64 pipe): the top 24 bits of the mantissa, one
-// unit more where the rest says so; a carry runs into the exponent as it
-// should.  Results outside the normal range take the conversion.
+// (float)x on the integer pipe, for the FP32 copies of coordinates (the
+// conversion issues on the FP64 pipe, also predicated off): round to nearest
+// even, the top 24 bits of the mantissa and one unit more where the rest says
+// so; a carry runs into the exponent as it should.  Below 2^-126 zero; from
+// 2^127 on infinity, NaN included (a non-finite copy is what the check of the
+// coordinates looks for).
 __device__ __forceinline__ float to_float(double x) {
   const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
   const unsigned mag = hi & 0x7fffffffu;
-  // 2^-126 <= |x| < 2^127
-  if (mag - 0x38100000u >= 0x47e00000u - 0x38100000u) return (float)x;
   unsigned f = __funnelshift_l(lo, mag, 3) - (0x380u << 23);
   const unsigned rest = lo & 0x1fffffffu;
   f += (rest + 0x0fffffffu + (f & 1u)) >> 29;
+  if (mag < 0x38100000u) f = 0u;
+  if (mag >= 0x47e00000u) f = 0x7f800000u;
   return __uint_as_float(f | (hi & 0x80000000u));
 }
 
 // FixGravity::post_force (src/fix_gravity.cpp:329-337) adds m*g after the pair
 // forces; starting the sum from it instead changes only the rounding order and
 // saves three FP64 additions.  A component of +0 gives +0 without a product.
+// The components that are not +0 come first in s.gaxis: a loop, not three
+// conditions, whose products would issue predicated off.
 __device__ __forceinline__ void gravity_force(const Sys &s, double m, double &fx, double &fy, double &fz) {
-  if (__double_as_longlong(s.g[0]) != 0) fx = __dmul_rn(m, s.g[0]);
-  if (__double_as_longlong(s.g[1]) != 0) fy = __dmul_rn(m, s.g[1]);
-  if (__double_as_longlong(s.g[2]) != 0) fz = __dmul_rn(m, s.g[2]);
+#pragma unroll 1
+  for (int k = 0; k < s.gcount; k++) {
+    const int d = s.gaxis[k];
+    const double f = __dmul_rn(m, s.g[d]);
+    if (d == 0) fx = f;
+    if (d == 1) fy = f;
+    if (d == 2) fz = f;
+  }
 }
 
 // nve/sphere, FP32 copy and displacement check of atom i with its summed force
@@ -1570,7 +1599,8 @@ __device__ __forceinline__ void particle_finish(const Sys &s, int i, bool gather
 // dependent loads; measured against one lane per atom sorted over a block of
 // 256 (pipe 42-50 % busy, its warps all waiting for the same phase): 1,000,000
 // atoms in a hopper 101 -> 77 us, 400,000 packed 81 -> 71, 526,000 of an
-// ensemble 46 -> 39.  More blocks per SM (48 registers), larger batches and
+// ensemble 46 -> 39; and with no conversion, doubling or product issued in vain
+// (a quarter of its FP64 instructions were predicated off) 74, 70 and 36.  More blocks per SM (48 registers), larger batches and
 // prefetches of the atom's state were slower.
 // Called by all lanes of a warp, each with its atom i (valid or none).
 template <int T>
