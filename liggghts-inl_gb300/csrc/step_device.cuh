@@ -336,19 +336,25 @@ struct BandRest {
 // contact laws run on full warps.  The warps' remainders merge into one
 // block batch at the end.  Each entry's result goes to its own slot and
 // depends on no other entry, so the order changes no value.
+// entry p of the list; code kHole: none
+__device__ __forceinline__ void pf_load(const Sys &s, int np, int p, int &i, int &j, int &code) {
+  const PairArrays &L = s.pairs[0];
+  const bool on = p < np;
+  code = on ? L.sh[p] : kHole;
+  i = on ? L.i[p] : 0;
+  j = on ? L.j[p] : 0;
+}
 // Phase 1 of the general kernel for entry p: the exact distance, the flags and
 // histories of an entry that does not touch; true when phase 2 has to see it.
 template <bool BOND>
-__device__ __forceinline__ bool band_test(const Sys &s, int np, int p, double cdm, bool may_create, double &delx,
-                                          double &dely, double &delz, double &rsq) {
+__device__ __forceinline__ bool band_near(const Sys &s, int np, int p, int i, int j, int code, double cdm,
+                                          bool may_create, double &delx, double &dely, double &delz, double &rsq) {
   const AtomArrays &A = s.atoms[0];
   const PairArrays &L = s.pairs[0];
   const size_t P = s.pcap;
   bool queue = false;
-  const int code = p < np ? L.sh[p] : kHole;
   if (code == kHole && p < np) s.active[p] = 0;  // an unused entry of an ensemble segment
   if (code != kHole) {
-    const int i = L.i[p], j = L.j[p];
     double xj = A.x[j], yj = A.y[j], zj = A.z[j];
     image(s, code, xj, yj, zj);
     delx = __dadd_rn(A.x[i], -xj);
@@ -378,6 +384,14 @@ __device__ __forceinline__ bool band_test(const Sys &s, int np, int p, double cd
   return queue;
 }
 
+template <bool BOND>
+__device__ __forceinline__ bool band_test(const Sys &s, int np, int p, double cdm, bool may_create, double &delx,
+                                          double &dely, double &delz, double &rsq) {
+  int i, j, code;
+  pf_load(s, np, p, i, j, code);
+  return band_near<BOND>(s, np, p, i, j, code, cdm, may_create, delx, dely, delz, rsq);
+}
+
 // cohesion bond/nonlinear: a bond can be created in this pass
 template <bool BOND>
 __device__ __forceinline__ bool band_may_create(const Sys &s, int shearupdate, long long ntimestep) {
@@ -395,10 +409,14 @@ __device__ __forceinline__ int band_tiles(const Sys &s, int np, int shearupdate,
   const unsigned below = (1u << lane) - 1u;
   const bool may_create = band_may_create<BOND>(s, shearupdate, ntimestep);
   int qn = 0;  // the same in every lane
-  for (int base = next(); base < np; base = next()) {
-    const int p = base + lane;
+  int base = next(), i = 0, j = 0, code = kHole;
+  if (base < np) pf_load(s, np, base + lane, i, j, code);
+  while (base < np) {
+    const int p = base + lane, pi = i, pj = j, pc = code;
+    base = next();
+    if (base < np) pf_load(s, np, base + lane, i, j, code);  // on its way during this tile's test
     double delx = 0., dely = 0., delz = 0., rsq = 0.;
-    const bool queue = band_test<BOND>(s, np, p, cdm, may_create, delx, dely, delz, rsq);
+    const bool queue = band_near<BOND>(s, np, p, pi, pj, pc, cdm, may_create, delx, dely, delz, rsq);
     const unsigned m = __ballot_sync(0xffffffffu, queue);
     if (queue) {
       const int slot = qn + __popc(m & below);
@@ -540,13 +558,6 @@ __device__ __forceinline__ bool pf_near(const Sys &s, int np, int p, int i, int 
   }
   if (!maybe && p < np) s.active[p] = 0;
   return maybe;
-}
-__device__ __forceinline__ void pf_load(const Sys &s, int np, int p, int &i, int &j, int &code) {
-  const PairArrays &L = s.pairs[0];
-  const bool on = p < np;
-  code = on ? L.sh[p] : kHole;
-  i = on ? L.i[p] : 0;
-  j = on ? L.j[p] : 0;
 }
 __device__ __forceinline__ bool pf_test(const Sys &s, int np, int p, int &i, int &j, int &code) {
   pf_load(s, np, p, i, j, code);
