@@ -8,7 +8,7 @@
 // runs step after step, with a grid barrier where a kernel boundary was:
 //
 //   A  per atom: gather, gravity, wall totals, nve/sphere, displacement test
-//      (particle_tile); moving meshes advance on the grid's last warps
+//      (particle_warp); moving meshes advance on the grid's last warps
 //   -- barrier; every block takes the same rebuild decision; a rebuild ends
 //      the launch (the graph's IF node rebuilds, the WHILE node comes back,
 //      and the launch resumes with B)
