@@ -1404,6 +1404,26 @@ int dem_setup(dem_handle *h) {
   return DEM_OK;
 }
 
+// Calls of up to this many steps of a fused system launch k_steps from the
+// host, without a graph: a graph launch costs some 10 us more, and building the
+// graph 0.17 ms once, but a rebuild then waits for the host (30 us; one in some
+// 50 steps and more).
+constexpr int kDirectSteps = 8;
+
+// n steps of a fused system from `phase`, rebuilding as they ask for it
+static int direct_steps(dem_handle *h, int n, int phase, bool *resumed) {
+  for (;;) {
+    CUDA_TRY(h, launch_steps_direct(h->s, h->lc, n, phase, h->st));
+    h->kt.kernel_launches++;
+    CUDA_TRY(h, cudaEventRecord(h->ev1, h->st));
+    int rc = recover(h, resumed);
+    if (rc || *resumed || h->host_ctrl.step_phase != kStepForces) return rc;
+    // (a halt in the rebuild makes the launch behind it a no-op)
+    h->kt.kernel_launches += launch_rebuild(h->s, h->lc, h->st, 0);
+    n = -1;
+  }
+}
+
 int dem_step(dem_handle *h, int nsteps) {
   if (!h || nsteps < 0) return DEM_ERR_BAD_ARG;
   if (!h->setup_done) return fail(h, DEM_ERR_BAD_ARG, "dem_setup must precede dem_step");
@@ -1412,7 +1432,9 @@ int dem_step(dem_handle *h, int nsteps) {
   int rc = DEM_OK;
   const long long ts0 = h->host_ctrl.ntimestep;
   const bool graph = h->use_graph && !h->profile;
-  if (graph && (rc = ensure_graph(h))) return rc;
+  h->lc.np = h->host_ctrl.np;
+  const bool direct = graph && nsteps <= kDirectSteps && fused_steps(h->s, h->lc);
+  if (graph && !direct && (rc = ensure_graph(h))) return rc;
   CUDA_TRY(h, cudaEventRecord(h->ev0, h->st));
   long long done = 0;  // steps whose rebuild+pair stage has been queued
   bool first = true;
@@ -1445,7 +1467,11 @@ int dem_step(dem_handle *h, int nsteps) {
     first = false;
     const long long rb0 = h->host_ctrl.nrebuilds;
     const bool launched = graph && chunk > k0;
-    if (launched) {
+    bool resumed = false;
+    if (launched && direct) {
+      rc = direct_steps(h, (int)(chunk - k0), phase, &resumed);
+      if (rc) return rc;
+    } else if (launched) {
       h->kt.kernel_launches += launch_set_loop(h->s, (int)(chunk - k0), phase, h->st);
       CUDA_TRY(h, cudaGraphLaunch(h->gexec, h->st));
       CUDA_TRY(h, cudaEventRecord(h->ev1, h->st));
@@ -1464,10 +1490,11 @@ int dem_step(dem_handle *h, int nsteps) {
       }
     }
     CUDA_TRY(h, cudaGetLastError());
-    bool resumed = false;
-    rc = recover(h, &resumed);
-    if (rc) return rc;
-    if (launched) {
+    if (!(launched && direct)) {
+      rc = recover(h, &resumed);
+      if (rc) return rc;
+    }
+    if (launched && !direct) {
       const StepCounts &gc = h->graph_counts;
       const long long iters = std::min<long long>(chunk - k0, h->host_ctrl.ntimestep - (ts0 + done + k0));
       h->kt.kernel_launches += gc.call + std::max<long long>(0, iters - 1) * gc.step +
@@ -1487,7 +1514,7 @@ int dem_step(dem_handle *h, int nsteps) {
           h->kt.kernel_launches += launch_wall_force(h->s, h->lc, 1, h->st);
         }
       }
-      if (graph && (rc = ensure_graph(h))) return rc;  // device pointers changed
+      if (graph && !direct && (rc = ensure_graph(h))) return rc;  // device pointers changed
       done = h->host_ctrl.ntimestep - ts0;
     } else {
       done += chunk;

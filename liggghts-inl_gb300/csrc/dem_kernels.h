@@ -85,6 +85,8 @@ bool fused_steps(const Sys &s, const LaunchCfg &lc);
 int step_loop_key(const Sys &s, const LaunchCfg &lc);
 cudaError_t launch_steps(const Sys &s, const LaunchCfg &lc, cudaGraphConditionalHandle hreb,
                          cudaGraphConditionalHandle hloop, cudaStream_t st);
+// the same from the host, without a graph: n steps from `phase`, or (n < 0) on from where Ctrl says
+cudaError_t launch_steps_direct(const Sys &s, const LaunchCfg &lc, int n, int phase, cudaStream_t st);
 // Executable graph of the step loop (WHILE node over steps, IF node around
 // the rebuild); see dem_kernels.cu.  launch_set_loop sets what it runs.
 struct StepCounts {  // kernels of a graph launch: per call, per further step, per rebuild

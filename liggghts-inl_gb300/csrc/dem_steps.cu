@@ -120,6 +120,20 @@ template <int NORMAL, bool ROLL>
 __device__ __forceinline__ void queue_entry(const Sys &s, const StepQueue<kPathTouch> &q, int e, long long) {
   pair_entry<NORMAL, ROLL>(s, q.p[e], q.i[e], q.j[e], q.code[e], 1);
 }
+// How a launch of k_steps is driven: by a graph's conditionals (in_graph), or
+// from the host; n >= 0: steps and phase to start with, else Ctrl's.
+struct StepCall {
+  int in_graph, n, phase;
+  cudaGraphConditionalHandle hreb, hloop;
+};
+
+// the launch ended with a rebuild due (reb), or done
+__device__ __forceinline__ void step_conditionals(const StepCall &call, int reb) {
+  if (!call.in_graph) return;
+  cudaGraphSetConditional(call.hreb, reb ? 1u : 0u);
+  cudaGraphSetConditional(call.hloop, reb ? 1u : 0u);
+}
+
 template <int NORMAL, bool ROLL, int PATH>
 __device__ __forceinline__ void queue_entry(const Sys &s, const StepQueue<PATH> &q, int e, long long ts) {
   band_entry<NORMAL, ROLL, PATH == kPathBond>(s, q.p[e], q.d[0][e], q.d[1][e], q.d[2][e], q.d[3][e], 1, ts);
@@ -127,8 +141,7 @@ __device__ __forceinline__ void queue_entry(const Sys &s, const StepQueue<PATH> 
 
 template <int NORMAL, bool ROLL, int PATH>
 __global__ void __launch_bounds__(kStepThreads, 1)
-    k_steps(const __grid_constant__ Sys s, int wall_cap, int limit, cudaGraphConditionalHandle hreb,
-            cudaGraphConditionalHandle hloop) {
+    k_steps(const __grid_constant__ Sys s, int wall_cap, int limit, StepCall call) {
   constexpr int kStepWarps = kStepThreads / 32;
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ StepFlags fl;
@@ -136,10 +149,7 @@ __global__ void __launch_bounds__(kStepThreads, 1)
   Ctrl *c = s.ctrl;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, G = gridDim.x;
   if (c->halt) {
-    if (blockIdx.x == 0 && tid == 0) {
-      cudaGraphSetConditional(hreb, 0);
-      cudaGraphSetConditional(hloop, 0);
-    }
+    if (blockIdx.x == 0 && tid == 0) step_conditionals(call, 0);
     return;
   }
   StepShared<PATH> &sh = *reinterpret_cast<StepShared<PATH> *>(dyn);
@@ -153,7 +163,7 @@ __global__ void __launch_bounds__(kStepThreads, 1)
   }
   // the launch's constants, and the decision's state: the same in every block
   const int n = c->n, np = c->np, nl = c->nmlist;
-  int left = c->loop_left, phase = c->step_phase, ago = c->ago, force = c->force_rebuild;
+  int left = call.n >= 0 ? call.n : c->loop_left, phase = call.n >= 0 ? call.phase : c->step_phase, ago = c->ago, force = c->force_rebuild;
   long long ts = c->ntimestep;
   int reb = 0;
   unsigned long long seen = 0;  // the barrier's count behind the last one
@@ -255,8 +265,7 @@ __global__ void __launch_bounds__(kStepThreads, 1)
   if (!ok) {  // a wait gave up: the host reads the status (the counts stay as they are until the next upload)
     atomicExch(&c->status, kStatTimeout);
     c->halt = 1;
-    cudaGraphSetConditional(hreb, 0);
-    cudaGraphSetConditional(hloop, 0);
+    step_conditionals(call, 0);
     return;
   }
   // the last block to leave: every other one has read and passed everything
@@ -272,13 +281,12 @@ __global__ void __launch_bounds__(kStepThreads, 1)
   c->mesh_moved = 0;
   c->loop_left = left;
   c->step_phase = reb ? kStepForces : kStepDone;
-  cudaGraphSetConditional(hreb, reb ? 1u : 0u);
-  cudaGraphSetConditional(hloop, reb ? 1u : 0u);
+  step_conditionals(call, reb);
 }
 
 namespace {
 
-typedef void (*StepKernel)(Sys, int, int, cudaGraphConditionalHandle, cudaGraphConditionalHandle);
+typedef void (*StepKernel)(Sys, int, int, StepCall);
 
 StepKernel step_kernel(const Sys &s, size_t *shared) {
   const int path = s.bond ? kPathBond : (s.cdf == 1.0 ? kPathTouch : kPathBand);
@@ -327,17 +335,13 @@ static int barrier_polls() {
 
 int step_loop_key(const Sys &s, const LaunchCfg &lc) { return fused_steps(s, lc) ? barrier_polls() : 0; }
 
-cudaError_t launch_steps(const Sys &s, const LaunchCfg &lc, cudaGraphConditionalHandle hreb,
-                         cudaGraphConditionalHandle hloop, cudaStream_t st) {
+static cudaError_t launch_call(const Sys &s, const LaunchCfg &lc, const StepCall &call, cudaStream_t st) {
   size_t shared = 0;
   StepKernel k = step_kernel(s, &shared);
   const int wall_cap = s.nmeshes > 0 ? wall_cap_per_atom() * kWallTile : 0;
   shared += (size_t)(kStepThreads / 32) * wall_cap * kWallQ;
   cudaError_t e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
   if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kStepThreads, shared)) != cudaSuccess) return e;
-  if (per_sm < 1) return cudaErrorLaunchOutOfResources;
   // one block per SM; fewer for systems of fewer warps
   const int grid = std::max(1, std::min((s.nmax + 31) / 32, lc.sms));
   cudaLaunchConfig_t cfg = {};
@@ -350,7 +354,16 @@ cudaError_t launch_steps(const Sys &s, const LaunchCfg &lc, cudaGraphConditional
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k, s, wall_cap, barrier_polls(), hreb, hloop);
+  return cudaLaunchKernelEx(&cfg, k, s, wall_cap, barrier_polls(), call);
+}
+
+cudaError_t launch_steps(const Sys &s, const LaunchCfg &lc, cudaGraphConditionalHandle hreb,
+                         cudaGraphConditionalHandle hloop, cudaStream_t st) {
+  return launch_call(s, lc, StepCall{1, -1, 0, hreb, hloop}, st);
+}
+
+cudaError_t launch_steps_direct(const Sys &s, const LaunchCfg &lc, int n, int phase, cudaStream_t st) {
+  return launch_call(s, lc, StepCall{0, n, phase, 0, 0}, st);
 }
 
 }  // namespace gb300
