@@ -338,14 +338,17 @@ int step_loop_key(const Sys &s, const LaunchCfg &lc) { return fused_steps(s, lc)
 static cudaError_t launch_call(const Sys &s, const LaunchCfg &lc, const StepCall &call, cudaStream_t st) {
   size_t shared = 0;
   StepKernel k = step_kernel(s, &shared);
-  const int most = wall_cap_per_atom() * kWallTile, wall_cap = s.nmeshes > 0 ? most : 0;
-  const size_t queue = (size_t)(kStepThreads / 32) * kWallQ;  // per entry of wall_cap
+  // wall queues as long as asked for, or as fit (a fuller tile takes the
+  // sequential path, with the same result; 1 KB is for the static part)
+  const size_t queue = (size_t)(kStepThreads / 32) * kWallTile * kWallQ;  // per entry of a tile's atom
+  const int most = (int)std::min<size_t>(wall_cap_per_atom(), (226 * 1024 - shared) / queue);
+  const int wall_cap = s.nmeshes > 0 ? most * kWallTile : 0;
   // the limit belongs to the function, not to the launch: the same for every
   // system, so that threads that step different ones do not undercut each other
   cudaError_t e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)std::min<size_t>(shared + queue * most, 227 * 1024));
+                                       (int)(shared + queue * most));
   if (e != cudaSuccess) return e;
-  shared += queue * wall_cap;
+  shared += (size_t)(kStepThreads / 32) * kWallQ * wall_cap;
   // one block per SM; fewer for systems of fewer warps
   const int grid = std::max(1, std::min((s.nmax + 31) / 32, lc.sms));
   cudaLaunchConfig_t cfg = {};
