@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <cstdlib>
 
+#include "barrier_count.cuh"
 #include "dem_kernels.h"
 #include "step_device.cuh"
 
@@ -70,37 +71,33 @@ struct StepFlags {  // what thread 0 read behind the barrier
 // Grid barrier: every block adds to one 64-bit count and polls it (one trip to
 // L2 to arrive, one to see the last arrival: 2.3k cycles with 152 blocks; a
 // separate release flag took 3.2k, a flag per block that all blocks poll
-// 5.8k).  The arrivals fill the low 32 bits; a block with an atom that moved
-// more than skin/2 adds 2^32 as well, one with such a mesh node 2^48, so that
-// the wait also brings the movement flags.  `seen` is the count behind the
-// last barrier, the same in every block; the difference holds at most two
-// barriers' arrivals (no block passes the next barrier before this one has
-// arrived there), and only the barrier after the movement adds flags, so the
-// fields cannot run into one another.  False when a wait gave up.
+// 5.8k).  MOVEMENT: the barrier behind phase A, whose arrivals bring the
+// movement flags (see barrier_count.cuh).  `seen` is the same in every block.
+// False when a wait gave up.
+template <bool MOVEMENT>
 __device__ __forceinline__ bool grid_barrier(Ctrl *c, int blocks, int limit, unsigned long long &seen, int flags,
                                              StepFlags &fl) {
-  flags = __syncthreads_or(flags & 1) | (__syncthreads_or(flags & 2) ? 2 : 0);
+  if (MOVEMENT) flags = __syncthreads_or(flags & 1) | (__syncthreads_or(flags & 2) ? 2 : 0);
+  else __syncthreads();
   if (threadIdx.x == 0) {
-    unsigned long long add = 1ull, now, d;
-    if (flags & 1) add += 1ull << 32;
-    if (flags & 2) add += 1ull << 48;
+    const unsigned long long add = barrier_arrival(MOVEMENT ? flags : 0);
+    unsigned long long now;
     int ok = 1, polls = 0;
     asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&c->bar), "l"(add) : "memory");
     for (;;) {
       asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(&c->bar) : "memory");
-      d = now - seen;
-      if ((unsigned)d >= (unsigned)blocks) break;
+      if (barrier_full(now, seen, blocks)) break;
       if (++polls >= limit || *(volatile int *)&c->bar_abort) {
         *(volatile int *)&c->bar_abort = 1;
         ok = 0;
         break;
       }
     }
-    const unsigned up = (unsigned)(d >> 32);
+    const BarrierPass p = barrier_pass(now, seen, blocks, MOVEMENT);
     fl.ok = ok;
-    fl.moved = (up & 0xffffu) != 0;
-    fl.mesh_moved = (up >> 16) != 0;
-    fl.seen = seen + (unsigned long long)blocks + ((unsigned long long)up << 32);
+    fl.moved = p.moved;
+    fl.mesh_moved = p.mesh_moved;
+    fl.seen = p.seen;
   }
   __syncthreads();
   seen = fl.seen;
@@ -194,7 +191,7 @@ __global__ void __launch_bounds__(kStepThreads, 1)
         const int w = G * kStepWarps - 1 - warp_id;
         for (int t0 = 2 * w; t0 < M.ntri; t0 += 2 * G * kStepWarps) mm |= mesh_move_part(s, M, t0 + (lane >> 4), lane & 15);
       }
-      if (!(ok = grid_barrier(c, G, limit, seen, (moved ? 1 : 0) | (mm ? 2 : 0), fl))) break;
+      if (!(ok = grid_barrier<true>(c, G, limit, seen, (moved ? 1 : 0) | (mm ? 2 : 0), fl))) break;
       // Neighbor::decide (see decide_rebuild)
       ts++;
       if (force) {
@@ -255,7 +252,7 @@ __global__ void __launch_bounds__(kStepThreads, 1)
       }
       __syncthreads();
     }
-    if (!(ok = grid_barrier(c, G, limit, seen, 0, fl))) break;
+    if (!(ok = grid_barrier<false>(c, G, limit, seen, 0, fl))) break;
     left--;
   }
   if (__any_sync(0xffffffffu, bad) && lane == 0) atomicExch(&c->status, kStatNan);
