@@ -179,13 +179,21 @@ static __device__ bool bond_nonlinear(const Sys &s, const BondIn &b, double *h, 
     const double kc1 = bond_tab(s, kBondKcfn1, tp), k2 = bond_tab(s, kBondKfn2, tp);
     const double ku2 = bond_tab(s, kBondKufn2, tp), kc2 = bond_tab(s, kBondKcfn2, tp);
     const double q1 = bond_tab(s, kBondRatioFn1, tp);
-    double f;
-    if (kd < 0) {
+    double f = 0.0;
+    // The law of tension reaches into compression where dmin or its product
+    // with the ratio lies above zero: the latter after tension with an unloading
+    // stiffness below the loading one (dmin is reset at the next step).
+    const long long kn = order_key(dmin);
+    bool tension = kd < 0;
+    if (!tension && kn != 0) tension = kn > 0 || __double_as_longlong(bond_tab(s, kBondRatioFn2, tp)) < 0;
+    if (tension) {
       const double dc2 = bond_tab(s, kBondRatioFn2, tp) * dmin;
-      if (kd < order_key(dmin)) f = k2 * A * disp;
+      if (kd < kn) f = k2 * A * disp;
       else if (kd < order_key(dc2)) f = ku2 * A * disp + (k2 - ku2) * A * dmin;
-      else f = -kc2 * A * disp;
-    } else {
+      else if (kd < 0) f = -kc2 * A * disp;
+      else tension = false;
+    }
+    if (!tension) {
       const double dc1 = q1 * q1 * dmax, root = sqrt(fabs(disp));
       if (kd < order_key(dc1)) f = -kc1 * root;
       else if (kd < order_key(dmax)) f = ku1 * root + (k1 - ku1) * sqrt(fabs(dmax));
@@ -257,8 +265,8 @@ static __device__ bool bond_nonlinear(const Sys &s, const BondIn &b, double *h, 
     const double ttm = sqrt(tt[0] * tt[0] + tt[1] * tt[1] + tt[2] * tt[2]);
     const double maxSigma = bond_tab(s, kBondMaxSigma, tp) *
                             (((fl & kBondUseRatioTC) && kd < -tiny) ? bond_tab(s, kBondRatioTC, tp) : 1.0);
-    const bool nstress = order_key(maxSigma) < order_key(nfm / A + ttm * rb / I);
-    const bool tstress = order_key(bond_tab(s, kBondMaxTau, tp)) < order_key(tfm / A + ntm * rb / J);
+    const bool nstress = key_lt(order_key(maxSigma), nfm / A + ttm * rb / I);
+    const bool tstress = key_lt(order_key(bond_tab(s, kBondMaxTau, tp)), tfm / A + ntm * rb / J);
     if ((nstress || tstress) && update_history) {
       *flag &= ~kContactCohesion;
       h[0] = 0.;

@@ -108,11 +108,18 @@ __device__ __forceinline__ bool gt_nonneg(double a, double b) {
   return __double_as_longlong(a) > __double_as_longlong(b);
 }
 
-// A key that orders doubles as the comparison does, -0 and +0 alike (a NaN lies
-// beyond the infinities), for comparisons of any sign on the integer pipe.
+// A key that orders doubles as the comparison does, -0 and +0 alike, for
+// comparisons of any sign on the integer pipe.  A NaN lies beyond the infinity
+// of its sign: where one may come, key_lt says no to it, as the comparison does.
 __device__ __forceinline__ long long order_key(double x) {
   const long long b = __double_as_longlong(x);
   return b < 0 ? (long long)(0x8000000000000000ull - (unsigned long long)b) : b;
+}
+constexpr long long kInfKey = 0x7ff0000000000000ll;
+// a < b for a's key and a b that may be NaN
+__device__ __forceinline__ bool key_lt(long long a, double b) {
+  const long long k = order_key(b);
+  return a < k && k <= kInfKey;
 }
 
 // shear[3] is the tangential history, updated in place when update_history.

@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <string>
 #include <vector>
 
@@ -699,13 +700,21 @@ int dem_set_bond_params(dem_handle *h, const double *tables, const dem_bond_sett
     std::vector<double> all(tables, tables + (size_t)kBondTables * m);
     all.resize((size_t)(kBondTables + kBondDerived) * m);
     auto T = [&](int t, size_t q) { return tables[(size_t)t * m + q]; };
+    // The hysteresis of a law, (Ku - K)/(Ku + Kc).  With Ku = Kc = 0 it is
+    // infinite, and its product with an extreme of zero a NaN, which no value
+    // lies beyond; the largest finite number in its place gives a zero there and
+    // the same decisions (the extreme of the other sign is zero then, and the
+    // value between them).  With K = 0 as well the law gives zero whatever it is.
+    auto ratio = [&](int k, int ku, int kc, size_t q) {
+      const double r = (T(ku, q) - T(k, q)) / (T(ku, q) + T(kc, q));
+      if (std::isfinite(r)) return r;
+      return std::isnan(r) ? 0.0 : std::copysign(std::numeric_limits<double>::max(), r);
+    };
     for (size_t q = 0; q < m; q++) {
-      all[(size_t)kBondRatioTn * m + q] = (T(kBondKutn, q) - T(kBondKtn, q)) / (T(kBondKutn, q) + T(kBondKctn, q));
-      all[(size_t)kBondRatioTt * m + q] = (T(kBondKutt, q) - T(kBondKtt, q)) / (T(kBondKutt, q) + T(kBondKctt, q));
-      all[(size_t)kBondRatioFn1 * m + q] =
-          (T(kBondKufn1, q) - T(kBondKfn1, q)) / (T(kBondKufn1, q) + T(kBondKcfn1, q));
-      all[(size_t)kBondRatioFn2 * m + q] =
-          (T(kBondKufn2, q) - T(kBondKfn2, q)) / (T(kBondKufn2, q) + T(kBondKcfn2, q));
+      all[(size_t)kBondRatioTn * m + q] = ratio(kBondKtn, kBondKutn, kBondKctn, q);
+      all[(size_t)kBondRatioTt * m + q] = ratio(kBondKtt, kBondKutt, kBondKctt, q);
+      all[(size_t)kBondRatioFn1 * m + q] = ratio(kBondKfn1, kBondKufn1, kBondKcfn1, q);
+      all[(size_t)kBondRatioFn2 * m + q] = ratio(kBondKfn2, kBondKufn2, kBondKcfn2, q);
     }
     CUDA_TRY(h, cudaMemcpyAsync(h->s.bondp, all.data(), all.size() * sizeof(double), cudaMemcpyHostToDevice, h->st));
   }
