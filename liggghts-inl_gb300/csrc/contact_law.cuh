@@ -103,23 +103,29 @@ struct ContactOut {
 
 // a > b for doubles that are not negative, on the integer pipe (their bit
 // patterns order the same way; a DSETP and the selects behind it hold the FP64
-// pipe for 108 cycles per warp)
+// pipe for 108 cycles per warp).  Unsigned: no a is above a NaN b (a distance),
+// whose sign may be either.
 __device__ __forceinline__ bool gt_nonneg(double a, double b) {
-  return __double_as_longlong(a) > __double_as_longlong(b);
+  return (unsigned long long)__double_as_longlong(a) > (unsigned long long)__double_as_longlong(b);
 }
 
 // A key that orders doubles as the comparison does, -0 and +0 alike, for
 // comparisons of any sign on the integer pipe.  A NaN lies beyond the infinity
-// of its sign: where one may come, key_lt says no to it, as the comparison does.
+// of its sign: where one may come, key_lt and key_gt say no to it, as the
+// comparison does.
 __device__ __forceinline__ long long order_key(double x) {
   const long long b = __double_as_longlong(x);
   return b < 0 ? (long long)(0x8000000000000000ull - (unsigned long long)b) : b;
 }
 constexpr long long kInfKey = 0x7ff0000000000000ll;
-// a < b for a's key and a b that may be NaN
+// a < b for a's key and a b that may be NaN; a > b for such an a and b's key
 __device__ __forceinline__ bool key_lt(long long a, double b) {
   const long long k = order_key(b);
   return a < k && k <= kInfKey;
+}
+__device__ __forceinline__ bool key_gt(double a, long long b) {
+  const long long k = order_key(a);
+  return k > b && k <= kInfKey;
 }
 
 // shear[3] is the tangential history, updated in place when update_history.

@@ -135,8 +135,9 @@ __device__ __forceinline__ double resolve_tri_sphere(const double *g, int meta, 
   bary[1] = __dadd_rn(a, -__dmul_rn(b, c)) / __dmul_rn(tri_el(g, 0), oneMinCSqr);
   bary[2] = __dadd_rn(__dmul_rn(a, c), -b) / __dmul_rn(tri_el(g, 2), oneMinCSqr);
   bary[0] = __dadd_rn(__dadd_rn(1., -bary[1]), -bary[2]);
+  // (a line's coordinates may be NaN, which is beyond no limit)
   const long long lim = order_key(tri_lim(g));
-  const int bs = (order_key(bary[0]) > lim) + 2 * (order_key(bary[1]) > lim) + 4 * (order_key(bary[2]) > lim);
+  const int bs = key_gt(bary[0], lim) + 2 * key_gt(bary[1], lim) + 4 * key_gt(bary[2], lim);
   barySign = bs;
   const int ob = obtuse_index(meta);
   double d;
