@@ -670,10 +670,15 @@ int dem_set_pair_params(dem_handle *h, int ntypes, const double *Yeff, const dou
   }
   CUDA_TRY(h, dalloc(h->allocs_misc, &h->s.params, tab.size()));
   CUDA_TRY(h, cudaMemcpyAsync(h->s.params, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, h->st));
+  const bool running = h->setup_done && ntypes >= h->s.ntypes;  // (every atom's type is in the tables)
   h->s.ntypes = ntypes;
   h->s.charVel = charVel;
   h->have_params = true;
   h->sys_gen++;
+  if (running) {
+    h->kt.kernel_launches += launch_wall_consts(h->s, h->lc, h->st);
+    CUDA_TRY(h, cudaGetLastError());
+  }
   return DEM_OK;
 }
 

@@ -986,6 +986,35 @@ __device__ __forceinline__ int find_old(const Sys &s, const PairArrays &L, int o
   return -1;
 }
 
+// The contact constants of atom i with the walls that it is near (bits: its
+// primitive walls); whether there are any.
+__device__ __forceinline__ bool wall_consts_form(const Sys &s, int i, unsigned bits) {
+  const AtomArrays &A = s.atoms[0];
+  bool has = (bits & 0x7fu) != 0;
+  for (int w = 0; w < s.nplanes + s.nmeshes; w++) {
+    const bool mesh = w >= s.nplanes;
+    // (plane 7 shares its bit with the list mark, so that the wall tiles
+    // look at it for every listed atom)
+    const bool near = mesh ? s.meshes[w - s.nplanes].cand_n[i] > 0 : (w == 7 || ((bits >> w) & 1u));
+    has |= mesh && near;
+    if (!near) continue;
+    const int wt = mesh ? s.meshes[w - s.nplanes].wall_type : s.planes[w].wall_type;
+    const TypePair tp = load_typepair(s.params, s.ntypes, A.type[i], wt ? wt : A.type[i]);
+    double c0, c1;
+    if (s.normal == kHertz) contact_consts<kHertz>(tp, A.m[i], A.r[i], s.charVel, s.tdamp, c0, c1);
+    else contact_consts<kHooke>(tp, A.m[i], A.r[i], s.charVel, s.tdamp, c0, c1);
+    s.wcon[(size_t)(2 * w) * s.nmax + i] = c0;
+    s.wcon[(size_t)(2 * w + 1) * s.nmax + i] = c1;
+  }
+  return has;
+}
+
+// new pair parameters between two builds: the walls' contacts take them at the
+// next step (the pairs' constants belong to the list and stay until its build)
+__global__ void k_wall_consts(Sys s) {
+  GRID_STRIDE(i, s.ctrl->n) wall_consts_form(s, i, s.atoms[0].wbits[i]);
+}
+
 // atoms in a primitive wall's neighbour list or with candidate triangles on
 // any mesh: bit 7 of wbits and the compact list the wall kernel walks (its
 // order does not matter: one thread computes all of an atom's wall forces)
@@ -1002,23 +1031,7 @@ __global__ void __launch_bounds__(256) k_wall_list(Sys s) {
     const int i = base + threadIdx.x;
     bool has = false;
     if (i < n) {
-      const unsigned bits = A.wbits[i];
-      has = (bits & 0x7fu) != 0;
-      for (int w = 0; w < s.nplanes + s.nmeshes; w++) {
-        const bool mesh = w >= s.nplanes;
-        // (plane 7 shares its bit with the list mark, so that the wall tiles
-        // look at it for every listed atom)
-        const bool near = mesh ? s.meshes[w - s.nplanes].cand_n[i] > 0 : (w == 7 || ((bits >> w) & 1u));
-        has |= mesh && near;
-        if (!near) continue;
-        const int wt = mesh ? s.meshes[w - s.nplanes].wall_type : s.planes[w].wall_type;
-        const TypePair tp = load_typepair(s.params, s.ntypes, A.type[i], wt ? wt : A.type[i]);
-        double c0, c1;
-        if (s.normal == kHertz) contact_consts<kHertz>(tp, A.m[i], A.r[i], s.charVel, s.tdamp, c0, c1);
-        else contact_consts<kHooke>(tp, A.m[i], A.r[i], s.charVel, s.tdamp, c0, c1);
-        s.wcon[(size_t)(2 * w) * s.nmax + i] = c0;
-        s.wcon[(size_t)(2 * w + 1) * s.nmax + i] = c1;
-      }
+      has = wall_consts_form(s, i, A.wbits[i]);
       A.wbits[i] = has ? (uint8_t)(A.wbits[i] | 0x80u) : (uint8_t)(A.wbits[i] & 0x7fu);
     }
     const unsigned m = __ballot_sync(0xffffffffu, has);
@@ -1878,6 +1891,12 @@ int scan_exclusive(const Sys &s, const int *in, int *out, int len, int *tmp, int
   k_scan_blocks<<<1, 1024, 0, st>>>(s, tmp, tmp, nb, nullptr, gate);
   k_scan_add<<<nb, 256, 0, st>>>(s, out, len, tmp, gate);
   return 3;
+}
+
+int launch_wall_consts(const Sys &s, const LaunchCfg &lc, cudaStream_t st) {
+  if (s.nplanes == 0 && s.nmeshes == 0) return 0;
+  k_wall_consts<<<grid_for(s.nmax, 256, lc.max_grid), 256, 0, st>>>(s);
+  return 1;
 }
 
 // one block: one thread per ensemble system (up to 256 at a time)

@@ -74,6 +74,8 @@ int launch_set_loop(const Sys &s, int n, int phase, cudaStream_t st);
 // wall (plane and mesh) forces of the current state, before the particle
 // kernel that gathers the step's forces; none without walls
 int launch_wall_force(const Sys &s, const LaunchCfg &lc, int shearupdate, cudaStream_t st, int gate = 0);
+// the wall contacts' constants anew (the pair parameters changed since the build)
+int launch_wall_consts(const Sys &s, const LaunchCfg &lc, cudaStream_t st);
 // fix move/mesh: moves the moving meshes by one step (after the drift)
 int launch_mesh_move(const Sys &s, const LaunchCfg &lc, cudaStream_t st, int gate = 0);
 // queue entries of the wall kernel per tile atom (LIGGGHTS_GB300_WALL_CAP)
