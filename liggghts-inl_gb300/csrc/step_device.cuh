@@ -711,6 +711,8 @@ __device__ __forceinline__ bool plane_contact_fast(const Sys &s, const AtomArray
   if (-deltan > s.cutneighmax) return true;
   double *h = A.whist + (size_t)(w * 3) * s.nmax + i;
   const size_t hs = s.nmax;
+  // a restart's history may have a normal part, which counts until the first update
+  if (!shearupdate && (__double_as_longlong(h[n * hs]) << 1) != 0) return false;
   if (!(deltan >= 0)) {  // not touching: the history ends (surfacesClose)
     h[0] = 0.0; h[hs] = 0.0; h[2 * hs] = 0.0;
     return true;
