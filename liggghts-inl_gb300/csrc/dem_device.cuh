@@ -75,8 +75,8 @@ struct AtomArrays {
   int *type, *tag;
   int *lidx;                // the atom's index in the caller's (reference's) local order
   double *whist;            // [(w*3+d)*nmax + i]
-  uint8_t *wbits;           // bit w: atom in primitive wall w's neighbour list;
-                            // bit 7: atom has candidate mesh triangles
+  uint8_t *wbits;           // bit w: atom in primitive wall w's neighbour list; bit 7 (behind k_wall_list):
+                            // atom listed for the wall tiles (the eighth plane is looked at for all of those)
   double *fmx, *fmy, *fmz, *tmx, *tmy, *tmz;  // mesh wall force/torque of the step (bit 7 atoms)
 };
 

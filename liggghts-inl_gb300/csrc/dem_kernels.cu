@@ -987,10 +987,12 @@ __device__ __forceinline__ int find_old(const Sys &s, const PairArrays &L, int o
 }
 
 // The contact constants of atom i with the walls that it is near (bits: its
-// primitive walls); whether there are any.
+// primitive walls); whether there are any.  Bit 7 is the eighth plane's behind
+// k_permute and the list mark behind k_wall_list (of a system that does not
+// rebuild, the mark of the build before): a reason to be listed either way.
 __device__ __forceinline__ bool wall_consts_form(const Sys &s, int i, unsigned bits) {
   const AtomArrays &A = s.atoms[0];
-  bool has = (bits & 0x7fu) != 0;
+  bool has = bits != 0;
   for (int w = 0; w < s.nplanes + s.nmeshes; w++) {
     const bool mesh = w >= s.nplanes;
     // (plane 7 shares its bit with the list mark, so that the wall tiles
