@@ -1503,7 +1503,7 @@ __device__ __forceinline__ double twice(double x) {
 // conversion issues on the FP64 pipe, also predicated off): round to nearest
 // even, the top 24 bits of the mantissa and one unit more where the rest says
 // so; a carry runs into the exponent as it should.  Below 2^-126 zero; from
-// 2^127 on infinity, NaN included (a non-finite copy is what the check of the
+// 2^128 on infinity, NaN included (a non-finite copy is what the check of the
 // coordinates looks for).
 __device__ __forceinline__ float to_float(double x) {
   const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
@@ -1512,7 +1512,7 @@ __device__ __forceinline__ float to_float(double x) {
   const unsigned rest = lo & 0x1fffffffu;
   f += (rest + 0x0fffffffu + (f & 1u)) >> 29;
   if (mag < 0x38100000u) f = 0u;
-  if (mag >= 0x47e00000u) f = 0x7f800000u;
+  if (mag >= 0x47f00000u) f = 0x7f800000u;
   return __uint_as_float(f | (hi & 0x80000000u));
 }
 
