@@ -92,6 +92,7 @@ struct dem_handle {
   cudaStream_t st2 = nullptr;
   cudaGraphExec_t gexec = nullptr;
   long long graph_gen = -1, sys_gen = 0;  // looked at again when something that it holds may have changed
+  int graph_key = 0;                       // its step_loop_key
   std::vector<unsigned char> graph_holds;  // what it was built from (see ensure_graph)
   StepCounts graph_counts;
   std::vector<MeshHost> mesh_host;
@@ -108,16 +109,17 @@ struct dem_handle {
 };
 
 static int ensure_graph(dem_handle *h) {
-  if (h->gexec && h->graph_gen == h->sys_gen) return DEM_OK;
-  h->lc.np = h->host_ctrl.np;
+  const int key = step_loop_key(h->lc);
+  if (h->gexec && h->graph_gen == h->sys_gen && h->graph_key == key) return DEM_OK;
   // the kernels' arguments and the launch settings: the same bytes give the
   // same graph (0.25 ms to build), as after the next upload of as many atoms
-  const int cfg[4] = {h->lc.max_grid, h->lc.particle_threads, h->lc.sms, step_loop_key(h->s, h->lc)};
+  const int cfg[4] = {h->lc.max_grid, h->lc.particle_threads, h->lc.sms, key};
   std::vector<unsigned char> holds(sizeof(Sys) + sizeof cfg);
   std::memcpy(holds.data(), &h->s, sizeof(Sys));
   std::memcpy(holds.data() + sizeof(Sys), cfg, sizeof cfg);
   if (h->gexec && holds == h->graph_holds) {
     h->graph_gen = h->sys_gen;
+    h->graph_key = key;
     return DEM_OK;
   }
   if (h->gexec) {
@@ -130,6 +132,7 @@ static int ensure_graph(dem_handle *h) {
     return DEM_ERR_CUDA;
   }
   h->graph_gen = h->sys_gen;
+  h->graph_key = key;
   h->graph_holds.swap(holds);
   return DEM_OK;
 }
@@ -1447,7 +1450,8 @@ int dem_step(dem_handle *h, int nsteps) {
   const long long ts0 = h->host_ctrl.ntimestep;
   const bool graph = h->use_graph && !h->profile;
   h->lc.np = h->host_ctrl.np;
-  const bool direct = graph && nsteps <= kDirectSteps && fused_steps(h->s, h->lc);
+  h->lc.fused = graph && fused_steps(h->s, h->lc);
+  const bool direct = h->lc.fused && nsteps <= kDirectSteps;
   if (graph && !direct && (rc = ensure_graph(h))) return rc;
   CUDA_TRY(h, cudaEventRecord(h->ev0, h->st));
   long long done = 0;  // steps whose rebuild+pair stage has been queued

@@ -2143,7 +2143,7 @@ cudaError_t build_step_graph(const Sys &s, const LaunchCfg &lc, cudaStream_t st,
   *counts = StepCounts{};
   cudaGraph_t body;
   if ((e = b.begin(b.g)) != cudaSuccess) return b.fail(e);
-  if (fused_steps(s, lc)) {
+  if (lc.fused) {
     if ((e = b.conditional(hloop, cudaGraphCondTypeWhile, &body)) != cudaSuccess) return b.fail(e);
     if ((e = b.end()) != cudaSuccess) return b.fail(e);
     if ((e = b.begin(body)) != cudaSuccess) return b.fail(e);

@@ -11,6 +11,7 @@ struct LaunchCfg {
   int particle_threads = 256;  // threads per block of the per-particle kernel (64, 128, 256)
   int sms = 152;               // multiprocessors of the device
   int np = 0;                  // list entries at the last build (what fused_steps goes by)
+  bool fused = false;          // the call runs in k_steps (dem_step's choice by fused_steps)
 };
 
 enum {
@@ -81,10 +82,11 @@ int launch_mesh_move(const Sys &s, const LaunchCfg &lc, cudaStream_t st, int gat
 // queue entries of the wall kernel per tile atom (LIGGGHTS_GB300_WALL_CAP)
 int wall_cap_per_atom();
 // Whether dem_step runs the steps in k_steps (dem_steps.cu) rather than as
-// separate kernels, and its launch inside the step graph.
+// separate kernels (lc.fused: the choice before), and its launch inside the
+// step graph.
 bool fused_steps(const Sys &s, const LaunchCfg &lc);
 // what else the step graph depends on: 0 for the separate kernels, else k_steps' limit
-int step_loop_key(const Sys &s, const LaunchCfg &lc);
+int step_loop_key(const LaunchCfg &lc);
 cudaError_t launch_steps(const Sys &s, const LaunchCfg &lc, cudaGraphConditionalHandle hreb,
                          cudaGraphConditionalHandle hloop, cudaStream_t st);
 // the same from the host, without a graph: n steps from `phase`, or (n < 0) on from where Ctrl says

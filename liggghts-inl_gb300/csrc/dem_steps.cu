@@ -317,12 +317,16 @@ StepKernel step_kernel(const Sys &s, size_t *shared) {
 // nodes' latency is small beside them; a mesh's wall kernel runs beside the pair
 // kernel, while here its tiles hold up the blocks that have them.  (With bonds
 // the pair law is the longer one.)  Ensembles decide per system
-// (decide_rebuild) and keep the separate kernels.
+// (decide_rebuild) and keep the separate kernels.  Asked at every call; a
+// system that runs fused stays so for another sixteenth (the two sides are a few
+// percent apart there), so that one at the limit does not build a graph (0.25
+// ms) call after call.
 // LIGGGHTS_GB300_FUSED_STEPS=0|1: never, always (tests).
 bool fused_steps(const Sys &s, const LaunchCfg &lc) {
   if (s.nsys) return false;
   if (const char *e = getenv("LIGGGHTS_GB300_FUSED_STEPS")) return atoi(e) != 0;
-  return lc.np <= (s.nmeshes > 0 && !s.bond ? 160000 : 330000);
+  const int limit = s.nmeshes > 0 && !s.bond ? 160000 : 330000;
+  return lc.np <= limit + (lc.fused ? limit / 16 : 0);
 }
 
 static int barrier_polls() {
@@ -330,7 +334,7 @@ static int barrier_polls() {
   return polls ? std::max(1, atoi(polls)) : kBarrierPolls;
 }
 
-int step_loop_key(const Sys &s, const LaunchCfg &lc) { return fused_steps(s, lc) ? barrier_polls() : 0; }
+int step_loop_key(const LaunchCfg &lc) { return lc.fused ? barrier_polls() : 0; }
 
 static cudaError_t launch_call(const Sys &s, const LaunchCfg &lc, const StepCall &call, cudaStream_t st) {
   size_t shared = 0;
