@@ -89,6 +89,7 @@ struct dem_handle {
   dem_kernel_times kt{};
   // graph-resident step loop
   bool use_graph = true;
+  bool steps_refused = false;  // a launch of k_steps was refused: the separate kernels from then on
   cudaStream_t st2 = nullptr;
   cudaGraphExec_t gexec = nullptr;
   long long graph_gen = -1, sys_gen = 0;  // looked at again when something that it holds may have changed
@@ -1403,6 +1404,7 @@ int dem_setup(dem_handle *h) {
   if (!h || !h->have_atoms) return DEM_ERR_BAD_ARG;
   cudaGetLastError();
   set_mesh_velocity_on(h, 0);  // FixMoveMesh::setup: node velocities 0
+  h->lc.coop = !h->steps_refused && (h->s.nsys || steps_resident(h->s, h->lc));
   h->kt.kernel_launches += launch_set_rebuild(h->s, 1, h->st);
   h->kt.kernel_launches += launch_rebuild(h->s, h->lc, h->st, 0);
   bool resumed = true;
@@ -1427,10 +1429,35 @@ int dem_setup(dem_handle *h) {
 // 50 steps and more).
 constexpr int kDirectSteps = 8;
 
-// n steps of a fused system from `phase`, rebuilding as they ask for it
+// The driver refused a launch of k_steps, or the graph with it (a grid that
+// cannot be resident, MPS, which allows no cooperative launch in a graph's
+// conditionals): nothing of it has run, and the separate kernels take over.
+static void leave_fused(dem_handle *h) {
+  cudaGetLastError();
+  h->steps_refused = true;
+  h->lc.coop = h->lc.fused = false;
+}
+
+// the step graph, of the separate kernels where that with k_steps cannot be had
+static int step_graph(dem_handle *h) {
+  int rc = ensure_graph(h);
+  if (rc && h->lc.fused) {
+    leave_fused(h);
+    rc = ensure_graph(h);
+  }
+  return rc;
+}
+
+// n steps of a fused system from `phase`, rebuilding as they ask for it.
+// lc.fused is off when a launch was refused: the first, before anything has
+// run, or (resumed) one behind a rebuild, whose step then lacks its forces.
 static int direct_steps(dem_handle *h, int n, int phase, bool *resumed) {
   for (;;) {
-    CUDA_TRY(h, launch_steps_direct(h->s, h->lc, n, phase, h->st));
+    if (launch_steps_direct(h->s, h->lc, n, phase, h->st) != cudaSuccess) {
+      leave_fused(h);
+      *resumed = n < 0;
+      return DEM_OK;
+    }
     h->kt.kernel_launches++;
     CUDA_TRY(h, cudaEventRecord(h->ev1, h->st));
     int rc = recover(h, resumed);
@@ -1451,8 +1478,8 @@ int dem_step(dem_handle *h, int nsteps) {
   const bool graph = h->use_graph && !h->profile;
   h->lc.np = h->host_ctrl.np;
   h->lc.fused = graph && fused_steps(h->s, h->lc);
-  const bool direct = h->lc.fused && nsteps <= kDirectSteps;
-  if (graph && !direct && (rc = ensure_graph(h))) return rc;
+  bool direct = h->lc.fused && nsteps <= kDirectSteps;
+  if (graph && !direct && (rc = step_graph(h))) return rc;
   CUDA_TRY(h, cudaEventRecord(h->ev0, h->st));
   long long done = 0;  // steps whose rebuild+pair stage has been queued
   bool first = true;
@@ -1489,11 +1516,24 @@ int dem_step(dem_handle *h, int nsteps) {
     if (launched && direct) {
       rc = direct_steps(h, (int)(chunk - k0), phase, &resumed);
       if (rc) return rc;
-    } else if (launched) {
+      if (!h->lc.fused) {
+        direct = false;
+        if ((rc = step_graph(h))) return rc;
+      }
+    }
+    const bool queued = launched && !direct && !resumed;
+    if (queued) {
       h->kt.kernel_launches += launch_set_loop(h->s, (int)(chunk - k0), phase, h->st);
-      CUDA_TRY(h, cudaGraphLaunch(h->gexec, h->st));
+      cudaError_t e = h->lc.fused && coop_refused(kCoopGraphLaunch) ? cudaErrorCooperativeLaunchTooLarge
+                                                                    : cudaGraphLaunch(h->gexec, h->st);
+      if (e != cudaSuccess && h->lc.fused) {
+        leave_fused(h);
+        if ((rc = step_graph(h))) return rc;
+        e = cudaGraphLaunch(h->gexec, h->st);
+      }
+      CUDA_TRY(h, e);
       CUDA_TRY(h, cudaEventRecord(h->ev1, h->st));
-    } else {
+    } else if (!launched) {
       for (long long k = k0; k < chunk; k++) {
         h->kt.kernel_launches += launch_particle(h->s, h->lc, kModeGatherFinalInitial, h->st);
         h->kt.kernel_launches += launch_mesh_move(h->s, h->lc, h->st);
@@ -1508,11 +1548,11 @@ int dem_step(dem_handle *h, int nsteps) {
       }
     }
     CUDA_TRY(h, cudaGetLastError());
-    if (!(launched && direct)) {
+    if (!launched || queued) {
       rc = recover(h, &resumed);
       if (rc) return rc;
     }
-    if (launched && !direct) {
+    if (queued) {
       const StepCounts &gc = h->graph_counts;
       const long long iters = std::min<long long>(chunk - k0, h->host_ctrl.ntimestep - (ts0 + done + k0));
       h->kt.kernel_launches += gc.call + std::max<long long>(0, iters - 1) * gc.step +
@@ -1532,7 +1572,7 @@ int dem_step(dem_handle *h, int nsteps) {
           h->kt.kernel_launches += launch_wall_force(h->s, h->lc, 1, h->st);
         }
       }
-      if (graph && !direct && (rc = ensure_graph(h))) return rc;  // device pointers changed
+      if (graph && !direct && (rc = step_graph(h))) return rc;  // device pointers changed
       done = h->host_ctrl.ntimestep - ts0;
     } else {
       done += chunk;

@@ -11,6 +11,7 @@ struct LaunchCfg {
   int particle_threads = 256;  // threads per block of the per-particle kernel (64, 128, 256)
   int sms = 152;               // multiprocessors of the device
   int np = 0;                  // list entries at the last build (what fused_steps goes by)
+  bool coop = true;            // k_steps' grid can be resident, and no launch of it was refused
   bool fused = false;          // the call runs in k_steps (dem_step's choice by fused_steps)
 };
 
@@ -85,6 +86,12 @@ int wall_cap_per_atom();
 // separate kernels (lc.fused: the choice before), and its launch inside the
 // step graph.
 bool fused_steps(const Sys &s, const LaunchCfg &lc);
+// whether all blocks of k_steps can be resident together, which its cooperative launch needs
+bool steps_resident(const Sys &s, const LaunchCfg &lc);
+// Refusals as the driver gives them (under MPS, say), for tests:
+// LIGGGHTS_GB300_COOP_REFUSE adds up what is refused.
+enum { kCoopGrid = 1, kCoopInGraph = 2, kCoopDirect = 4, kCoopResume = 8, kCoopGraphLaunch = 16 };
+bool coop_refused(int what);
 // what else the step graph depends on: 0 for the separate kernels, else k_steps' limit
 int step_loop_key(const LaunchCfg &lc);
 cudaError_t launch_steps(const Sys &s, const LaunchCfg &lc, cudaGraphConditionalHandle hreb,

@@ -323,7 +323,7 @@ StepKernel step_kernel(const Sys &s, size_t *shared) {
 // ms) call after call.
 // LIGGGHTS_GB300_FUSED_STEPS=0|1: never, always (tests).
 bool fused_steps(const Sys &s, const LaunchCfg &lc) {
-  if (s.nsys) return false;
+  if (s.nsys || !lc.coop) return false;
   if (const char *e = getenv("LIGGGHTS_GB300_FUSED_STEPS")) return atoi(e) != 0;
   const int limit = s.nmeshes > 0 && !s.bond ? 160000 : 330000;
   return lc.np <= limit + (lc.fused ? limit / 16 : 0);
@@ -336,33 +336,68 @@ static int barrier_polls() {
 
 int step_loop_key(const LaunchCfg &lc) { return lc.fused ? barrier_polls() : 0; }
 
-static cudaError_t launch_call(const Sys &s, const LaunchCfg &lc, const StepCall &call, cudaStream_t st) {
+bool coop_refused(int what) {
+  const char *e = getenv("LIGGGHTS_GB300_COOP_REFUSE");
+  return e && (atoi(e) & what);
+}
+
+namespace {
+
+struct StepLaunch {
+  StepKernel kernel = nullptr;
+  int grid = 0, wall_cap = 0;
   size_t shared = 0;
-  StepKernel k = step_kernel(s, &shared);
+};
+
+cudaError_t step_launch(const Sys &s, const LaunchCfg &lc, StepLaunch *l) {
+  size_t shared = 0;
+  l->kernel = step_kernel(s, &shared);
   // wall queues as long as asked for, or as fit (a fuller tile takes the
   // sequential path, with the same result; 1 KB is for the static part)
   const size_t queue = (size_t)(kStepThreads / 32) * kWallTile * kWallQ;  // per entry of a tile's atom
   const int most = (int)std::min<size_t>(wall_cap_per_atom(), (226 * 1024 - shared) / queue);
-  const int wall_cap = s.nmeshes > 0 ? most * kWallTile : 0;
+  l->wall_cap = s.nmeshes > 0 ? most * kWallTile : 0;
+  l->shared = shared + (size_t)(kStepThreads / 32) * kWallQ * l->wall_cap;
+  // one block per SM; fewer for systems of fewer warps
+  l->grid = std::max(1, std::min((s.nmax + 31) / 32, lc.sms));
   // the limit belongs to the function, not to the launch: the same for every
   // system, so that threads that step different ones do not undercut each other
-  cudaError_t e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)(shared + queue * most));
+  return cudaFuncSetAttribute((const void *)l->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)(shared + queue * most));
+}
+
+}  // namespace
+
+bool steps_resident(const Sys &s, const LaunchCfg &lc) {
+  if (coop_refused(kCoopGrid)) return false;
+  StepLaunch l;
+  int device = 0, coop = 0, blocks = 0;
+  const bool ok = cudaGetDevice(&device) == cudaSuccess &&
+                  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) == cudaSuccess &&
+                  step_launch(s, lc, &l) == cudaSuccess &&
+                  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, (const void *)l.kernel, kStepThreads,
+                                                                l.shared) == cudaSuccess;
+  if (!ok) cudaGetLastError();
+  return ok && coop && (long)blocks * lc.sms >= l.grid;
+}
+
+static cudaError_t launch_call(const Sys &s, const LaunchCfg &lc, const StepCall &call, cudaStream_t st) {
+  if (coop_refused(call.in_graph ? kCoopInGraph : (call.n < 0 ? kCoopResume : kCoopDirect)))
+    return cudaErrorCooperativeLaunchTooLarge;
+  StepLaunch l;
+  cudaError_t e = step_launch(s, lc, &l);
   if (e != cudaSuccess) return e;
-  shared += (size_t)(kStepThreads / 32) * kWallQ * wall_cap;
-  // one block per SM; fewer for systems of fewer warps
-  const int grid = std::max(1, std::min((s.nmax + 31) / 32, lc.sms));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = dim3(l.grid);
   cfg.blockDim = dim3(kStepThreads);
-  cfg.dynamicSmemBytes = shared;
+  cfg.dynamicSmemBytes = l.shared;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k, s, wall_cap, barrier_polls(), call);
+  return cudaLaunchKernelEx(&cfg, l.kernel, s, l.wall_cap, barrier_polls(), call);
 }
 
 cudaError_t launch_steps(const Sys &s, const LaunchCfg &lc, cudaGraphConditionalHandle hreb,
