@@ -1798,6 +1798,7 @@ struct dem_adjoint {
   cudaStream_t st2 = nullptr;
   cudaEvent_t evq[4] = {nullptr, nullptr, nullptr, nullptr};
   std::string err;
+  int device = 0;
   double *x0 = nullptr, *v0 = nullptr, *w0 = nullptr, *r0 = nullptr;  // initial state
   double rmax0 = 0.0;
   double *xref = nullptr;  // positions at the last build
@@ -2045,6 +2046,7 @@ int dem_adjoint_create(const dem_adjoint_config *cfg, dem_adjoint **out) {
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return DEM_ERR_NO_DEVICE;
   dem_adjoint *h = new dem_adjoint();
   h->cfg = *cfg;
+  cudaGetDevice(&h->device);
   bool ok = cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking) == cudaSuccess &&
             cudaStreamCreateWithFlags(&h->st2, cudaStreamNonBlocking) == cudaSuccess &&
             cudaEventCreate(&h->ev[0]) == cudaSuccess && cudaEventCreate(&h->ev[1]) == cudaSuccess;
@@ -2297,6 +2299,7 @@ static int adj_run(dem_adjoint *h, double E, double e, double mu, const double *
       !(mu >= 0))
     return DEM_ERR_BAD_ARG;
   if (backward && (!gE || !ge || !gmu || !gr)) return DEM_ERR_BAD_ARG;
+  DeviceCall call(h->device);
   ADev &s = h->s;
   const int n = h->n;
   const cudaStream_t st = h->st;

@@ -91,11 +91,14 @@ struct dem_handle {
   bool use_graph = true;
   bool steps_refused = false;  // a launch of k_steps was refused: the separate kernels from then on
   cudaStream_t st2 = nullptr;
-  cudaGraphExec_t gexec = nullptr;
-  long long graph_gen = -1, sys_gen = 0;  // looked at again when something that it holds may have changed
-  int graph_key = 0;                       // its step_loop_key
-  std::vector<unsigned char> graph_holds;  // what it was built from (see ensure_graph)
-  StepCounts graph_counts;
+  struct StepGraph {
+    cudaGraphExec_t exec = nullptr;
+    long long gen = -1;  // sys_gen when last looked at
+    int key = 0;         // its step_loop_key
+    std::vector<unsigned char> holds;  // what it was built from (see ensure_graph)
+    StepCounts counts;
+  } graphs[2];            // of the separate kernels, of k_steps
+  long long sys_gen = 0;  // counts changes of what a graph may hold
   std::vector<MeshHost> mesh_host;
   std::vector<double> bond_tables;  // host copy for the cutoff derivation
   double cell_scale = 1.0;          // neighbour cell edge / cutneighmax (dem_set_tuning)
@@ -110,31 +113,28 @@ struct dem_handle {
 };
 
 static int ensure_graph(dem_handle *h) {
+  dem_handle::StepGraph &g = h->graphs[h->lc.fused];
   const int key = step_loop_key(h->lc);
-  if (h->gexec && h->graph_gen == h->sys_gen && h->graph_key == key) return DEM_OK;
+  if (g.exec && g.gen == h->sys_gen && g.key == key) return DEM_OK;
   // the kernels' arguments and the launch settings: the same bytes give the
   // same graph (0.25 ms to build), as after the next upload of as many atoms
   const int cfg[4] = {h->lc.max_grid, h->lc.particle_threads, h->lc.sms, key};
   std::vector<unsigned char> holds(sizeof(Sys) + sizeof cfg);
   std::memcpy(holds.data(), &h->s, sizeof(Sys));
   std::memcpy(holds.data() + sizeof(Sys), cfg, sizeof cfg);
-  if (h->gexec && holds == h->graph_holds) {
-    h->graph_gen = h->sys_gen;
-    h->graph_key = key;
-    return DEM_OK;
+  if (!g.exec || holds != g.holds) {
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    g.exec = nullptr;
+    cudaError_t e = build_step_graph(h->s, h->lc, h->st, h->st2, &g.exec, &g.counts);
+    if (e != cudaSuccess) {
+      g.exec = nullptr;
+      h->err = std::string("build_step_graph: ") + cudaGetErrorString(e);
+      return DEM_ERR_CUDA;
+    }
+    g.holds.swap(holds);
   }
-  if (h->gexec) {
-    cudaGraphExecDestroy(h->gexec);
-    h->gexec = nullptr;
-  }
-  cudaError_t e = build_step_graph(h->s, h->lc, h->st, h->st2, &h->gexec, &h->graph_counts);
-  if (e != cudaSuccess) {
-    h->err = std::string("build_step_graph: ") + cudaGetErrorString(e);
-    return DEM_ERR_CUDA;
-  }
-  h->graph_gen = h->sys_gen;
-  h->graph_key = key;
-  h->graph_holds.swap(holds);
+  g.gen = h->sys_gen;
+  g.key = key;
   return DEM_OK;
 }
 
@@ -625,7 +625,8 @@ int dem_destroy(dem_handle *h) {
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);
   for (auto &e : h->evpool) cudaEventDestroy(e);
-  if (h->gexec) cudaGraphExecDestroy(h->gexec);
+  for (dem_handle::StepGraph &g : h->graphs)
+    if (g.exec) cudaGraphExecDestroy(g.exec);
   if (h->st) cudaStreamDestroy(h->st);
   if (h->st2) cudaStreamDestroy(h->st2);
   delete h;
@@ -1428,6 +1429,12 @@ int dem_setup(dem_handle *h) {
 // graph 0.17 ms once, but a rebuild then waits for the host (30 us; one in some
 // 50 steps and more).
 constexpr int kDirectSteps = 8;
+// Calls of up to this many steps take turns with another's k_steps (their host
+// part overlaps with it), longer ones run in the separate kernels beside it (see
+// DeviceCall).  Two handles, us per step of one-step calls, in turns / beside: 10,000
+// spheres 48 / 67, 50,000 69 / 83, 100,000 129 / 112; of eight-step calls 35 /
+// 32, 54 / 49, 100 / 76.
+constexpr int kTurnSteps = 2;
 
 // The driver refused a launch of k_steps, or the graph with it (a grid that
 // cannot be resident, MPS, which allows no cooperative launch in a graph's
@@ -1476,10 +1483,16 @@ int dem_step(dem_handle *h, int nsteps) {
   int rc = DEM_OK;
   const long long ts0 = h->host_ctrl.ntimestep;
   const bool graph = h->use_graph && !h->profile;
-  h->lc.np = h->host_ctrl.np;
-  h->lc.fused = graph && fused_steps(h->s, h->lc);
-  bool direct = h->lc.fused && nsteps <= kDirectSteps;
-  if (graph && !direct && (rc = step_graph(h))) return rc;
+  DeviceCall call(h->device);
+  bool direct = false;
+  const auto choose = [&](long long steps) {
+    h->lc.np = h->host_ctrl.np;
+    h->lc.fused = call.ask(graph && fused_steps(h->s, h->lc) ? steps_grid(h->s, h->lc) : 0,
+                           steps <= kTurnSteps ? 2 * h->lc.sms : h->lc.sms);
+    direct = h->lc.fused && steps <= kDirectSteps;
+    return graph && !direct ? step_graph(h) : DEM_OK;
+  };
+  if ((rc = choose(nsteps))) return rc;
   CUDA_TRY(h, cudaEventRecord(h->ev0, h->st));
   long long done = 0;  // steps whose rebuild+pair stage has been queued
   bool first = true;
@@ -1525,11 +1538,11 @@ int dem_step(dem_handle *h, int nsteps) {
     if (queued) {
       h->kt.kernel_launches += launch_set_loop(h->s, (int)(chunk - k0), phase, h->st);
       cudaError_t e = h->lc.fused && coop_refused(kCoopGraphLaunch) ? cudaErrorCooperativeLaunchTooLarge
-                                                                    : cudaGraphLaunch(h->gexec, h->st);
+                                                                    : cudaGraphLaunch(h->graphs[h->lc.fused].exec, h->st);
       if (e != cudaSuccess && h->lc.fused) {
         leave_fused(h);
         if ((rc = step_graph(h))) return rc;
-        e = cudaGraphLaunch(h->gexec, h->st);
+        e = cudaGraphLaunch(h->graphs[h->lc.fused].exec, h->st);
       }
       CUDA_TRY(h, e);
       CUDA_TRY(h, cudaEventRecord(h->ev1, h->st));
@@ -1553,7 +1566,7 @@ int dem_step(dem_handle *h, int nsteps) {
       if (rc) return rc;
     }
     if (queued) {
-      const StepCounts &gc = h->graph_counts;
+      const StepCounts &gc = h->graphs[h->lc.fused].counts;
       const long long iters = std::min<long long>(chunk - k0, h->host_ctrl.ntimestep - (ts0 + done + k0));
       h->kt.kernel_launches += gc.call + std::max<long long>(0, iters - 1) * gc.step +
                                (h->host_ctrl.nrebuilds - rb0) * gc.rebuild;
@@ -1574,6 +1587,9 @@ int dem_step(dem_handle *h, int nsteps) {
       }
       if (graph && !direct && (rc = step_graph(h))) return rc;  // device pointers changed
       done = h->host_ctrl.ntimestep - ts0;
+    } else if (queued && h->lc.fused && h->host_ctrl.step_phase == kStepGather) {  // the launch's turn is over
+      done = h->host_ctrl.ntimestep - ts0;
+      if ((rc = choose(nsteps - done))) return rc;
     } else {
       done += chunk;
       closed = launched;

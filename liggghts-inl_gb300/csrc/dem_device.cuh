@@ -115,6 +115,7 @@ struct Ctrl {
   long long ntimestep, nrebuilds;
   int halt_step;
   int loop_left;    // steps left for the device-side step loop (graph WHILE node)
+  int turn;         // of them, steps until k_steps returns to the host, which looks who else needs the device
   int mesh_moved;   // a moving mesh node travelled > skin/2 since the last build
   int force_rebuild;  // rebuild at the next decide (FixMesh next_reneighbor)
   int nmlist;         // atoms with candidate mesh triangles (Sys::mlist)

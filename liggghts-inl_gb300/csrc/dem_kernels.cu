@@ -117,8 +117,9 @@ __global__ void k_decide_loop(Sys s, LoopCond lp) {
   if (threadIdx.x == 0) loop_decided(c, lp, reb);
 }
 
-__global__ void k_set_loop(Ctrl *c, int n, int phase) {
+__global__ void k_set_loop(Ctrl *c, int n, int phase, int turn) {
   c->loop_left = n;
+  c->turn = turn;
   c->step_phase = phase;
 }
 
@@ -2219,8 +2220,14 @@ int launch_mesh_move(const Sys &s, const LaunchCfg &lc, cudaStream_t st, int gat
   return nl;
 }
 
+// Steps of a graph launch after which k_steps returns and the host looks whether
+// the system is still alone on the device (see DeviceCall): 20 us, 0.1 % of the
+// smallest systems' turn; LIGGGHTS_GB300_TURN sets it (tests)
+constexpr int kTurn = 2048;
+
 int launch_set_loop(const Sys &s, int n, int phase, cudaStream_t st) {
-  k_set_loop<<<1, 1, 0, st>>>(s.ctrl, n, phase);
+  const char *turn = getenv("LIGGGHTS_GB300_TURN");
+  k_set_loop<<<1, 1, 0, st>>>(s.ctrl, n, phase, turn ? std::max(1, atoi(turn)) : kTurn);
   return 1;
 }
 

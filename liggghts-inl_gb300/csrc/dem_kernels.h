@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <mutex>
+
 #include "dem_device.cuh"
 
 namespace gb300 {
@@ -72,6 +74,7 @@ int launch_set_rebuild(const Sys &s, int v, cudaStream_t st);
 int launch_rebuild(const Sys &s, const LaunchCfg &lc, cudaStream_t st, int stage);
 int launch_pair(const Sys &s, const LaunchCfg &lc, int shearupdate, cudaStream_t st, int gate = 0);
 int launch_particle(const Sys &s, const LaunchCfg &lc, int mode, cudaStream_t st);
+// the graph's next launch: n steps from `phase` (k_steps returns after some 2,000, see Ctrl::turn)
 int launch_set_loop(const Sys &s, int n, int phase, cudaStream_t st);
 // wall (plane and mesh) forces of the current state, before the particle
 // kernel that gathers the step's forces; none without walls
@@ -82,12 +85,29 @@ int launch_wall_consts(const Sys &s, const LaunchCfg &lc, cudaStream_t st);
 int launch_mesh_move(const Sys &s, const LaunchCfg &lc, cudaStream_t st, int gate = 0);
 // queue entries of the wall kernel per tile atom (LIGGGHTS_GB300_WALL_CAP)
 int wall_cap_per_atom();
-// Whether dem_step runs the steps in k_steps (dem_steps.cu) rather than as
-// separate kernels (lc.fused: the choice before), and its launch inside the
-// step graph.
+// Whether a system runs its steps in k_steps (dem_steps.cu) rather than as
+// separate kernels, its grid, and its launch inside the step graph.
 bool fused_steps(const Sys &s, const LaunchCfg &lc);
+int steps_grid(const Sys &s, const LaunchCfg &lc);
 // whether all blocks of k_steps can be resident together, which its cooperative launch needs
 bool steps_resident(const Sys &s, const LaunchCfg &lc);
+
+// A call that keeps the device busy, for as long as it lives.  k_steps holds
+// its SMs until its launch ends, so calls from several threads would take turns
+// where the separate kernels overlap: it is granted only beside other k_steps,
+// and only up to `room` blocks of all together (the SMs: all are resident).
+class DeviceCall {
+ public:
+  explicit DeviceCall(int device);
+  ~DeviceCall();
+  DeviceCall(const DeviceCall &) = delete;
+  DeviceCall &operator=(const DeviceCall &) = delete;
+  bool ask(int blocks, int room);  // k_steps with so many blocks (0: none); gives back what was granted before
+
+ private:
+  void give_back();
+  int device_, blocks_ = 0;  // blocks_: granted
+};
 // Refusals as the driver gives them (under MPS, say), for tests:
 // LIGGGHTS_GB300_COOP_REFUSE adds up what is refused.
 enum { kCoopGrid = 1, kCoopInGraph = 2, kCoopDirect = 4, kCoopResume = 8, kCoopGraphLaunch = 16 };

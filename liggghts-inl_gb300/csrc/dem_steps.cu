@@ -25,6 +25,7 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <mutex>
 
 #include "barrier_count.cuh"
 #include "dem_kernels.h"
@@ -160,7 +161,8 @@ __global__ void __launch_bounds__(kStepThreads, 1)
   }
   // the launch's constants, and the decision's state: the same in every block
   const int n = c->n, np = c->np, nl = c->nmlist;
-  int left = call.n >= 0 ? call.n : c->loop_left, phase = call.n >= 0 ? call.phase : c->step_phase, ago = c->ago, force = c->force_rebuild;
+  int left = call.n >= 0 ? call.n : c->loop_left, phase = call.n >= 0 ? call.phase : c->step_phase, turn = c->turn;
+  int ago = c->ago, force = c->force_rebuild;
   long long ts = c->ntimestep;
   int reb = 0;
   unsigned long long seen = 0;  // the barrier's count behind the last one
@@ -254,6 +256,7 @@ __global__ void __launch_bounds__(kStepThreads, 1)
     }
     if (!(ok = grid_barrier<false>(c, G, limit, seen, 0, fl))) break;
     left--;
+    if (call.in_graph && left > 0 && --turn <= 0) break;
   }
   if (__any_sync(0xffffffffu, bad) && lane == 0) atomicExch(&c->status, kStatNan);
   if (__any_sync(0xffffffffu, meshbad) && lane == 0) atomicExch(&c->status, kStatMeshSlots);
@@ -277,7 +280,8 @@ __global__ void __launch_bounds__(kStepThreads, 1)
   c->moved = 0;
   c->mesh_moved = 0;
   c->loop_left = left;
-  c->step_phase = reb ? kStepForces : kStepDone;
+  c->turn = turn;
+  c->step_phase = reb ? kStepForces : (left > 0 ? kStepGather : kStepDone);
   step_conditionals(call, reb);
 }
 
@@ -317,17 +321,16 @@ StepKernel step_kernel(const Sys &s, size_t *shared) {
 // nodes' latency is small beside them; a mesh's wall kernel runs beside the pair
 // kernel, while here its tiles hold up the blocks that have them.  (With bonds
 // the pair law is the longer one.)  Ensembles decide per system
-// (decide_rebuild) and keep the separate kernels.  Asked at every call; a
-// system that runs fused stays so for another sixteenth (the two sides are a few
-// percent apart there), so that one at the limit does not build a graph (0.25
-// ms) call after call.
+// (decide_rebuild) and keep the separate kernels.  Asked at every call.
 // LIGGGHTS_GB300_FUSED_STEPS=0|1: never, always (tests).
 bool fused_steps(const Sys &s, const LaunchCfg &lc) {
   if (s.nsys || !lc.coop) return false;
   if (const char *e = getenv("LIGGGHTS_GB300_FUSED_STEPS")) return atoi(e) != 0;
-  const int limit = s.nmeshes > 0 && !s.bond ? 160000 : 330000;
-  return lc.np <= limit + (lc.fused ? limit / 16 : 0);
+  return lc.np <= (s.nmeshes > 0 && !s.bond ? 160000 : 330000);
 }
+
+// one block per SM; fewer for systems of fewer warps
+int steps_grid(const Sys &s, const LaunchCfg &lc) { return std::max(1, std::min((s.nmax + 31) / 32, lc.sms)); }
 
 static int barrier_polls() {
   const char *polls = getenv("LIGGGHTS_GB300_BARRIER_POLLS");
@@ -335,6 +338,56 @@ static int barrier_polls() {
 }
 
 int step_loop_key(const LaunchCfg &lc) { return lc.fused ? barrier_polls() : 0; }
+
+// Us per step of 1, 2 and 4 handles in as many threads, 50 steps a call: the
+// separate kernels; k_steps in turns; by DeviceCall's rule:
+//   2,000 spheres   21  23  24    16  16  30    16  16  24
+//   10,000          22  24  27    18  34  68    18  26  28
+//   50,000          31  40  56    26  50  99    25  40  57
+//   100,000         42  59 104    45  89 177    44  60 105
+namespace {
+struct DeviceLoad {
+  std::mutex m;
+  int calls = 0, fused = 0, blocks = 0;  // in flight; those that run k_steps, and their blocks
+};
+constexpr int kMaxDevices = 64;
+DeviceLoad &device_load(int device) {
+  static DeviceLoad loads[kMaxDevices];
+  return loads[device >= 0 ? device % kMaxDevices : 0];
+}
+}  // namespace
+
+DeviceCall::DeviceCall(int device) : device_(device) {
+  DeviceLoad &d = device_load(device_);
+  std::lock_guard<std::mutex> lock(d.m);
+  d.calls++;
+}
+
+DeviceCall::~DeviceCall() {
+  DeviceLoad &d = device_load(device_);
+  std::lock_guard<std::mutex> lock(d.m);
+  give_back();
+  d.calls--;
+}
+
+void DeviceCall::give_back() {
+  DeviceLoad &d = device_load(device_);
+  d.fused -= blocks_ > 0 ? 1 : 0;
+  d.blocks -= blocks_;
+  blocks_ = 0;
+}
+
+bool DeviceCall::ask(int blocks, int room) {
+  DeviceLoad &d = device_load(device_);
+  std::lock_guard<std::mutex> lock(d.m);
+  give_back();
+  // (this call is one of those that run no k_steps)
+  if (blocks <= 0 || d.calls - d.fused > 1 || d.blocks + blocks > room) return false;
+  blocks_ = blocks;
+  d.fused++;
+  d.blocks += blocks;
+  return true;
+}
 
 bool coop_refused(int what) {
   const char *e = getenv("LIGGGHTS_GB300_COOP_REFUSE");
@@ -358,8 +411,7 @@ cudaError_t step_launch(const Sys &s, const LaunchCfg &lc, StepLaunch *l) {
   const int most = (int)std::min<size_t>(wall_cap_per_atom(), (226 * 1024 - shared) / queue);
   l->wall_cap = s.nmeshes > 0 ? most * kWallTile : 0;
   l->shared = shared + (size_t)(kStepThreads / 32) * kWallQ * l->wall_cap;
-  // one block per SM; fewer for systems of fewer warps
-  l->grid = std::max(1, std::min((s.nmax + 31) / 32, lc.sms));
+  l->grid = steps_grid(s, lc);
   // the limit belongs to the function, not to the launch: the same for every
   // system, so that threads that step different ones do not undercut each other
   return cudaFuncSetAttribute((const void *)l->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
