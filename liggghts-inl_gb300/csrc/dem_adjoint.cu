@@ -1378,10 +1378,12 @@ __global__ void ka_kick_drift(ADev s, const double *xref, int wrap, double *tx, 
 
 // ------------------------------------------------------------------ backward
 
-// The second half-kick v' = vh + a F', w' = wh + b T' of an evaluation, in
-// reverse: Fb += a vb, Tb += b wb and the radius and mass adjoints; then
-// gravity's mass adjoint.  fv = F'.vb, tw = T'.wb.  fresh: Fb, Tb start from
-// the next step's first half-kick (the same a vb, b wb), else from zero.
+// The half-kicks v' = v + a F, w' = w + b T with the forces of one evaluation,
+// in reverse: first, the next step's first half-kick; second, the second one of
+// the step whose forces they are.  Both see the same vb and wb, so that Fb and
+// Tb are set to once or twice a vb and b wb; rb and mb come with the other
+// radius and mass adjoints of the atom, and the half-kicks' and gravity's join
+// them.  fv = F.vb, tw = T.wb.
 __device__ __forceinline__ void kick_back(const ADev &s, const ABar &B, int i, const double vb[3], const double wb[3],
                                           bool first, bool second, double fv, double tw, double rb, double mb) {
   const double c = (first ? 1.0 : 0.0) + (second ? 1.0 : 0.0);

@@ -668,7 +668,8 @@ __global__ void k_cell_sort(Sys s) {
 
 // The copies of a rebuild load an item's values before they store the first:
 // a store may alias the loads behind it, so that a copy value by value waits
-// XX
+// for every load in turn (526,000 atoms: k_permute 61 -> 46 us, k_copy_atoms 44 ->
+// 27, k_copy_pairs 69 -> 35).
 template <int N, class T>
 __device__ __forceinline__ void copy_values(T *const (&to)[N], const T *const (&from)[N], size_t i, size_t o) {
   T v[N];

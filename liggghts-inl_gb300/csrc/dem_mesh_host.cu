@@ -312,7 +312,7 @@ int mesh_prepare(int ntri, const double *nodes, const uint8_t *ea_in, const uint
     d[36] = g.rb[t];
     // resolveTriSphereContactBary's limit, in its operations
     const double invlen = 1. / (2. * g.rb[t]);
-    d[37] = -1e-8 * invlen;
+    d[37] = -kPrecision * invlen;
     int m = g.obtuse[t] + 1;
     for (int q = 0; q < 3; q++) {
       if (tp.ea[3 * t + q]) m |= 1 << (2 + q);

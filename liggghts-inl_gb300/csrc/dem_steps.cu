@@ -4,16 +4,18 @@
 // separate graph nodes (per-atom kernel, rebuild decision, IF node, pair and
 // wall kernels side by side, WHILE iteration) about 14 us of every step pass
 // between the kernels, and each kernel fetches its parameters, its code and
-// its atoms anew.  k_steps keeps one block (or two) resident on every SM and
-// runs step after step, with a grid barrier where a kernel boundary was:
+// its atoms anew.  k_steps keeps one block resident on every SM (fewer blocks
+// for systems of fewer warps) and runs step after step, with a grid barrier
+// where a kernel boundary was:
 //
 //   A  per atom: gather, gravity, wall totals, nve/sphere, displacement test
 //      (particle_warp); moving meshes advance on the grid's last warps
 //   -- barrier; every block takes the same rebuild decision; a rebuild ends
 //      the launch (the graph's IF node rebuilds, the WHILE node comes back,
 //      and the launch resumes with B)
-//   B  wall tiles, then pair tiles, by warps (wall_tile, pf_tiles/band_tiles)
-//   -- barrier
+//   B  by warps, the tests of the block's list tiles (pf_test, band_test), then
+//      its wall tiles (wall_tile) and the laws of the entries that passed
+//   -- barrier; after a call's last step, and every 2,048, the launch ends
 //
 // The tiles are those of the separate kernels, and every atom's and entry's
 // result goes to its own slot, so the results are the same bits.

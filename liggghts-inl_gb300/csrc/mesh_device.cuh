@@ -16,7 +16,6 @@ namespace gb300 {
 
 constexpr double kTriSmall = 1.e-10;    // SMALL_TRIMESH
 constexpr double kTriLarge = 1000000;   // LARGE_TRIMESH
-constexpr double kMeshPrecision = 1e-8; // EPSILON_PRECISION
 
 __device__ __forceinline__ double dot3_rn(const double *a, const double *b) {
   return __dadd_rn(__dadd_rn(__dmul_rn(a[0], b[0]), __dmul_rn(a[1], b[1])), __dmul_rn(a[2], b[2]));

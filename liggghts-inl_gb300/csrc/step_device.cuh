@@ -330,12 +330,6 @@ struct BandRest {
   int n;
 };
 
-// Phase 1 runs per lane on 32 consecutive entries of a warp at a time; the
-// entries that need phase 2 wait in the warp's shared-memory queue (with
-// their exact test's delta and rsq) until 32 have gathered, so the bond and
-// contact laws run on full warps.  The warps' remainders merge into one
-// block batch at the end.  Each entry's result goes to its own slot and
-// depends on no other entry, so the order changes no value.
 // entry p of the list; code kHole: none
 __device__ __forceinline__ void pf_load(const Sys &s, int np, int p, int &i, int &j, int &code) {
   const PairArrays &L = s.pairs[0];
@@ -398,6 +392,12 @@ __device__ __forceinline__ bool band_may_create(const Sys &s, int shearupdate, l
   return BOND && shearupdate && ((s.bond_flags & kBondCreateAlways) || ntimestep == s.bond_ts_create);
 }
 
+// Phase 1 runs per lane on 32 consecutive entries of a warp at a time; the
+// entries that need phase 2 wait in the warp's shared-memory queue (with
+// their exact test's delta and rsq) until 32 have gathered, so the bond and
+// contact laws run on full warps.  The warps' remainders merge into one
+// block batch at the end (band_rest).  Each entry's result goes to its own slot
+// and depends on no other entry, so the order changes no value.
 // next() gives the first entry of the warp's next 32 (np or more: none left).
 template <int NORMAL, bool ROLL, bool BOND, class Next>
 __device__ __forceinline__ int band_tiles(const Sys &s, int np, int shearupdate, long long ntimestep, BandQueue &q,
@@ -968,7 +968,7 @@ __device__ __noinline__ bool mesh_contacts(const Sys &s, int i, int k, int shear
 // candidates and contacts):
 //   A  per atom, FP32: the candidates the triangle bounds cannot reject
 //      (tri_candidate_f), queued in ascending order;
-//   B  per queued candidate: exact plane test and closest feature
+//   B  per queued candidate: closest feature
 //      (TriMesh::resolveTriSphereContactBary), kept when touching;
 //   C  per atom, integer work in candidate order: FixContactHistoryMesh's
 //      slot semantics (handleContact, coplanarContactAlready); an atom whose
@@ -1106,7 +1106,7 @@ __device__ __forceinline__ void wall_tile(const Sys &s, const AtomArrays &A, int
       }
     }
     __syncwarp();
-    // ---- B: exact plane test and closest feature per queued candidate
+    // ---- B: closest feature per queued candidate
     for (int e = a; e < total; e += kWallTile) {
       const int ie = s.mlist[base + w.qa[e]];
       const int t = M.cand[(size_t)w.qq[e] * nmax + ie];
@@ -1608,13 +1608,14 @@ __device__ __forceinline__ void particle_finish(const Sys &s, int i, bool gather
 // lanes of a warp run loops of nearly equal length and a record is read by
 // neighbouring lanes.  Warps work on their own: they reach the FP64 pipe at
 // different times.  Each sum keeps its order, so the result does not depend on
-// any of this.  Bound by the FP64 pipe (55 % busy) and the latency of its four
-// dependent loads; measured against one lane per atom sorted over a block of
-// 256 (pipe 42-50 % busy, its warps all waiting for the same phase): 1,000,000
-// atoms in a hopper 101 -> 77 us, 400,000 packed 81 -> 71, 526,000 of an
-// ensemble 46 -> 39; and with no conversion, doubling or product issued in vain
-// (a quarter of its FP64 instructions were predicated off) 74, 70 and 36.  More blocks per SM (48 registers), larger batches and
-// prefetches of the atom's state were slower.
+// any of this.  Bound by the latency of its four dependent loads (FP64 pipe 44 %
+// busy on the hopper, 48 % on the packed bed); measured against one lane per
+// atom sorted over a block of 256 (pipe 42-50 % busy, its warps all waiting for
+// the same phase): 1,000,000 atoms in a hopper 101 -> 77 us, 400,000 packed 81 ->
+// 71, 526,000 of an ensemble 46 -> 39; and with no conversion, doubling or product
+// issued in vain (a quarter of its FP64 instructions were predicated off) 74, 70
+// and 36.  More blocks per SM (48 registers), larger batches and prefetches of
+// the atom's state were slower.
 // Called by all lanes of a warp, each with its atom i (valid or none).
 template <int T>
 __device__ __forceinline__ void particle_tile(const Sys &s, ParticleShared<T> &sm, int i, bool valid, bool gather,
