@@ -1436,7 +1436,7 @@ constexpr int kDirectSteps = 8;
 // 32, 54 / 49, 100 / 76.
 constexpr int kTurnSteps = 2;
 
-// The driver refused a launch of k_steps, or the graph with it (a grid that
+// CUDA refused a launch of k_steps, or the graph with it (a grid that
 // cannot be resident, MPS, which allows no cooperative launch in a graph's
 // conditionals): nothing of it has run, and the separate kernels take over.
 static void leave_fused(dem_handle *h) {

@@ -108,7 +108,7 @@ class DeviceCall {
   void give_back();
   int device_, blocks_ = 0;  // blocks_: granted
 };
-// Refusals as the driver gives them (under MPS, say), for tests:
+// Refusals as CUDA gives them (under MPS, say), for tests:
 // LIGGGHTS_GB300_COOP_REFUSE adds up what is refused.
 enum { kCoopGrid = 1, kCoopInGraph = 2, kCoopDirect = 4, kCoopResume = 8, kCoopGraphLaunch = 16 };
 bool coop_refused(int what);
